@@ -198,6 +198,29 @@ def test_varlen_forward_backward(ext, request, d, causal, lens_q, lens_k, h, hk,
         assert lse[i, :, lens_q[i]:].abs().max().item() == 0 if lens_q[i] < max(lens_q) else True
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_varlen_backward_of_many_short_sequences(ext, d, causal):
+    # Items of one to four key blocks, nearly all with a ragged last block, several per CTA: the loads of an item run
+    # under the products of the one before it.  Every launch bit for bit equal to dense launches per sequence.
+    h, hk = 8, 4
+    lens = [(37 * i + 11) % 511 + 1 for i in range(96)]
+    q, k, v, dout, cq, _ = _varlen_case(77 + d, lens, lens, h, hk, d)
+    q, k, v, dout, cu = (x.to(DEV) for x in (q, k, v, dout, cq))
+    args = (cu, cu, max(lens), max(lens), d ** -0.5, causal)
+    out, lse = ext.varlen_fwd(q, k, v, *args)
+    grads = ext.varlen_bwd(q, k, v, out, lse, dout, *args)
+    for _ in range(30):
+        for got, want in zip(ext.varlen_bwd(q, k, v, out, lse, dout, *args), grads):
+            assert torch.equal(got, want)
+    for i in range(0, len(lens), 7):
+        a, b = int(cq[i]), int(cq[i + 1])
+        one = [x[None, a:b] for x in (q, k, v)]
+        o, l = ext.fwd(*one, d ** -0.5, causal)
+        for got, want in zip(grads, ext.bwd(*one, o, l, dout[None, a:b], d ** -0.5, causal)):
+            assert torch.equal(got[a:b], want[0])
+
+
 def test_varlen_packed_variants(ext):
     from flash_attention_turing_b200 import (flash_attn_varlen_func, flash_attn_varlen_kvpacked_func,
                                              flash_attn_varlen_qkvpacked_func)
