@@ -3,7 +3,7 @@
 //   1. preprocess   -delta[b,h,i] = -sum_d dO*O (fp32) and -lse2 = -LSE*log2(e) (stored negated so that
 //                   the consumers need only fused multiply-adds), both padded to a multiple of 128 rows
 //                   per (b, h); padded rows get -lse2 = -inf so that they produce P = 0.
-//   2. dQ kernel    one CTA per 128-row Q tile; loops over K/V blocks:
+//   2. dQ kernel    items = 128-row Q tiles; loops over K/V blocks:
 //                     S  = Q K_j^T, dP = dO V_j^T            (tcgen05 SS, fp32 in TMEM)
 //                     P  = exp2(S*c - lse2), dS = P o (dP - delta) -> fp16, written to TMEM columns of its own
 //                     dQ += dS K_j                            (tcgen05 TS, K_j as MN-major B operand)
@@ -111,55 +111,60 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) 
 // is persistent: one CTA per SM takes items from a global counter (heaviest causal tile of a head first) and
 // keeps its barriers, its TMEM allocation and the K / V rings across items: every barrier phase is derived from
 // the cumulative block count G (or the item count), the Q / dO tiles and the row statistics of the next item are
-// loaded as soon as the last dP product of the current item has read them, and the first S product of the next
-// item is issued under the last elementwise block and the epilogue of the current one.  The row statistics come
-// through shared memory with the Q / dO tiles (no global load at the start of an item).  Scheduling as in the
-// forward kernel: an item is claimed two blocks before the current one ends.  Measured against one CTA per item
-// (bit-identical results): S = 8192 1.4 % faster, S = 4096 5 %, S = 1024 19 %, D = 64 S = 4096 11 %.
-constexpr int kDqpThreads = 640;  // + one scheduler warp: 20 warps, five on one sub-partition -> 96 registers
-constexpr int kDqpSchedWarp = 19;
-constexpr int kDqpReaders = kComputeWarps + 3;  // elementwise warps, producer warp, two MMA threads
-static_assert((kDqpThreads / 32 + 3) / 4 * 32 * 96 <= 16384, "register file of one SM sub-partition");
+// loaded as soon as the current item has read its own for the last time, and the first S product of the next
+// item is issued under the last elementwise block and the epilogue of the current one.  An item is claimed two blocks
+// before the current one ends; the scheduler thread derives everything the roles need from it once and leaves it in
+// shared memory (decoding it in five roles was code the instruction cache had to hold).
+//
+// Bound by the issue of its products: 16 SS MMAs of about 88 clocks (operand fetches share the shared-memory port with
+// the arriving tiles) and 8 TS MMAs of about 75, of 1536 clocks at the tensor peak.  S and dP of a block are issued back
+// to back, fetched into registers together and handed back together, so that the whole arithmetic of the block runs
+// under the next S / dP: ONE wait and one hand-back per block where waiting for S and dP in turn took two of each, at
+// 150-300 clocks apiece for warps in lock-step.  The hand-back has to leave before the arithmetic starts (see
+// schedule_barrier: without it 55 % slower).  Measured per 128 x 128 block at B4 S8192 H32 D128 causal: 2511 -> 2226 clocks;
+// launch, SM clocks: D128 S8192 4520 -> 4005 k, D128 S1024 462 -> 436 k, D64 S16384 3417 -> 3189 k.
+constexpr int kDqThreads = 640;
+constexpr int kDqSchedWarp = 19;
+constexpr int kDqReaders = kComputeWarps + 3;  // elementwise warps, producer warp, two MMA threads
+static_assert((kDqThreads / 32 + 3) / 4 * 32 * 96 <= 16384, "register file of one SM sub-partition");
 
-struct DqpItem {
-  int batch, head, mblk, pad;  // mblk < 0: no more work
+// A work item with everything the roles derive from it, filled in once by the scheduler thread.
+struct __align__(16) DqItem {
+  int nb;  // key blocks to visit; < 0: no more work
+  int sk, shift, row0;
+  int q_off, k_off, sq, bq;
+  int batch, head, head_k, fix_k_tail;  // fix_k_tail: rows of the last K tile belong to the next sequence
 };
-struct DqpBarriers {
+struct DqBarriers {
   BBarriers b;
   uint64_t q_free;          // the Q / dO tiles (last dP products) and the statistics (elementwise warps) have been read
   uint64_t sched_full[2], sched_empty[2], sched_go;
-  DqpItem items[2];
+  DqItem items[2];
 };
-static_assert(sizeof(DqpBarriers) <= 512, "barrier block");
+static_assert(sizeof(DqBarriers) <= 1024, "barrier block");
 
-struct DqpWork {
-  int batch, head, head_k, bq, q_off, k_off, sq, sk, row0, nkb, nb, shift;
-  bool fix_k_tail;
-};
-__device__ __forceinline__ DqpWork dqp_decode(const BwdKernelParams& p, const DqpItem& it) {
-  DqpWork w;
+__device__ __forceinline__ void dq_make_item(const BwdKernelParams& p, int batch, int head, int mblk, DqItem& w) {
   const bool varlen = p.cu_seqlens_q != nullptr;
-  w.batch = it.batch, w.head = it.head;
-  w.q_off = varlen ? p.cu_seqlens_q[it.batch] : 0;
-  w.sq = varlen ? p.cu_seqlens_q[it.batch + 1] - w.q_off : p.seqlen_q;
-  w.k_off = varlen ? p.cu_seqlens_k[it.batch] : 0;
-  w.sk = varlen ? p.cu_seqlens_k[it.batch + 1] - w.k_off : p.seqlen_k;
-  w.row0 = it.mblk * kBlock;
-  w.bq = varlen ? 0 : it.batch;
-  w.head_k = it.head / (p.h / p.h_k);
-  w.nkb = (w.sk + kBlock - 1) / kBlock;
+  w.batch = batch, w.head = head;
+  w.q_off = varlen ? p.cu_seqlens_q[batch] : 0;
+  w.sq = varlen ? p.cu_seqlens_q[batch + 1] - w.q_off : p.seqlen_q;
+  w.k_off = varlen ? p.cu_seqlens_k[batch] : 0;
+  w.sk = varlen ? p.cu_seqlens_k[batch + 1] - w.k_off : p.seqlen_k;
+  w.row0 = mblk * kBlock;
+  w.bq = varlen ? 0 : batch;
+  w.head_k = head / (p.h / p.h_k);
+  const int nkb = (w.sk + kBlock - 1) / kBlock;
   w.shift = (p.is_causal == 2) ? p.causal_shift : w.sk - w.sq;
-  w.nb = w.nkb;
+  w.nb = nkb;
   if (p.is_causal) {
     const int x = w.row0 + kBlock + w.shift;
-    w.nb = x <= 0 ? 0 : min(w.nkb, (x + kBlock - 1) / kBlock);
+    w.nb = x <= 0 ? 0 : min(nkb, (x + kBlock - 1) / kBlock);
   }
-  w.fix_k_tail = varlen && (w.sk % kBlock) != 0 && w.nb == w.nkb && w.nb > 0;
-  return w;
+  w.fix_k_tail = varlen && (w.sk % kBlock) != 0 && w.nb == nkb && w.nb > 0;
 }
 
 template <int D>
-__global__ void __launch_bounds__(kDqpThreads, 1)
+__global__ void __launch_bounds__(kDqThreads, 1)
 bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
   using C = BCfg<D>;
   extern __shared__ uint8_t smem_raw[];
@@ -172,7 +177,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
   uint8_t* sK = sdO + C::kTileBytes;
   uint8_t* sV = sK + C::kStagesK * C::kTileBytes;
   float* sStats = reinterpret_cast<float*>(sV + C::kStagesV * C::kTileBytes);  // lse2[128] | delta[128]
-  DqpBarriers* xb = reinterpret_cast<DqpBarriers*>(reinterpret_cast<uint8_t*>(sStats) + 1024);
+  DqBarriers* xb = reinterpret_cast<DqBarriers*>(reinterpret_cast<uint8_t*>(sStats) + 1024);
   BBarriers* bars = &xb->b;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -181,7 +186,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
     mbar_init(&xb->q_free, 1 + kComputeWarps);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&xb->sched_full[i], 1);
-      mbar_init(&xb->sched_empty[i], kDqpReaders);
+      mbar_init(&xb->sched_empty[i], kDqReaders);
     }
     mbar_init(&xb->sched_go, 1);
     fence_mbar_init();
@@ -196,15 +201,11 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
   const uint32_t tmem_base = bars->tmem_base;
   WaitCtx ctx{&bars->abort_flag, p.status};
 
-  auto read_item = [&](int n, DqpItem& it) -> bool {
-    if (!mbar_wait(&xb->sched_full[n & 1], (n >> 1) & 1, ctx)) return false;
-    it = xb->items[n & 1];
-    return true;
-  };
+  auto wait_item = [&](int n) -> bool { return mbar_wait(&xb->sched_full[n & 1], (n >> 1) & 1, ctx); };
   auto release_item = [&](int n) { mbar_arrive(&xb->sched_empty[n & 1]); };
 
   if (stop) {
-  } else if (warp == kDqpSchedWarp) {
+  } else if (warp == kDqSchedWarp) {
     if (lane == 0) {
       bool finished = false;
       int seq = 0;
@@ -214,8 +215,8 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
           if (!mbar_wait(&xb->sched_go, (n - 1) & 1, ctx)) break;
           next = gridDim.x + atomicAdd(p.sched, 1);
         }
-        DqpItem it;
-        it.batch = 0, it.head = 0, it.mblk = -1, it.pad = 0;
+        DqItem it;
+        it.nb = -1;
         while (next < p.total_items) {
           int batch, head, mblk, sq;
           if (p.cu_seqlens_q == nullptr) {
@@ -230,7 +231,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
             if (head >= p.h) mblk = -1;
           }
           if (mblk >= 0 && mblk * kBlock < sq) {
-            it.batch = batch, it.head = head, it.mblk = mblk;
+            dq_make_item(p, batch, head, mblk, it);
             break;
           }
           next = gridDim.x + atomicAdd(p.sched, 1);
@@ -238,7 +239,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
         if (!mbar_wait(&xb->sched_empty[n & 1], ((n >> 1) & 1) ^ 1, ctx)) break;
         xb->items[n & 1] = it;
         mbar_arrive(&xb->sched_full[n & 1]);
-        if (it.mblk < 0) {
+        if (it.nb < 0) {
           finished = true;
           break;
         }
@@ -254,13 +255,12 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
   } else if (warp == kProducerWarp) {
     int G = 0, ni = 0, nf = 0;
     for (int n = 0;; ++n) {
-      DqpItem it;
-      bool ok = read_item(n, it);
+      bool ok = wait_item(n);
       if (!__all_sync(0xffffffffu, ok)) break;
+      const DqItem w = xb->items[n & 1];
       __syncwarp();
       if (lane == 0) release_item(n);
-      if (it.mblk < 0) break;
-      const DqpWork w = dqp_decode(p, it);
+      if (w.nb < 0) break;
       if (w.nb == 0) continue;
       if (lane == 0) {
         ok = mbar_wait(&xb->q_free, (ni & 1) ^ 1, ctx);
@@ -293,9 +293,9 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       }
       if (!__all_sync(0xffffffffu, ok)) break;
       if (w.fix_k_tail) {
-        const int g = G + w.nkb - 1, s = g % C::kStagesK;
+        const int g = G + w.nb - 1, s = g % C::kStagesK;
         if (!mbar_wait_warp(&bars->a_full[s], (g / C::kStagesK) & 1, ctx)) break;
-        zero_tile_rows_from<D>(sK + s * C::kTileBytes, w.sk - (w.nkb - 1) * kBlock, lane);
+        zero_tile_rows_from<D>(sK + s * C::kTileBytes, w.sk - (w.nb - 1) * kBlock, lane);
         // Two barriers in turn: with short items this warp can be a whole item ahead of the accumulating thread, and
         // on one barrier that thread would then wait for a phase that is over and comes round only after it has
         // moved on.  It cannot be two ahead: item n + 2 is published when the epilogue of item n is done.
@@ -310,42 +310,36 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       constexpr uint32_t idesc_nn = make_idesc_f16(128, kBlock, false, false);
       const uint32_t q_addr = smem_u32(sQ), do_addr = smem_u32(sdO);
       auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, ctx); };
-      auto k_tile = [&](int g) { return smem_u32(sK + (g % C::kStagesK) * C::kTileBytes); };
-      auto v_tile = [&](int g) { return smem_u32(sV + (g % C::kStagesV) * C::kTileBytes); };
-      auto k_full = [&](int g) { return wait(&bars->a_full[g % C::kStagesK], (g / C::kStagesK) & 1); };
-      auto v_full = [&](int g) { return wait(&bars->b_full[g % C::kStagesV], (g / C::kStagesV) & 1); };
       int G = 0, ni = 0;
       bool ok = true;
       for (int n = 0; ok; ++n) {
-        DqpItem it;
-        if (!(ok = read_item(n, it))) break;
+        if (!(ok = wait_item(n))) break;
+        const int nb = xb->items[n & 1].nb;
         release_item(n);
-        if (it.mblk < 0) break;
-        const DqpWork w = dqp_decode(p, it);
-        if (w.nb <= 2) mbar_arrive(&xb->sched_go);  // short item: claim the next one right away
-        if (w.nb == 0) continue;
-        ok = wait(&bars->fixed_full, ni & 1) && k_full(G);
-        for (int j = 0; ok && j < w.nb; ++j) {
-          const int g = G + j;
+        if (nb < 0) break;
+        if (nb <= 2) mbar_arrive(&xb->sched_go);  // short item: claim the next one right away
+        if (nb == 0) continue;
+        ok = wait(&bars->fixed_full, ni & 1);
+        for (int j = 0; ok && j < nb; ++j) {
+          const int g = G + j, s = g % C::kStagesK, sv = g % C::kStagesV;
+          // the loads are polled before the hand-back of S and dP, while nothing could be issued anyway
+          if (!(ok = wait(&bars->a_full[s], (g / C::kStagesK) & 1))) break;
+          if (!(ok = wait(&bars->b_full[sv], (g / C::kStagesV) & 1))) break;
           if (g > 0 && !(ok = wait(&bars->s_loaded, (g - 1) & 1))) break;
-          // S(g) complete tells the elementwise warps that packed-dS buffer g&1 is free again
-          if (g >= 2 && !(ok = wait(&bars->ds_free[g & 1], ((g >> 1) - 1) & 1))) break;
           tc_fence_after_sync();
-          ok = gemm_ss<D>(tmem_base + kColS, q_addr, k_tile(g), idesc_nn, [&] { return v_full(g); });
-          if (!ok) break;
-          tc_commit(&bars->s_full);
-          tc_commit(&bars->a_empty[g % C::kStagesK]);  // second reader: the dQ MMAs of this block
-          if (g > 0 && !(ok = wait(&bars->dp_loaded, (g - 1) & 1))) break;
-          tc_fence_after_sync();
-          ok = gemm_ss<D>(tmem_base + kColDP, do_addr, v_tile(g), idesc_nn,
-                          [&] { return j + 1 >= w.nb || k_full(g + 1); });
+          gemm_ss<D>(tmem_base + kColS, q_addr, smem_u32(sK + s * C::kTileBytes), idesc_nn);
+          // dP(g) complete tells the elementwise warps that packed-dS buffer g & 1 is free again (dQ(g-2) ends about
+          // when S(g) starts)
+          ok = gemm_ss<D>(tmem_base + kColDP, do_addr, smem_u32(sV + sv * C::kTileBytes), idesc_nn,
+                          [&] { return g < 2 || wait(&bars->ds_free[g & 1], ((g >> 1) - 1) & 1); });
           if (!ok) break;
           tc_commit(&bars->dp_full);
-          tc_commit(&bars->b_empty[g % C::kStagesV]);
-          if (j + 1 == w.nb) tc_commit(&xb->q_free);  // Q and dO may be replaced
-          if (w.nb > 2 && j + 3 == w.nb) mbar_arrive(&xb->sched_go);
+          tc_commit(&bars->a_empty[s]);  // second reader: the dQ MMAs of this block
+          tc_commit(&bars->b_empty[sv]);
+          if (j + 1 == nb) tc_commit(&xb->q_free);  // Q and dO may be replaced
+          if (nb > 2 && j + 3 == nb) mbar_arrive(&xb->sched_go);
         }
-        G += w.nb;
+        G += nb;
         ++ni;
       }
     }
@@ -355,17 +349,19 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       int G = 0, nf = 0;
       bool ok = true;
       for (int n = 0; ok; ++n) {
-        DqpItem it;
-        if (!(ok = read_item(n, it))) break;
+        if (!(ok = wait_item(n))) break;
+        const int nb = xb->items[n & 1].nb, fix_k_tail = xb->items[n & 1].fix_k_tail;
         release_item(n);
-        if (it.mblk < 0) break;
-        const DqpWork w = dqp_decode(p, it);
-        if (w.nb == 0) continue;
-        for (int j = 0; ok && j < w.nb; ++j) {
+        if (nb < 0) break;
+        if (nb == 0) continue;
+        for (int j = 0; ok && j < nb; ++j) {
           const int g = G + j, s = g % C::kStagesK;
-          if (!(ok = mbar_wait(&bars->a_full[s], (g / C::kStagesK) & 1, ctx))) break;
+          // dS(g) written implies that K(g) has landed: S(g) read it, and the elementwise warps have seen S(g)
           if (!(ok = mbar_wait(&bars->ds_full, g & 1, ctx))) break;
-          if (w.fix_k_tail && j == w.nkb - 1 && !(ok = mbar_wait(&bars->tail_fixed[nf & 1], (nf >> 1) & 1, ctx))) break;
+          if (fix_k_tail && j == nb - 1) {
+            if (!(ok = mbar_wait(&bars->tail_fixed[nf & 1], (nf >> 1) & 1, ctx))) break;
+            ++nf;
+          }
           tc_fence_after_sync();
           gemm_ts<D>(tmem_base + kColAcc, tmem_base + kColPacked + (g & 1) * 64, smem_u32(sK + s * C::kTileBytes),
                      idesc_acc, j == 0);
@@ -373,8 +369,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
           tc_commit(&bars->ds_free[g & 1]);
         }
         if (ok) tc_commit(&bars->acc_full);
-        G += w.nb;
-        if (w.fix_k_tail) ++nf;
+        G += nb;
       }
     }
   } else if (warp < kComputeWarps) {
@@ -386,28 +381,23 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
     const uint32_t tDP = tmem_base + lane_base + kColDP + cq * 32;
     const float c = p.scale_log2;
     const float2 c2 = make_float2(c, c);
-    const bool varlen = p.cu_seqlens_q != nullptr;
     int G = 0, ni = 0;
     bool ok = true;
     for (int n = 0; ok; ++n) {
-      int nb, sk, shift, row;
-      {
-        DqpItem it;
-        ok = read_item(n, it);
-        if (!(ok = __all_sync(0xffffffffu, ok))) break;
-        if (it.mblk < 0) break;
-        const DqpWork w = dqp_decode(p, it);
-        nb = w.nb, sk = w.sk, shift = w.shift, row = w.row0 + row_in_tile;
-      }
+      ok = wait_item(n);
+      if (!(ok = __all_sync(0xffffffffu, ok))) break;
+      const DqItem* it = &xb->items[n & 1];  // stays in its slot until this warp releases it
+      const int nb = it->nb, sk = it->sk, shift = it->shift, row = it->row0 + row_in_tile;
+      if (nb < 0) break;
       float2 nl2 = make_float2(0.f, 0.f), nd2 = make_float2(0.f, 0.f);
-      bool s_ready = false;
       for (int j = 0; j < nb; ++j) {
         const int g = G + j;
-        if (!(ok = warp_wait_unless(s_ready, &bars->s_full, g & 1, ctx))) break;
+        // dP(g) complete: S and dP are there and packed-dS buffer g & 1 is free.  S and dP are fetched at once and handed back together, then the arithmetic of the block runs under the next products.
+        if (!(ok = mbar_wait_warp(&bars->dp_full, g & 1, ctx))) break;
         tc_fence_after_sync();
-        uint32_t sr[32];
+        uint32_t sr[32], dr[32];
         tmem_ld32(tS, sr);
-        const bool dp_ready = warp_probe(&bars->dp_full, g & 1);  // dP(j) follows S(j) through the pipe
+        tmem_ld32(tDP, dr);
         if (j == 0) {  // S(0) of the item was issued after its statistics had landed
           const float l = sStats[row_in_tile], dl = sStats[128 + row_in_tile];
           nl2 = make_float2(l, l), nd2 = make_float2(dl, dl);
@@ -415,6 +405,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
         tmem_wait_ld();
         warp_arrive_loaded(&bars->s_loaded, lane);
         if (j == 0 && lane == 0) mbar_arrive(&xb->q_free);  // the statistics are in registers
+        schedule_barrier(lane);
         const int col0 = j * kBlock + cq * 32;
         int limit = sk - 1 - col0;
         if (p.is_causal) limit = min(limit, row + shift - col0);
@@ -431,16 +422,10 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
             if (2 * i + 1 > limit) pr[i].y = 0.f;
           }
         }
-        if (!(ok = warp_wait_unless(dp_ready, &bars->dp_full, g & 1, ctx))) break;
-        tc_fence_after_sync();
-        tmem_ld32(tDP, sr);
-        s_ready = j + 1 < nb && warp_probe(&bars->s_full, (g + 1) & 1);  // S(j+1) ran under the exponentials
-        tmem_wait_ld();
-        warp_arrive_loaded(&bars->dp_loaded, lane);
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float2 d = fmul2(pr[i], fadd2(make_float2(__uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1])), nd2));
+          const float2 d = fmul2(pr[i], fadd2(make_float2(__uint_as_float(dr[2 * i]), __uint_as_float(dr[2 * i + 1])), nd2));
           pk[i] = pack_half2(d.x, d.y);
         }
         if (limit < 31) {  // by selection: dP of a masked column may be NaN/Inf (rows of the next sequence in V)
@@ -454,17 +439,11 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
         warp_arrive(&bars->ds_full, lane);
       }
       if (!ok) break;
-      // ---- epilogue: dQ = scale * acc; what it needs of the item is derived again from the ring slot ----
-      DqpItem it;
-      {
-        const volatile int* src = reinterpret_cast<const volatile int*>(&xb->items[n & 1]);
-        it.batch = src[0], it.head = src[1], it.mblk = src[2], it.pad = 0;
-      }
-      const DqpWork w = dqp_decode(p, it);
+      // ---- epilogue: dQ = scale * acc ----
       const bool stores = cq < D / 32;
-      const int64_t dq_idx = (varlen ? static_cast<int64_t>(w.q_off + row) * p.dq_row_stride
-                                     : w.batch * p.dq_batch_stride + static_cast<int64_t>(row) * p.dq_row_stride) +
-                             w.head * p.dq_head_stride + cq * 32;
+      const int64_t dq_idx = it->bq * p.dq_batch_stride + static_cast<int64_t>(it->q_off + row) * p.dq_row_stride +
+                             it->head * p.dq_head_stride + cq * 32;
+      const int sq = it->sq;
       if (nb > 0) {
         if (!(ok = mbar_wait_warp(&bars->acc_full, ni & 1, ctx))) break;
         ++ni;
@@ -476,8 +455,8 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
           tmem_ld32(tmem_base + lane_base + kColAcc + cq * 32, r);
           tmem_wait_ld();
           tc_fence_before_sync();
-          if (row < w.sq) store_row_fp16(p.dq + dq_idx, r, p.scale);
-        } else if (row < w.sq) {
+          if (row < sq) store_row_fp16(p.dq + dq_idx, r, p.scale);
+        } else if (row < sq) {
           const uint4 z = make_uint4(0, 0, 0, 0);
 #pragma unroll
           for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(p.dq + dq_idx + i * 8) = z;
@@ -514,6 +493,10 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
 // loaded as soon as the last dP^T product of the current item has read them, and its first S^T product is issued
 // under the last elementwise iteration and the epilogue of the current one.  Dense batches only: packed (varlen)
 // batches go to bwd_dkdv_packed_kernel below.
+constexpr int kDkvThreads = 640;  // + one scheduler warp: 20 warps, five on one sub-partition -> 96 registers
+constexpr int kDkvSchedWarp = 19;
+constexpr int kDkvReaders = kComputeWarps + 3;  // elementwise warps, producer warp, two MMA threads
+static_assert((kDkvThreads / 32 + 3) / 4 * 32 * 96 <= 16384, "register file of one SM sub-partition");
 struct DkvItem {
   int batch, head_k, nblk, pad;  // nblk < 0: no more work
 };
@@ -548,7 +531,7 @@ __device__ __forceinline__ DkvWork dkv_decode(const BwdKernelParams& p, const Dk
 }
 
 template <int D>
-__global__ void __launch_bounds__(kDqpThreads, 1)
+__global__ void __launch_bounds__(kDkvThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
   using C = BCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -574,7 +557,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
     mbar_init(&xb->kv_free, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&xb->sched_full[i], 1);
-      mbar_init(&xb->sched_empty[i], kDqpReaders);
+      mbar_init(&xb->sched_empty[i], kDkvReaders);
     }
     mbar_init(&xb->sched_go, 1);
     fence_mbar_init();
@@ -597,7 +580,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
   auto release_item = [&](int n) { mbar_arrive(&xb->sched_empty[n & 1]); };
 
   if (stop) {
-  } else if (warp == kDqpSchedWarp) {
+  } else if (warp == kDkvSchedWarp) {
     if (lane == 0) {
       bool finished = false;
       for (int n = 0;; ++n) {
@@ -1301,7 +1284,7 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
     FA_CHECK_ARG(total < (1ll << 30), "fa_bwd: too many work items");
     kq.total_items = static_cast<int>(total);
     const int grid = kq.total_items < sms ? kq.total_items : sms;
-    bwd_dq_kernel<D><<<grid, kDqpThreads, C::kSmemBytesDq + 1024, stream>>>(kq);
+    bwd_dq_kernel<D><<<grid, kDqThreads, C::kSmemBytesDq + 1024, stream>>>(kq);
     FA_CHECK_CUDA(cudaGetLastError());
   }
   if (stage_mask & 4) {
@@ -1319,7 +1302,7 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
       FA_CHECK_ARG(total < (1ll << 30), "fa_bwd: too many work items");
       kk.total_items = static_cast<int>(total);
       const int grid = kk.total_items < sms ? kk.total_items : sms;
-      bwd_dkdv_kernel<D><<<grid, kDqpThreads, C::kSmemBytesDkdv, stream>>>(kk);
+      bwd_dkdv_kernel<D><<<grid, kDkvThreads, C::kSmemBytesDkdv, stream>>>(kk);
     }
     FA_CHECK_CUDA(cudaGetLastError());
   }
