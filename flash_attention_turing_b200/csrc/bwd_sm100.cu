@@ -53,6 +53,7 @@ struct PreParams {
 // of each statistic.  grid (ceil(items / items_per_block), 1, b).
 constexpr int kPreRows = 8;
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const PreParams p) {
+  grid_launch_dependents();
   const int tpr = p.d / 8;  // threads per item: 8 or 16
   const int item = blockIdx.x * (256 / tpr) + threadIdx.x / tpr;
   const int sub = threadIdx.x % tpr;
@@ -190,6 +191,8 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
     }
     mbar_init(&xb->sched_go, 1);
     fence_mbar_init();
+    grid_dependency_wait();  // the row statistics; everything behind the synchronisation below may read them
+    grid_launch_dependents();
   }
   if (warp == kMmaWarp) {
     tmem_alloc(&bars->tmem_base, kTmemCols);
@@ -548,6 +551,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
   BBarriers* bars = &xb->b;
   if (smem - smem_raw > C::kAlignPadDkdv) {  // uniform over the CTA: nothing has been set up yet
     if (threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusSmemLayout);
+    grid_dependency_wait();
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -909,6 +913,8 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
     }
     __syncthreads();
   }
+  // the dQ kernel may still be running: this launch must not complete before it (see launch_bwd)
+  if (blockIdx.x == 0 && threadIdx.x == 0) grid_dependency_wait();
   if (warp == kMmaWarp) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
@@ -936,7 +942,11 @@ bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
   const int k_off = varlen ? p.cu_seqlens_k[batch] : 0;
   const int sk = varlen ? p.cu_seqlens_k[batch + 1] - k_off : p.seqlen_k;
   const int key0 = nblk * kBlock;
-  if (key0 >= sk) return;
+  const bool first_cta = (blockIdx.x | blockIdx.y | blockIdx.z) == 0;
+  if (key0 >= sk) {
+    if (first_cta) grid_dependency_wait();
+    return;
+  }
   const int stop_probe = stop_probe_begin(p.status);
   const int bq = varlen ? 0 : batch;
   const int group = p.h / p.h_k;
@@ -961,6 +971,7 @@ bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
   static_assert(sizeof(BBarriers) <= 512, "barrier block");
   if (smem - smem_raw > C::kAlignPadDkdv) {  // uniform over the CTA: nothing has been set up yet
     if (threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusSmemLayout);
+    if (first_cta) grid_dependency_wait();
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1145,6 +1156,9 @@ bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
       tmem_ld32(tA, sr);
       tmem_wait_ld();
       warp_arrive_loaded(&bars->s_loaded, lane);  // region A may now receive dP^T
+      // D = 128: 1650 -> 1600 us for 16 packed documents (Hq32 Hkv8); nothing at D = 64, nor in the dense kernel, where
+      // the other products of the pipe are in the way of the earlier dP^T
+      if constexpr (D == 128) schedule_barrier(lane);
       // columns below cmin are masked by causality; columns from cmax on are query rows past the end of the
       // sequence (last Q tile of a packed sequence).  Both clamped to [0, 32] and packed into one register.
       const int cmask = max(0, min(32, cmin0 - i_rel * kBlock)) |
@@ -1243,6 +1257,7 @@ bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
     }
     __syncthreads();
   }
+  if (first_cta && threadIdx.x == 0) grid_dependency_wait();  // as in bwd_dkdv_kernel
   if (warp == kMmaWarp) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
@@ -1284,13 +1299,27 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
     FA_CHECK_ARG(total < (1ll << 30), "fa_bwd: too many work items");
     kq.total_items = static_cast<int>(total);
     const int grid = kq.total_items < sms ? kq.total_items : sms;
-    bwd_dq_kernel<D><<<grid, kDqThreads, C::kSmemBytesDq + 1024, stream>>>(kq);
-    FA_CHECK_CUDA(cudaGetLastError());
+    if (stage_mask & 1) {
+      FA_CHECK_CUDA(launch_overlapped(bwd_dq_kernel<D>, dim3(grid), kDqThreads, C::kSmemBytesDq + 1024, stream, kq));
+    } else {
+      bwd_dq_kernel<D><<<grid, kDqThreads, C::kSmemBytesDq + 1024, stream>>>(kq);
+      FA_CHECK_CUDA(cudaGetLastError());
+    }
   }
   if (stage_mask & 4) {
+    // The dK/dV kernel reads nothing that the dQ kernel writes.  It starts on the SMs that the dQ kernel leaves idle (fewer
+    // items than SMs, the last wave) and ends after it: every CTA of the dQ kernel lets it go only when the preprocess
+    // kernel has finished, and its CTA 0 waits for the dQ kernel before it exits.  Whole backward, three launches in turn
+    // against overlapped: B3 S197 H12 D64 28.3 -> 17.0 us, B2 S512 H8 D64 32.4 -> 17.7, B1 S1000 H16 D128 causal
+    // 49.5 -> 43.6, B2 S2047 Hq16 Hkv4 D128 causal 195 -> 182, B16 S1024 H32 805 -> 786, B4 S8192 H32 7317 -> 7135.
+    const bool overlap = (stage_mask & 2) != 0;
     if (kp.cu_seqlens_q != nullptr) {  // packed sequences: one CTA per key tile (see bwd_dkdv_packed_kernel)
       dim3 grid_k((p->seqlen_k + kBlock - 1) / kBlock, p->h_k, p->b);
-      bwd_dkdv_packed_kernel<D, true><<<grid_k, kNumThreads, C::kSmemBytesDkdv, stream>>>(kp);
+      if (overlap) {
+        FA_CHECK_CUDA(launch_overlapped(bwd_dkdv_packed_kernel<D, true>, grid_k, kNumThreads, C::kSmemBytesDkdv, stream, kp));
+      } else {
+        bwd_dkdv_packed_kernel<D, true><<<grid_k, kNumThreads, C::kSmemBytesDkdv, stream>>>(kp);
+      }
     } else {
       BwdKernelParams kk = kp;
       const int sms = device_sm_count();
@@ -1302,7 +1331,11 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
       FA_CHECK_ARG(total < (1ll << 30), "fa_bwd: too many work items");
       kk.total_items = static_cast<int>(total);
       const int grid = kk.total_items < sms ? kk.total_items : sms;
-      bwd_dkdv_kernel<D><<<grid, kDkvThreads, C::kSmemBytesDkdv, stream>>>(kk);
+      if (overlap) {
+        FA_CHECK_CUDA(launch_overlapped(bwd_dkdv_kernel<D>, dim3(grid), kDkvThreads, C::kSmemBytesDkdv, stream, kk));
+      } else {
+        bwd_dkdv_kernel<D><<<grid, kDkvThreads, C::kSmemBytesDkdv, stream>>>(kk);
+      }
     }
     FA_CHECK_CUDA(cudaGetLastError());
   }

@@ -53,6 +53,26 @@ int* next_sched_slot();
 // Number of SMs of the current device (cached); 0 on error.
 int device_sm_count();
 
+// Launches a kernel that may start before the previous kernel of the stream has finished, as soon as that one lets it
+// (grid_launch_dependents() in ptx.cuh): its set-up and launch latency then run under the predecessor.  The kernel has to
+// call grid_dependency_wait() before it touches anything the predecessor writes, and in at least one CTA in any case, so
+// that its own completion implies that of everything before it.
+template <class Params>
+cudaError_t launch_overlapped(void (*kernel)(Params), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                              const Params& params) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, params);
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace fa

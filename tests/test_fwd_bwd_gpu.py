@@ -3,6 +3,8 @@ binding (which calls the C ABI).  Shapes follow the reference's grid (test_flash
 Cy-47/flash-attention-turing: odd lengths, Sq != Sk both ways, GQA/MQA head pairs, both head dims,
 causal on/off, explicit scale) plus MHA cases for the packed variants, which the reference's grid
 never reaches (all of its head pairs have Hq != Hk)."""
+import ctypes
+
 import pytest
 import torch
 
@@ -647,3 +649,73 @@ def test_package_reports_the_device_status_word(ext):
 
     assert fa.device_status() == 0
     assert fa.device_status(reset=True) == 0
+
+
+def _bwd_params_for(ext, b, s, h, hk, d, causal, lens):
+    """Inputs, outputs and filled FaBwdParams of a dense batch, or of packed sequences of the given lengths."""
+    from flash_attention_turing_b200 import capi
+
+    torch.manual_seed(0)
+    rows = (sum(lens),) if lens else (b, s)
+    q, k, v, dout = (torch.randn(*rows, n, d, device=DEV, dtype=torch.float16) for n in (h, hk, hk, h))
+    cu = torch.tensor([0] + list(lens), dtype=torch.int32, device=DEV).cumsum(0, dtype=torch.int32) if lens else None
+    extra = () if cu is None else (cu, cu, s, s)
+    scale = d ** -0.5
+    out, lse = ext.fwd(q, k, v, scale, causal) if cu is None else ext.varlen_fwd(q, k, v, *extra, scale, causal)
+    grads = [torch.empty_like(x) for x in (q, k, v)]
+    four_d = [x if cu is None else x.unsqueeze(0) for x in (q, k, v, out, dout, *grads)]
+    p = capi.bwd_params(*four_d[:5], lse, *four_d[5:], None, scale, causal)
+    p.b, p.seqlen_q, p.seqlen_k = b, s, s
+    if cu is not None:
+        p.cu_seqlens_q = p.cu_seqlens_k = cu.data_ptr()
+        p.total_q = p.total_k = sum(lens)
+    ws = torch.empty(capi.lib().fa_bwd_workspace_bytes(ctypes.byref(p)), dtype=torch.uint8, device=DEV)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    return p, grads, ws, (q, k, v, out, dout, lse, cu)  # the last: kept alive by the caller
+
+
+@pytest.mark.parametrize("b,s,h,hk,d,causal,lens", [
+    (1, 1, 1, 1, 64, False, ()),          # one item in every kernel
+    (3, 197, 12, 12, 64, False, ()),      # fewer items than SMs: the dK/dV kernel runs beside the dQ kernel
+    (2, 640, 16, 4, 128, True, ()),       # a few more items than SMs in the dQ kernel
+    (1, 4096, 8, 8, 128, True, ()),
+    (3, 300, 4, 2, 128, True, (300, 1, 129)),
+    (2, 700, 24, 24, 64, True, (700, 256)),
+])
+def test_overlapped_backward_launches_equal_separate_ones(ext, b, s, h, hk, d, causal, lens):
+    """dQ starts under the preprocess kernel and dK/dV under dQ; a kernel that did not wait for the row statistics would
+    read the NaN pattern that the workspace is filled with before every call.  Bit for bit, also replayed from a graph."""
+    from flash_attention_turing_b200 import capi
+
+    lib = capi.lib()
+    p, grads, ws, keep = _bwd_params_for(ext, b, s, h, hk, d, causal, lens)
+
+    def stream():
+        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    for stage in (1, 2, 4):
+        capi.check(lib.fa_bwd_stages(ctypes.byref(p), stage, stream()))
+        torch.cuda.synchronize()
+    want = [g.clone() for g in grads]
+    assert all(torch.isfinite(g).all() for g in want)
+    got = []
+    for _ in range(20):
+        ws.fill_(255)
+        for g in grads:
+            g.fill_(float("nan"))
+        capi.check(lib.fa_bwd(ctypes.byref(p), stream()))
+        got.append([g.clone() for g in grads])  # on the stream, right behind the last kernel
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ws.fill_(255)
+        capi.check(lib.fa_bwd(ctypes.byref(p), stream()))
+        copies = [g.clone() for g in grads]
+    for _ in range(5):
+        for g in grads:
+            g.fill_(float("nan"))
+        graph.replay()
+        got.append([c.clone() for c in copies])
+    torch.cuda.synchronize()
+    assert lib.fa_device_status(0) == 0
+    for run in got:
+        assert all(torch.equal(a, w) for a, w in zip(run, want))
