@@ -2,7 +2,7 @@
 //
 // One warp per output row.  The split LSEs are spread over the lanes and reduced with warp
 // shuffles (max, then sum of exponentials); each lane then owns D/32 consecutive output columns
-// and streams the fp32 partial rows with 8- or 16-byte loads, so a row of every split is one
+// and streams the fp32 partial rows with 8- or 16-byte loads, four rows at a time, so a row of every split is one
 // fully coalesced 256/512-byte read.  HBM-bound: bytes = splits*rows*(D+1)*4 + rows*(2*D+4).
 //
 // Replaces kvcache_combine_kernel / kvcache_combine_kernel_legacy of the reference
@@ -18,25 +18,35 @@ namespace {
 
 constexpr int kWarpsPerBlock = 8;
 
+struct CombineArgs {
+  const float* o_accum;
+  const float* lse_accum;
+  __half* o;
+  float* lse;
+  int64_t rows, o_batch_stride, o_row_stride, o_head_stride;
+  int num_splits, h, seqlen_q;
+};
+
 template <int D>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-combine_kernel(const float* __restrict__ o_accum, const float* __restrict__ lse_accum,
-               __half* __restrict__ o, float* __restrict__ lse, int64_t rows, int num_splits,
-               int h, int seqlen_q, int64_t o_batch_stride, int64_t o_row_stride,
-               int64_t o_head_stride) {
+__global__ void __launch_bounds__(kWarpsPerBlock * 32) combine_kernel(const __grid_constant__ CombineArgs a) {
   constexpr int kPerLane = D / 32;  // 2 or 4 consecutive columns
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (row >= rows) return;
+  grid_dependency_wait();  // the partials
+  if (row >= a.rows) return;
 
   // log-sum-exp over splits: lanes stride over the splits, shuffles reduce
-  float mx = -INFINITY;
-  for (int s = lane; s < num_splits; s += 32) mx = fmaxf(mx, lse_accum[s * rows + row]);
+  const float* lse_row = a.lse_accum + row;
+  const float first = lane < a.num_splits ? lse_row[lane * a.rows] : -INFINITY;
+  float mx = first;
+  for (int s = lane + 32; s < a.num_splits; s += 32) mx = fmaxf(mx, lse_row[s * a.rows]);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   float sum = 0.f;
-  if (mx != -INFINITY)
-    for (int s = lane; s < num_splits; s += 32) sum += __expf(lse_accum[s * rows + row] - mx);
+  if (mx != -INFINITY) {
+    if (lane < a.num_splits) sum += __expf(first - mx);
+    for (int s = lane + 32; s < a.num_splits; s += 32) sum += __expf(lse_row[s * a.rows] - mx);
+  }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
   const bool empty = (mx == -INFINITY) || (sum == 0.f);
@@ -45,33 +55,49 @@ combine_kernel(const float* __restrict__ o_accum, const float* __restrict__ lse_
   float acc[kPerLane];
 #pragma unroll
   for (int i = 0; i < kPerLane; ++i) acc[i] = 0.f;
-  if (!empty) {
-    for (int s = 0; s < num_splits; ++s) {
-      const float ls = lse_accum[s * rows + row];  // same address for all lanes: one broadcast load
-      if (ls == -INFINITY) continue;
-      const float w = __expf(ls - lse_total);
-      const float* src = o_accum + (static_cast<int64_t>(s) * rows + row) * D + lane * kPerLane;
-      if constexpr (kPerLane == 4) {
-        const float4 x = *reinterpret_cast<const float4*>(src);
-        acc[0] = fmaf(w, x.x, acc[0]);
-        acc[1] = fmaf(w, x.y, acc[1]);
-        acc[2] = fmaf(w, x.z, acc[2]);
-        acc[3] = fmaf(w, x.w, acc[3]);
-      } else {
-        const float2 x = *reinterpret_cast<const float2*>(src);
-        acc[0] = fmaf(w, x.x, acc[0]);
-        acc[1] = fmaf(w, x.y, acc[1]);
+  // Weights of 32 splits sit in the lanes; the partial rows of the live ones are fetched four at a time (one load after
+  // another was a chain of one memory latency per split).  Added in the order of the splits.
+  for (int base = 0; !empty && base < a.num_splits; base += 32) {
+    const int s = base + lane;
+    const float ls = base == 0 ? first : (s < a.num_splits ? lse_row[s * a.rows] : -INFINITY);
+    const float w = ls == -INFINITY ? 0.f : __expf(ls - lse_total);
+    const float* src = a.o_accum + (base * a.rows + row) * D + lane * kPerLane;
+    uint32_t live = __ballot_sync(0xffffffffu, ls != -INFINITY);
+    while (live != 0) {
+      int idx[4];
+      float x[4][kPerLane];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        idx[u] = __ffs(live) - 1;  // -1: none left
+        live &= live - 1;
+        if (idx[u] >= 0) {
+          const float* from = src + idx[u] * a.rows * D;
+          if constexpr (kPerLane == 4) {
+            const float4 v = *reinterpret_cast<const float4*>(from);
+            x[u][0] = v.x, x[u][1] = v.y, x[u][2] = v.z, x[u][3] = v.w;
+          } else {
+            const float2 v = *reinterpret_cast<const float2*>(from);
+            x[u][0] = v.x, x[u][1] = v.y;
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (idx[u] >= 0) {
+          const float wu = __shfl_sync(0xffffffffu, w, idx[u]);
+#pragma unroll
+          for (int i = 0; i < kPerLane; ++i) acc[i] = fmaf(wu, x[u][i], acc[i]);
+        }
       }
     }
   }
 
   // rows are ordered (b, h, seqlen_q)
-  const int64_t bh = row / seqlen_q;
-  const int q_pos = static_cast<int>(row - bh * seqlen_q);
-  const int64_t batch = bh / h;
-  const int head = static_cast<int>(bh - batch * h);
-  __half* dst = o + batch * o_batch_stride + q_pos * o_row_stride + head * o_head_stride +
-                lane * kPerLane;
+  const int64_t bh = row / a.seqlen_q;
+  const int q_pos = static_cast<int>(row - bh * a.seqlen_q);
+  const int64_t batch = bh / a.h;
+  const int head = static_cast<int>(bh - batch * a.h);
+  __half* dst = a.o + batch * a.o_batch_stride + q_pos * a.o_row_stride + head * a.o_head_stride + lane * kPerLane;
   if constexpr (kPerLane == 4) {
     uint2 v;
     v.x = pack_half2(acc[0], acc[1]);
@@ -80,7 +106,7 @@ combine_kernel(const float* __restrict__ o_accum, const float* __restrict__ lse_
   } else {
     *reinterpret_cast<uint32_t*>(dst) = pack_half2(acc[0], acc[1]);
   }
-  if (lse != nullptr && lane == 0) lse[row] = empty ? 0.f : lse_total;
+  if (a.lse != nullptr && lane == 0) a.lse[row] = empty ? 0.f : lse_total;
 }
 
 // Merge over ranks with the partials read in place (possibly from peer GPUs): D/8 lanes per output row
@@ -244,18 +270,17 @@ sum_gather_kernel(const __grid_constant__ SumArgs a, __half* __restrict__ out, i
 
 int launch_combine(const float* o_accum, const float* lse_accum, void* o, float* lse, int64_t rows,
                    int num_splits, int h, int seqlen_q, int d, int64_t o_batch_stride,
-                   int64_t o_row_stride, int64_t o_head_stride, cudaStream_t stream) {
+                   int64_t o_row_stride, int64_t o_head_stride, cudaStream_t stream, bool overlap) {
   if (rows == 0) return FA_OK;
   const unsigned blocks = static_cast<unsigned>((rows + kWarpsPerBlock - 1) / kWarpsPerBlock);
-  if (d == 128) {
-    combine_kernel<128><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(
-        o_accum, lse_accum, static_cast<__half*>(o), lse, rows, num_splits, h, seqlen_q,
-        o_batch_stride, o_row_stride, o_head_stride);
-  } else {
-    combine_kernel<64><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(
-        o_accum, lse_accum, static_cast<__half*>(o), lse, rows, num_splits, h, seqlen_q,
-        o_batch_stride, o_row_stride, o_head_stride);
+  const CombineArgs a{o_accum, lse_accum, static_cast<__half*>(o), lse, rows, o_batch_stride, o_row_stride, o_head_stride,
+                      num_splits, h, seqlen_q};
+  const auto kernel = d == 128 ? combine_kernel<128> : combine_kernel<64>;
+  if (overlap) {
+    FA_CHECK_CUDA(launch_overlapped(kernel, dim3(blocks), kWarpsPerBlock * 32, 0, stream, a));
+    return FA_OK;
   }
+  kernel<<<blocks, kWarpsPerBlock * 32, 0, stream>>>(a);
   FA_CHECK_CUDA(cudaGetLastError());
   return FA_OK;
 }

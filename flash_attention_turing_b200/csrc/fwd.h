@@ -5,7 +5,8 @@
 
 namespace fa {
 
-// Same as fa_fwd(); seqused_k_add is added to every seqused_k[b] on the device.
-int run_fwd(const FaFwdParams* p, int seqused_k_add, cudaStream_t stream);
+// Same as fa_fwd(); seqused_k_add is added to every seqused_k[b] on the device.  overlap: the previous kernel of the stream
+// lets this one start early (launch_overlapped).
+int run_fwd(const FaFwdParams* p, int seqused_k_add, cudaStream_t stream, bool overlap = false);
 
 }  // namespace fa

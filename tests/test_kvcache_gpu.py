@@ -220,3 +220,64 @@ def test_device_side_capacity_clamp_without_host_check(ext):
     with pytest.raises(ValueError, match="cache capacity is insufficient"):
         iface.flash_attn_with_kvcache(q.to(DEV), kc.to(DEV), vc.to(DEV), cache_seqlens=lens_bad.to(DEV),
                                       block_table=table.to(DEV), causal=True)
+
+
+@pytest.mark.parametrize("b,new,h,hk,d,length,capacity,page,splits", [
+    (1, 1, 8, 2, 128, 700, 1024, 0, 0),     # append, attend and merge overlap
+    (1, 1, 4, 4, 64, 63, 512, 256, 1),      # no merge; the appended token starts a tile
+    (3, 4, 8, 2, 64, 250, 512, 256, 4),     # the new tokens straddle a page
+    (2, 64, 4, 2, 128, 190, 512, 256, 0),   # tiled path
+])
+def test_overlapped_steps_see_the_appended_rows(ext, b, new, h, hk, d, length, capacity, page, splits):
+    """The attend kernel starts under the append kernel and the merge under the attend kernel.  The rows that are appended
+    hold NaN before every call, so a kernel that did not wait would not return the same bits; also replayed from a graph."""
+    torch.manual_seed(0)
+    half = lambda *s: torch.randn(*s, device=DEV, dtype=torch.float16)  # noqa: E731
+    q, kn, vn = half(b, new, h, d), half(b, new, hk, d), half(b, new, hk, d)
+    rows = (b * (capacity // page), page) if page else (b, capacity)
+    kc, vc = half(*rows, hk, d), half(*rows, hk, d)
+    table = torch.arange(rows[0], dtype=torch.int32, device=DEV).view(b, -1) if page else None
+    lens = torch.full((b,), length, dtype=torch.int32, device=DEV)
+    flat_k, flat_v = kc.view(b, -1, hk, d), vc.view(b, -1, hk, d)
+
+    def step():
+        flat_k[:, length:] = float("nan")
+        flat_v[:, length:] = float("nan")
+        return ext.fwd_kvcache(q, kc, vc, kn, vn, lens, None, None, None, None, table, None, None, d ** -0.5, True, -1, -1,
+                               0.0, True, splits)
+
+    want, want_lse = step()
+    torch.cuda.synchronize()
+    assert torch.isfinite(want).all() and torch.equal(flat_k[:, length:length + new], kn)
+    got = [step() for _ in range(20)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step()
+    for _ in range(5):
+        graph.replay()
+        got.append([x.clone() for x in captured])
+    torch.cuda.synchronize()
+    for out, lse in got:
+        assert torch.equal(out, want) and torch.equal(lse, want_lse)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("splits", [1, 3, 4, 5, 31, 32, 33, 64, 67])
+def test_merge_at_the_edges_of_its_batches(ext, d, splits):
+    """Partials are fetched four at a time and weights held for 32 splits; empty splits (LSE = -inf, NaN rows) lie between."""
+    gen = torch.Generator().manual_seed(splits)
+    b, h, sq = 2, 3, 3
+    rows = b * h * sq
+    o_acc, l_acc = torch.randn(splits, rows, d, generator=gen), torch.randn(splits, rows, generator=gen) * 3
+    dead = torch.rand(splits, rows, generator=gen) < 0.4
+    dead[:, 0], dead[:, 1] = False, True
+    l_acc[dead], o_acc[dead] = float("-inf"), float("nan")
+    out, lse = ext.combine(o_acc.to(DEV), l_acc.to(DEV), b, sq, h)
+    want = torch.logsumexp(l_acc.double(), 0)
+    weight = torch.where(dead, 0.0, torch.exp(l_acc.double() - want))
+    o_ref = (weight[..., None] * torch.nan_to_num(o_acc).double()).sum(0)
+    want[dead.all(0)] = 0  # nothing to attend to
+    got = out.float().cpu().permute(0, 2, 1, 3).reshape(rows, d)
+    # half an fp16 ulp of the result, and 1e-5 for the exponentials and the fp32 sums
+    assert ((got - o_ref).abs() <= o_ref.abs() * 2 ** -11 + 1e-5).all()
+    assert err_stats(lse.view(-1), want)[0] <= 1e-5
