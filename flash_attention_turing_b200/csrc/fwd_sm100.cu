@@ -280,7 +280,7 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
             const int len = p.cu_seqlens_q[seq + 1] - p.cu_seqlens_q[seq];
             batch = seq, head = rel / cnt;
             mpair = (len + kTiles * kBlockM - 1) / (kTiles * kBlockM) - 1 - rel % cnt;  // < 0: the spare slot
-            if (head >= p.h) mpair = -1;  // past the last sequence
+            if (rel < 0 || head >= p.h) mpair = -1;  // before the first sequence (cu_seqlens_q[0] >= 256), past the last one
           }
           const int sq = p.cu_seqlens_q ? p.cu_seqlens_q[batch + 1] - p.cu_seqlens_q[batch] : p.seqlen_q;
           if (mpair >= 0 && mpair * (kTiles * kBlockM) < sq) {

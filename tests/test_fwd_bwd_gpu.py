@@ -719,3 +719,24 @@ def test_overlapped_backward_launches_equal_separate_ones(ext, b, s, h, hk, d, c
     assert lib.fa_device_status(0) == 0
     for run in got:
         assert all(torch.equal(a, w) for a, w in zip(run, want))
+
+
+@pytest.mark.parametrize("before", [127, 128, 255, 256, 700])
+def test_packed_sequences_that_start_past_the_first_tiles(ext, before):
+    """cu_seqlens[0] > 0: the work indices below the first sequence's are spare ones.  Bit for bit what the sequences give
+    when they start at row 0."""
+    gen = torch.Generator().manual_seed(6)
+    lens, h, hk, d = (300, 1, 70), 4, 2, 64
+    used, scale = sum(lens), d ** -0.5
+    q, k, v, dout = (randn_half(gen, before + used, n, d).to(DEV) for n in (h, hk, hk, h))
+    cu = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0, dtype=torch.int32).to(DEV)
+
+    def run(q, k, v, dout, cu):
+        out, lse = ext.varlen_fwd(q, k, v, cu, cu, max(lens), max(lens), scale, True)
+        return (out, *ext.varlen_bwd(q, k, v, out, lse, dout, cu, cu, max(lens), max(lens), scale, True))
+
+    got = run(q, k, v, dout, cu + before)
+    want = run(*(x[before:].contiguous() for x in (q, k, v, dout)), cu)
+    for a, b in zip(got, want):
+        assert torch.equal(a[before:], b) and a[:before].abs().sum() == 0
+    assert ext.device_status(True) == 0
