@@ -45,7 +45,7 @@ class FaFwdParams(C.Structure):
            ("softmax_scale", _f32), ("is_causal", _i32), ("cu_seqlens_q", _vp), ("cu_seqlens_k", _vp),
            ("seqused_k", _vp), ("cache_batch_idx", _vp), ("block_table", _vp),
            ("block_table_batch_stride", _i64), ("page_size", _i32), ("block_table_cols", _i32),
-           ("causal_shift", _i32), ("reserved0", _i32)]
+           ("causal_shift", _i32), ("flags", _i32)]
     )
 
 
@@ -61,7 +61,9 @@ class FaBwdParams(C.Structure):
     )
 
 
+FA_FWD_ZERO_UNUSED_ROWS = 1
 FA_BWD_SINGLE_KERNEL = 1
+FA_BWD_ZERO_UNUSED_ROWS = 2
 FA_CAUSAL_SHIFT = 2
 
 

@@ -138,11 +138,12 @@ std::vector<at::Tensor> mha_varlen_fwd(at::Tensor q, at::Tensor k, at::Tensor v,
   const int64_t num_heads = q.size(1), num_heads_k = k.size(1), head_size = q.size(2);
   c10::cuda::CUDAGuard guard(q.device());
 
-  at::Tensor out = torch::zeros_like(q);  // rows outside every sequence stay zero, as in the reference
+  at::Tensor out = torch::empty_like(q);
   at::Tensor l = torch::zeros({batch_size, num_heads, max_seqlen_q}, q.options().dtype(torch::kFloat32));
-  if (q.size(0) == 0 || k.size(0) == 0 || max_seqlen_q <= 0) return {out, l};
+  if (q.size(0) == 0 || k.size(0) == 0 || max_seqlen_q <= 0) return {out.zero_(), l};
 
   FaFwdParams p = {};
+  p.flags = FA_FWD_ZERO_UNUSED_ROWS;  // rows outside every sequence are zero, as in the reference
   p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr(); p.o = out.data_ptr();
   p.lse = l.data_ptr<float>();
   p.q_row_stride = q.stride(0); p.q_head_stride = q.stride(1); p.q_batch_stride = 0;
@@ -259,11 +260,14 @@ std::vector<at::Tensor> mha_varlen_bwd(at::Tensor q, at::Tensor k, at::Tensor v,
               "l must be a contiguous float32 CUDA tensor");
   c10::cuda::CUDAGuard guard(q.device());
 
-  // rows outside every sequence stay zero, as in the reference (torch::zeros_like, :462-464)
-  at::Tensor dq = grad_destination(dq_, q, "dq", true);
-  at::Tensor dk = grad_destination(dk_, k, "dk", true);
-  at::Tensor dv = grad_destination(dv_, v, "dv", true);
-  if (q.size(0) == 0 || k.size(0) == 0 || max_seqlen_q <= 0 || max_seqlen_k <= 0) return {dq, dk, dv};
+  // rows outside every sequence are zero, as in the reference (torch::zeros_like, :462-464); the default path clears
+  // them itself, a whole pass over the gradients less
+  const bool empty = q.size(0) == 0 || k.size(0) == 0 || max_seqlen_q <= 0 || max_seqlen_k <= 0;
+  const bool zero_all = empty || (g_bwd_flags & FA_BWD_SINGLE_KERNEL) != 0;
+  at::Tensor dq = grad_destination(dq_, q, "dq", zero_all);
+  at::Tensor dk = grad_destination(dk_, k, "dk", zero_all);
+  at::Tensor dv = grad_destination(dv_, v, "dv", zero_all);
+  if (empty) return {dq, dk, dv};
 
   FaBwdParams p = {};
   p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr(); p.o = out.data_ptr();
@@ -285,7 +289,7 @@ std::vector<at::Tensor> mha_varlen_bwd(at::Tensor q, at::Tensor k, at::Tensor v,
   p.is_causal = is_causal;
   p.cu_seqlens_q = cu_seqlens_q.data_ptr<int>();
   p.cu_seqlens_k = cu_seqlens_k.data_ptr<int>();
-  p.flags = g_bwd_flags;
+  p.flags = zero_all ? g_bwd_flags : g_bwd_flags | FA_BWD_ZERO_UNUSED_ROWS;
   const size_t ws = fa_bwd_workspace_bytes(&p);
   at::Tensor workspace = torch::empty({static_cast<int64_t>(ws)}, q.options().dtype(torch::kUInt8));
   p.workspace = workspace.data_ptr();

@@ -31,6 +31,10 @@ extern "C" {
 /* Same underlying type as cudaStream_t (struct CUstream_st*); void* keeps the header CUDA-free. */
 typedef void* fa_stream_t;
 
+/* FaFwdParams.flags: packed (varlen) calls also set the rows of o outside every sequence to zero; without it they are left
+ * as they are.  FA_BWD_ZERO_UNUSED_ROWS does the same for dq, dk, dv (and for keys past max_seqlen_k). */
+#define FA_FWD_ZERO_UNUSED_ROWS 1
+
 #define FA_CAUSAL_SHIFT 2 /* value of is_causal: the causal diagonal is given by causal_shift */
 
 enum {
@@ -116,7 +120,7 @@ typedef struct FaFwdParams {
   int32_t page_size;           /* tokens per page (multiple of 128) when block_table != NULL    */
   int32_t block_table_cols;    /* columns of block_table (0 = unknown: seqused_k is trusted)    */
   int32_t causal_shift;        /* used when is_causal == FA_CAUSAL_SHIFT                        */
-  int32_t reserved0;
+  int32_t flags;               /* FA_FWD_* bits, 0 by default                                   */
 } FaFwdParams;
 
 int fa_fwd(const FaFwdParams* p, fa_stream_t stream);
@@ -142,6 +146,7 @@ int fa_fwd(const FaFwdParams* p, fa_stream_t stream);
 /* (heads x padded rows x d).  The size depends on `flags`.                                      */
 /* ------------------------------------------------------------------------------------------- */
 #define FA_BWD_SINGLE_KERNEL 1
+#define FA_BWD_ZERO_UNUSED_ROWS 2 /* packed calls, default path: see FA_FWD_ZERO_UNUSED_ROWS */
 typedef struct FaBwdParams {
   const void* q;
   const void* k;
@@ -169,7 +174,7 @@ typedef struct FaBwdParams {
   const int32_t* cu_seqlens_k;
   void* workspace;
   size_t workspace_bytes;
-  int32_t flags;      /* 0 or FA_BWD_SINGLE_KERNEL */
+  int32_t flags;      /* FA_BWD_* bits, 0 by default */
   int32_t causal_shift; /* used when is_causal == FA_CAUSAL_SHIFT */
 } FaBwdParams;
 

@@ -740,3 +740,43 @@ def test_packed_sequences_that_start_past_the_first_tiles(ext, before):
     for a, b in zip(got, want):
         assert torch.equal(a[before:], b) and a[:before].abs().sum() == 0
     assert ext.device_status(True) == 0
+
+
+@pytest.mark.parametrize("path", ["default", "single_kernel"])
+@pytest.mark.parametrize("d,before,after,lens,max_k", [
+    (64, 0, 0, (5, 300, 128), 300),      # nothing to clear
+    (64, 3, 0, (130,), 130),
+    (128, 0, 1, (1, 257), 600),
+    (128, 140, 77, (64, 0, 200), 256),   # an empty sequence in between
+])
+def test_rows_outside_every_packed_sequence_are_zero(ext, request, path, d, before, after, lens, max_k):
+    """cu_seqlens may start above 0 and end below the last row: O, dQ, dK, dV are zero there, whatever the memory held, and
+    the sequences come out as they do without the extra rows, bit for bit."""
+    if path == "single_kernel":
+        request.getfixturevalue("single_kernel_backward")
+    gen = torch.Generator().manual_seed(5)
+    h, hk, used = 4, 2, sum(lens)
+    total = before + used + after
+    q, k, v, dout = (randn_half(gen, total, n, d).to(DEV) for n in (h, hk, hk, h))
+    inner = slice(before, before + used)
+    cu0 = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0, dtype=torch.int32).to(DEV)
+    cu = cu0 + before
+    max_q, scale = max(lens), d ** -0.5
+    torch.cuda.empty_cache()
+    junk = [torch.full_like(x, float("nan")) for x in (q, q, k, v)]
+    grads = [torch.full_like(x, float("nan")) for x in (q, k, v)]
+    del junk  # the allocator hands this memory out for O
+    out, lse = ext.varlen_fwd(q, k, v, cu, cu, max_q, max_k, scale, True)
+    ext.varlen_bwd(q, k, v, out, lse, dout, cu, cu, max_q, max_k, scale, True, *grads)
+    qi, ki, vi, di = (x[inner].contiguous() for x in (q, k, v, dout))
+    want, want_lse = ext.varlen_fwd(qi, ki, vi, cu0, cu0, max_q, max_k, scale, True)
+    want_grads = ext.varlen_bwd(qi, ki, vi, want, want_lse, di, cu0, cu0, max_q, max_k, scale, True)
+    assert torch.equal(out[inner], want) and torch.equal(lse, want_lse)
+    for i, (got, ref) in enumerate(zip(grads, want_grads)):
+        if i == 0 and path == "single_kernel":  # summed in no fixed order: an fp16 ulp, and fp32 noise where it cancels
+            torch.testing.assert_close(got[inner], ref, rtol=2 ** -10, atol=1e-4)
+        else:
+            assert torch.equal(got[inner], ref)
+    for x in (out, *grads):
+        assert x[:before].abs().sum() == 0 and x[before + used:].abs().sum() == 0
+    assert ext.device_status(True) == 0
