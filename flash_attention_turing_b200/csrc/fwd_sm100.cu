@@ -80,7 +80,7 @@ struct FwdKernelParams {
   int page_size;
   int* status;
   int* sched;         // {next item - gridDim.x, CTAs finished}: both zero at launch and again at the end
-  int items_x;        // dense: work items per (sequence, head) = ceil(seqlen_q / 256)
+  int items_x;        // dense: work items per (sequence, head) = ceil(seqlen_q / rows of an item)
   int total_items;    // dense: items_x * h * b; packed sequences: h * (total_q / 256 + b), see the scheduler
   int b;              // sequences
 };
@@ -135,6 +135,7 @@ struct Work {
   bool fix_v_tail;
 };
 
+template <int kItemRows>
 __device__ __forceinline__ Work decode_work(const FwdKernelParams& p, const WorkItem& it) {
   Work w;
   w.batch = it.batch;
@@ -149,12 +150,13 @@ __device__ __forceinline__ Work decode_work(const FwdKernelParams& p, const Work
     // clamped to what the K/V tensor (or the block table) can hold; the scheduler thread reports a clamp
     w.sk = max(0, min(p.seqused_k[w.batch] + p.seqused_k_add, p.k_capacity));
   }
-  w.row0 = it.mpair * (kTiles * kBlockM);
+  w.row0 = it.mpair * kItemRows;
   w.bq = varlen_q ? 0 : w.batch;
   w.bk = varlen_k ? 0 : (p.cache_batch_idx ? p.cache_batch_idx[w.batch] : w.batch);
   w.head_k = w.head / (p.h / p.h_k);
   // causal diagonal: key j is visible to query i iff j <= i + shift
   w.shift = (p.is_causal == 2) ? p.causal_shift : w.sk - w.sq;
+  if (kItemRows == kBlockM) w.sq = min(w.sq, w.row0 + kBlockM);  // the rows after the item's only tile are not its own
   // number of K/V blocks each tile visits
   w.nkb = (w.sk + kBlockN - 1) / kBlockN;
 #pragma unroll
@@ -177,7 +179,9 @@ __device__ __forceinline__ Work decode_work(const FwdKernelParams& p, const Work
   return w;
 }
 
-template <int D>
+// kItemRows = 256: two Q tiles per item.  kItemRows = 128: one, the second tile's warps have nothing to do (dense batches, chosen
+// in launch_fwd).
+template <int D, int kItemRows>
 __global__ void __maxnreg__(168)
 fwd_kernel(const __grid_constant__ FwdKernelParams p) {
   using C = Cfg<D>;
@@ -284,7 +288,7 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
             if (rel < 0 || head >= p.h) mpair = -1;  // before the first sequence (cu_seqlens_q[0] >= 256), past the last one
           }
           const int sq = p.cu_seqlens_q ? p.cu_seqlens_q[batch + 1] - p.cu_seqlens_q[batch] : p.seqlen_q;
-          if (mpair >= 0 && mpair * (kTiles * kBlockM) < sq) {
+          if (mpair >= 0 && mpair * kItemRows < sq) {
             it.batch = batch, it.head = head, it.mpair = mpair;
             if (p.seqused_k && p.status && head == 0 && mpair == 0) {
               const int raw = p.seqused_k[batch] + p.seqused_k_add;
@@ -324,7 +328,7 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
       __syncwarp();
       if (lane == 0) release_item(n);
       if (it.mpair < 0) break;
-      const Work w = decode_work(p, it);
+      const Work w = decode_work<kItemRows>(p, it);
       if (w.nb_max == 0) continue;
       if (lane == 0) {
         ok = mbar_wait(&bars->q_empty, (nq & 1) ^ 1, ctx);
@@ -437,7 +441,7 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
         if (!(ok = read_item(n, it, ctx))) break;
         release_item(n);
         if (it.mpair < 0) break;
-        const Work w = decode_work(p, it);
+        const Work w = decode_work<kItemRows>(p, it);
         const int nb0 = w.nb[0], nb1 = w.nb[1], nb_max = w.nb_max;
         if (nb_max <= 2) mbar_arrive(&bars->sched_go);  // short item: claim the next one right away
         if (nb_max == 0) continue;
@@ -524,7 +528,7 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
         ok = read_item(n, it, ctx);
         if (!(ok = __all_sync(0xffffffffu, ok))) break;
         if (it.mpair < 0) break;
-        const Work w = decode_work(p, it);
+        const Work w = decode_work<kItemRows>(p, it);
         row = w.row0 + t * kBlockM + row_in_tile;
         nbt = t ? w.nb[1] : w.nb[0], sk = w.sk, shift = w.shift, nb_max = w.nb_max;
       }
@@ -656,7 +660,7 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
         const volatile int* src = reinterpret_cast<const volatile int*>(&bars->items[n % kSchedDepth]);
         it.batch = src[0], it.head = src[1], it.mpair = src[2], it.pad = 0;
       }
-      const Work w = decode_work(p, it);
+      const Work w = decode_work<kItemRows>(p, it);
       const bool row_valid = row < w.sq;
       int64_t o_index;
       if (varlen_q) {
@@ -733,21 +737,21 @@ __global__ void __launch_bounds__(256) clear_unused_rows_kernel(const __grid_con
   clear_unused_rows(t, static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x, static_cast<int64_t>(gridDim.x) * blockDim.x);
 }
 
-template <int D>
-int launch_fwd(FwdKernelParams& kp, int b, int h, int seqlen_q, int64_t total_q, bool overlap, cudaStream_t stream) {
+template <int D, int kItemRows>
+int launch_items(FwdKernelParams& kp, int b, int h, int seqlen_q, int64_t total_q, bool overlap, cudaStream_t stream) {
   using C = Cfg<D>;
   static bool configured[64] = {};
   int dev = 0;
   FA_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    FA_CHECK_CUDA(cudaFuncSetAttribute(fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    FA_CHECK_CUDA(cudaFuncSetAttribute(fwd_kernel<D, kItemRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        C::kSmemBytes));
     configured[dev & 63] = true;
   }
   const int sms = device_sm_count();
   kp.sched = next_sched_slot();
   if (sms <= 0 || kp.sched == nullptr) return set_error(FA_ERR_CUDA, "fa_fwd: device attributes not available");
-  kp.items_x = (seqlen_q + kTiles * kBlockM - 1) / (kTiles * kBlockM);
+  kp.items_x = (seqlen_q + kItemRows - 1) / kItemRows;
   kp.b = b;
   const int64_t total = kp.cu_seqlens_q ? static_cast<int64_t>(h) * (total_q / (kTiles * kBlockM) + b)
                                         : static_cast<int64_t>(kp.items_x) * h * b;
@@ -755,12 +759,23 @@ int launch_fwd(FwdKernelParams& kp, int b, int h, int seqlen_q, int64_t total_q,
   kp.total_items = static_cast<int>(total);
   const int grid = kp.total_items < sms ? kp.total_items : sms;  // one CTA per SM (202 KB of shared memory each)
   if (overlap) {
-    FA_CHECK_CUDA(launch_overlapped(fwd_kernel<D>, dim3(grid), kNumThreads, C::kSmemBytes, stream, kp));
+    FA_CHECK_CUDA(launch_overlapped(fwd_kernel<D, kItemRows>, dim3(grid), kNumThreads, C::kSmemBytes, stream, kp));
   } else {
-    fwd_kernel<D><<<grid, kNumThreads, C::kSmemBytes, stream>>>(kp);
+    fwd_kernel<D, kItemRows><<<grid, kNumThreads, C::kSmemBytes, stream>>>(kp);
     FA_CHECK_CUDA(cudaGetLastError());
   }
   return FA_OK;
+}
+
+// The two tiles of an item share a tensor core, an exponential unit and their K/V blocks.  A dense batch with no more 128-row tiles
+// than the chip has SMs gets an SM for every tile instead: B2 S512 H8 D64 15.1 -> 13.6 us, B1 S1000 H16 D128 causal 24.8 -> 21.8, B1 S2304
+// H8 D128 43.8 -> 38.1; with more tiles than SMs some SMs would run two items in turn, which takes longer than a pair.
+template <int D>
+int launch_fwd(FwdKernelParams& kp, int b, int h, int seqlen_q, int64_t total_q, bool overlap, cudaStream_t stream) {
+  const int64_t tiles = static_cast<int64_t>((seqlen_q + kBlockM - 1) / kBlockM) * h * b;
+  if (kp.cu_seqlens_q == nullptr && tiles <= device_sm_count())
+    return launch_items<D, kBlockM>(kp, b, h, seqlen_q, total_q, overlap, stream);
+  return launch_items<D, kTiles * kBlockM>(kp, b, h, seqlen_q, total_q, overlap, stream);
 }
 
 }  // namespace

@@ -780,3 +780,26 @@ def test_rows_outside_every_packed_sequence_are_zero(ext, request, path, d, befo
     for x in (out, *grads):
         assert x[:before].abs().sum() == 0 and x[before + used:].abs().sum() == 0
     assert ext.device_status(True) == 0
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("b,sq,sk,h,hk,causal", [
+    (1, 1, 1, 1, 1, False),
+    (1, 129, 300, 4, 2, True),       # a second tile of one row
+    (1, 128 * 37, 700, 4, 4, True),  # 148 tiles: one item per SM, rows past sk without a visible key on the way
+    (1, 128 * 37 + 1, 257, 4, 4, False),  # 152 tiles: pairs again
+    (2, 500, 90, 3, 1, True),        # rows that see no key
+])
+def test_forward_items_of_one_tile(ext, d, b, sq, sk, h, hk, causal):
+    """A small dense batch gets a work item per 128-row tile.  A row does not depend on how rows are grouped, so the result
+    equals, bit for bit, that of the same batch among copies of itself (more tiles than SMs: items of two tiles)."""
+    q, k, v, _ = (x.to(DEV) for x in _inputs(11, b, sq, sk, h, hk, d))
+    out, lse = torch.full_like(q, float("nan")), torch.full((b, h, sq), float("nan"), device=DEV)
+    ext.fwd(q, k, v, d ** -0.5, causal, out=out, lse=lse)
+    n = 149
+    many = [x[:1].repeat(n, 1, 1, 1) for x in (q, k, v)]
+    want, want_lse = ext.fwd(*many, d ** -0.5, causal)
+    assert torch.equal(out[0], want[0]) and torch.equal(lse[0], want_lse[0])
+    o_ref, lse_ref = orc.attention_forward(*(x.cpu() for x in (q, k, v)), None, causal)
+    assert err_stats(out, o_ref)[0] <= 2e-3 and err_stats(lse, lse_ref)[0] <= LSE_TOL
+    assert ext.device_status(True) == 0
