@@ -803,3 +803,59 @@ def test_forward_items_of_one_tile(ext, d, b, sq, sk, h, hk, causal):
     o_ref, lse_ref = orc.attention_forward(*(x.cpu() for x in (q, k, v)), None, causal)
     assert err_stats(out, o_ref)[0] <= 2e-3 and err_stats(lse, lse_ref)[0] <= LSE_TOL
     assert ext.device_status(True) == 0
+
+
+def _shortest_us(fn, runs=9, calls=4):
+    best = float("inf")
+    for _ in range(runs + 1):  # the first is a warm-up
+        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        start.record()
+        for _ in range(calls):
+            fn()
+        end.record()
+        end.synchronize()
+        best = min(best, start.elapsed_time(end) * 1e3 / calls)
+    return best
+
+
+@pytest.mark.parametrize("h,d,lens", [(16, 64, (64,) * 64), (1, 64, (64,) * 64), (8, 128, (100,))])
+def test_rows_without_a_sequence_cost_no_more_than_a_full_clear(ext, h, d, lens):
+    """A buffer of fixed capacity, mostly unused (normal under CUDA graphs).  Bound: what the used rows take in a buffer of their
+    own, and clearing whole tensors, with half as much again and 20 us for the spread of the timings."""
+    torch.manual_seed(0)
+    used, rows, scale = sum(lens), 32768, d ** -0.5
+    cu = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0, dtype=torch.int32).to(DEV)
+    args = (cu, cu, max(lens), max(lens), scale, True)
+
+    def times(rows):
+        q, k, v, dout = (torch.randn(rows, h, d, device=DEV, dtype=torch.float16) for _ in range(4))
+        grads = [torch.empty_like(x) for x in (q, k, v)]
+        out, lse = ext.varlen_fwd(q, k, v, *args)
+        return (_shortest_us(lambda: ext.varlen_fwd(q, k, v, *args)),
+                _shortest_us(lambda: ext.varlen_bwd(q, k, v, out, lse, dout, *args, *grads)),
+                _shortest_us(lambda: [g.zero_() for g in grads]))
+
+    fwd, bwd, _ = times(used)
+    fwd_spare, bwd_spare, clear = times(rows)
+    assert fwd_spare <= 1.5 * (fwd + clear / 3) + 20, (fwd_spare, fwd, clear)
+    assert bwd_spare <= 1.5 * (bwd + clear) + 20, (bwd_spare, bwd, clear)
+
+
+@pytest.mark.parametrize("h,hk,d", [(1, 1, 64), (3, 1, 64), (5, 5, 128), (16, 4, 128)])
+@pytest.mark.parametrize("before,after", [(0, 9001), (4097, 3), (2500, 2500)])
+def test_thousands_of_unused_rows_in_strided_gradients_are_zero(ext, h, hk, d, before, after):
+    """More unused rows than threads that clear, in gradients that are slices of a wider tensor; the rest of that tensor stays."""
+    gen = torch.Generator().manual_seed(9)
+    lens, scale = (70, 129), d ** -0.5
+    total = before + sum(lens) + after
+    q, k, v, dout = (randn_half(gen, total, n, d).to(DEV) for n in (h, hk, hk, h))
+    cu = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0, dtype=torch.int32).to(DEV) + before
+    args = (cu, cu, max(lens), max(lens), scale, True)
+    out, lse = ext.varlen_fwd(q, k, v, *args)
+    wide = torch.full((total, h + 2 * hk + 1, d), float("nan"), device=DEV, dtype=torch.float16)
+    grads = [wide[:, :h], wide[:, h:h + hk], wide[:, h + hk:h + 2 * hk]]
+    ext.varlen_bwd(q, k, v, out, lse, dout, *args, *grads)
+    for x in (out, *grads):
+        assert x[:before].abs().sum() == 0 and x[before + sum(lens):].abs().sum() == 0
+        assert torch.isfinite(x).all() and x.abs().sum() > 0
+    assert torch.isnan(wide[:, h + 2 * hk]).all()
