@@ -58,8 +58,11 @@ struct PreParams {
 // the threads of a block read neighbouring heads of the same rows, i.e. contiguous memory when the heads of a
 // row are adjacent, every thread has 2 * kPreRows loads in flight, and an item writes one full 32-byte sector
 // of each statistic.  grid (ceil(items / items_per_block), 1, b).
+// Bound by memory, with three blocks per SM (80 registers; the clearing code of packed calls takes 86 and is left out of the other
+// instantiation: two blocks, 98.8 instead of 82.2 us at B4 S8192 H32 D128, 5560 against 6680 GB/s).
 constexpr int kPreRows = 8;
 static_assert(kClearThreads == 256, "the clearing threads are those of the preprocess kernel");
+template <bool kClear>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_constant__ PreParams p) {
   grid_launch_dependents();
   const int tpr = p.d / 8;  // threads per item: 8 or 16
@@ -110,7 +113,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
     p.delta[idx] = valid ? -mine : 0.f;
     p.lse2[idx] = valid ? -my_lse * kLog2e : -INFINITY;
   }
-  if (p.clear[0].base != nullptr) {  // the other kernels write all other rows of dq, dk, dv
+  if constexpr (kClear) {  // the other kernels write all other rows of dq, dk, dv
     // The blocks of all sequences share the unused rows: those of one sequence are too few when the buffer is much larger than
     // what it holds.  Backward of 64 texts of 64 tokens, H16 D64, in 32768 rows: 1270 us with one sequence's blocks and a
     // division per store, 115 now; 79 in 4096 rows, and clearing the three whole tensors takes 62.
@@ -1461,7 +1464,8 @@ extern "C" int fa_bwd_stages(const FaBwdParams* p, int stage_mask, fa_stream_t s
   }
   dim3 grid_pre(static_cast<unsigned>(pre_blocks), 1, p->b);
   if (stage_mask & 1) {
-    bwd_preprocess_kernel<<<grid_pre, 256, 0, stream>>>(pp);
+    const auto preprocess = clears ? bwd_preprocess_kernel<true> : bwd_preprocess_kernel<false>;
+    preprocess<<<grid_pre, 256, 0, stream>>>(pp);
     FA_CHECK_CUDA(cudaGetLastError());
   }
   const bool fused = (p->flags & FA_BWD_SINGLE_KERNEL) != 0;

@@ -859,3 +859,16 @@ def test_thousands_of_unused_rows_in_strided_gradients_are_zero(ext, h, hk, d, b
         assert x[:before].abs().sum() == 0 and x[before + sum(lens):].abs().sum() == 0
         assert torch.isfinite(x).all() and x.abs().sum() > 0
     assert torch.isnan(wide[:, h + 2 * hk]).all()
+
+
+def test_row_statistics_are_read_at_the_rate_of_a_copy(ext):
+    """The first stage of a dense backward reads O and dO once.  Bound: a copy that moves as many bytes on the same GPU, and 10 %
+    (with two blocks per SM in place of three it took 18 % more)."""
+    from flash_attention_turing_b200 import capi
+
+    p, _, ws, keep = _bwd_params_for(ext, 4, 8192, 32, 32, 128, True, ())
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    stage = _shortest_us(lambda: capi.check(capi.lib().fa_bwd_stages(ctypes.byref(p), 1, stream)))
+    out, dst = keep[3], torch.empty_like(keep[3])
+    copy = _shortest_us(lambda: dst.copy_(out))  # reads one tensor and writes one, where the stage reads two
+    assert stage <= 1.1 * copy, (stage, copy)
