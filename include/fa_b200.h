@@ -144,6 +144,8 @@ int fa_fwd(const FaFwdParams* p, fa_stream_t stream);
 /* Scratch: `workspace` (256-byte aligned) must hold fa_bwd_workspace_bytes() bytes: fp32         */
 /* rowsum(dO*O) and the LSE in base-2 units, and for FA_BWD_SINGLE_KERNEL the fp32 dQ accumulator */
 /* (heads x padded rows x d).  The size depends on `flags`.                                      */
+/* dk and dv may lie over k and v (either over either, with the same strides): the dK/dV kernel then starts when  */
+/* the dQ kernel has ended, not beside it.  No other output may overlap an input that a kernel still reads. */
 /* ------------------------------------------------------------------------------------------- */
 #define FA_BWD_SINGLE_KERNEL 1
 #define FA_BWD_ZERO_UNUSED_ROWS 2 /* packed calls, default path: see FA_FWD_ZERO_UNUSED_ROWS */

@@ -872,3 +872,27 @@ def test_row_statistics_are_read_at_the_rate_of_a_copy(ext):
     out, dst = keep[3], torch.empty_like(keep[3])
     copy = _shortest_us(lambda: dst.copy_(out))  # reads one tensor and writes one, where the stage reads two
     assert stage <= 1.1 * copy, (stage, copy)
+
+
+@pytest.mark.parametrize("b,s,h,hk,d,causal,lens", [
+    (2, 197, 12, 12, 64, False, ()),    # fewer items than SMs: the dK/dV kernel could start at once
+    (1, 4096, 8, 2, 128, True, ()),
+    (3, 300, 4, 2, 128, True, (300, 1, 129)),
+])
+@pytest.mark.parametrize("swapped", [False, True])
+def test_gradients_may_be_written_over_keys_and_values(ext, b, s, h, hk, d, causal, lens, swapped):
+    """dK and dV in the memory of K and V (or of V and K): bit for bit the gradients in memory of their own."""
+    from flash_attention_turing_b200 import capi
+
+    lib = capi.lib()
+    p, grads, ws, keep = _bwd_params_for(ext, b, s, h, hk, d, causal, lens)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    capi.check(lib.fa_bwd(ctypes.byref(p), stream))
+    k, v = keep[1], keep[2]
+    k0, v0 = k.clone(), v.clone()
+    dk, dv = (v, k) if swapped else (k, v)
+    p.dk, p.dv = dk.data_ptr(), dv.data_ptr()
+    for _ in range(10):
+        k.copy_(k0), v.copy_(v0)
+        capi.check(lib.fa_bwd(ctypes.byref(p), stream))
+        assert torch.equal(dk, grads[1]) and torch.equal(dv, grads[2])
