@@ -732,9 +732,9 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
 }
 
 // FA_FWD_ZERO_UNUSED_ROWS.  Runs beside the forward kernel, which writes all other rows.
-__global__ void __launch_bounds__(kClearThreads) clear_unused_rows_kernel(const __grid_constant__ PackedRows t) {
+__global__ void __launch_bounds__(kClearThreads) clear_unused_rows_kernel(const __grid_constant__ PackedRows t, const int* status) {
   grid_launch_dependents();
-  clear_unused_rows(t, blockIdx.x * kClearThreads + threadIdx.x, gridDim.x * kClearThreads);
+  clear_unused_rows(t, wait_timed_out(status), blockIdx.x * kClearThreads + threadIdx.x, gridDim.x * kClearThreads);
 }
 
 template <int D, int kItemRows>
@@ -867,7 +867,7 @@ int run_fwd(const FaFwdParams* p, int seqused_k_add, cudaStream_t stream, bool o
     const PackedRows rows{kp.o, kp.o_row_stride, kp.o_head_stride, p->total_q, p->h, p->d, p->cu_seqlens_q, p->b};
     const int sms = device_sm_count();
     if (sms <= 0) return set_error(FA_ERR_CUDA, "fa_fwd: device attributes not available");
-    clear_unused_rows_kernel<<<sms, kClearThreads, 0, stream>>>(rows);
+    clear_unused_rows_kernel<<<sms, kClearThreads, 0, stream>>>(rows, kp.status);
     FA_CHECK_CUDA(cudaGetLastError());
     overlap = true;
   }

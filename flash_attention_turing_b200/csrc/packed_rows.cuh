@@ -44,9 +44,12 @@ __device__ __forceinline__ void clear_rows(const PackedRows& t, int64_t first, i
   }
 }
 
-__device__ __forceinline__ void clear_unused_rows(const PackedRows& t, uint32_t worker, uint32_t workers) {
-  const int64_t begin = min(t.total, static_cast<int64_t>(max(t.cu_seqlens[0], 0)));
-  const int64_t end = max(begin, min(t.total, static_cast<int64_t>(t.cu_seqlens[t.b])));
+// all: clear every row.  Once a wait has timed out the kernels that write the other rows return at once, and a caller that has
+// not looked at the status word would find what the memory held before.
+__device__ __forceinline__ void clear_unused_rows(const PackedRows& t, bool all, uint32_t worker, uint32_t workers) {
+  const int first_used = t.cu_seqlens[0], end_used = t.cu_seqlens[t.b];
+  const int64_t begin = min(t.total, all ? t.total : static_cast<int64_t>(max(first_used, 0)));
+  const int64_t end = max(begin, min(t.total, static_cast<int64_t>(end_used)));
   clear_rows(t, 0, begin, worker, workers);
   clear_rows(t, end, t.total, worker, workers);
 }

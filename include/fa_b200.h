@@ -63,7 +63,8 @@ int fa_abi_version(void);
  * no room for an alignment pad) and did no work, so dK and dV of that launch are invalid; negative =
  * FA_ERR_*.  With
  * reset != 0 the word is cleared afterwards.  Bit 0 is STICKY: while it is set, every later forward, backward
- * or decode launch on that device returns without doing any work (its outputs stay as they were) although the
+ * or decode launch on that device returns without doing any work (its outputs stay as they were; those of a packed
+ * call that asks for zeros outside its sequences become zero) although the
  * host call reports FA_OK, until this function clears the word -- a host that wants to detect the condition
  * polls it.  When a wait gave up, bits 8-31 of the word identify the first one that did: bits 8-15 the warp
  * role that waited, bits 16-23 the index of the barrier in the kernel's barrier block, bit 24 the phase

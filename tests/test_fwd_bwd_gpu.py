@@ -896,3 +896,33 @@ def test_gradients_may_be_written_over_keys_and_values(ext, b, s, h, hk, d, caus
         k.copy_(k0), v.copy_(v0)
         capi.check(lib.fa_bwd(ctypes.byref(p), stream))
         assert torch.equal(dk, grads[1]) and torch.equal(dv, grads[2])
+
+
+def test_packed_outputs_after_a_time_out_are_zero(ext):
+    """While the time-out bit of the status word is set the kernels return at once.  The outputs of a packed call are zero then,
+    not what the memory held before."""
+    from flash_attention_turing_b200 import capi
+
+    gen = torch.Generator().manual_seed(8)
+    lens, h, hk, d = (300, 1, 129), 4, 2, 64
+    total, scale = sum(lens) + 40, d ** -0.5
+    q, k, v, dout = (randn_half(gen, total, n, d).to(DEV) for n in (h, hk, hk, h))
+    cu = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0, dtype=torch.int32).to(DEV) + 9
+    args = (cu, cu, max(lens), max(lens), scale, True)
+    want, want_lse = ext.varlen_fwd(q, k, v, *args)
+    grads = [torch.full_like(x, float("nan")) for x in (q, k, v)]
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    capi.check(capi.lib().fa_selftest_wait_timeout(1000, stream))
+    torch.cuda.synchronize()
+    try:
+        junk = torch.full_like(q, float("nan"))
+        torch.cuda.synchronize()
+        del junk  # the allocator hands this memory out for O
+        out, _ = ext.varlen_fwd(q, k, v, *args)
+        ext.varlen_bwd(q, k, v, want, want_lse, dout, *args, *grads)
+        torch.cuda.synchronize()
+    finally:
+        assert ext.device_status(True) & 1
+    for x in (out, *grads):
+        assert (x == 0).all()
+    assert torch.equal(ext.varlen_fwd(q, k, v, *args)[0], want)
