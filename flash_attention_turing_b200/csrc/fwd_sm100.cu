@@ -863,7 +863,7 @@ int run_fwd(const FaFwdParams* p, int seqused_k_add, cudaStream_t stream, bool o
   kp.block_table_batch_stride = p->block_table_batch_stride;
   kp.page_size = p->page_size;
   kp.status = device_status_ptr();
-  if ((p->flags & FA_FWD_ZERO_UNUSED_ROWS) && varlen_q) {
+  if (p->flags == FA_FWD_ZERO_UNUSED_ROWS && varlen_q) {  // no other value: see the header
     const PackedRows rows{kp.o, kp.o_row_stride, kp.o_head_stride, p->total_q, p->h, p->d, p->cu_seqlens_q, p->b};
     const int sms = device_sm_count();
     if (sms <= 0) return set_error(FA_ERR_CUDA, "fa_fwd: device attributes not available");

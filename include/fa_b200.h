@@ -121,7 +121,8 @@ typedef struct FaFwdParams {
   int32_t page_size;           /* tokens per page (multiple of 128) when block_table != NULL    */
   int32_t block_table_cols;    /* columns of block_table (0 = unknown: seqused_k is trusted)    */
   int32_t causal_shift;        /* used when is_causal == FA_CAUSAL_SHIFT                        */
-  int32_t flags;               /* FA_FWD_* bits, 0 by default                                   */
+  int32_t flags;               /* 0 or FA_FWD_ZERO_UNUSED_ROWS; any other value counts as 0 (the field was reserved0 in earlier */
+                               /* headers of this ABI version, and hosts built with those may leave it unset)                */
 } FaFwdParams;
 
 int fa_fwd(const FaFwdParams* p, fa_stream_t stream);

@@ -926,3 +926,26 @@ def test_packed_outputs_after_a_time_out_are_zero(ext):
     for x in (out, *grads):
         assert (x == 0).all()
     assert torch.equal(ext.varlen_fwd(q, k, v, *args)[0], want)
+
+
+@pytest.mark.parametrize("flags", [0, 2, 3, -1, 0x7fffffff])
+def test_forward_flags_of_no_meaning_leave_unused_rows_alone(ext, flags):
+    """The field was a reserved one before: whatever a host of that time left in it clears nothing."""
+    from flash_attention_turing_b200 import capi
+
+    gen = torch.Generator().manual_seed(3)
+    lens, h, d, spare = (70, 129), 2, 64, 11
+    q, k, v = (randn_half(gen, sum(lens) + spare, h, d).to(DEV) for _ in range(3))
+    cu = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0, dtype=torch.int32).to(DEV)
+    out = torch.full_like(q, 7.0)
+    lse = torch.zeros(len(lens), h, max(lens), device=DEV)
+    p = capi.fwd_params(*(x[None] for x in (q, k, v, out)), lse, d ** -0.5, False)
+    p.b, p.seqlen_q, p.seqlen_k, p.lse_row_stride = len(lens), max(lens), max(lens), max(lens)
+    p.cu_seqlens_q = p.cu_seqlens_k = cu.data_ptr()
+    p.total_q = p.total_k = q.shape[0]
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for value in (flags, capi.FA_FWD_ZERO_UNUSED_ROWS):
+        p.flags = value
+        capi.check(capi.lib().fa_fwd(ctypes.byref(p), stream))
+        assert (out[sum(lens):] == (0 if value == capi.FA_FWD_ZERO_UNUSED_ROWS else 7)).all()
+        assert torch.equal(out[:sum(lens)], ext.varlen_fwd(q, k, v, cu, cu, max(lens), max(lens), d ** -0.5, False)[0][:sum(lens)])
