@@ -226,6 +226,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
     mbar_init(&xb->sched_go, 1);
     fence_mbar_init();
     grid_dependency_wait();  // the row statistics; everything behind the synchronisation below may read them
+    fence_acq_rel_gpu();     // ... and so may the dK/dV kernel, which starts behind the next line without a wait of its own
     grid_launch_dependents();
   }
   if (warp == kMmaWarp) {

@@ -56,7 +56,8 @@ int device_sm_count();
 // Launches a kernel that may start before the previous kernel of the stream has finished, as soon as that one lets it
 // (grid_launch_dependents() in ptx.cuh): its set-up and launch latency then run under the predecessor.  The kernel has to
 // call grid_dependency_wait() before it touches anything the predecessor writes, and in at least one CTA in any case, so
-// that its own completion implies that of everything before it.
+// that its own completion implies that of everything before it.  A kernel that reads, without such a wait, what a kernel further
+// back has written (dK/dV: the row statistics) needs its predecessor to wait, fence_acq_rel_gpu() and only then let it start.
 template <class Params>
 cudaError_t launch_overlapped(void (*kernel)(Params), dim3 grid, int threads, size_t smem, cudaStream_t stream,
                               const Params& params) {

@@ -101,6 +101,7 @@ __device__ __forceinline__ uint32_t mbar_test_nonblocking(uint64_t* bar, uint32_
 // depends on have finished and their writes are visible, at once in a plain launch; the other call lets the next kernel
 // start once every CTA has made it or has exited.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Per-CTA abort state shared by all waits of a kernel.
