@@ -31,7 +31,6 @@ struct BwdKernelParams {
   const int* cu_seqlens_q;
   const int* cu_seqlens_k;
   int* status;
-  int reserved0;
   // single-kernel backward: fp32 dQ accumulator (heads, dq_acc_rows, d), rows grouped in 128-row tiles;
   // the tiles of sequence b start at row dq_acc_tile_base(b) * 128
   float* dq_acc;
@@ -109,12 +108,12 @@ struct BBarriers {
   uint64_t a_empty[4];
   uint64_t b_full[4];      // ring B (dQ: V, dK/dV: dO)
   uint64_t b_empty[4];
-  uint64_t s_full;         // S (or S^T) accumulator ready
+  uint64_t s_full;         // S^T accumulator ready (not used by the dQ kernel, whose dp_full covers both)
   uint64_t dp_full;        // dP (or dP^T) accumulator ready
   uint64_t p_full;         // packed P^T written to TMEM (dK/dV kernel)
   uint64_t ds_full;        // packed dS (or dS^T) written to TMEM
-  uint64_t s_loaded;       // S (S^T) sits in registers: its TMEM region may be overwritten
-  uint64_t dp_loaded;      // dP (dP^T) sits in registers
+  uint64_t s_loaded;       // S^T (dQ kernel: S and dP) sits in registers: its TMEM region may be overwritten
+  uint64_t dp_loaded;      // dP^T sits in registers (dQ kernel: s_loaded covers both)
   uint64_t p_free;         // dV MMAs of the previous tile have consumed the packed P^T
   uint64_t ds_free[2];     // dK/dV kernel [0]: dK MMAs of the previous tile have consumed the packed dS^T;
                            // dQ kernel [u]: the dQ MMAs have consumed packed-dS buffer u
