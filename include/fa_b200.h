@@ -87,7 +87,7 @@ int fa_selftest_wait_timeout(uint32_t limit_us, fa_stream_t stream);
 /* (src/flash_fwd_launch_template.h:49-93) and flash_fwd_kernel (src/flash_fwd_kernel.h:23-664). */
 /* Also serves the tiled path of mha_fwd_kvcache (flash_api.cpp:686-714) through seqused_k,      */
 /* cache_batch_idx and block_table, without the index_select copy the reference makes.           */
-/* The kernel is persistent: one CTA per SM takes 256-row work items from a counter in device    */
+/* The kernel is persistent: one CTA per SM takes items of 256 (small dense batches: 128) rows from a counter in device */
 /* memory (a pool of 1024 counter pairs inside the library; a launch takes the next pair and     */
 /* leaves it zero), where the reference launches one CTA per row block of a max_seqlen-sized     */
 /* grid (src/flash_fwd_launch_template.h:60-75).  Nothing for the host to manage: launches may   */
