@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 // to back, fetched into registers together and handed back together, so that the whole arithmetic of the block runs
 // under the next S / dP: ONE wait and one hand-back per block where waiting for S and dP in turn took two of each, at
 // 150-300 clocks apiece for warps in lock-step.  The hand-back has to leave before the arithmetic starts (see
-// schedule_barrier: without it 55 % slower).  Measured per 128 x 128 block at B4 S8192 H32 D128 causal: 2511 -> 2226 clocks;
+// schedule_barrier: without it 40 % slower, 267 against 188 us at B2 S4096 H16 D128 causal).  Measured per 128 x 128 block at B4 S8192 H32 D128 causal: 2511 -> 2226 clocks;
 // launch, SM clocks: D128 S8192 4520 -> 4005 k, D128 S1024 462 -> 436 k, D64 S16384 3417 -> 3189 k.
 constexpr int kDqThreads = 640;
 constexpr int kDqSchedWarp = 19;
