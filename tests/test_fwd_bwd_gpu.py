@@ -963,3 +963,32 @@ def test_compiler_keeps_the_hand_back_of_the_dq_kernel_ahead_of_its_arithmetic(e
     capi.check(lib.fa_bwd_stages(ctypes.byref(p), 1, stream))
     dq, dkdv = (_shortest_us(lambda: capi.check(lib.fa_bwd_stages(ctypes.byref(p), stage, stream))) for stage in (2, 4))
     assert dq <= 0.87 * dkdv, (dq, dkdv)
+
+
+@pytest.mark.parametrize("max_k", [128, 130, 384])
+@pytest.mark.parametrize("d,lens", [(64, (300, 520)), (128, (520, 300, 1)), (128, (700,))])
+def test_key_gradients_past_the_given_maximum_are_zero(ext, d, lens, max_k):
+    """A max_seqlen_k below a sequence's length: dK and dV are written for the whole tiles within it and zero from there on, in
+    a sequence in between as in the last one, whatever the memory held.  O and dQ do not depend on it."""
+    gen = torch.Generator().manual_seed(12)
+    h, hk, scale = 4, 2, d ** -0.5
+    q, k, v, dout = (randn_half(gen, sum(lens), n, d).to(DEV) for n in (h, hk, hk, h))
+    cu = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0, dtype=torch.int32).to(DEV)
+
+    def run(max_k):
+        args = (cu, cu, max(lens), max_k, scale, True)
+        out, lse = ext.varlen_fwd(q, k, v, *args)
+        grads = [torch.full_like(x, float("nan")) for x in (q, k, v)]
+        ext.varlen_bwd(q, k, v, out, lse, dout, *args, *grads)
+        return out, *grads
+
+    out, dq, dk, dv = run(max_k)
+    want_out, want_dq, want_dk, want_dv = run(max(lens))
+    assert torch.equal(out, want_out) and torch.equal(dq, want_dq)
+    written = -(-max_k // 128) * 128
+    for got, want in ((dk, want_dk), (dv, want_dv)):
+        first = 0
+        for n in lens:
+            assert torch.equal(got[first:first + min(n, written)], want[first:first + min(n, written)])
+            assert (got[first + min(n, written):first + n] == 0).all()
+            first += n

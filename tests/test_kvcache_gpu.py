@@ -281,3 +281,44 @@ def test_merge_at_the_edges_of_its_batches(ext, d, splits):
     # half an fp16 ulp of the result, and 1e-5 for the exponentials and the fp32 sums
     assert ((got - o_ref).abs() <= o_ref.abs() * 2 ** -11 + 1e-5).all()
     assert err_stats(lse.view(-1), want)[0] <= 1e-5
+
+
+def _more_tiles_than_sms(b, sq, h):
+    return b * h * -(-sq // 128) > torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("layout", ["contiguous", "paged", "batch_idx"])
+def test_chunks_of_more_tiles_than_sms(ext, d, causal, layout):
+    """What a serving batch uses: items of two 128-row tiles over a cache (smaller chunks, as in the tests above, get an item per
+    tile).  A ragged second tile, an odd number of tiles, an empty cache, and NaN behind the used part of a contiguous one."""
+    b, sq, h, hk = 4, 300, 16, 4
+    assert _more_tiles_than_sms(b, sq, h)
+    _run(b, sq, h, hk, d, 1280, [0, 129, 700, 955], sq, paged=layout == "paged", batch_idx=layout == "batch_idx",
+         causal=causal, poison_tail=True)
+    _run(b, sq, h, hk, d, 1280, [300, 1, 700, 1280], 0, paged=layout == "paged", batch_idx=layout == "batch_idx",
+         causal=causal, poison_tail=True)
+
+
+@pytest.mark.parametrize("b,sq,h", [(2, 100, 4), (4, 300, 16)])  # an item per tile, items of two tiles
+def test_tiled_path_clamps_lengths_to_the_capacity_and_reports_it(ext, b, sq, h):
+    from flash_attention_turing_b200 import flash_attention_interface as iface
+
+    assert _more_tiles_than_sms(b, sq, h) == (b == 4)
+    gen = torch.Generator().manual_seed(4)
+    hk, d, page, per = 2, 64, 256, 2
+    kc, vc = randn_half(gen, b * per, page, hk, d), randn_half(gen, b * per, page, hk, d)
+    table = torch.randperm(b * per, generator=gen).to(torch.int32).view(b, per)
+    q = randn_half(gen, b, sq, h, d)
+    lens_bad = torch.tensor([9999, 300, 512, 1][:b], dtype=torch.int32)
+    o_ref, _ = orc.kvcache_forward(q, kc.clone(), vc.clone(), None, None, lens_bad.clamp(max=page * per), None, table, None, True)
+    iface.HOST_CAPACITY_CHECK = False
+    try:
+        out = iface.flash_attn_with_kvcache(q.to(DEV), kc.to(DEV), vc.to(DEV), cache_seqlens=lens_bad.to(DEV),
+                                            block_table=table.to(DEV), causal=True)
+        status = ext.device_status(True)
+    finally:
+        iface.HOST_CAPACITY_CHECK = True
+    assert status == 2
+    assert err_stats(out, o_ref)[0] <= O_TOL
