@@ -344,7 +344,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       ++ni;
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_nn = make_idesc_f16(128, kBlock, false, false);
       const uint32_t q_addr = smem_u32(sQ), do_addr = smem_u32(sdO);
       auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, ctx); };
@@ -382,7 +382,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       }
     }
   } else if (warp == kAccMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_acc = make_idesc_f16(128, D, false, true);
       int G = 0, nf = 0;
       bool ok = true;
@@ -705,7 +705,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
       ++ni;
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_nn = make_idesc_f16(128, kBlock, false, false);
       const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV);
       // One accumulator region A holds S^T(T) and then dP^T(T): dP^T(T) is issued as soon as S^T(T)
@@ -760,7 +760,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
       }
     }
   } else if (warp == kAccMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       // dV += P^T dO as soon as the packed P^T is written, dK += dS^T Q likewise.
       constexpr uint32_t idesc_acc = make_idesc_f16(128, D, false, true);
       const uint32_t tP = tmem_base + kColDP, tDS = tmem_base + kColDP + 64;
@@ -1088,7 +1088,7 @@ bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
       }
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0 && n_it > 0) {
+    if (elect_one() && n_it > 0) {
       constexpr uint32_t idesc_nn = make_idesc_f16(128, kBlock, false, false);
       const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV);
       // One accumulator region A holds S^T(it) and then dP^T(it): dP^T(it) is issued as soon as S^T(it)
@@ -1125,7 +1125,7 @@ bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
       }
     }
   } else if (warp == kAccMmaWarp) {
-    if (lane == 0 && n_it > 0) {
+    if (elect_one() && n_it > 0) {
       // dV += P^T(it) dO(it) as soon as the packed P^T is written, dK += dS^T(it) Q(it) likewise.
       constexpr uint32_t idesc_acc = make_idesc_f16(128, D, false, true);
       const uint32_t tP = tmem_base + kColDP, tDS = tmem_base + kColDP + 64;

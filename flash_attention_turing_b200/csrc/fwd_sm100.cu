@@ -394,7 +394,7 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================
     const WaitCtx ctx{&bars->abort_flag, p.status, 3, bars};
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_f16(128, kBlockN, false, false);
       constexpr uint32_t idesc_pv = make_idesc_f16(128, D, false, true);
       const uint32_t sQ_addr = smem_u32(sQ);
