@@ -92,19 +92,21 @@ struct BCfg {
                                       1024 /*alignment*/;
   // dK/dV kernel: a Q tile lives from the S^T MMAs of its iteration to the dK MMAs issued one iteration
   // later, a dO tile for less than one iteration; the row statistics have a ring of their own (2 x 1 KB)
-  // that the elementwise warps release.  At D = 128 the tiles take 224 KB, which leaves no room for an
+  // that the elementwise warps release, or at D = 64 stages beside those of the Q tiles.  At D = 128 the tiles take 224 KB, which leaves no room for an
   // alignment pad: the kernel checks that the dynamic shared memory starts on a 1024-byte boundary.
   static constexpr int kStagesQ = kStages + 1;
   static constexpr int kStagesDO = kStages;
+  static constexpr bool kStatsWithQ = D == 64;
+  static constexpr int kStatsStages = kStatsWithQ ? kStagesQ : 2;
   static constexpr int kAlignPadDkdv = (D == 128) ? 0 : 1024;
-  static constexpr int kSmemBytesDkdv = 2 * kTileBytes + (kStagesQ + kStagesDO) * kTileBytes + 2048 /*stats*/ +
+  static constexpr int kSmemBytesDkdv = 2 * kTileBytes + (kStagesQ + kStagesDO) * kTileBytes + kStatsStages * 1024 +
                                         512 /*barriers*/ + kAlignPadDkdv;
   static_assert(kSmemBytesDq <= 227 * 1024 && kSmemBytesDkdv <= 227 * 1024, "shared memory budget");
 };
 
 struct BBarriers {
   uint64_t fixed_full;     // the tiles loaded once (Q,dO or K,V)
-  uint64_t a_full[4];      // ring A (dQ: K, dK/dV: Q + stats)
+  uint64_t a_full[4];      // ring A (dQ: K, dK/dV: Q, at D = 64 with its row statistics)
   uint64_t a_empty[4];
   uint64_t b_full[4];      // ring B (dQ: V, dK/dV: dO)
   uint64_t b_empty[4];
@@ -117,7 +119,7 @@ struct BBarriers {
   uint64_t p_free;         // dV MMAs of the previous tile have consumed the packed P^T
   uint64_t ds_free[2];     // dK/dV kernel [0]: dK MMAs of the previous tile have consumed the packed dS^T;
                            // dQ kernel [u]: the dQ MMAs have consumed packed-dS buffer u
-  uint64_t st_full[2];     // dK/dV kernel: row statistics (lse, delta) of a Q tile loaded
+  uint64_t st_full[2];     // dK/dV kernel at D = 128: row statistics (lse, delta) of a Q tile loaded
   uint64_t st_empty[2];    // ... and read by all elementwise warps
   uint64_t tail_fixed[4];  // rows past the end of a packed sequence have been zeroed in an operand tile
                            // (dK/dV kernel: one barrier per dO stage -- up to 3 at head size 64 -- so that

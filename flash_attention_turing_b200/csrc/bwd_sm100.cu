@@ -529,14 +529,20 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
 // kernel: one CTA per SM takes items from the work counter (heaviest causal key tile first), every barrier phase
 // is derived from the cumulative iteration count T (or the item count), the K / V tiles of the next item are
 // loaded as soon as the last dP^T product of the current item has read them, and its first S^T product is issued
-// under the last elementwise iteration and the epilogue of the current one.  Dense batches only: packed (varlen)
-// batches go to bwd_dkdv_packed_kernel below.
+// under the last elementwise iteration and the epilogue of the current one.  Bound by the chain of a tile through the sixteen
+// elementwise warps (about 3250 clocks a tile at D = 128, of 2048 at the tensor peak; 2250 at D = 64).
+//   D = 64: the row statistics of a tile arrive on the barrier of its Q tile (there is shared memory for as many stages of them),
+// which the thread that issues S^T waits for anyway: the elementwise warps, which have seen S^T, need no wait and no release of
+// their own.  2600 -> 2510 us at B2 S16384 H16 causal, 377 -> 364 at B4 S4096, 49.2 -> 47.1 at B4 Sq333 Sk2047.
+//   kVarlen: packed sequences.  A Q tile can hold rows of the neighbouring sequence; this form carries the code that guards
+// against them.  D = 64, and D = 128 without grouped heads; the rest goes to bwd_dkdv_packed_kernel (see there).
 constexpr int kDkvThreads = 640;  // + one scheduler warp: 20 warps, five on one sub-partition -> 96 registers
 constexpr int kDkvSchedWarp = 19;
 constexpr int kDkvReaders = kComputeWarps + 3;  // elementwise warps, producer warp, two MMA threads
 static_assert((kDkvThreads / 32 + 3) / 4 * 32 * 96 <= 16384, "register file of one SM sub-partition");
-struct DkvItem {
-  int batch, head_k, nblk, pad;  // nblk < 0: no more work
+struct __align__(16) DkvItem {
+  int batch, head_k, nblk, q_off;  // nblk < 0: no more work
+  int k_off, sq, sk, pad;          // the extents of the sequence: from cu_seqlens_* for packed batches
 };
 struct DkvBarriers {
   BBarriers b;
@@ -547,13 +553,15 @@ struct DkvBarriers {
 static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 
 struct DkvWork {
-  int batch, head_k, sq, sk, key0, group, nq, i_min, shift, per_head, n_it;
+  int batch, head_k, q_off, k_off, sq, sk, key0, group, nq, i_min, shift, per_head, n_it;
 };
+template <bool kVarlen>
 __device__ __forceinline__ DkvWork dkv_decode(const BwdKernelParams& p, const DkvItem& it) {
   DkvWork w;
   w.batch = it.batch, w.head_k = it.head_k;
-  w.sq = p.seqlen_q;
-  w.sk = p.seqlen_k;
+  w.q_off = kVarlen ? it.q_off : 0, w.k_off = kVarlen ? it.k_off : 0;
+  w.sq = kVarlen ? it.sq : p.seqlen_q;
+  w.sk = kVarlen ? it.sk : p.seqlen_k;
   w.key0 = it.nblk * kBlock;
   w.group = p.h / p.h_k;
   w.nq = (w.sq + kBlock - 1) / kBlock;
@@ -568,7 +576,7 @@ __device__ __forceinline__ DkvWork dkv_decode(const BwdKernelParams& p, const Dk
   return w;
 }
 
-template <int D>
+template <int D, bool kVarlen>
 __global__ void __launch_bounds__(kDkvThreads, 1)
 bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
   using C = BCfg<D>;
@@ -582,7 +590,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
   uint8_t* sQ = sV + C::kTileBytes;
   uint8_t* sdO = sQ + C::kStagesQ * C::kTileBytes;
   float* sStats = reinterpret_cast<float*>(sdO + C::kStagesDO * C::kTileBytes);  // [2][lse2 128 | delta 128]
-  DkvBarriers* xb = reinterpret_cast<DkvBarriers*>(reinterpret_cast<uint8_t*>(sStats) + 2048);
+  DkvBarriers* xb = reinterpret_cast<DkvBarriers*>(reinterpret_cast<uint8_t*>(sStats) + C::kStatsStages * 1024);
   BBarriers* bars = &xb->b;
   if (smem - smem_raw > C::kAlignPadDkdv) {  // uniform over the CTA: nothing has been set up yet
     if (threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusSmemLayout);
@@ -622,6 +630,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
   } else if (warp == kDkvSchedWarp) {
     if (lane == 0) {
       bool finished = false;
+      int seq = 0;  // packed sequences: the sequence of the last claimed index
       for (int n = 0;; ++n) {
         int next = blockIdx.x;
         if (n > 0) {
@@ -629,10 +638,29 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
           next = gridDim.x + atomicAdd(p.sched, 1);
         }
         DkvItem it;
-        it.batch = 0, it.head_k = 0, it.nblk = -1, it.pad = 0;
-        if (next < p.total_items) {  // every index is a live item: key tile 0 of a head is the heaviest
-          const int x = next % p.items_x, rest = next / p.items_x;
-          it.head_k = rest % p.h_k, it.batch = rest / p.h_k, it.nblk = x;
+        it.batch = 0, it.head_k = 0, it.nblk = -1, it.pad = 0, it.q_off = 0, it.k_off = 0;
+        it.sq = p.seqlen_q, it.sk = p.seqlen_k;
+        if constexpr (!kVarlen) {
+          if (next < p.total_items) {  // every index is a live item: key tile 0 of a head is the heaviest
+            const int x = next % p.items_x, rest = next / p.items_x;
+            it.head_k = rest % p.h_k, it.batch = rest / p.h_k, it.nblk = x;
+          }
+        } else {
+          while (next < p.total_items) {  // slots per sequence from cu_seqlens_k / 128 (see the forward kernel)
+            while (seq + 1 < p.b && p.h_k * ((p.cu_seqlens_k[seq + 1] >> 7) + seq + 1) <= next) ++seq;
+            const int k0 = p.cu_seqlens_k[seq], k1 = p.cu_seqlens_k[seq + 1];
+            const int v0 = (k0 >> 7) + seq, v1 = (k1 >> 7) + seq + 1;
+            const int rel = next - p.h_k * v0, cnt = v1 - v0;
+            const int x = rel % cnt;
+            // items_x: key tiles up to the maximum the caller gave; later ones are not computed
+            if (rel >= 0 && rel / cnt < p.h_k && x < p.items_x && x * kBlock < k1 - k0) {
+              it.batch = seq, it.head_k = rel / cnt, it.nblk = x;
+              it.q_off = p.cu_seqlens_q[seq], it.sq = p.cu_seqlens_q[seq + 1] - it.q_off;
+              it.k_off = k0, it.sk = k1 - k0;
+              break;
+            }
+            next = gridDim.x + atomicAdd(p.sched, 1);
+          }
         }
         if (!mbar_wait(&xb->sched_empty[n & 1], ((n >> 1) & 1) ^ 1, ctx)) break;
         xb->items[n & 1] = it;
@@ -659,7 +687,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
       __syncwarp();
       if (lane == 0) release_item(n);
       if (item.nblk < 0) break;
-      const DkvWork w = dkv_decode(p, item);
+      const DkvWork w = dkv_decode<kVarlen>(p, item);
       if (w.n_it == 0) continue;
       // Q tile, row statistics and dO tile of iteration `it` of the item into the rings at position T0 + it
       auto load_q_do = [&](int it) -> bool {
@@ -668,22 +696,28 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
         const uint32_t phq = (T / C::kStagesQ) & 1, phd = (T / C::kStagesDO) & 1, phs = (T >> 1) & 1;
         const int head = w.head_k * w.group + it / w.per_head;
         const int i = w.i_min + it % w.per_head;
-        const int qrow = i * kBlock;
+        const int qrow = w.q_off + i * kBlock;
         const int64_t stat = (static_cast<int64_t>(w.batch) * p.h + head) * p.sq_pad + i * kBlock;
         if (!mbar_wait(&bars->a_empty[sq_], phq ^ 1, ctx)) return false;
-        mbar_arrive_expect_tx(&bars->a_full[sq_], C::kTileBytes);
+        mbar_arrive_expect_tx(&bars->a_full[sq_], C::kTileBytes + (C::kStatsWithQ ? 1024 : 0));
+        if constexpr (C::kStatsWithQ) {
+          bulk_load_1d(sStats + sq_ * 256, p.lse2 + stat, 512, &bars->a_full[sq_]);
+          bulk_load_1d(sStats + sq_ * 256 + 128, p.delta + stat, 512, &bars->a_full[sq_]);
+        }
 #pragma unroll
         for (int c = 0; c < C::kChunks; ++c)
-          tma_load_4d(sQ + sq_ * C::kTileBytes + c * C::kChunkBytes, &p.tm_q, &bars->a_full[sq_], c * 64, head, qrow, w.batch);
-        if (!mbar_wait(&bars->st_empty[ss], phs ^ 1, ctx)) return false;
-        mbar_arrive_expect_tx(&bars->st_full[ss], 1024);
-        bulk_load_1d(sStats + ss * 256, p.lse2 + stat, 512, &bars->st_full[ss]);
-        bulk_load_1d(sStats + ss * 256 + 128, p.delta + stat, 512, &bars->st_full[ss]);
+          tma_load_4d(sQ + sq_ * C::kTileBytes + c * C::kChunkBytes, &p.tm_q, &bars->a_full[sq_], c * 64, head, qrow, kVarlen ? 0 : w.batch);
+        if constexpr (!C::kStatsWithQ) {
+          if (!mbar_wait(&bars->st_empty[ss], phs ^ 1, ctx)) return false;
+          mbar_arrive_expect_tx(&bars->st_full[ss], 1024);
+          bulk_load_1d(sStats + ss * 256, p.lse2 + stat, 512, &bars->st_full[ss]);
+          bulk_load_1d(sStats + ss * 256 + 128, p.delta + stat, 512, &bars->st_full[ss]);
+        }
         if (!mbar_wait(&bars->b_empty[sd], phd ^ 1, ctx)) return false;
         mbar_arrive_expect_tx(&bars->b_full[sd], C::kTileBytes);
 #pragma unroll
         for (int c = 0; c < C::kChunks; ++c)
-          tma_load_4d(sdO + sd * C::kTileBytes + c * C::kChunkBytes, &p.tm_do, &bars->b_full[sd], c * 64, head, qrow, w.batch);
+          tma_load_4d(sdO + sd * C::kTileBytes + c * C::kChunkBytes, &p.tm_do, &bars->b_full[sd], c * 64, head, qrow, kVarlen ? 0 : w.batch);
         return true;
       };
       if (lane == 0) {
@@ -692,13 +726,31 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
           mbar_arrive_expect_tx(&bars->fixed_full, 2 * C::kTileBytes);
 #pragma unroll
           for (int c = 0; c < C::kChunks; ++c) {
-            tma_load_4d(sK + c * C::kChunkBytes, &p.tm_k, &bars->fixed_full, c * 64, w.head_k, w.key0, w.batch);
-            tma_load_4d(sV + c * C::kChunkBytes, &p.tm_v, &bars->fixed_full, c * 64, w.head_k, w.key0, w.batch);
+            tma_load_4d(sK + c * C::kChunkBytes, &p.tm_k, &bars->fixed_full, c * 64, w.head_k, w.k_off + w.key0, kVarlen ? 0 : w.batch);
+            tma_load_4d(sV + c * C::kChunkBytes, &p.tm_v, &bars->fixed_full, c * 64, w.head_k, w.k_off + w.key0, kVarlen ? 0 : w.batch);
           }
         }
       }
-      if (lane == 0) {
-        for (int it = 0; ok && it < w.n_it; ++it) ok = load_q_do(it);
+      if (!kVarlen || (w.sq % kBlock) == 0) {
+        if (lane == 0) {
+          for (int it = 0; ok && it < w.n_it; ++it) ok = load_q_do(it);
+        }
+      } else {
+        // the whole warp walks the tiles: lane 0 issues the loads, all lanes zero the rows of the next sequence
+        ok = __all_sync(0xffffffffu, ok);
+        for (int it = 0; ok && it < w.n_it; ++it) {
+          if (lane == 0) ok = load_q_do(it);
+          if (!(ok = __all_sync(0xffffffffu, ok))) break;
+          if (it % w.per_head == w.per_head - 1) {  // the last Q tile of this head
+            const int T = T0 + it, sq_ = T % C::kStagesQ, sd = T % C::kStagesDO;
+            if (!(ok = mbar_wait_warp(&bars->a_full[sq_], (T / C::kStagesQ) & 1, ctx))) break;
+            if (!(ok = mbar_wait_warp(&bars->b_full[sd], (T / C::kStagesDO) & 1, ctx))) break;
+            const int q_tail_rows = w.sq - (w.nq - 1) * kBlock;
+            zero_tile_rows_from<D>(sQ + sq_ * C::kTileBytes, q_tail_rows, lane);
+            zero_tile_rows_from<D>(sdO + sd * C::kTileBytes, q_tail_rows, lane);
+            if (lane == 0) mbar_arrive(&bars->tail_fixed[sd]);
+          }
+        }
       }
       if (!__all_sync(0xffffffffu, ok)) break;
       T0 += w.n_it;
@@ -725,7 +777,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
         if (!(ok = read_item(n, item))) break;
         release_item(n);
         if (item.nblk < 0) break;
-        const DkvWork w = dkv_decode(p, item);
+        const DkvWork w = dkv_decode<kVarlen>(p, item);
         // the next item is claimed kGoAhead iterations before this one ends; a shorter item: right away
         constexpr int kGoAhead = 2;
         if (w.n_it <= kGoAhead) mbar_arrive(&xb->sched_go);
@@ -767,18 +819,23 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
       const uint32_t tDV = tmem_base + kColAcc, tDK = tmem_base + kColAcc + D;
       bool ok = true;
       int T0 = 0;
+      uint32_t tail_phase = 0;  // bit sd: parity of the next tail_fixed[sd] phase to wait for
       for (int n = 0; ok; ++n) {
         DkvItem item;
         if (!(ok = read_item(n, item))) break;
         release_item(n);
         if (item.nblk < 0) break;
-        const DkvWork w = dkv_decode(p, item);
+        const DkvWork w = dkv_decode<kVarlen>(p, item);
         if (w.n_it == 0) continue;
         for (int it = 0; ok && it < w.n_it; ++it) {
           const int T = T0 + it;
           const int sq_ = T % C::kStagesQ, sd = T % C::kStagesDO;
           if (!(ok = mbar_wait(&bars->b_full[sd], (T / C::kStagesDO) & 1, ctx))) break;
           if (!(ok = mbar_wait(&bars->p_full, T & 1, ctx))) break;
+          if (kVarlen && (w.sq % kBlock) != 0 && it % w.per_head == w.per_head - 1) {
+            if (!(ok = mbar_wait(&bars->tail_fixed[sd], (tail_phase >> sd) & 1, ctx))) break;
+            tail_phase ^= 1u << sd;
+          }
           tc_fence_after_sync();
           gemm_ts<D>(tDV, tP, smem_u32(sdO + sd * C::kTileBytes), idesc_acc, it == 0);
           tc_commit(&bars->b_empty[sd]);
@@ -807,14 +864,16 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
     int T0 = 0, ni = 0;
     bool ok = true;
     for (int n = 0; ok; ++n) {
-      int n_it, per_head, cmin0;
+      int n_it, per_head, cmin0, cmax_last;
       {
         DkvItem item;
         ok = read_item(n, item);
         if (!(ok = __all_sync(0xffffffffu, ok))) break;
         if (item.nblk < 0) break;
-        const DkvWork w = dkv_decode(p, item);
+        const DkvWork w = dkv_decode<kVarlen>(p, item);
         n_it = w.n_it, per_head = w.per_head;
+        // valid columns in the last Q tile
+        cmax_last = kVarlen ? max(0, min(32, w.sq - (w.nq - 1) * kBlock - cq * 32)) : 32;
         // causal: query column q of tile i is masked for this key when key > q + shift, i.e. the columns of
         // this thread's quarter below  key - shift - (i * 128 + cq * 32)  are masked
         cmin0 = p.is_causal ? (w.key0 + row_in_tile) - w.shift - (w.i_min * kBlock + cq * 32) : 0;
@@ -822,8 +881,10 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
       int i_rel = 0;  // Q tile within the current head
       for (int it = 0; it < n_it; ++it) {
         const int T = T0 + it;
-        const int ss = T & 1;
-        if (!(ok = mbar_wait_warp(&bars->st_full[ss], (T >> 1) & 1, ctx))) break;
+        const int ss = C::kStatsWithQ ? T % C::kStagesQ : T & 1;
+        if constexpr (!C::kStatsWithQ) {
+          if (!(ok = mbar_wait_warp(&bars->st_full[ss], (T >> 1) & 1, ctx))) break;
+        }
         // D = 128: the LSE of this thread's 32 query columns is fetched while the warp waits for S^T anyway.
         // Read after the wait, these shared-memory loads compete with the operand fetches of the dP^T MMAs, which
         // take the whole shared-memory bandwidth (measured: 4.5-7 % of the kernel; at D = 64 the MMAs are half as
@@ -842,9 +903,10 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
         tmem_ld32(tA, sr);
         tmem_wait_ld();
         warp_arrive_loaded(&bars->s_loaded, lane);  // region A may now receive dP^T
+        if constexpr (kVarlen && D == 128) schedule_barrier(lane);
         // columns below cmin are masked by causality (clamped to [0, 32])
-        const int cmin = max(0, min(32, cmin0 - i_rel * kBlock));
-        const bool col_masked = cmin != 0;
+        const int cmask = max(0, min(32, cmin0 - i_rel * kBlock)) | (((kVarlen && i_rel == per_head - 1) ? cmax_last : 32) << 8);
+        const bool col_masked = cmask != (32 << 8);
         if (++i_rel == per_head) i_rel = 0;
         float2 pr[16];
         uint32_t pk[16];
@@ -857,10 +919,11 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
                                           c2, make_float2(l.z, l.w)));
         }
         if (col_masked) {
+          const int cmin = cmask & 0xff, cmax = kVarlen ? cmask >> 8 : 32;
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            if (2 * e < cmin) pr[e].x = 0.f;
-            if (2 * e + 1 < cmin) pr[e].y = 0.f;
+            if (2 * e < cmin || 2 * e >= cmax) pr[e].x = 0.f;
+            if (2 * e + 1 < cmin || 2 * e + 1 >= cmax) pr[e].y = 0.f;
           }
         }
 #pragma unroll
@@ -885,16 +948,18 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
           pk[2 * e] = pack_half2(d0.x, d0.y);
           pk[2 * e + 1] = pack_half2(d1.x, d1.y);
         }
-        if (col_masked) {  // by selection, like P^T
+        if (col_masked) {  // by selection: dP of a masked column may be NaN/Inf (dO rows of the next sequence)
+          const int cmin = cmask & 0xff, cmax = kVarlen ? cmask >> 8 : 32;
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            if (2 * e < cmin) pk[e] &= 0xffff0000u;
-            if (2 * e + 1 < cmin) pk[e] &= 0x0000ffffu;
+            if (2 * e < cmin || 2 * e >= cmax) pk[e] &= 0xffff0000u;
+            if (2 * e + 1 < cmin || 2 * e + 1 >= cmax) pk[e] &= 0x0000ffffu;
           }
         }
-        // the statistics of this tile are in use no longer
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->st_empty[ss]);
+        if constexpr (!C::kStatsWithQ) {  // the statistics of this tile are in use no longer
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->st_empty[ss]);
+        }
         if (T > 0 && !(ok = mbar_wait_warp(&bars->ds_free[0], (T - 1) & 1, ctx))) break;
         tmem_st16(tP + 64, pk);  // packed dS^T
         warp_arrive(&bars->ds_full, lane);
@@ -905,9 +970,10 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
       DkvItem item;
       {
         const volatile int* src = reinterpret_cast<const volatile int*>(&xb->items[n & 1]);
-        item.batch = src[0], item.head_k = src[1], item.nblk = src[2], item.pad = 0;
+        item.batch = src[0], item.head_k = src[1], item.nblk = src[2], item.q_off = src[3];
+        item.k_off = src[4], item.sq = src[5], item.sk = src[6], item.pad = 0;
       }
-      const DkvWork w = dkv_decode(p, item);
+      const DkvWork w = dkv_decode<kVarlen>(p, item);
       const int key = w.key0 + row_in_tile;
       const int which = cq >> 1;        // 0 = dV, 1 = dK
       const int col_half = cq & 1;      // which D/2 columns
@@ -915,7 +981,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
       const int64_t bs = (which == 0) ? p.dv_batch_stride : p.dk_batch_stride;
       const int64_t rs = (which == 0) ? p.dv_row_stride : p.dk_row_stride;
       const int64_t hs = (which == 0) ? p.dv_head_stride : p.dk_head_stride;
-      __half* dst = dst_base + w.batch * bs + static_cast<int64_t>(key) * rs + w.head_k * hs + col_half * (D / 2);
+      __half* dst = dst_base + (kVarlen ? 0 : w.batch * bs) + static_cast<int64_t>(w.k_off + key) * rs + w.head_k * hs + col_half * (D / 2);
       const float mul = (which == 0) ? 1.f : p.scale;
       if (n_it > 0) {
         if (!(ok = mbar_wait_warp(&bars->acc_full, ni & 1, ctx))) break;
@@ -960,9 +1026,11 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
 // 4. dK/dV kernel for packed sequences, one CTA per (sequence, KV head, key tile)
 // =============================================================================================
 // The same products and hand-offs as bwd_dkdv_kernel, but launched as a grid of max_seqlen_k / 128 x h_k x b CTAs
-// that each set up, process one key tile and exit.  Kept for packed (varlen) batches: there the persistent form
-// was measured 8-16 % SLOWER (16 sequences of 256-4096 tokens, Hq32 Hkv8 D128; 8 % with equal lengths) although it
-// is 3-11 % faster on dense batches of the same sizes, and the cause was not found in the time there was.
+// that each set up, process one key tile and exit.  Kept for packed batches with grouped heads at D = 128, whose items are several
+// times as long and gain little from running into one another: this kernel against the persistent one, 16 documents of 256-4096 tokens
+// Hq32 Hkv8 1556 : 1650 us, 24 of 700-1700 Hq16 Hkv4 430 : 456, 4 of 4096-8192 1066 : 1126.  The other way round without
+// groups (64 texts of 130-640 tokens H16 308 : 254, 24 of 700-1700 not causal 812 : 782) and at D = 64 (64 texts of 130-640 H16
+// 227 : 168, 16 documents 609 : 528, 32 of 500-1500 Hq16 Hkv4 457 : 438).
 // A Q tile of a packed batch can hold rows of the neighbouring sequence; this kernel carries the code that guards
 // against them (kVarlen is always true here).
 template <int D, bool kVarlen>
@@ -1336,8 +1404,10 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
   int dev = 0;
   FA_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    FA_CHECK_CUDA(cudaFuncSetAttribute(bwd_dkdv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytesDkdv));
-    FA_CHECK_CUDA(cudaFuncSetAttribute(bwd_dkdv_packed_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytesDkdv));
+    FA_CHECK_CUDA(cudaFuncSetAttribute(bwd_dkdv_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytesDkdv));
+    FA_CHECK_CUDA(cudaFuncSetAttribute(bwd_dkdv_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytesDkdv));
+    if constexpr (D == 128)
+      FA_CHECK_CUDA(cudaFuncSetAttribute(bwd_dkdv_packed_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytesDkdv));
     configured[dev & 63] = true;
   }
   if (stage_mask & 2) {
@@ -1374,12 +1444,14 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
     // dK and dV may be written over K and V (a CTA reads its own tile before it writes it): then the dQ kernel, which reads
     // K and V too, has to be over first.
     const bool overlap = (stage_mask & 2) != 0 && !gradients_over_keys(p);
-    if (kp.cu_seqlens_q != nullptr) {  // packed sequences: one CTA per key tile (see bwd_dkdv_packed_kernel)
-      dim3 grid_k((p->seqlen_k + kBlock - 1) / kBlock, p->h_k, p->b);
-      if (overlap) {
-        FA_CHECK_CUDA(launch_overlapped(bwd_dkdv_packed_kernel<D, true>, grid_k, kNumThreads, C::kSmemBytesDkdv, stream, kp));
-      } else {
-        bwd_dkdv_packed_kernel<D, true><<<grid_k, kNumThreads, C::kSmemBytesDkdv, stream>>>(kp);
+    if (D == 128 && kp.cu_seqlens_q != nullptr && p->h != p->h_k) {  // one CTA per key tile: see bwd_dkdv_packed_kernel
+      if constexpr (D == 128) {
+        dim3 grid_k((p->seqlen_k + kBlock - 1) / kBlock, p->h_k, p->b);
+        if (overlap) {
+          FA_CHECK_CUDA(launch_overlapped(bwd_dkdv_packed_kernel<D, true>, grid_k, kNumThreads, C::kSmemBytesDkdv, stream, kp));
+        } else {
+          bwd_dkdv_packed_kernel<D, true><<<grid_k, kNumThreads, C::kSmemBytesDkdv, stream>>>(kp);
+        }
       }
     } else {
       BwdKernelParams kk = kp;
@@ -1388,14 +1460,16 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
       if (sms <= 0 || kk.sched == nullptr) return set_error(FA_ERR_CUDA, "fa_bwd: device attributes not available");
       kk.items_x = (p->seqlen_k + kBlock - 1) / kBlock;
       kk.b = p->b;
-      const int64_t total = static_cast<int64_t>(kk.items_x) * p->h_k * p->b;
+      const int64_t total = kk.cu_seqlens_k ? static_cast<int64_t>(p->h_k) * (p->total_k / kBlock + p->b)
+                                            : static_cast<int64_t>(kk.items_x) * p->h_k * p->b;
       FA_CHECK_ARG(total < (1ll << 30), "fa_bwd: too many work items");
       kk.total_items = static_cast<int>(total);
       const int grid = kk.total_items < sms ? kk.total_items : sms;
+      const auto kernel = kk.cu_seqlens_q ? bwd_dkdv_kernel<D, true> : bwd_dkdv_kernel<D, false>;
       if (overlap) {
-        FA_CHECK_CUDA(launch_overlapped(bwd_dkdv_kernel<D>, dim3(grid), kDkvThreads, C::kSmemBytesDkdv, stream, kk));
+        FA_CHECK_CUDA(launch_overlapped(kernel, dim3(grid), kDkvThreads, C::kSmemBytesDkdv, stream, kk));
       } else {
-        bwd_dkdv_kernel<D><<<grid, kDkvThreads, C::kSmemBytesDkdv, stream>>>(kk);
+        kernel<<<grid, kDkvThreads, C::kSmemBytesDkdv, stream>>>(kk);
       }
     }
     FA_CHECK_CUDA(cudaGetLastError());

@@ -223,6 +223,26 @@ def test_varlen_backward_of_many_short_sequences(ext, d, causal):
             assert torch.equal(got[a:b], want[0])
 
 
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("d,h,hk", [(64, 6, 6), (64, 6, 2), (128, 6, 6), (128, 6, 2)])
+def test_packed_key_gradients_equal_dense_ones(ext, d, h, hk, causal):
+    # Key tiles and Q tiles of one row, whole ones and one row more, more queries than keys and the reverse, several key tiles
+    # per CTA: both dK/dV kernels of packed batches against the one of dense batches, bit for bit.
+    lens_q = [1, 128, 129, 500, 127, 257, 40, 256, 300] * 6
+    lens_k = [300, 129, 128, 1, 127, 640, 256, 40, 300] * 6
+    q, k, v, dout, cq, ck = _varlen_case(91 + d, lens_q, lens_k, h, hk, d)
+    q, k, v, dout, cq_d, ck_d = (x.to(DEV) for x in (q, k, v, dout, cq, ck))
+    args = (cq_d, ck_d, max(lens_q), max(lens_k), d ** -0.5, causal)
+    out, lse = ext.varlen_fwd(q, k, v, *args)
+    grads = ext.varlen_bwd(q, k, v, out, lse, dout, *args)
+    for i in list(range(9)) + [30, 49, 53]:
+        rq, rk = slice(int(cq[i]), int(cq[i + 1])), slice(int(ck[i]), int(ck[i + 1]))
+        o, l = ext.fwd(q[None, rq], k[None, rk], v[None, rk], d ** -0.5, causal)
+        dense = ext.bwd(q[None, rq], k[None, rk], v[None, rk], o, l, dout[None, rq], d ** -0.5, causal)
+        for got, want, rows in zip(grads, dense, (rq, rk, rk)):
+            assert torch.equal(got[rows], want[0])
+
+
 def test_varlen_packed_variants(ext):
     from flash_attention_turing_b200 import (flash_attn_varlen_func, flash_attn_varlen_kvpacked_func,
                                              flash_attn_varlen_qkvpacked_func)
