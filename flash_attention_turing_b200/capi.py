@@ -23,6 +23,7 @@ EXPORTED_SYMBOLS = (
     "fa_kvcache_num_splits",
     "fa_kvcache_workspace_bytes",
     "fa_kvcache",
+    "fa_kvcache_checked",
     "fa_kvcache_noalloc",
     "fa_combine",
     "fa_combine_gather",

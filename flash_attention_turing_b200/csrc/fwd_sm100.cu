@@ -72,6 +72,7 @@ struct FwdKernelParams {
   const int* cu_seqlens_q;
   const int* cu_seqlens_k;
   const int* seqused_k;
+  int checked;        // the host refuses lengths beyond the capacity: not reported
   int seqused_k_add;  // added to seqused_k[b] (tokens appended to a cache in the same call)
   int k_capacity;     // upper bound for seqused_k: rows of k, or block_table columns * page_size
   const int* cache_batch_idx;
@@ -292,7 +293,7 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
             it.batch = batch, it.head = head, it.mpair = mpair;
             if (p.seqused_k && p.status && head == 0 && mpair == 0) {
               const int raw = p.seqused_k[batch] + p.seqused_k_add;
-              if (raw < 0 || raw > p.k_capacity) atomicOr(p.status, kStatusCapacityClamped);
+              if (raw < 0 || (raw > p.k_capacity && !p.checked)) atomicOr(p.status, kStatusCapacityClamped);
             }
             break;
           }
@@ -784,7 +785,7 @@ int launch_fwd(FwdKernelParams& kp, int b, int h, int seqlen_q, int64_t total_q,
 
 namespace fa {
 
-int run_fwd(const FaFwdParams* p, int seqused_k_add, cudaStream_t stream, bool overlap) {
+int run_fwd(const FaFwdParams* p, int seqused_k_add, cudaStream_t stream, bool overlap, bool checked) {
   FA_CHECK_ARG(p != nullptr, "fa_fwd: params is NULL");
   FA_CHECK_ARG(p->q && p->k && p->v && p->o && p->lse, "fa_fwd: q, k, v, o, lse must be non-NULL");
   if (p->d != 64 && p->d != 128)
@@ -857,6 +858,7 @@ int run_fwd(const FaFwdParams* p, int seqused_k_add, cudaStream_t stream, bool o
   kp.cu_seqlens_k = p->cu_seqlens_k;
   kp.seqused_k = p->seqused_k;
   kp.seqused_k_add = seqused_k_add;
+  kp.checked = checked;
   kp.k_capacity = (p->block_table && p->block_table_cols > 0) ? p->block_table_cols * p->page_size
                   : (p->block_table ? 0x7fffffff : static_cast<int>(k_rows));
   kp.cache_batch_idx = p->cache_batch_idx;

@@ -57,6 +57,7 @@ struct DecodeParams {
   int page_size;     // tokens per page (paged) or capacity per cache row (contiguous)
   int capacity;      // tokens a sequence can hold: max_blocks_per_seq * page_size, or the cache row length
   int num_splits;    // grid.x
+  int checked;       // the host refuses lengths beyond the capacity: not reported
   int chunk_tiles;   // > 0: split s owns tiles [s*chunk, (s+1)*chunk); 0: proportional ranges
   int* status;
 };
@@ -124,7 +125,7 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
   // a clamp is reported through the status word.
   const int len_raw = p.cache_seqlens[batch] + p.seqlen_new;
   const int len = max(0, min(len_raw, p.capacity));
-  if (len != len_raw && threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusCapacityClamped);
+  if (len != len_raw && (len_raw < 0 || !p.checked) && threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusCapacityClamped);
   const int n_tiles = (len + kTileTokens - 1) / kTileTokens;
   int tile_begin, tile_end;
   if (p.chunk_tiles > 0) {
@@ -465,10 +466,36 @@ struct AppendParams {
   const int* block_table;
   int64_t block_table_batch_stride;
   int max_blocks_per_seq;
+  // fa_kvcache_checked(): nothing is written unless every length is at most max_length
+  int* verdict;
+  int token;
+  int64_t max_length;
 };
+
+// By all threads of a block.
+__device__ __forceinline__ bool lengths_fit(const int* lengths, int b, int64_t max_length) {
+  bool over = false;
+  for (int i = threadIdx.x; i < b; i += blockDim.x) over |= lengths[i] > max_length;
+  return !__syncthreads_or(over);
+}
+__device__ __forceinline__ void tell_host(int* verdict, int token, bool fits) {
+  *reinterpret_cast<volatile int*>(verdict) = 2 * token + (fits ? 0 : 1);
+  __threadfence_system();
+}
+
+// fa_kvcache_checked() without new tokens
+__global__ void __launch_bounds__(256) check_lengths_kernel(const int* lengths, int b, int64_t max_length, int* verdict, int token) {
+  const bool fits = lengths_fit(lengths, b, max_length);
+  if (threadIdx.x == 0) tell_host(verdict, token, fits);
+}
 
 __global__ void __launch_bounds__(256) append_kernel(const AppendParams p) {
   grid_launch_dependents();
+  if (p.verdict != nullptr) {  // every block looks at all lengths: a few hundred of them at most, and no launch in between
+    const bool fits = lengths_fit(p.cache_seqlens, p.b, p.max_length);
+    if (blockIdx.x == 0 && threadIdx.x == 0) tell_host(p.verdict, p.token, fits);
+    if (!fits) return;
+  }
   const int units_per_row = p.d / 8;  // 16-byte units per (token, head)
   const int64_t total = static_cast<int64_t>(p.b) * p.seqlen_new * p.h_k * units_per_row;
   for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
@@ -609,9 +636,10 @@ extern "C" size_t fa_kvcache_workspace_bytes(const FaKvcacheParams* p) {
          align_up(static_cast<size_t>(splits) * rows * sizeof(float), 256);
 }
 
-extern "C" int fa_kvcache(const FaKvcacheParams* p, fa_stream_t stream_) {
-  using namespace fa;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+namespace fa {
+namespace {
+// verdict: see fa_kvcache_checked(); NULL: lengths are clamped to the capacity
+int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t stream) {
   int rc = validate(p, "fa_kvcache");
   if (rc != FA_OK) return rc;
   FA_CHECK_ARG(p->q && p->k_cache && p->v_cache && p->o && p->lse && p->cache_seqlens,
@@ -630,6 +658,11 @@ extern "C" int fa_kvcache(const FaKvcacheParams* p, fa_stream_t stream_) {
   // sequence of 1500 tokens (Hq32 Hkv8 D128) 21.2 -> 14.6 us, four of up to 4000 24.8 -> 20.7, 16 of up to 8000 77.6 -> 71.4.
   // ---- 1. append ----
   const bool appends = p->k_new && p->seqlen_new > 0;
+  const int64_t max_length = (p->block_table ? static_cast<int64_t>(p->max_blocks_per_seq) : 1) * p->seqlen_cache - p->seqlen_new;
+  if (verdict != nullptr && !appends) {
+    check_lengths_kernel<<<1, 256, 0, stream>>>(p->cache_seqlens, p->b, max_length, verdict, token);
+    FA_CHECK_CUDA(cudaGetLastError());
+  }
   if (appends) {
     FA_CHECK_ARG(aligned16(p->k_new) && aligned16(p->v_new) && aligned16(p->k_cache) && aligned16(p->v_cache),
                  "fa_kvcache: k_new, v_new and the caches must be 16-byte aligned");
@@ -652,6 +685,7 @@ extern "C" int fa_kvcache(const FaKvcacheParams* p, fa_stream_t stream_) {
     ap.cache_seqlens = p->cache_seqlens; ap.cache_batch_idx = p->cache_batch_idx;
     ap.block_table = p->block_table; ap.block_table_batch_stride = p->block_table_batch_stride;
     ap.max_blocks_per_seq = p->max_blocks_per_seq;
+    ap.verdict = verdict; ap.token = token; ap.max_length = max_length;
     const int64_t total = static_cast<int64_t>(p->b) * p->seqlen_new * p->h_k * (p->d / 8);
     const int blocks = static_cast<int>(std::min<int64_t>((total + 255) / 256, 148 * 8));
     append_kernel<<<blocks, 256, 0, stream>>>(ap);
@@ -678,7 +712,7 @@ extern "C" int fa_kvcache(const FaKvcacheParams* p, fa_stream_t stream_) {
     f.block_table_batch_stride = p->block_table_batch_stride;
     f.page_size = p->block_table ? p->seqlen_cache : 0;
     f.block_table_cols = p->block_table ? p->max_blocks_per_seq : 0;
-    return run_fwd(&f, p->seqlen_new, stream, appends);
+    return run_fwd(&f, p->seqlen_new, stream, appends, verdict != nullptr);
   }
 
   int splits, chunk;
@@ -723,6 +757,7 @@ extern "C" int fa_kvcache(const FaKvcacheParams* p, fa_stream_t stream_) {
   dp.capacity = capacity_tokens(p);
   dp.num_splits = splits;
   dp.chunk_tiles = chunk;
+  dp.checked = verdict != nullptr;
   dp.status = device_status_ptr();
   rc = (p->d == 128) ? launch_decode<128>(dp, p->b, p->h_k, appends, stream) : launch_decode<64>(dp, p->b, p->h_k, appends, stream);
   if (rc != FA_OK) return rc;
@@ -732,6 +767,18 @@ extern "C" int fa_kvcache(const FaKvcacheParams* p, fa_stream_t stream_) {
     return launch_combine(dp.o_accum, dp.lse_accum, p->o, p->lse, rows_total, splits, p->h, p->seqlen_q, p->d,
                           p->o_batch_stride, p->o_row_stride, p->o_head_stride, stream, true);
   return FA_OK;
+}
+}  // namespace
+}  // namespace fa
+
+extern "C" int fa_kvcache(const FaKvcacheParams* p, fa_stream_t stream) {
+  return fa::run_kvcache(p, nullptr, 0, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int fa_kvcache_checked(const FaKvcacheParams* p, int32_t* verdict, int32_t token, fa_stream_t stream) {
+  using namespace fa;
+  FA_CHECK_ARG(verdict != nullptr && token >= 0 && token < (1 << 30), "fa_kvcache_checked: verdict is NULL or token out of range");
+  return run_kvcache(p, verdict, token, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -298,9 +298,44 @@ std::vector<at::Tensor> mha_varlen_bwd(at::Tensor q, at::Tensor k, at::Tensor v,
   return {dq, dk, dv};
 }
 
+// The word of pinned host memory in which the device answers fa_kvcache_checked(): one per thread, which waits for its answer
+// before it makes the next call.
+struct Verdict {
+  int32_t* word = nullptr;
+  int32_t token = 0;
+  ~Verdict() {
+    if (word) cudaFreeHost(word);
+  }
+  void next() {
+    if (!word) {
+      C10_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&word), sizeof(int32_t), cudaHostAllocPortable));
+      *word = -1;
+    }
+    token = (token + 1) & 0xfffff;
+  }
+  // After an error the device may still write the word, so it is not used again (nor freed).
+  void abandon() { word = nullptr; }
+  // Waits until the device has answered; whether all lengths fit.  The stream is asked now and then, so that a failed launch or
+  // device ends the wait with its error.
+  bool wait(cudaStream_t stream) {
+    const volatile int32_t* w = word;
+    for (unsigned n = 1; *w >> 1 != token; ++n) {
+      if (n % 4096 != 0) continue;
+      const cudaError_t state = cudaStreamQuery(stream);
+      if (state == cudaErrorNotReady) continue;
+      if (state == cudaSuccess && *w >> 1 == token) break;
+      abandon();
+      C10_CUDA_CHECK(state);
+      TORCH_CHECK(false, "fa_kvcache_checked gave no answer");
+    }
+    return (*w & 1) == 0;
+  }
+};
+
 // ---- KV-cache forward (mha_fwd_kvcache, flash_api.cpp:508-715) ----
-std::vector<at::Tensor> mha_fwd_kvcache(at::Tensor q, at::Tensor k_cache, at::Tensor v_cache, py::object k_obj,
-                                        py::object v_obj, at::Tensor cache_seqlens, py::object rotary_cos_obj,
+// checked: see fwd_kvcache_checked().
+std::vector<at::Tensor> kvcache_forward(Verdict* checked, at::Tensor q, at::Tensor k_cache, at::Tensor v_cache,
+                                        py::object k_obj, py::object v_obj, at::Tensor cache_seqlens, py::object rotary_cos_obj,
                                         py::object rotary_sin_obj, py::object cache_batch_idx_obj,
                                         py::object cache_leftpad_obj, py::object block_table_obj,
                                         py::object alibi_slopes_obj, py::object out_obj,
@@ -432,8 +467,52 @@ std::vector<at::Tensor> mha_fwd_kvcache(at::Tensor q, at::Tensor k_cache, at::Te
   at::Tensor workspace = torch::empty({static_cast<int64_t>(ws)}, q.options().dtype(torch::kUInt8));
   p.workspace = ws ? workspace.data_ptr() : nullptr;
   p.workspace_bytes = ws;
-  check_rc(fa_kvcache(&p, current_stream()), "fa_kvcache");
+  if (checked) {
+    checked->next();
+    const int rc = fa_kvcache_checked(&p, checked->word, checked->token, current_stream());
+    if (rc != FA_OK) checked->abandon();
+    check_rc(rc, "fa_kvcache_checked");
+  } else {
+    check_rc(fa_kvcache(&p, current_stream()), "fa_kvcache");
+  }
   return {out, lse};
+}
+
+std::vector<at::Tensor> mha_fwd_kvcache(at::Tensor q, at::Tensor k_cache, at::Tensor v_cache, py::object k_obj,
+                                        py::object v_obj, at::Tensor cache_seqlens, py::object rotary_cos_obj,
+                                        py::object rotary_sin_obj, py::object cache_batch_idx_obj,
+                                        py::object cache_leftpad_obj, py::object block_table_obj,
+                                        py::object alibi_slopes_obj, py::object out_obj,
+                                        const double softmax_scale, bool is_causal, int64_t window_size_left,
+                                        int64_t window_size_right, const double softcap,
+                                        bool rotary_interleaved, int64_t num_splits) {
+  return kvcache_forward(nullptr, q, k_cache, v_cache, k_obj, v_obj, cache_seqlens, rotary_cos_obj, rotary_sin_obj,
+                         cache_batch_idx_obj, cache_leftpad_obj, block_table_obj, alibi_slopes_obj, out_obj, softmax_scale,
+                         is_causal, window_size_left, window_size_right, softcap, rotary_interleaved, num_splits);
+}
+
+// fwd_kvcache that writes nothing to the cache when a length does not fit it: out, lse and whether all did.  The kernels are
+// launched first and the answer is waited for under them.  None when the call has to be checked beforehand: no work to
+// launch, or a stream that is being captured.
+py::object fwd_kvcache_checked(at::Tensor q, at::Tensor k_cache, at::Tensor v_cache, py::object k, py::object v,
+                               at::Tensor cache_seqlens, py::object cache_batch_idx, py::object block_table,
+                               double softmax_scale, bool is_causal, int64_t num_splits) {
+  if (!q.is_cuda() || q.numel() == 0 || cache_seqlens.device() != q.device()) return py::none();
+  c10::cuda::CUDAGuard guard(q.device());
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+  C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone) return py::none();
+  static thread_local Verdict verdict;
+  const std::vector<at::Tensor> r =
+      kvcache_forward(&verdict, q, k_cache, v_cache, k, v, cache_seqlens, py::none(), py::none(), cache_batch_idx, py::none(),
+                      block_table, py::none(), py::none(), softmax_scale, is_causal, -1, -1, 0.0, true, num_splits);
+  bool fits;
+  {
+    py::gil_scoped_release release;
+    fits = verdict.wait(stream);
+  }
+  return py::make_tuple(r[0], r[1], fits);
 }
 
 // ---- stand-alone LSE merge (no counterpart binding in the reference; used after the NCCL exchange
@@ -552,6 +631,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("max_seqlen_q"), py::arg("max_seqlen_k"), py::arg("softmax_scale"), py::arg("is_causal"),
         py::arg("dq") = py::none(), py::arg("dk") = py::none(), py::arg("dv") = py::none());
   m.def("fwd_kvcache", &mha_fwd_kvcache, "KV-cache forward pass");
+  m.def("fwd_kvcache_checked", &fwd_kvcache_checked, "KV-cache forward pass that refuses lengths beyond the capacity");
   m.def("combine", &combine, "Merge split partials (O fp32, LSE) with log-sum-exp weights");
   m.def("combine_gather", &combine_gather, "Merge per-rank partial (O fp16, LSE) read in place, peer memory allowed");
   m.def("sum_gather", &sum_gather, "Sum per-rank partial dQ (fp16) read in place, peer memory allowed", py::arg("parts"),

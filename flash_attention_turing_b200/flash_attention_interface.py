@@ -24,7 +24,8 @@ from . import _ext
 
 # The reference reads cache_seqlens back to the host to check the cache capacity on every call
 # (``int(cache_seqlens.max().item())``, its :855) -- a device synchronisation per decode step.  The check
-# is part of the reference's error contract, so it stays on by default.  A serving loop that guarantees
+# is part of the reference's error contract, so it stays on by default; the device makes it, writes nothing to the cache when
+# a length does not fit, and the host waits for the answer under the kernels instead of before they are launched.  A serving loop that guarantees
 # capacity itself can set this to False: the kernels then clamp every length to the capacity on the device
 # (never reading or writing out of bounds) and report a clamp through ``device_status()`` bit 1.
 HOST_CAPACITY_CHECK = True
@@ -80,10 +81,14 @@ def _flash_attn_varlen_backward(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlen
 
 
 def _flash_attn_kvcache_forward(q, k_cache, v_cache, k, v, cache_seqlens, cache_batch_idx, block_table,
-                                softmax_scale: float, causal: bool, num_splits: int):
+                                softmax_scale: float, causal: bool, num_splits: int, checked: bool = False):
+    """``checked``: (out, lse, whether all lengths fit the cache), or None when that has to be found out beforehand."""
     q, k_cache, v_cache, k, v, cache_seqlens, cache_batch_idx, block_table = (
         maybe_contiguous(t) for t in (q, k_cache, v_cache, k, v, cache_seqlens, cache_batch_idx, block_table)
     )
+    if checked:
+        return _gpu().fwd_kvcache_checked(q, k_cache, v_cache, k, v, cache_seqlens, cache_batch_idx, block_table,
+                                          softmax_scale, causal, num_splits)
     # 20-argument binding of the reference (flash_api.cpp:508-528); unsupported features are None.
     out, lse = _gpu().fwd_kvcache(q, k_cache, v_cache, k, v, cache_seqlens, None, None, cache_batch_idx,
                                   None, block_table, None, None, softmax_scale, causal, -1, -1, 0.0, True,
@@ -388,6 +393,18 @@ def flash_attn_with_kvcache(
         seqlen_new = k.shape[1]
     # Capacity is checked before the device/dtype checks, on whatever device the lengths live
     # (the reference does the same, :855-858, and its tests rely on that order with CPU tensors).
+    scale = _default_scale(q, softmax_scale)
+    if HOST_CAPACITY_CHECK and cache_batch_idx is None and all(t.is_cuda for t in (q, k_cache, v_cache, cache_seqlens)):
+        try:
+            r = _flash_attn_kvcache_forward(q, k_cache, v_cache, k, v, cache_seqlens, cache_batch_idx, block_table, scale,
+                                            causal, num_splits, checked=True)
+        except RuntimeError:
+            r = None  # whatever is wrong, a capacity that is insufficient comes first
+        if r is not None:
+            out, lse, fits = r
+            if not fits:
+                raise ValueError("cache capacity is insufficient for the requested append length")
+            return (out, lse) if return_softmax_lse else out
     if HOST_CAPACITY_CHECK or not cache_seqlens.is_cuda:
         used = int(cache_seqlens.max().item()) if cache_seqlens.numel() > 0 else 0
         if used + seqlen_new > capacity:
@@ -404,5 +421,5 @@ def flash_attn_with_kvcache(
             raise RuntimeError("k and v must be float16 tensors")
 
     out, lse = _flash_attn_kvcache_forward(q, k_cache, v_cache, k, v, cache_seqlens, cache_batch_idx,
-                                           block_table, _default_scale(q, softmax_scale), causal, num_splits)
+                                           block_table, scale, causal, num_splits)
     return (out, lse) if return_softmax_lse else out

@@ -322,3 +322,54 @@ def test_tiled_path_clamps_lengths_to_the_capacity_and_reports_it(ext, b, sq, h)
         iface.HOST_CAPACITY_CHECK = True
     assert status == 2
     assert err_stats(out, o_ref)[0] <= O_TOL
+
+
+@pytest.mark.parametrize("b,sq,new,d,capacity,page", [
+    (1, 1, 1, 128, 512, 0),      # append kernel of one block
+    (300, 1, 1, 64, 256, 256),   # more lengths than threads of a block
+    (3, 2, 0, 128, 512, 0),      # nothing to append: a kernel of its own looks at the lengths
+    (2, 64, 64, 64, 512, 256),   # tiled path
+])
+def test_lengths_beyond_the_capacity_write_nothing(ext, b, sq, new, d, capacity, page):
+    """The device finds out whether the lengths fit, under kernels that are already launched: one token too many in the last
+    sequence leaves the cache and the status word as they were, and the calls before and after it are not affected."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from flash_attention_turing_b200 import flash_attn_with_kvcache
+
+    torch.manual_seed(b)
+    h, hk = 4, 2
+    half = lambda *s: torch.randn(*s, device=DEV, dtype=torch.float16)  # noqa: E731
+    rows = (b * (capacity // page), page) if page else (b, capacity)
+    q, kn, vn, kc, vc = half(b, sq, h, d), half(b, new, hk, d), half(b, new, hk, d), half(*rows, hk, d), half(*rows, hk, d)
+    kwargs = dict(k=kn if new else None, v=vn if new else None, causal=True, return_softmax_lse=True,
+                  block_table=torch.arange(rows[0], dtype=torch.int32, device=DEV).view(b, -1) if page else None)
+    full = torch.full((b,), capacity - new, dtype=torch.int32, device=DEV)  # the last token fits exactly
+    over = full.clone()
+    over[-1] += 1
+    kw, vw = kc.clone(), vc.clone()
+    want = flash_attn_with_kvcache(q, kw, vw, cache_seqlens=full, **kwargs)
+    k0, v0 = kc.clone(), vc.clone()
+    for _ in range(3):
+        with pytest.raises(ValueError, match="cache capacity is insufficient"):
+            flash_attn_with_kvcache(q, kc, vc, cache_seqlens=over, **kwargs)
+    assert torch.equal(kc, k0) and torch.equal(vc, v0)
+    assert ext.device_status(False) == 0
+
+    def step(i):
+        k, v = kc.clone(), vc.clone()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+            if i % 2:
+                with pytest.raises(ValueError, match="cache capacity is insufficient"):
+                    flash_attn_with_kvcache(q, k, v, cache_seqlens=over, **kwargs)
+                out = None
+            else:
+                out = flash_attn_with_kvcache(q, k, v, cache_seqlens=full, **kwargs)
+            torch.cuda.current_stream().synchronize()
+        return out, k, v
+
+    with ThreadPoolExecutor(4) as pool:  # every thread waits for an answer of its own
+        for i, (out, k, v) in enumerate(pool.map(step, range(16))):
+            assert torch.equal(k, k0 if i % 2 else kw) and torch.equal(v, v0 if i % 2 else vw)
+            assert out is None or (torch.equal(out[0], want[0]) and torch.equal(out[1], want[1]))
