@@ -172,13 +172,11 @@ __device__ __forceinline__ uint64_t kmajor_slice(uint64_t tile_desc, int k) {
 }
 __device__ __forceinline__ uint64_t mnmajor_slice(uint64_t tile_desc, int k) { return desc_advance(tile_desc, k * 2048); }
 
-// A thread that issues tcgen05.mma is held for the duration of each MMA (about 66 clocks for
-// 128x128x16), and whatever else it executes -- a barrier poll costs 60-80 clocks even when the barrier
-// completed long ago, a commit about 50 -- is time in which it feeds nothing to the tensor pipe.  Two
-// measures keep the pipe busy: the products are issued by two warps (kMmaWarp, kAccMmaWarp), so that one
-// polls while the other issues, and a product takes a hook that runs after half of its MMAs for waits on
-// TMA loads of the NEXT product, which are satisfied long before and cost only the poll.  A hook returns
-// false when a bounded wait gave up; the rest of the product is then skipped.
+// Whatever the thread that issues the products executes between them -- a barrier poll costs 60-80 clocks even when the
+// barrier completed long ago, a commit about 50 -- holds back what it issues next.  Two measures keep the pipe busy: the products
+// are issued by two warps (kMmaWarp, kAccMmaWarp), so that one polls while the other issues, and a product takes a hook that runs
+// after half of its MMAs for waits on TMA loads of the NEXT product, which are satisfied long before and cost only the poll.  A hook
+// returns false when a bounded wait gave up; the rest of the product is then skipped.
 // C = A[smem, K-major] * B[smem, K-major]^T over D, both 128-row tiles.
 template <int D, class Hook>
 __device__ __forceinline__ bool gemm_ss(uint32_t d_tmem, uint32_t a_tile, uint32_t b_tile, uint32_t idesc,
