@@ -151,8 +151,9 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 // before the current one ends; the scheduler thread derives everything the roles need from it once and leaves it in
 // shared memory (decoding it in five roles was code the instruction cache had to hold).
 //
-// Bound by the issue of its products: 16 SS MMAs of about 88 clocks (operand fetches share the shared-memory port with
-// the arriving tiles) and 8 TS MMAs of about 75, of 1536 clocks at the tensor peak.  S and dP of a block are issued back
+// Bound by the chain products -> fetch and hand-back -> products: 16 SS MMAs (1060 clocks), about 250 until their result is seen,
+// 300 until it is in registers and handed back, and the dQ product of the block before (512), which comes in between; 2070
+// clocks a block at D = 128, of 1536 at the tensor peak (2230 before its loops ran under elect_one()).  S and dP of a block are issued back
 // to back, fetched into registers together and handed back together, so that the whole arithmetic of the block runs
 // under the next S / dP: ONE wait and one hand-back per block where waiting for S and dP in turn took two of each, at
 // 150-300 clocks apiece for warps in lock-step.  The hand-back has to leave before the arithmetic starts (see
@@ -1038,13 +1039,31 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
 // 227 : 168, 16 documents 609 : 528, 32 of 500-1500 Hq16 Hkv4 457 : 438).
 // A Q tile of a packed batch can hold rows of the neighbouring sequence; this kernel carries the code that guards
 // against them (kVarlen is always true here).
+// The z-th largest sequence by the pairs of a head, for up to 32 of them; otherwise the z-th.  Called by whole warps.
+// Blocks start in the order of the grid, and an item of the longest sequence can take a tenth of the launch: begun last, it runs on
+// alone: 16 documents of 256-4096 tokens Hq32 Hkv8 1557 -> 1538 us, 4 of 4096-8192 Hq16 Hkv4 1034 -> 995, 24 of 700-1700 the same.
+// (32: one lane of a warp each.  The forward gained nothing from the same order over the sequences of a cache.)
+__device__ __forceinline__ int sequence_by_size(const int* cu_q, const int* cu_k, int b, int z) {
+  if (b > 32) return z;
+  const int lane = threadIdx.x & 31;
+  float size = -1.f;
+  if (lane < b) size = static_cast<float>(cu_q[lane + 1] - cu_q[lane]) * static_cast<float>(cu_k[lane + 1] - cu_k[lane]);
+  int rank = 0;
+  for (int j = 0; j < b; ++j) {
+    const float other = __shfl_sync(0xffffffffu, size, j);
+    rank += other > size || (other == size && j < lane);
+  }
+  return __ffs(__ballot_sync(0xffffffffu, lane < b && rank == z)) - 1;
+}
+
 template <int D, bool kVarlen>
 __global__ void __launch_bounds__(kNumThreads, 1)
 bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
   using C = BCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  const int batch = blockIdx.z, head_k = blockIdx.y, nblk = blockIdx.x;
   constexpr bool varlen = kVarlen;
+  const int batch = varlen ? sequence_by_size(p.cu_seqlens_q, p.cu_seqlens_k, p.b, blockIdx.z) : blockIdx.z;
+  const int head_k = blockIdx.y, nblk = blockIdx.x;
   const int q_off = varlen ? p.cu_seqlens_q[batch] : 0;
   const int sq = varlen ? p.cu_seqlens_q[batch + 1] - q_off : p.seqlen_q;
   const int k_off = varlen ? p.cu_seqlens_k[batch] : 0;
