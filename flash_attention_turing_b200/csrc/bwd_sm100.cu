@@ -151,9 +151,9 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 // before the current one ends; the scheduler thread derives everything the roles need from it once and leaves it in
 // shared memory (decoding it in five roles was code the instruction cache had to hold).
 //
-// Bound by the chain products -> fetch and hand-back -> products: 16 SS MMAs (1060 clocks), about 250 until their result is seen,
-// 300 until it is in registers and handed back, and the dQ product of the block before (512), which comes in between; 2070
-// clocks a block at D = 128, of 1536 at the tensor peak (2230 before its loops ran under elect_one()).  S and dP of a block are issued back
+// Bound by the issue of its products: 16 SS MMAs of about 88 clocks and 8 TS MMAs of about 75, of 1536 clocks at the tensor peak.
+// Its two issuing loops run under lane == 0 and not under elect_one() as elsewhere: that was 7-9 % faster, but at D = 64 about one
+// test run in ten then found wrong dQ; the cause is not known.  S and dP of a block are issued back
 // to back, fetched into registers together and handed back together, so that the whole arithmetic of the block runs
 // under the next S / dP: ONE wait and one hand-back per block where waiting for S and dP in turn took two of each, at
 // 150-300 clocks apiece for warps in lock-step.  The hand-back has to leave before the arithmetic starts (see
@@ -345,7 +345,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       ++ni;
     }
   } else if (warp == kMmaWarp) {
-    if (elect_one()) {
+    if (lane == 0) {
       constexpr uint32_t idesc_nn = make_idesc_f16(128, kBlock, false, false);
       const uint32_t q_addr = smem_u32(sQ), do_addr = smem_u32(sdO);
       auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, ctx); };
@@ -383,7 +383,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       }
     }
   } else if (warp == kAccMmaWarp) {
-    if (elect_one()) {
+    if (lane == 0) {
       constexpr uint32_t idesc_acc = make_idesc_f16(128, D, false, true);
       int G = 0, nf = 0;
       bool ok = true;
