@@ -113,7 +113,7 @@ struct BBarriers {
   uint64_t s_full;         // S^T accumulator ready (not used by the dQ kernel, whose dp_full covers both)
   uint64_t dp_full;        // dP (or dP^T) accumulator ready
   uint64_t p_full;         // packed P^T written to TMEM (dK/dV kernel)
-  uint64_t ds_full;        // packed dS (or dS^T) written to TMEM
+  uint64_t ds_full;        // packed dS^T written to TMEM (the dQ kernel has two of its own)
   uint64_t s_loaded;       // S^T (dQ kernel: S and dP) sits in registers: its TMEM region may be overwritten
   uint64_t dp_loaded;      // dP^T sits in registers (dQ kernel: s_loaded covers both)
   uint64_t p_free;         // dV MMAs of the previous tile have consumed the packed P^T

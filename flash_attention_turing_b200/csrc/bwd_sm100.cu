@@ -152,8 +152,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 // shared memory (decoding it in five roles was code the instruction cache had to hold).
 //
 // Bound by the issue of its products: 16 SS MMAs of about 88 clocks and 8 TS MMAs of about 75, of 1536 clocks at the tensor peak.
-// Its two issuing loops run under lane == 0 and not under elect_one() as elsewhere: that was 7-9 % faster, but at D = 64 about one
-// test run in ten then found wrong dQ; the cause is not known.  S and dP of a block are issued back
+// Its two issuing loops run under lane == 0 and not under elect_one() as elsewhere.  S and dP of a block are issued back
 // to back, fetched into registers together and handed back together, so that the whole arithmetic of the block runs
 // under the next S / dP: ONE wait and one hand-back per block where waiting for S and dP in turn took two of each, at
 // 150-300 clocks apiece for warps in lock-step.  The hand-back has to leave before the arithmetic starts (see
@@ -174,6 +173,10 @@ struct __align__(16) DqItem {
 struct DqBarriers {
   BBarriers b;
   uint64_t q_free;          // the Q / dO tiles (last dP products) and the statistics (elementwise warps) have been read
+  // dS(g) is whole in packed buffer g & 1.  Two barriers in turn: a warp may be at the end of block g + 1 while another is still in
+  // the arithmetic of block g (S and dP are handed back before it), and on one barrier its second arrival would stand for the other
+  // warp's first: dQ(g) on half a dS.  For block g + 2, the next on the same barrier, dP(g+2) has waited for dQ(g).
+  uint64_t ds_full[2];
   uint64_t sched_full[2], sched_empty[2], sched_go;
   DqItem items[2];
 };
@@ -221,6 +224,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
     init_barriers(bars, C::kStagesK, 2, 1);
     mbar_init(&xb->q_free, 1 + kComputeWarps);
     for (int i = 0; i < 2; ++i) {
+      mbar_init(&xb->ds_full[i], kComputeWarps);
       mbar_init(&xb->sched_full[i], 1);
       mbar_init(&xb->sched_empty[i], kDqReaders);
     }
@@ -396,7 +400,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
         for (int j = 0; ok && j < nb; ++j) {
           const int g = G + j, s = g % C::kStagesK;
           // dS(g) written implies that K(g) has landed: S(g) read it, and the elementwise warps have seen S(g)
-          if (!(ok = mbar_wait(&bars->ds_full, g & 1, ctx))) break;
+          if (!(ok = mbar_wait(&xb->ds_full[g & 1], (g >> 1) & 1, ctx))) break;
           if (fix_k_tail && j == nb - 1) {
             if (!(ok = mbar_wait(&bars->tail_fixed[nf & 1], (nf >> 1) & 1, ctx))) break;
             ++nf;
@@ -475,7 +479,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
           }
         }
         tmem_st16(tmem_base + lane_base + kColPacked + (g & 1) * 64 + cq * 16, pk);
-        warp_arrive(&bars->ds_full, lane);
+        warp_arrive(&xb->ds_full[g & 1], lane);
       }
       if (!ok) break;
       // ---- epilogue: dQ = scale * acc ----

@@ -297,6 +297,49 @@ def test_run_to_run_determinism(ext):
 
 
 @pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("b,sq,sk,h,hk,causal", [
+    (2, 897, 1024, 4, 4, False),   # items of eight whole key blocks, a ragged last Q tile
+    (1, 2048, 2048, 16, 4, True),  # items of one block up to sixteen
+    (3, 197, 197, 12, 12, False),  # fewer items than SMs
+    (40, 130, 260, 8, 2, True),    # several items per SM, each of three blocks or fewer
+])
+def test_repeated_launches_are_bit_identical(ext, d, b, sq, sk, h, hk, causal):
+    # No accumulation order depends on timing, so a hand-over that does (a product issued before its operand is whole) shows as a
+    # difference between launches: rarely in one of them, hence 200, back to back.
+    q, k, v, dout = _inputs(511 + sq, b, sq, sk, h, hk, d)
+    qd, kd, vd, dd = (x.to(DEV) for x in (q, k, v, dout))
+    scale = d ** -0.5
+    out, lse = ext.fwd(qd, kd, vd, scale, causal)
+    first = [out, lse, *ext.bwd(qd, kd, vd, out, lse, dd, scale, causal)]
+    differ = torch.zeros(5, dtype=torch.int64, device=DEV)
+    for _ in range(200):
+        o, l = ext.fwd(qd, kd, vd, scale, causal)
+        again = [o, l, *ext.bwd(qd, kd, vd, out, lse, dd, scale, causal)]
+        differ += torch.stack([(x != y).any() for x, y in zip(again, first)])
+    assert differ.tolist() == [0] * 5
+    refs = (orc.attention_forward(q, k, v, scale, causal)[0], *orc.attention_backward(q, k, v, dout, scale, causal))
+    em = emulate_reference_kernel(q, k, v, dout, scale, causal)
+    for name, got, want, emul in zip(("O", "dQ", "dK", "dV"), [first[0], *first[2:]], refs, (em.out, em.dq, em.dk, em.dv)):
+        _check(name, got, want, emul)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("h,hk,causal", [(8, 8, True), (8, 2, True), (8, 2, False)])
+def test_repeated_packed_launches_are_bit_identical(ext, d, h, hk, causal):
+    lens_q = [130, 1, 640, 257, 129, 40, 1500, 384] * 3
+    lens_k = [130, 300, 640, 129, 257, 1, 1500, 300] * 3
+    q, k, v, dout, cq, ck = (x.to(DEV) for x in _varlen_case(17 + d, lens_q, lens_k, h, hk, d))
+    args = (cq, ck, max(lens_q), max(lens_k), d ** -0.5, causal)
+    out, lse = ext.varlen_fwd(q, k, v, *args)
+    first = [out, *ext.varlen_bwd(q, k, v, out, lse, dout, *args)]
+    differ = torch.zeros(4, dtype=torch.int64, device=DEV)
+    for _ in range(200):
+        again = [ext.varlen_fwd(q, k, v, *args)[0], *ext.varlen_bwd(q, k, v, out, lse, dout, *args)]
+        differ += torch.stack([(x != y).any() for x, y in zip(again, first)])
+    assert differ.tolist() == [0] * 4
+
+
+@pytest.mark.parametrize("d", [64, 128])
 def test_both_backward_paths_agree(ext, d):
     # the single-kernel and the two-kernel backward compute the same sums with the same rounding points:
     # dK and dV agree bit for bit or within an ulp (different accumulation chunks), dQ within an ulp
