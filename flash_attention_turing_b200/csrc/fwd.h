@@ -10,4 +10,18 @@ namespace fa {
 // tell of them.
 int run_fwd(const FaFwdParams* p, int seqused_k_add, cudaStream_t stream, bool overlap = false, bool checked = false);
 
+#ifdef __CUDACC__
+// What a sequence of a cache holds, limited to what it can hold.  In 64 bits: a length may be any int32.
+struct CacheLength {
+  int len;
+  bool report;  // it was limited, and the host does not refuse the call for that
+};
+__device__ __forceinline__ CacheLength cache_length(int cached, int added, int capacity, bool checked) {
+  const int64_t n = static_cast<int64_t>(cached) + added;
+  if (n < 0) return {0, true};
+  if (n > capacity) return {capacity, !checked};
+  return {static_cast<int>(n), false};
+}
+#endif
+
 }  // namespace fa

@@ -147,7 +147,7 @@ __device__ __forceinline__ void make_work(const FwdKernelParams& p, int batch, i
   w.sk = varlen_k ? p.cu_seqlens_k[w.batch + 1] - w.k_off : p.seqlen_k;
   if (p.seqused_k) {
     // clamped to what the K/V tensor (or the block table) can hold; the scheduler thread reports a clamp
-    w.sk = max(0, min(p.seqused_k[w.batch] + p.seqused_k_add, p.k_capacity));
+    w.sk = cache_length(p.seqused_k[w.batch], p.seqused_k_add, p.k_capacity, p.checked).len;
   }
   w.row0 = mpair * kItemRows;
   w.bq = varlen_q ? 0 : w.batch;
@@ -285,10 +285,9 @@ fwd_kernel(const __grid_constant__ FwdKernelParams p) {
           const int sq = p.cu_seqlens_q ? p.cu_seqlens_q[batch + 1] - p.cu_seqlens_q[batch] : p.seqlen_q;
           if (mpair >= 0 && mpair * kItemRows < sq) {
             make_work<kItemRows>(p, batch, head, mpair, it);
-            if (p.seqused_k && p.status && head == 0 && mpair == 0) {
-              const int raw = p.seqused_k[batch] + p.seqused_k_add;
-              if (raw < 0 || (raw > p.k_capacity && !p.checked)) atomicOr(p.status, kStatusCapacityClamped);
-            }
+            if (p.seqused_k && p.status && head == 0 && mpair == 0 &&
+                cache_length(p.seqused_k[batch], p.seqused_k_add, p.k_capacity, p.checked).report)
+              atomicOr(p.status, kStatusCapacityClamped);
             break;
           }
           next = gridDim.x + atomicAdd(p.sched, 1);  // a spare slot: skip

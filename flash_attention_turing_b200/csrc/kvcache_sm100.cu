@@ -123,9 +123,9 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
   // ---- this CTA's token range ----
   // Lengths are clamped to the cache capacity on the device (the host does not have to read them back);
   // a clamp is reported through the status word.
-  const int len_raw = p.cache_seqlens[batch] + p.seqlen_new;
-  const int len = max(0, min(len_raw, p.capacity));
-  if (len != len_raw && (len_raw < 0 || !p.checked) && threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusCapacityClamped);
+  const CacheLength length = cache_length(p.cache_seqlens[batch], p.seqlen_new, p.capacity, p.checked);
+  const int len = length.len;
+  if (length.report && threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusCapacityClamped);
   const int n_tiles = (len + kTileTokens - 1) / kTileTokens;
   int tile_begin, tile_end;
   if (p.chunk_tiles > 0) {
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(256) append_kernel(const AppendParams p) {
     rest /= p.h_k;
     const int t = static_cast<int>(rest % p.seqlen_new);
     const int batch = static_cast<int>(rest / p.seqlen_new);
-    const int pos = p.cache_seqlens[batch] + t;
+    const int pos = static_cast<int>(static_cast<uint32_t>(p.cache_seqlens[batch]) + t);  // past 2^31: negative, not written
     int64_t blk, row;
     if (p.block_table) {
       const int slot = pos / p.seqlen_cache;

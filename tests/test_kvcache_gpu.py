@@ -373,3 +373,31 @@ def test_lengths_beyond_the_capacity_write_nothing(ext, b, sq, new, d, capacity,
         for i, (out, k, v) in enumerate(pool.map(step, range(16))):
             assert torch.equal(k, k0 if i % 2 else kw) and torch.equal(v, v0 if i % 2 else vw)
             assert out is None or (torch.equal(out[0], want[0]) and torch.equal(out[1], want[1]))
+
+
+@pytest.mark.parametrize("sq,new", [(1, 1), (2, 2), (64, 64)])  # decode kernel, tiled kernel
+def test_lengths_near_the_largest_int_do_not_wrap_around(ext, sq, new):
+    """cache_seqlens + seqlen_new past 2^31 is beyond the capacity, not negative: refused without a mark in the status word, or
+    with HOST_CAPACITY_CHECK off clamped to the capacity like any other length."""
+    from flash_attention_turing_b200 import flash_attention_interface as iface
+
+    gen = torch.Generator().manual_seed(sq)
+    b, h, hk, d, cap = 2, 4, 2, 64, 256
+    q, kn, vn = (randn_half(gen, b, n, x, d).to(DEV) for n, x in ((sq, h), (new, hk), (new, hk)))
+    kc, vc = randn_half(gen, b, cap, hk, d).to(DEV), randn_half(gen, b, cap, hk, d).to(DEV)
+    k0, v0 = kc.clone(), vc.clone()
+    lens = torch.tensor([100, 2 ** 31 - 1], dtype=torch.int32, device=DEV)
+    with pytest.raises(ValueError, match="cache capacity is insufficient"):
+        iface.flash_attn_with_kvcache(q, kc, vc, kn, vn, cache_seqlens=lens, causal=True)
+    assert ext.device_status(False) == 0
+    assert torch.equal(kc, k0) and torch.equal(vc, v0)
+    want = iface.flash_attn_with_kvcache(q[1:], k0[1:], v0[1:], cache_seqlens=cap, causal=True)
+    iface.HOST_CAPACITY_CHECK = False
+    try:
+        out = iface.flash_attn_with_kvcache(q, kc, vc, kn, vn, cache_seqlens=lens, causal=True)
+        status = ext.device_status(True)
+    finally:
+        iface.HOST_CAPACITY_CHECK = True
+    assert status == 2
+    assert torch.equal(kc[1], k0[1]) and torch.equal(vc[1], v0[1])
+    assert torch.equal(out[1:], want)
