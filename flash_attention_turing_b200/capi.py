@@ -127,6 +127,8 @@ def lib() -> C.CDLL:
             fn = getattr(l, name)
             fn.restype = C.c_int
             fn.argtypes = [C.POINTER(struct), _vp]
+        l.fa_kvcache_checked.restype = C.c_int
+        l.fa_kvcache_checked.argtypes = [C.POINTER(FaKvcacheParams), _vp, _i32, _vp]
         l.fa_combine_gather.restype = C.c_int
         l.fa_combine_gather.argtypes = [C.POINTER(FaCombineGatherParams), _vp]
         l.fa_sum_gather.restype = C.c_int

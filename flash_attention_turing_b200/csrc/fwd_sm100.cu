@@ -72,7 +72,7 @@ struct FwdKernelParams {
   const int* cu_seqlens_q;
   const int* cu_seqlens_k;
   const int* seqused_k;
-  int checked;        // the host refuses lengths beyond the capacity: not reported
+  int checked;        // the host refuses lengths beyond the capacity: neither read nor reported
   int seqused_k_add;  // added to seqused_k[b] (tokens appended to a cache in the same call)
   int k_capacity;     // upper bound for seqused_k: rows of k, or block_table columns * page_size
   const int* cache_batch_idx;
@@ -146,7 +146,7 @@ __device__ __forceinline__ void make_work(const FwdKernelParams& p, int batch, i
   w.k_off = varlen_k ? p.cu_seqlens_k[w.batch] : 0;
   w.sk = varlen_k ? p.cu_seqlens_k[w.batch + 1] - w.k_off : p.seqlen_k;
   if (p.seqused_k) {
-    // clamped to what the K/V tensor (or the block table) can hold; the scheduler thread reports a clamp
+    // limited to what the K/V tensor (or the block table) can hold; the scheduler thread reports a clamp
     w.sk = cache_length(p.seqused_k[w.batch], p.seqused_k_add, p.k_capacity, p.checked).len;
   }
   w.row0 = mpair * kItemRows;

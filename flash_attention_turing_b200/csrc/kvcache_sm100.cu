@@ -57,7 +57,7 @@ struct DecodeParams {
   int page_size;     // tokens per page (paged) or capacity per cache row (contiguous)
   int capacity;      // tokens a sequence can hold: max_blocks_per_seq * page_size, or the cache row length
   int num_splits;    // grid.x
-  int checked;       // the host refuses lengths beyond the capacity: not reported
+  int checked;       // the host refuses lengths beyond the capacity: neither read nor reported
   int chunk_tiles;   // > 0: split s owns tiles [s*chunk, (s+1)*chunk); 0: proportional ranges
   int* status;
 };

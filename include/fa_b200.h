@@ -242,9 +242,10 @@ int fa_kvcache(const FaKvcacheParams* p, fa_stream_t stream);
 
 /* fa_kvcache() for hosts that refuse a call whose lengths do not fit the cache, without a round trip to the device before  */
 /* the launches: no key or value is written unless cache_seqlens[i] + seqlen_new <= capacity for every i, and *verdict      */
-/* becomes 2 * token when all fit and 2 * token + 1 when one does not, as soon as the device has come to the call.  The     */
-/* other outputs of a refused call are undefined.  verdict: host memory that the device can write (cudaHostAlloc), not      */
-/* shared with another call in flight; token >= 0: what tells this call's answer from an older one in the same word.        */
+/* becomes 2 * token when all fit and 2 * token + 1 when one does not, as soon as the device has come to the call.  In a    */
+/* refused call a sequence that does not fit counts as empty (nothing of it is read, its rows of o are zero) and the rows of */
+/* the others are undefined.  verdict: host memory that the device can write (cudaHostAlloc), not shared with another call  */
+/* in flight; token >= 0: what tells this call's answer from an older one in the same word.                                 */
 int fa_kvcache_checked(const FaKvcacheParams* p, int32_t* verdict, int32_t token, fa_stream_t stream);
 
 /* KV-cache step for hosts that cannot allocate device memory.  No counterpart in the reference.   */

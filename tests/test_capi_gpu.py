@@ -200,6 +200,49 @@ def test_fa_kvcache_raw_paged():
     assert lib.fa_device_status(1) == 0
 
 
+@pytest.mark.parametrize("sq,new,splits", [(1, 1, 0), (1, 0, 0), (2, 2, 3), (64, 64, 0)])  # decode kernel, tiled kernel
+@pytest.mark.parametrize("page", [0, 256])
+def test_fa_kvcache_checked_reads_nothing_of_a_sequence_that_does_not_fit(sq, new, splits, page):
+    """Columns of the block table that the caller has not filled in are -1, and the cache rows behind the used ones NaN: a refused
+    call makes nothing of them, and the call that is accepted next is not affected."""
+    from flash_attention_turing_b200 import capi
+
+    lib = capi.lib()
+    b, h, hk, d, cap = 2, 4, 2, 64, 1024
+    gen = torch.Generator().manual_seed(sq)
+    rows = (b * (cap // page), page) if page else (b, cap)
+    q, kn, vn = (randn_half(gen, b, n, x, d).to(DEV) for n, x in ((sq, h), (max(new, 1), hk), (max(new, 1), hk)))
+    kc, vc = randn_half(gen, *rows, hk, d).to(DEV), randn_half(gen, *rows, hk, d).to(DEV)
+    flat_k, flat_v = kc.view(b, cap, hk, d), vc.view(b, cap, hk, d)
+    flat_k[1, 300:], flat_v[1, 300:] = float("nan"), float("nan")
+    table = torch.arange(rows[0], dtype=torch.int32, device=DEV).view(b, -1) if page else None
+    if page:
+        table[1, 2:] = -1
+    out, lse = torch.full_like(q, 7.0), torch.full((b, h, sq), 7.0, dtype=torch.float32, device=DEV)
+    word = torch.full((1,), -1, dtype=torch.int32).pin_memory()
+
+    def call(lengths, token):
+        lens = torch.tensor(lengths, dtype=torch.int32, device=DEV)
+        p = capi.kvcache_params(q, kc, vc, kn if new else None, vn if new else None, out, lse, lens, table, d ** -0.5, True, splits)
+        need = lib.fa_kvcache_workspace_bytes(ctypes.byref(p))
+        ws = torch.empty(max(int(need), 16), dtype=torch.uint8, device=DEV)
+        p.workspace, p.workspace_bytes = ws.data_ptr(), need
+        capi.check(lib.fa_kvcache_checked(ctypes.byref(p), word.data_ptr(), token, _stream()))
+        torch.cuda.synchronize()
+        return int(word[0])
+
+    before = kc.clone(), vc.clone()
+    for token, length in ((3, cap - new + 1), (4, 2 ** 31 - 1)):
+        assert call([200, length], token) == 2 * token + 1
+        assert bool((out[1] == 0).all()) and bool((lse[1] <= 0).all())
+        assert torch.equal(torch.nan_to_num(kc), torch.nan_to_num(before[0]))
+        assert torch.equal(torch.nan_to_num(vc), torch.nan_to_num(before[1]))
+    # as far as they were filled: the last accepted step of a sequence of 300 tokens
+    assert call([200, 300 - new], 5) == 10
+    assert torch.isfinite(out).all()
+    assert lib.fa_device_status(1) == 0
+
+
 def test_a_wait_that_runs_out_is_reported_and_the_context_stays_usable():
     """Failure detection without a failure: fa_selftest_wait_timeout() makes one bounded wait run out after
     2 ms (a barrier nobody arrives on, the kernels' own wait routine with a short limit).  The kernel returns by
