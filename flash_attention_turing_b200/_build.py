@@ -29,6 +29,9 @@ EXT_NAME = "_fa_b200_torch"
 EXT_PATH = PKG_DIR / f"{EXT_NAME}.so"
 
 CUDA_SOURCES = ["common.cu", "fwd_sm100.cu", "bwd_sm100.cu", "bwd_fused_sm100.cu", "kvcache_sm100.cu", "combine.cu"]
+# Ahead of the compiler's own -lstdc++, which is an archive in some installations: a second C++ runtime in the extension takes the
+# place of a part of the one torch uses, and formatting a number for an exception then crashes the process.
+CXX_RUNTIME = "-l:libstdc++.so.6"
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo", "--use_fast_math",
@@ -99,7 +102,7 @@ def build_torch_extension(force: bool = False, verbose: bool = False) -> Path:
     src = CSRC / "torch_ext.cpp"
     deps = [src, *INCLUDE.glob("*.h"), LIB_PATH]
     stamp = OBJ_DIR / "torch_ext.stamp"
-    tag = f"{torch.__version__}|{sys.version_info[:2]}"
+    tag = f"{torch.__version__}|{sys.version_info[:2]}|{CXX_RUNTIME}"
     if not force and _newer(EXT_PATH, deps) and stamp.exists() and stamp.read_text() == tag:
         return EXT_PATH
     OBJ_DIR.mkdir(exist_ok=True)
@@ -113,6 +116,7 @@ def build_torch_extension(force: bool = False, verbose: bool = False) -> Path:
         f"-D_GLIBCXX_USE_CXX11_ABI={cxx11}",
         *[f"-I{i}" for i in inc],
         str(src), "-o", str(EXT_PATH),
+        CXX_RUNTIME,
         f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
         f"-L{PKG_DIR}", "-lfa_b200",
         "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}",

@@ -47,6 +47,17 @@ def test_struct_layouts_match_the_header(tmp_path):
     assert got == want
 
 
+def test_binding_uses_the_shared_cxx_runtime():
+    """With a C++ runtime of its own (an archive linked into it) the binding crashed where it should have raised RuntimeError with
+    the library's error code: streams and locales of two runtimes were mixed."""
+    from flash_attention_turing_b200 import _build
+
+    names = subprocess.run(["nm", "-D", "--defined-only", str(_build.EXT_PATH)], capture_output=True, text=True, check=True).stdout
+    defined = {line.split()[-1] for line in names.splitlines()}
+    assert any(name.startswith("PyInit_") for name in defined)
+    assert not defined & {"_ZNSo9_M_insertIlEERSoT_", "_ZNSolsEi", "_ZNSt6locale7classicEv"}  # std::ostream, std::locale
+
+
 def test_host_side_argument_checks_need_no_gpu():
     lib = capi.lib()
     p = capi.FaFwdParams()

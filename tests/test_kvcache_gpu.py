@@ -401,3 +401,21 @@ def test_lengths_near_the_largest_int_do_not_wrap_around(ext, sq, new):
     assert status == 2
     assert torch.equal(kc[1], k0[1]) and torch.equal(vc[1], v0[1])
     assert torch.equal(out[1:], want)
+
+
+def test_errors_of_the_library_become_exceptions(ext):
+    """What only the library refuses (an address that is not a multiple of 16 bytes) comes back as RuntimeError with its code and
+    message, from each of the bindings."""
+    q = torch.randn(2 * 16 * 4 * 64 + 1, device=DEV, dtype=torch.float16)[1:].view(2, 16, 4, 64)
+    kv = torch.randn(2, 256, 4, 64, device=DEV, dtype=torch.float16)
+    lens = torch.tensor([16, 100], dtype=torch.int32, device=DEV)
+    cu = torch.tensor([0, 16, 32], dtype=torch.int32, device=DEV)
+    lse = torch.zeros(2, 4, 16, device=DEV)
+    flat = q.flatten(0, 1)
+    for call in (lambda: ext.fwd(q, kv, kv, 0.125, True),
+                 lambda: ext.bwd(q, kv, kv, q, lse, q, 0.125, True),
+                 lambda: ext.varlen_fwd(flat, flat, flat, cu, cu, 16, 16, 0.125, True),
+                 lambda: ext.fwd_kvcache(q, kv, kv, None, None, lens, None, None, None, None, None, None, None, 0.125, True, -1, -1,
+                                         0.0, True, 0)):
+        with pytest.raises(RuntimeError, match=r"failed \(-1\): .*16-byte aligned"):
+            call()
