@@ -7,6 +7,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <atomic>
 #include <vector>
 
 #include "../../include/fa_b200.h"
@@ -300,21 +301,30 @@ std::vector<at::Tensor> mha_varlen_bwd(at::Tensor q, at::Tensor k, at::Tensor v,
 
 // The word of pinned host memory in which the device answers fa_kvcache_checked(): one per thread, which waits for its answer
 // before it makes the next call.
+std::atomic<int64_t> g_verdict_words{0};  // alive in all threads
+
 struct Verdict {
   int32_t* word = nullptr;
   int32_t token = 0;
   ~Verdict() {
-    if (word) cudaFreeHost(word);
+    if (!word) return;
+    cudaFreeHost(word);
+    --g_verdict_words;
   }
   void next() {
     if (!word) {
       C10_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&word), sizeof(int32_t), cudaHostAllocPortable));
+      ++g_verdict_words;
       *word = -1;
     }
     token = (token + 1) & 0xfffff;
   }
-  // After an error the device may still write the word, so it is not used again (nor freed).
-  void abandon() { word = nullptr; }
+  // After an error of fa_kvcache_checked(), which may have launched a part of the call: waits for that, so that the word can be used
+  // again.  When the device itself has failed it is neither used nor freed any more.
+  void settle(cudaStream_t stream) {
+    py::gil_scoped_release release;
+    if (cudaStreamSynchronize(stream) != cudaSuccess) word = nullptr;
+  }
   // Waits until the device has answered; whether all lengths fit.  The stream is asked now and then, so that a failed launch or
   // device ends the wait with its error.
   bool wait(cudaStream_t stream) {
@@ -324,7 +334,7 @@ struct Verdict {
       const cudaError_t state = cudaStreamQuery(stream);
       if (state == cudaErrorNotReady) continue;
       if (state == cudaSuccess && *w >> 1 == token) break;
-      abandon();
+      if (state != cudaSuccess) word = nullptr;  // the device may still write it
       C10_CUDA_CHECK(state);
       TORCH_CHECK(false, "fa_kvcache_checked gave no answer");
     }
@@ -470,7 +480,7 @@ std::vector<at::Tensor> kvcache_forward(Verdict* checked, at::Tensor q, at::Tens
   if (checked) {
     checked->next();
     const int rc = fa_kvcache_checked(&p, checked->word, checked->token, current_stream());
-    if (rc != FA_OK) checked->abandon();
+    if (rc != FA_OK) checked->settle(at::cuda::getCurrentCUDAStream().stream());
     check_rc(rc, "fa_kvcache_checked");
   } else {
     check_rc(fa_kvcache(&p, current_stream()), "fa_kvcache");
@@ -632,6 +642,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("dq") = py::none(), py::arg("dk") = py::none(), py::arg("dv") = py::none());
   m.def("fwd_kvcache", &mha_fwd_kvcache, "KV-cache forward pass");
   m.def("fwd_kvcache_checked", &fwd_kvcache_checked, "KV-cache forward pass that refuses lengths beyond the capacity");
+  m.def("kvcache_answer_words", [] { return g_verdict_words.load(); },
+        "Pinned words that fwd_kvcache_checked holds: one per thread that called it and is alive");
   m.def("combine", &combine, "Merge split partials (O fp32, LSE) with log-sum-exp weights");
   m.def("combine_gather", &combine_gather, "Merge per-rank partial (O fp16, LSE) read in place, peer memory allowed");
   m.def("sum_gather", &sum_gather, "Sum per-rank partial dQ (fp16) read in place, peer memory allowed", py::arg("parts"),

@@ -419,3 +419,45 @@ def test_errors_of_the_library_become_exceptions(ext):
                                          0.0, True, 0)):
         with pytest.raises(RuntimeError, match=r"failed \(-1\): .*16-byte aligned"):
             call()
+
+
+def test_refused_arguments_cost_no_answer_word(ext):
+    """Each thread has one word for the device's answer.  A call that is refused for its arguments, before or after the append kernel
+    was launched, keeps it, and it goes with its thread."""
+    import time
+    from concurrent.futures import ThreadPoolExecutor
+
+    from flash_attention_turing_b200 import flash_attn_with_kvcache
+
+    torch.manual_seed(0)
+    b, h, hk, d, cap = 2, 4, 2, 64, 256
+    half = lambda *s: torch.randn(*s, device=DEV, dtype=torch.float16)  # noqa: E731
+    q, kn, vn, kc, vc = half(b, 1, h, d), half(b, 1, hk, d), half(b, 1, hk, d), half(b, cap, hk, d), half(b, cap, hk, d)
+    fits = torch.tensor([100, cap - 1], dtype=torch.int32, device=DEV)
+    over = fits + 1
+
+    def call(query=q, cache=kc, lens=fits):
+        return flash_attn_with_kvcache(query, cache, vc, kn, vn, cache_seqlens=lens, causal=True)
+
+    want = call()
+    unaligned = half(b * h * d + 1)[1:].view(b, 1, h, d)  # refused before anything is launched
+    one_head = half(b, cap, 1, d).expand(b, cap, hk, d)   # refused by the attend step, behind the append kernel
+    words = ext.kvcache_answer_words()
+    for _ in range(20):
+        with pytest.raises(RuntimeError, match="16-byte aligned"):
+            call(query=unaligned)
+        with pytest.raises(RuntimeError, match="strides must be positive"):
+            call(cache=one_head)
+        for wrong in (dict(query=unaligned), dict(cache=one_head), dict(query=q.float()), {}):
+            with pytest.raises(ValueError, match="cache capacity is insufficient"):  # told of first, whatever else is wrong
+                call(lens=over, **wrong)
+        assert torch.equal(call(), want)
+    assert ext.kvcache_answer_words() == words
+
+    with ThreadPoolExecutor(4) as pool:
+        for out in pool.map(lambda _: call(), range(32)):
+            assert torch.equal(out, want)
+    deadline = time.monotonic() + 10
+    while ext.kvcache_answer_words() != words and time.monotonic() < deadline:
+        time.sleep(0.01)
+    assert ext.kvcache_answer_words() == words
