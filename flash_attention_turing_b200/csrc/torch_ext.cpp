@@ -306,6 +306,7 @@ std::atomic<int64_t> g_verdict_words{0};  // alive in all threads
 struct Verdict {
   int32_t* word = nullptr;
   int32_t token = 0;
+  bool refused_by_host = true;  // no error of the current call came from the device or from a launch
   ~Verdict() {
     if (!word) return;
     cudaFreeHost(word);
@@ -480,6 +481,7 @@ std::vector<at::Tensor> kvcache_forward(Verdict* checked, at::Tensor q, at::Tens
   if (checked) {
     checked->next();
     const int rc = fa_kvcache_checked(&p, checked->word, checked->token, current_stream());
+    checked->refused_by_host = rc != FA_ERR_CUDA;
     if (rc != FA_OK) checked->settle(at::cuda::getCurrentCUDAStream().stream());
     check_rc(rc, "fa_kvcache_checked");
   } else {
@@ -503,7 +505,8 @@ std::vector<at::Tensor> mha_fwd_kvcache(at::Tensor q, at::Tensor k_cache, at::Te
 
 // fwd_kvcache that writes nothing to the cache when a length does not fit it: out, lse and whether all did.  The kernels are
 // launched first and the answer is waited for under them.  None when the call has to be checked beforehand: no work to
-// launch, or a stream that is being captured.
+// launch, a stream that is being captured, or arguments that are refused (a capacity that is insufficient is told of first, whatever
+// else is wrong).  What fails in a launch or on the device is an error of this call.
 py::object fwd_kvcache_checked(at::Tensor q, at::Tensor k_cache, at::Tensor v_cache, py::object k, py::object v,
                                at::Tensor cache_seqlens, py::object cache_batch_idx, py::object block_table,
                                double softmax_scale, bool is_causal, int64_t num_splits) {
@@ -514,9 +517,15 @@ py::object fwd_kvcache_checked(at::Tensor q, at::Tensor k_cache, at::Tensor v_ca
   C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &capture));
   if (capture != cudaStreamCaptureStatusNone) return py::none();
   static thread_local Verdict verdict;
-  const std::vector<at::Tensor> r =
-      kvcache_forward(&verdict, q, k_cache, v_cache, k, v, cache_seqlens, py::none(), py::none(), cache_batch_idx, py::none(),
-                      block_table, py::none(), py::none(), softmax_scale, is_causal, -1, -1, 0.0, true, num_splits);
+  std::vector<at::Tensor> r;
+  verdict.refused_by_host = true;
+  try {
+    r = kvcache_forward(&verdict, q, k_cache, v_cache, k, v, cache_seqlens, py::none(), py::none(), cache_batch_idx, py::none(),
+                        block_table, py::none(), py::none(), softmax_scale, is_causal, -1, -1, 0.0, true, num_splits);
+  } catch (const std::exception&) {
+    if (!verdict.refused_by_host) throw;
+    return py::none();
+  }
   bool fits;
   {
     py::gil_scoped_release release;

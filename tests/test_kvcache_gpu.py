@@ -461,3 +461,22 @@ def test_refused_arguments_cost_no_answer_word(ext):
     while ext.kvcache_answer_words() != words and time.monotonic() < deadline:
         time.sleep(0.01)
     assert ext.kvcache_answer_words() == words
+
+
+def test_an_error_behind_the_launch_is_not_hidden_by_a_second_try(ext, monkeypatch):
+    """A failed launch or an answer that never comes is an error of the call: repeating the step on the path that checks beforehand
+    would append and attend again and report nothing."""
+    from flash_attention_turing_b200 import flash_attention_interface as iface
+
+    class NoAnswer:
+        def __getattr__(self, name):
+            return getattr(ext, name)
+
+        def fwd_kvcache_checked(self, *args):
+            raise RuntimeError("fa_kvcache_checked gave no answer")
+
+    q, kv = torch.zeros(1, 1, 2, 64, device=DEV, dtype=torch.float16), torch.zeros(1, 256, 2, 64, device=DEV, dtype=torch.float16)
+    lens = torch.tensor([5], dtype=torch.int32, device=DEV)
+    monkeypatch.setattr(iface, "_gpu", NoAnswer)
+    with pytest.raises(RuntimeError, match="gave no answer"):
+        iface.flash_attn_with_kvcache(q, kv, kv.clone(), cache_seqlens=lens)
