@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(256) check_lengths_kernel(const int* lengths, 
 
 __global__ void __launch_bounds__(256) append_kernel(const AppendParams p) {
   grid_launch_dependents();
-  if (p.verdict != nullptr) {  // every block looks at all lengths: a few hundred of them at most, and no launch in between
+  if (p.verdict != nullptr) {  // every block looks at all lengths (b loads by its 256 threads, from L2 but for the first): no launch in between
     const bool fits = lengths_fit(p.cache_seqlens, p.b, p.max_length);
     if (blockIdx.x == 0 && threadIdx.x == 0) tell_host(p.verdict, p.token, fits);
     if (!fits) return;
