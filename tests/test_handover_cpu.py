@@ -1,32 +1,35 @@
-"""The hand-over of dS in the dQ kernel (bwd_dq_kernel, csrc/bwd_sm100.cu), walked through exhaustively.
+"""Two hand-overs of the kernels, walked through exhaustively: every interleaving of small models that have the kernels' waits and
+arrivals.  Barriers behave as mbarriers do: a phase ends with the last expected arrival, and a wait sees only the parity of the
+phase.  How many barriers a hand-over has is read from the kernels' source.
 
-The model has the kernel's waits and arrivals for one long item: two elementwise warps, the thread that issues S and dP, the one
-that issues dQ, and the tensor pipe, which completes each thread's products in order and as late as it likes.  Barriers behave as
-mbarriers do: a phase ends with the last expected arrival, and a wait sees only the parity of the phase.  Every interleaving is
-visited.  The number of ds_full barriers is read from the kernel's source.
+dS in the dQ kernel (bwd_dq_kernel, csrc/bwd_sm100.cu), one long item: two elementwise warps, the thread that issues S and dP, the
+one that issues dQ, and the tensor pipe, which completes each thread's products in order and as late as it likes.
+
+The zeroed tail of V in the forward (fwd_kernel, csrc/fwd_sm100.cu), short items that all need it: the producer warp, the thread that
+issues the products, and the tensor pipe.
 """
 import re
 from pathlib import Path
 
 import pytest
 
-SOURCE = Path(__file__).resolve().parents[1] / "flash_attention_turing_b200" / "csrc" / "bwd_sm100.cu"
+CSRC = Path(__file__).resolve().parents[1] / "flash_attention_turing_b200" / "csrc"
 WARPS = 2
 BLOCKS = 6
+ITEMS = 6
 
 
-def _ds_full_barriers():
-    text = SOURCE.read_text()
-    fields = re.search(r"struct DqBarriers \{(.*?)\n\};", text, re.S).group(1)
-    own = re.search(r"\bds_full\[(\d+)\]", fields)
-    return int(own.group(1)) if own else 1
+def _barriers(source, struct, name):
+    fields = re.search(rf"struct {struct} \{{(.*?)\n\}};", (CSRC / source).read_text(), re.S).group(1)
+    several = re.search(rf"\b{name}\[(\d+)\]", fields)
+    return int(several.group(1)) if several else 1
 
 
 class _Fault(Exception):
     pass
 
 
-def _walk(n_ds):
+def _walk_dq(n_ds):
     """Visits all states; raises _Fault for a product on a packed-dS buffer that is not whole, or for a state without a way on."""
     # barriers: name -> (index in the state, arrivals per phase)
     names = ["dp_full", "s_loaded", "ds_free0", "ds_free1"] + [f"ds_full{i}" for i in range(n_ds)]
@@ -100,10 +103,46 @@ def _walk(n_ds):
     return len(seen)
 
 
-def test_no_interleaving_breaks_the_hand_over():
-    assert _walk(_ds_full_barriers()) > 100
+def _walk_v_tail(n_fixed):
+    """Items of one block, the shortest way from one tail to the next.  The loads and the zeroing are the producer's step itself."""
+    # barriers with one arrival a phase: the number of phases completed
+    start = (0, 0, 0, (0,) * n_fixed, 0)  # producer item, issuing thread (2 * item + step), S products in flight, phases
+    seen, todo = {start}, [start]
+    while todo:
+        item, issue, flying, fixed, q_empty = todo.pop()
+        nexts = []
+        # wait for q_empty of the item before, load Q, K and V, zero the tail, arrive
+        if item < ITEMS and (item == 0 or q_empty % 2 != (item - 1) % 2) and item <= issue // 2 + 1:  # two items are published
+            u = item % n_fixed
+            nexts.append((item + 1, issue, flying, fixed[:u] + (fixed[u] + 1,) + fixed[u + 1:], q_empty))
+        n, step = divmod(issue, 2)
+        if n < ITEMS:
+            if step == 0 and item > n:  # the tiles are there: issue S, commit q_empty
+                nexts.append((item, issue + 1, flying + 1, fixed, q_empty))
+            elif step == 1 and fixed[n % n_fixed] % 2 != (n // n_fixed) % 2:  # issue PV
+                if fixed[n % n_fixed] <= n // n_fixed:
+                    raise _Fault(f"PV of item {n} issued on a tail that is not zeroed")
+                nexts.append((item, issue + 1, flying, fixed, q_empty))
+        if flying:
+            nexts.append((item, issue, flying - 1, fixed, q_empty + 1))
+        if not nexts and n < ITEMS:
+            raise _Fault(f"stuck: item {n} waits for its tail, the producer is at item {item}")
+        for s in nexts:
+            if s not in seen:
+                seen.add(s)
+                todo.append(s)
+    return len(seen)
 
 
-def test_one_barrier_for_all_blocks_would_not_do():
+HANDOVERS = [(_walk_dq, "bwd_sm100.cu", "DqBarriers", "ds_full"), (_walk_v_tail, "fwd_sm100.cu", "Barriers", "v_fixed")]
+
+
+@pytest.mark.parametrize("walk,source,struct,name", HANDOVERS)
+def test_no_interleaving_breaks_the_hand_over(walk, source, struct, name):
+    assert walk(_barriers(source, struct, name)) > 20
+
+
+@pytest.mark.parametrize("walk,source,struct,name", HANDOVERS)
+def test_one_barrier_would_not_do(walk, source, struct, name):
     with pytest.raises(_Fault):
-        _walk(1)
+        walk(1)
