@@ -41,6 +41,8 @@ struct BwdKernelParams {
   int items_x;      // dense: 128-row Q tiles per (sequence, head)
   int total_items;  // dense: items_x * h * b; packed sequences: h * (total_q / 128 + b)
   int b;
+  int section_rows;  // see section_item()
+  int group;         // query heads per key head
 };
 
 // Launchers of the single-kernel backward (bwd_fused_sm100.cu), called from fa_bwd_stages().

@@ -33,6 +33,7 @@
 #include <algorithm>
 
 #include "packed_rows.cuh"
+#include "work_order.cuh"
 
 namespace fa {
 namespace {
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 // =============================================================================================
 // A work item is one 128-row Q tile of one (sequence, query head): S = Q K^T and dP = dO V^T per key block (SS),
 // P and dS in the elementwise warps, dQ += dS K (TS, A = packed dS in TMEM, two alternating buffers).  The kernel
-// is persistent: one CTA per SM takes items from a global counter (heaviest causal tile of a head first) and
+// is persistent: one CTA per SM takes items from a global counter (heaviest causal tiles first, see section_item()) and
 // keeps its barriers, its TMEM allocation and the K / V rings across items: every barrier phase is derived from
 // the cumulative block count G (or the item count), the Q / dO tiles and the row statistics of the next item are
 // loaded as soon as the current item has read its own for the last time, and the first S product of the next
@@ -193,7 +194,7 @@ __device__ __forceinline__ void dq_make_item(const BwdKernelParams& p, int batch
   w.sk = varlen ? p.cu_seqlens_k[batch + 1] - w.k_off : p.seqlen_k;
   w.row0 = mblk * kBlock;
   w.bq = varlen ? 0 : batch;
-  w.head_k = head / (p.h / p.h_k);
+  w.head_k = head / p.group;
   const int nkb = (w.sk + kBlock - 1) / kBlock;
   w.shift = (p.is_causal == 2) ? p.causal_shift : w.sk - w.sq;
   w.nb = nkb;
@@ -265,15 +266,18 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
         while (next < p.total_items) {
           int batch, head, mblk, sq;
           if (p.cu_seqlens_q == nullptr) {
-            const int x = next % p.items_x, rest = next / p.items_x;
-            head = rest % p.h, batch = rest / p.h, mblk = p.items_x - 1 - x, sq = p.seqlen_q;
+            const HeadPlace at = section_item(next, p.h * p.b, p.items_x, p.group, p.seqlen_k, p.section_rows);
+            batch = at.head / p.h, head = at.head - batch * p.h, mblk = p.items_x - 1 - at.place, sq = p.seqlen_q;
           } else {  // slots per sequence from cu_seqlens_q / 128 (at most one spare slot per sequence and head)
             while (seq + 1 < p.b && p.h * ((p.cu_seqlens_q[seq + 1] >> 7) + seq + 1) <= next) ++seq;
             const int v0 = (p.cu_seqlens_q[seq] >> 7) + seq, v1 = (p.cu_seqlens_q[seq + 1] >> 7) + seq + 1;
             const int rel = next - p.h * v0, cnt = v1 - v0;
             sq = p.cu_seqlens_q[seq + 1] - p.cu_seqlens_q[seq];
-            batch = seq, head = rel / cnt, mblk = (sq + kBlock - 1) / kBlock - 1 - rel % cnt;
-            if (rel < 0 || head >= p.h) mblk = -1;  // before the first sequence (cu_seqlens_q[0] >= 128), past the last one
+            batch = seq, head = 0, mblk = -1;
+            if (rel >= 0 && rel < p.h * cnt) {  // else before the first sequence (cu_seqlens_q[0] >= 128) or past the last one
+              const HeadPlace at = section_item(rel, p.h, cnt, p.group, p.cu_seqlens_k[seq + 1] - p.cu_seqlens_k[seq], p.section_rows);
+              head = at.head, mblk = (sq + kBlock - 1) / kBlock - 1 - at.place;
+            }
           }
           if (mblk >= 0 && mblk * kBlock < sq) {
             dq_make_item(p, batch, head, mblk, it);
@@ -533,7 +537,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
 // A work item is one 128-key tile of one (sequence, KV head): the CTA loops over the query heads of the GQA group
 // and their Q tiles (iterations), S^T = K Q^T and dP^T = V dO^T per iteration (SS), P^T and dS^T in the elementwise
 // warps, dV += P^T dO and dK += dS^T Q (TS) accumulated in TMEM over the whole group.  Persistent like the dQ
-// kernel: one CTA per SM takes items from the work counter (heaviest causal key tile first), every barrier phase
+// kernel: one CTA per SM takes items from the work counter (heaviest causal key tiles first), every barrier phase
 // is derived from the cumulative iteration count T (or the item count), the K / V tiles of the next item are
 // loaded as soon as the last dP^T product of the current item has read them, and its first S^T product is issued
 // under the last elementwise iteration and the epilogue of the current one.  Bound by the chain of a tile through the sixteen
@@ -570,7 +574,7 @@ __device__ __forceinline__ DkvWork dkv_decode(const BwdKernelParams& p, const Dk
   w.sq = kVarlen ? it.sq : p.seqlen_q;
   w.sk = kVarlen ? it.sk : p.seqlen_k;
   w.key0 = it.nblk * kBlock;
-  w.group = p.h / p.h_k;
+  w.group = p.group;
   w.nq = (w.sq + kBlock - 1) / kBlock;
   w.i_min = 0;
   w.shift = (p.is_causal == 2) ? p.causal_shift : w.sk - w.sq;  // key j visible to query i iff j <= i + shift
@@ -653,8 +657,8 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
         it.sq = p.seqlen_q, it.sk = p.seqlen_k;
         if constexpr (!kVarlen) {
           if (next < p.total_items) {  // every index is a live item: key tile 0 of a head is the heaviest
-            const int x = next % p.items_x, rest = next / p.items_x;
-            it.head_k = rest % p.h_k, it.batch = rest / p.h_k, it.nblk = x;
+            const HeadPlace at = section_item(next, p.h_k * p.b, p.items_x, 1, p.seqlen_q, p.section_rows);
+            it.batch = at.head / p.h_k, it.head_k = at.head - it.batch * p.h_k, it.nblk = at.place;
           }
         } else {
           while (next < p.total_items) {  // slots per sequence from cu_seqlens_k / 128 (see the forward kernel)
@@ -662,13 +666,15 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
             const int k0 = p.cu_seqlens_k[seq], k1 = p.cu_seqlens_k[seq + 1];
             const int v0 = (k0 >> 7) + seq, v1 = (k1 >> 7) + seq + 1;
             const int rel = next - p.h_k * v0, cnt = v1 - v0;
-            const int x = rel % cnt;
-            // items_x: key tiles up to the maximum the caller gave; later ones are not computed
-            if (rel >= 0 && rel / cnt < p.h_k && x < p.items_x && x * kBlock < k1 - k0) {
-              it.batch = seq, it.head_k = rel / cnt, it.nblk = x;
+            if (rel >= 0 && rel < p.h_k * cnt) {
               it.q_off = p.cu_seqlens_q[seq], it.sq = p.cu_seqlens_q[seq + 1] - it.q_off;
-              it.k_off = k0, it.sk = k1 - k0;
-              break;
+              const HeadPlace at = section_item(rel, p.h_k, cnt, 1, it.sq, p.section_rows);
+              // items_x: key tiles up to the maximum the caller gave; later ones are not computed
+              if (at.place < p.items_x && at.place * kBlock < k1 - k0) {
+                it.batch = seq, it.head_k = at.head, it.nblk = at.place;
+                it.k_off = k0, it.sk = k1 - k0;
+                break;
+              }
             }
             next = gridDim.x + atomicAdd(p.sched, 1);
           }
@@ -1074,19 +1080,19 @@ bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
   static_assert(kColDPT<D> == kColS && !C::kStatsWithQ, "S^T and dP^T share a region, the statistics have a ring of their own");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int batch = sequence_by_size(p.cu_seqlens_q, p.cu_seqlens_k, p.b, blockIdx.z);
-  const int head_k = blockIdx.y, nblk = blockIdx.x;
+  const int nblk = blockIdx.x / p.h_k, head_k = blockIdx.x - nblk * p.h_k;  // the heaviest key tiles of all heads first
   const int q_off = p.cu_seqlens_q[batch];
   const int sq = p.cu_seqlens_q[batch + 1] - q_off;
   const int k_off = p.cu_seqlens_k[batch];
   const int sk = p.cu_seqlens_k[batch + 1] - k_off;
   const int key0 = nblk * kBlock;
-  const bool first_cta = (blockIdx.x | blockIdx.y | blockIdx.z) == 0;
+  const bool first_cta = (blockIdx.x | blockIdx.z) == 0;
   if (key0 >= sk) {
     if (first_cta) grid_dependency_wait();
     return;
   }
   const int stop_probe = stop_probe_begin(p.status);
-  const int group = p.h / p.h_k;
+  const int group = p.group;
   const int nq = (sq + kBlock - 1) / kBlock;
   int i_min = 0;
   const int shift = sk - sq;  // key j visible to query i iff j <= i + shift (FA_CAUSAL_SHIFT is for dense batches)
@@ -1445,6 +1451,7 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
     if (sms <= 0 || kq.sched == nullptr) return set_error(FA_ERR_CUDA, "fa_bwd: device attributes not available");
     kq.items_x = (p->seqlen_q + kBlock - 1) / kBlock;
     kq.b = p->b;
+    kq.section_rows = section_rows(p->is_causal != 0, 4 * p->d);
     const int64_t total = kq.cu_seqlens_q ? static_cast<int64_t>(p->h) * (p->total_q / kBlock + p->b)
                                           : static_cast<int64_t>(kq.items_x) * p->h * p->b;
     FA_CHECK_ARG(total < (1ll << 30), "fa_bwd: too many work items");
@@ -1468,7 +1475,7 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
     const bool overlap = (stage_mask & 2) != 0 && !gradients_over_keys(p);
     if (D == 128 && kp.cu_seqlens_q != nullptr && p->h != p->h_k) {  // one CTA per key tile: see bwd_dkdv_packed_kernel
       if constexpr (D == 128) {
-        dim3 grid_k((p->seqlen_k + kBlock - 1) / kBlock, p->h_k, p->b);
+        dim3 grid_k((p->seqlen_k + kBlock - 1) / kBlock * p->h_k, 1, p->b);
         if (overlap) {
           FA_CHECK_CUDA(launch_overlapped(bwd_dkdv_packed_kernel, grid_k, kNumThreads, C::kSmemBytesDkdv, stream, kp));
         } else {
@@ -1482,6 +1489,7 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
       if (sms <= 0 || kk.sched == nullptr) return set_error(FA_ERR_CUDA, "fa_bwd: device attributes not available");
       kk.items_x = (p->seqlen_k + kBlock - 1) / kBlock;
       kk.b = p->b;
+      kk.section_rows = section_rows(p->is_causal != 0, 4 * p->d * kp.group);
       const int64_t total = kk.cu_seqlens_k ? static_cast<int64_t>(p->h_k) * (p->total_k / kBlock + p->b)
                                             : static_cast<int64_t>(kk.items_x) * p->h_k * p->b;
       FA_CHECK_ARG(total < (1ll << 30), "fa_bwd: too many work items");
@@ -1628,6 +1636,7 @@ extern "C" int fa_bwd_stages(const FaBwdParams* p, int stage_mask, fa_stream_t s
   kp.lse2 = lse2;
   kp.sq_pad = sq_pad;
   kp.seqlen_q = p->seqlen_q; kp.seqlen_k = p->seqlen_k; kp.h = p->h; kp.h_k = p->h_k;
+  kp.group = p->h / p->h_k;
   kp.scale = p->softmax_scale;
   kp.scale_log2 = p->softmax_scale * kLog2e;
   kp.is_causal = p->is_causal;

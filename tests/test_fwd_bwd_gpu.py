@@ -1055,3 +1055,31 @@ def test_key_gradients_past_the_given_maximum_are_zero(ext, d, lens, max_k):
             assert torch.equal(got[first:first + min(n, written)], want[first:first + min(n, written)])
             assert (got[first + min(n, written):first + n] == 0).all()
             first += n
+
+
+@pytest.mark.parametrize("d,lens,h,hk", [(128, (2048,) * 5, 7, 7), (128, (4096,) * 3, 18, 9), (64, (4096,) * 5, 14, 14),
+                                         (128, (300, 8192, 5000), 18, 9), (64, (16384, 129), 9, 9)])
+def test_heads_of_several_sections_equal_heads_by_themselves(ext, d, lens, h, hk):
+    """More heads than one section of the work order holds, and a last section that is not full: every item runs once and its
+    result does not depend on the others (bitwise)."""
+    gen = torch.Generator(device=DEV).manual_seed(21)
+    total, group, scale = sum(lens), h // hk, d ** -0.5
+    q, k, v, dout = (torch.randn(total, n, d, generator=gen, device=DEV, dtype=torch.half) for n in (h, hk, hk, h))
+    cu = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0, dtype=torch.int32).to(DEV)
+
+    def run(kv_heads):
+        heads = slice(kv_heads.start * group, kv_heads.stop * group)
+        qq, kk, vv, dd = q[:, heads], k[:, kv_heads], v[:, kv_heads], dout[:, heads]
+        if len(set(lens)) > 1:
+            args = (cu, cu, max(lens), max(lens), scale, True)
+            out, lse = ext.varlen_fwd(qq, kk, vv, *args)
+            return out, *ext.varlen_bwd(qq, kk, vv, out, lse, dd, *args)
+        qq, kk, vv, dd = (x.unflatten(0, (len(lens), -1)) for x in (qq, kk, vv, dd))
+        out, lse = ext.fwd(qq, kk, vv, scale, True)
+        return tuple(x.flatten(0, 1) for x in (out, *ext.bwd(qq, kk, vv, out, lse, dd, scale, True)))
+
+    got = run(slice(0, hk))
+    for i in range(hk):
+        for x, want in zip(got, run(slice(i, i + 1))):
+            n = want.shape[1]
+            assert torch.equal(x[:, i * n:(i + 1) * n], want)
