@@ -153,13 +153,12 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 // before the current one ends; the scheduler thread derives everything the roles need from it once and leaves it in
 // shared memory (decoding it in five roles was code the instruction cache had to hold).
 //
-// Bound by the issue of its products: 16 SS MMAs of about 88 clocks and 8 TS MMAs of about 75, of 1536 clocks at the tensor peak.
-// Its two issuing loops run under lane == 0 and not under elect_one() as elsewhere (which was measured, and 7-9 % faster, when ds_full
-// was one barrier and its results were wrong now and then).  S and dP of a block are issued back
+// Bound by its products (1536 clocks a block at the tensor peak) and, above S = 4096, by the power cap.  Under elect_one() against
+// lane == 0 the issuing loops took B4 S4096 H32 D128 792 -> 728 us, S8192 2835 -> 2614, 64 texts H16 D64 110 -> 103.  S and dP of a block are issued back
 // to back, fetched into registers together and handed back together, so that the whole arithmetic of the block runs
 // under the next S / dP: ONE wait and one hand-back per block where waiting for S and dP in turn took two of each, at
 // 150-300 clocks apiece for warps in lock-step.  The hand-back has to leave before the arithmetic starts (see
-// schedule_barrier: without it 40 % slower, 267 against 188 us at B2 S4096 H16 D128 causal).  Measured per 128 x 128 block at B4 S8192 H32 D128 causal: 2511 -> 2226 clocks;
+// schedule_barrier: without it 40 % slower, 267 against 188 us at B2 S4096 H16 D128 causal).  Measured (loops under lane == 0) per 128 x 128 block at B4 S8192 H32 D128 causal: 2511 -> 2226 clocks;
 // launch, SM clocks: D128 S8192 4520 -> 4005 k, D128 S1024 462 -> 436 k, D64 S16384 3417 -> 3189 k.
 constexpr int kDqThreads = 640;
 constexpr int kDqSchedWarp = 19;
@@ -355,7 +354,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       ++ni;
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_nn = make_idesc_f16(128, kBlock, false, false);
       const uint32_t q_addr = smem_u32(sQ), do_addr = smem_u32(sdO);
       auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, ctx); };
@@ -393,7 +392,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       }
     }
   } else if (warp == kAccMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_acc = make_idesc_f16(128, D, false, true);
       int G = 0, nf = 0;
       bool ok = true;

@@ -31,10 +31,10 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 
-// One lane of a converged warp.  The loops that issue tcgen05.mma run under this and not under `lane == 0` (but see the dQ kernel):
+// One lane of a converged warp.  The loops that issue tcgen05.mma run under this and not under `lane == 0`:
 // only with elect.sync does the compiler know that a single thread is active, which the instruction's uniform operands need.  Same
 // loops, `lane == 0` against this: forward B4 S8192 H32 D128 causal 2247 -> 2069 us, B16 S1024 230 -> 211 us, 64 texts of 130-640
-// tokens (H16 D64) 114.6 -> 101.7 us, D = 64 S = 16384 unchanged; dK/dV 2 % and less, 4 % for the texts.
+// tokens (H16 D64) 114.6 -> 101.7 us, D = 64 S = 16384 unchanged; dK/dV 2 % and less, 4 % for the texts; dQ 6-9 %.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
