@@ -61,12 +61,13 @@ struct PreParams {
 // the threads of a block read neighbouring heads of the same rows, i.e. contiguous memory when the heads of a
 // row are adjacent, every thread has 2 * kPreRows loads in flight, and an item writes one full 32-byte sector
 // of each statistic.  grid (ceil(items / items_per_block), 1, b).
-// Bound by memory, with three blocks per SM (80 registers; the clearing code of packed calls takes 100 and is left out of the other
-// instantiation: two blocks, 98.8 instead of 82.2 us at B4 S8192 H32 D128, 5560 against 6680 GB/s).
+// Bound by memory, with three blocks per SM: 80 registers, which the clearing code of packed calls is held to as well (one spill; left
+// to itself it takes 100, two blocks).  That and the padding of short sequences left out: 16 documents of 256-4096 tokens (Hq32 D128)
+// 142 -> 112 us, 64 texts of 130-640 (H16 D64) 23.2 -> 21.1, (D128) 43.6 -> 39.5.
 constexpr int kPreRows = 8;
 static_assert(kClearThreads == 256, "the clearing threads are those of the preprocess kernel");
 template <bool kClear>
-__global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_constant__ PreParams p) {
+__global__ void __launch_bounds__(256, 3) bwd_preprocess_kernel(const __grid_constant__ PreParams p) {
   grid_launch_dependents();
   const bool stopped = kClear && wait_timed_out(p.status);  // read here, under the row loads
   const int tpr = p.d / 8;  // threads per item: 8 or 16
@@ -81,41 +82,44 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
                          head * p.o_head_stride + sub * 8;
   const int64_t do_base = (p.cu_seqlens_q ? static_cast<int64_t>(q_off) * p.do_row_stride : batch * p.do_batch_stride) +
                           head * p.do_head_stride + sub * 8;
-  uint4 a[kPreRows], b[kPreRows];
+  // the padding of a sequence much shorter than the longest: nothing reads statistics past its last 128-row tile
+  if (__any_sync(0xffffffffu, row0 < (sq + kBlock - 1) / kBlock * kBlock)) {
+    uint4 a[kPreRows], b[kPreRows];
 #pragma unroll
-  for (int i = 0; i < kPreRows; ++i) {
-    a[i] = make_uint4(0, 0, 0, 0);
-    b[i] = make_uint4(0, 0, 0, 0);
-    if (row0 + i < sq) {
-      a[i] = *reinterpret_cast<const uint4*>(p.o + o_base + static_cast<int64_t>(row0 + i) * p.o_row_stride);
-      b[i] = *reinterpret_cast<const uint4*>(p.dout + do_base + static_cast<int64_t>(row0 + i) * p.do_row_stride);
+    for (int i = 0; i < kPreRows; ++i) {
+      a[i] = make_uint4(0, 0, 0, 0);
+      b[i] = make_uint4(0, 0, 0, 0);
+      if (row0 + i < sq) {
+        a[i] = *reinterpret_cast<const uint4*>(p.o + o_base + static_cast<int64_t>(row0 + i) * p.o_row_stride);
+        b[i] = *reinterpret_cast<const uint4*>(p.dout + do_base + static_cast<int64_t>(row0 + i) * p.do_row_stride);
+      }
     }
-  }
-  // lane `sub` of the item keeps the statistics of row `sub` (sub < kPreRows <= tpr)
-  const int64_t bh = static_cast<int64_t>(batch) * p.h + head;
-  float my_lse = 0.f;
-  if (sub < kPreRows && row0 + sub < sq) my_lse = p.lse[bh * p.lse_row_stride + row0 + sub];
-  float mine = 0.f;
+    // lane `sub` of the item keeps the statistics of row `sub` (sub < kPreRows <= tpr)
+    const int64_t bh = static_cast<int64_t>(batch) * p.h + head;
+    float my_lse = 0.f;
+    if (sub < kPreRows && row0 + sub < sq) my_lse = p.lse[bh * p.lse_row_stride + row0 + sub];
+    float mine = 0.f;
 #pragma unroll
-  for (int i = 0; i < kPreRows; ++i) {
-    const __half2* ah = reinterpret_cast<const __half2*>(&a[i]);
-    const __half2* bh2 = reinterpret_cast<const __half2*>(&b[i]);
-    float acc = 0.f;
+    for (int i = 0; i < kPreRows; ++i) {
+      const __half2* ah = reinterpret_cast<const __half2*>(&a[i]);
+      const __half2* bh2 = reinterpret_cast<const __half2*>(&b[i]);
+      float acc = 0.f;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 x = __half22float2(ah[k]), y = __half22float2(bh2[k]);
-      acc = fmaf(x.x, y.x, acc);
-      acc = fmaf(x.y, y.y, acc);
+      for (int k = 0; k < 4; ++k) {
+        const float2 x = __half22float2(ah[k]), y = __half22float2(bh2[k]);
+        acc = fmaf(x.x, y.x, acc);
+        acc = fmaf(x.y, y.y, acc);
+      }
+      // sum over the tpr (8 or 16) consecutive lanes of the item; every lane ends up with the total
+      for (int off = tpr / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+      if (sub == i) mine = acc;
     }
-    // sum over the tpr (8 or 16) consecutive lanes of the item; every lane ends up with the total
-    for (int off = tpr / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (sub == i) mine = acc;
-  }
-  if (sub < kPreRows && row0 + sub < p.sq_pad) {
-    const int64_t idx = bh * p.sq_pad + row0 + sub;
-    const bool valid = row0 + sub < sq;
-    p.delta[idx] = valid ? -mine : 0.f;
-    p.lse2[idx] = valid ? -my_lse * kLog2e : -INFINITY;
+    if (sub < kPreRows && row0 + sub < p.sq_pad) {
+      const int64_t idx = bh * p.sq_pad + row0 + sub;
+      const bool valid = row0 + sub < sq;
+      p.delta[idx] = valid ? -mine : 0.f;
+      p.lse2[idx] = valid ? -my_lse * kLog2e : -INFINITY;
+    }
   }
   if constexpr (kClear) {  // the other kernels write all other rows of dq, dk, dv
     // The blocks of all sequences share the unused rows: those of one sequence are too few when the buffer is much larger than
