@@ -244,24 +244,33 @@ class FlashAttnVarlenKVPackedFunc(torch.autograd.Function):
 # --------------------------------------------------------------------------------------------
 # public functions (reference :448-614)
 # --------------------------------------------------------------------------------------------
+# Ordinary calls go to the native autograd node of the binding, which is the same forward and backward without the round trips
+# through Python; it returns None for what only the classes above answer (functorch transforms, forward-mode AD, tracing, modes,
+# tensor subclasses, CPU tensors and other inputs that are refused).
+_SEPARATE, _KV_PACKED, _QKV_PACKED = 0, 1, 2
+
+
 def flash_attn_func(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, softmax_scale: Optional[float] = None,
                     causal: bool = False) -> torch.Tensor:
     """q (batch, seqlen_q, nheads, d); k, v (batch, seqlen_k, nheads_k, d) -> out like q.
     nheads must be a multiple of nheads_k (GQA/MQA); d is 64 or 128; fp16.  ``causal`` masks with
     bottom-right alignment.  ``softmax_scale`` defaults to d ** -0.5."""
-    return FlashAttnFunc.apply(q, k, v, softmax_scale, causal, torch.is_grad_enabled())
+    out = _gpu().attention_dense(_SEPARATE, q, k, v, softmax_scale, causal)
+    return FlashAttnFunc.apply(q, k, v, softmax_scale, causal, torch.is_grad_enabled()) if out is None else out
 
 
 def flash_attn_qkvpacked_func(qkv: torch.Tensor, softmax_scale: Optional[float] = None,
                               causal: bool = False) -> torch.Tensor:
     """qkv (batch, seqlen, 3, nheads, d) -> out (batch, seqlen, nheads, d)."""
-    return FlashAttnQKVPackedFunc.apply(qkv, softmax_scale, causal, torch.is_grad_enabled())
+    out = _gpu().attention_dense(_QKV_PACKED, qkv, None, None, softmax_scale, causal)
+    return FlashAttnQKVPackedFunc.apply(qkv, softmax_scale, causal, torch.is_grad_enabled()) if out is None else out
 
 
 def flash_attn_kvpacked_func(q: torch.Tensor, kv: torch.Tensor, softmax_scale: Optional[float] = None,
                              causal: bool = False) -> torch.Tensor:
     """q (batch, seqlen_q, nheads, d); kv (batch, seqlen_k, 2, nheads_k, d) -> out like q."""
-    return FlashAttnKVPackedFunc.apply(q, kv, softmax_scale, causal, torch.is_grad_enabled())
+    out = _gpu().attention_dense(_KV_PACKED, q, kv, None, softmax_scale, causal)
+    return FlashAttnKVPackedFunc.apply(q, kv, softmax_scale, causal, torch.is_grad_enabled()) if out is None else out
 
 
 def flash_attn_varlen_func(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens_q: torch.Tensor,
@@ -269,6 +278,9 @@ def flash_attn_varlen_func(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu
                            softmax_scale: Optional[float] = None, causal: bool = False) -> torch.Tensor:
     """Packed sequences: q (total_q, nheads, d); k, v (total_k, nheads_k, d); cu_seqlens_* int32
     (batch + 1,) cumulative offsets; max_seqlen_* the longest sequence.  -> out (total_q, nheads, d)."""
+    out = _gpu().attention_varlen(_SEPARATE, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_scale, causal)
+    if out is not None:
+        return out
     return FlashAttnVarlenFunc.apply(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
                                      softmax_scale, causal, torch.is_grad_enabled())
 
@@ -276,6 +288,9 @@ def flash_attn_varlen_func(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu
 def flash_attn_varlen_qkvpacked_func(qkv: torch.Tensor, cu_seqlens: torch.Tensor, max_seqlen: int,
                                      softmax_scale: Optional[float] = None, causal: bool = False) -> torch.Tensor:
     """qkv (total, 3, nheads, d) with one cu_seqlens for q and k -> out (total, nheads, d)."""
+    out = _gpu().attention_varlen(_QKV_PACKED, qkv, None, None, cu_seqlens, cu_seqlens, max_seqlen, max_seqlen, softmax_scale, causal)
+    if out is not None:
+        return out
     return FlashAttnVarlenQKVPackedFunc.apply(qkv, cu_seqlens, max_seqlen, softmax_scale, causal,
                                               torch.is_grad_enabled())
 
@@ -284,6 +299,9 @@ def flash_attn_varlen_kvpacked_func(q: torch.Tensor, kv: torch.Tensor, cu_seqlen
                                     cu_seqlens_k: torch.Tensor, max_seqlen_q: int, max_seqlen_k: int,
                                     softmax_scale: Optional[float] = None, causal: bool = False) -> torch.Tensor:
     """q (total_q, nheads, d); kv (total_k, 2, nheads_k, d) -> out (total_q, nheads, d)."""
+    out = _gpu().attention_varlen(_KV_PACKED, q, kv, None, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_scale, causal)
+    if out is not None:
+        return out
     return FlashAttnVarlenKVPackedFunc.apply(q, kv, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
                                              softmax_scale, causal, torch.is_grad_enabled())
 

@@ -1083,3 +1083,91 @@ def test_heads_of_several_sections_equal_heads_by_themselves(ext, d, lens, h, hk
         for x, want in zip(got, run(slice(i, i + 1))):
             n = want.shape[1]
             assert torch.equal(x[:, i * n:(i + 1) * n], want)
+
+
+def _public_calls(d, grad):
+    """(name, native function, class, inputs, further arguments) of the six public functions with an autograd class."""
+    import flash_attention_turing_b200.flash_attention_interface as fi
+
+    gen = torch.Generator().manual_seed(5)
+    r = lambda *s: randn_half(gen, *s).to(DEV).requires_grad_(grad)  # noqa: E731
+    cu = torch.tensor([0, 70, 199], dtype=torch.int32, device=DEV)
+    dense, var = (None, True), (129, 129, None, True)
+    return [
+        ("dense", fi.flash_attn_func, fi.FlashAttnFunc, [r(2, 130, 4, d), r(2, 150, 2, d), r(2, 150, 2, d)], (), dense),
+        ("qkv", fi.flash_attn_qkvpacked_func, fi.FlashAttnQKVPackedFunc, [r(2, 130, 3, 4, d)], (), dense),
+        ("kv", fi.flash_attn_kvpacked_func, fi.FlashAttnKVPackedFunc, [r(2, 130, 4, d), r(2, 150, 2, 2, d)], (), dense),
+        ("varlen", fi.flash_attn_varlen_func, fi.FlashAttnVarlenFunc, [r(199, 4, d), r(199, 2, d), r(199, 2, d)], (cu, cu), var),
+        ("varlen qkv", fi.flash_attn_varlen_qkvpacked_func, fi.FlashAttnVarlenQKVPackedFunc, [r(199, 3, 4, d)], (cu,), var[1:]),
+        ("varlen kv", fi.flash_attn_varlen_kvpacked_func, fi.FlashAttnVarlenKVPackedFunc, [r(199, 4, d), r(199, 2, 2, d)], (cu, cu), var),
+    ]
+
+
+@pytest.mark.parametrize("which", range(6))
+@pytest.mark.parametrize("d", [64, 128])
+def test_native_autograd_node_equals_the_class(ext, d, which):
+    """Outputs, gradients, what is saved (as saved-tensor hooks see it), no gradients, a second backward, a transposed dout."""
+    _, fn, cls, inputs, extra, rest = _public_calls(d, True)[which]
+
+    def run(call, *tail):
+        seen = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append((t.shape, t.stride(), t.dtype)) or t, lambda t: t):
+            out = call(*inputs, *extra, *rest, *tail)
+        dout = torch.linspace(-1, 1, out.numel(), device=DEV).half().view(out.mT.shape).mT  # last dimension not contiguous
+        first = torch.autograd.grad(out, inputs, dout, retain_graph=True)
+        again = torch.autograd.grad(out, inputs, dout)
+        with pytest.raises(RuntimeError, match="second time"):
+            torch.autograd.grad(out, inputs, dout)
+        assert all(torch.equal(x, y) for x, y in zip(first, again))
+        return seen, (out.detach(), *first)
+
+    saved, got = run(fn)
+    saved_class, want = run(cls.apply, True)
+    assert saved == saved_class
+    assert all(torch.equal(x, y) and x.stride() == y.stride() for x, y in zip(got, want))
+    with torch.no_grad():
+        out = fn(*inputs, *extra, *rest)
+    assert not out.requires_grad and torch.equal(out, want[0])
+    # a gradient of some inputs only, and a mutated input
+    inputs[-1].requires_grad_(False)
+    if len(inputs) > 1:
+        out = fn(*inputs, *extra, *rest)
+        g = torch.autograd.grad(out, inputs[0], torch.ones_like(out), retain_graph=True)[0]
+        assert g.shape == inputs[0].shape
+        inputs[-1].add_(1)
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            torch.autograd.grad(out, inputs[0], torch.ones_like(out))
+
+
+@pytest.mark.parametrize("which", range(6))
+def test_transforms_and_modes_still_go_to_the_class(ext, which):
+    """What the native node does not know: functorch transforms and forward-mode AD are refused as by the class, a traced call is
+    recorded, a tensor subclass and a mode reach the class."""
+    from torch.overrides import TorchFunctionMode
+
+    name, fn, cls, inputs, extra, rest = _public_calls(64, False)[which]
+    call = lambda *x: fn(*x, *extra, *rest)  # noqa: E731
+    with pytest.raises(RuntimeError, match="functorch transforms"):
+        torch.func.vmap(call)(*(x[None] for x in inputs))
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(inputs[0], torch.ones_like(inputs[0]))
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            call(dual, *inputs[1:])
+    applied = []
+    real = cls.apply
+    try:
+        cls.apply = classmethod(lambda c, *a: applied.append(1) or real(*a))
+
+        class Mode(TorchFunctionMode):
+            def __torch_function__(self, func, types, args=(), kwargs=None):
+                return func(*args, **(kwargs or {}))
+
+        with Mode():
+            call(*inputs)
+        call(inputs[0].as_subclass(type("Sub", (torch.Tensor,), {})), *inputs[1:])
+        assert len(applied) == 2
+        call(*inputs)
+        assert len(applied) == 2
+    finally:
+        del cls.apply
+    assert torch.equal(call(*inputs), cls.apply(*inputs, *extra, *rest, False))
