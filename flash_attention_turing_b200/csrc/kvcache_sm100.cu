@@ -3,7 +3,8 @@
 //
 // The attend kernel is HBM-bound (every cached K and V byte is read exactly once per KV head; the
 // query heads of a GQA group share the read), so it is built around the memory system:
-//   * one CTA per (split, KV head, sequence); a producer warp streams 64-token K and V tiles with
+//   * one CTA per (split, KV head, sequence), or for num_splits = 0 per even share of the batch (decode_balanced_kernel); a producer
+//     warp streams 64-token K and V tiles with
 //     TMA (16-byte aligned bulk copies, 128-byte swizzle, no multicast) through a ring of
 //     mbarrier-guarded stages, pages looked up in block_table per tile;
 //   * four consumer warps each take 16 tokens of every tile: S = Q K^T and O += P V run on
@@ -58,7 +59,8 @@ struct DecodeParams {
   int capacity;      // tokens a sequence can hold: max_blocks_per_seq * page_size, or the cache row length
   int num_splits;    // grid.x
   int checked;       // the host refuses lengths beyond the capacity: neither read nor reported
-  int chunk_tiles;   // > 0: split s owns tiles [s*chunk, (s+1)*chunk); 0: proportional ranges
+  int b;             // sequences
+  int* arrivals;     // balanced kernel: one zeroed counter per CTA, zero again at the end
   int* status;
 };
 
@@ -70,16 +72,24 @@ struct DCfg {
   static constexpr int kStages = (D == 128) ? 3 : 6;
   static constexpr int kStageBytes = 2 * kTileBytes;
   static constexpr int kMergeBytes = kConsumerWarps * kMaxRows * (D + 2) * 4;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*barriers*/ + 1024 /*align*/;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 2048 /*barriers, (m, l)*/ + 1024 /*align*/;
   static_assert(kMergeBytes <= kStages * kStageBytes, "merge buffer aliases the stage ring");
+  static_assert(kConsumerWarps * 16 * D * 4 <= kStageBytes, "balanced kernel: the merge buffers are one stage");
 };
 
 struct DBarriers {
   uint64_t full[8];
   uint64_t empty[8];
   int abort_flag;
+  int last;  // balanced kernel: this CTA merges the parts of the sequence
 };
+static_assert(sizeof(DBarriers) % 8 == 0 && sizeof(DBarriers) + 2 * kConsumerWarps * kMaxRows * 8 <= 2048, "barrier block");
 
+__device__ __forceinline__ int atomic_add_acq_rel_gpu(int* p, int v) {
+  int old;
+  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2,
                                             uint32_t& r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -107,9 +117,144 @@ __device__ __forceinline__ uint32_t tile_offset(int r, int c8) {
   return (c8 >> 3) * DCfg<D>::kChunkBytes + r * 128 + (((c8 & 7) ^ (r & 7)) << 4);
 }
 
+// What a consumer warp holds of its (up to 16) query rows: the Q fragments and the running (maximum, sum, O) over its tokens.
+template <int D>
+struct WarpRows {
+  uint32_t qa[D / 16][4];
+  int lim0, lim1;         // last visible key of fragment rows g and g + 8
+  float oacc[D / 8][4];
+  float m0, m1;           // reference maxima (raw score units)
+  float l0, l1;           // per-thread partial row sums
+
+  __device__ __forceinline__ void begin(const DecodeParams& p, int batch, int head_k, int len, int rows, int lane) {
+    const int g = lane >> 2;   // fragment row (and row + 8)
+    const int t4 = lane & 3;   // fragment column pair
+    // Q fragments (A operand, 16 x D), straight from global memory; rows >= `rows` are zero.
+    {
+      auto q_ptr = [&](int r) -> const __half* {
+        const int q_pos = r / p.group;
+        const int head = head_k * p.group + (r - q_pos * p.group);
+        return p.q + batch * p.q_batch_stride + q_pos * p.q_row_stride + head * p.q_head_stride;
+      };
+      const __half* r0p = g < rows ? q_ptr(g) : nullptr;
+      const __half* r1p = (g + 8) < rows ? q_ptr(g + 8) : nullptr;
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k) {
+        const int c = k * 16 + t4 * 2;
+        qa[k][0] = r0p ? *reinterpret_cast<const uint32_t*>(r0p + c) : 0u;
+        qa[k][1] = r1p ? *reinterpret_cast<const uint32_t*>(r1p + c) : 0u;
+        qa[k][2] = r0p ? *reinterpret_cast<const uint32_t*>(r0p + c + 8) : 0u;
+        qa[k][3] = r1p ? *reinterpret_cast<const uint32_t*>(r1p + c + 8) : 0u;
+      }
+    }
+    // causal limit per fragment row: key j visible iff j <= q_pos + len - seqlen_q
+    lim0 = lim1 = len - 1;
+    if (p.is_causal) {
+      lim0 = min(lim0, g / p.group + len - p.seqlen_q);
+      lim1 = min(lim1, (g + 8) / p.group + len - p.seqlen_q);
+    }
+#pragma unroll
+    for (int n = 0; n < D / 8; ++n) oacc[n][0] = oacc[n][1] = oacc[n][2] = oacc[n][3] = 0.f;
+    m0 = m1 = -INFINITY;
+    l0 = l1 = 0.f;
+  }
+
+  // 16 tokens of a tile, the first of them token tok0 < len; sK, sV: the tiles, v_tile: the V tile's address, c: scale * log2(e)
+  __device__ __forceinline__ void tokens(uint32_t sK, uint32_t sV, uint8_t* v_tile, int tok_in_tile, int tok0, int len, float c,
+                                         int lane) {
+    const int t4 = lane & 3;
+    // ---- S = Q K^T for 16 tokens: two n8 tiles ----
+    float sacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k) {
+      uint32_t b0, b1, b2, b3;
+      const int mi = lane >> 3, rr = lane & 7;
+      ldmatrix_x4(sK + tile_offset<D>(tok_in_tile + (mi >> 1) * 8 + rr, k * 2 + (mi & 1)), b0, b1,
+                  b2, b3);
+      mma_16816(sacc[0], qa[k], b0, b1);
+      mma_16816(sacc[1], qa[k], b2, b3);
+    }
+    // ---- mask the tail / causal limit ----
+    if (tok0 + 15 > min(lim0, lim1)) {
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const int col = tok0 + n * 8 + t4 * 2;
+        if (col > lim0) sacc[n][0] = -INFINITY;
+        if (col + 1 > lim0) sacc[n][1] = -INFINITY;
+        if (col > lim1) sacc[n][2] = -INFINITY;
+        if (col + 1 > lim1) sacc[n][3] = -INFINITY;
+      }
+    }
+    // Rows of V past the end of the sequence may hold anything (uninitialised cache memory):
+    // zero them so that 0 * garbage cannot produce NaN.  Only this warp reads these rows.
+    // (warp-uniform condition)
+    if (tok0 + 15 >= len) {
+      for (int idx = lane; idx < 16 * (D / 8); idx += 32) {
+        const int r = idx / (D / 8), c8 = idx - r * (D / 8);
+        if (tok0 + r >= len)
+          *reinterpret_cast<uint4*>(v_tile +
+                                    tile_offset<D>(tok_in_tile + r, c8)) = make_uint4(0, 0, 0, 0);
+      }
+      fence_proxy_async_smem();  // order these generic writes before the next TMA refill
+      __syncwarp();
+    }
+    // ---- online softmax with a lazy reference maximum ----
+    float mx0 = fmaxf(fmaxf(sacc[0][0], sacc[0][1]), fmaxf(sacc[1][0], sacc[1][1]));
+    float mx1 = fmaxf(fmaxf(sacc[0][2], sacc[0][3]), fmaxf(sacc[1][2], sacc[1][3]));
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+    float a0 = 1.f, a1 = 1.f;
+    bool need = false;
+    if (mx0 > m0) {
+      if (m0 == -INFINITY) m0 = mx0;
+      else if ((mx0 - m0) * c > 8.f) { a0 = ex2f((m0 - mx0) * c); m0 = mx0; need = true; }
+    }
+    if (mx1 > m1) {
+      if (m1 == -INFINITY) m1 = mx1;
+      else if ((mx1 - m1) * c > 8.f) { a1 = ex2f((m1 - mx1) * c); m1 = mx1; need = true; }
+    }
+    if (__any_sync(0xffffffffu, need)) {
+      l0 *= a0;
+      l1 *= a1;
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n) {
+        oacc[n][0] *= a0; oacc[n][1] *= a0;
+        oacc[n][2] *= a1; oacc[n][3] *= a1;
+      }
+    }
+    const float nm0 = (m0 == -INFINITY) ? 0.f : -m0 * c;
+    const float nm1 = (m1 == -INFINITY) ? 0.f : -m1 * c;
+    uint32_t pa[4];
+    {
+      const float p00 = ex2f(fmaf(sacc[0][0], c, nm0)), p01 = ex2f(fmaf(sacc[0][1], c, nm0));
+      const float p02 = ex2f(fmaf(sacc[0][2], c, nm1)), p03 = ex2f(fmaf(sacc[0][3], c, nm1));
+      const float p10 = ex2f(fmaf(sacc[1][0], c, nm0)), p11 = ex2f(fmaf(sacc[1][1], c, nm0));
+      const float p12 = ex2f(fmaf(sacc[1][2], c, nm1)), p13 = ex2f(fmaf(sacc[1][3], c, nm1));
+      l0 += (p00 + p01) + (p10 + p11);
+      l1 += (p02 + p03) + (p12 + p13);
+      pa[0] = pack_half2(p00, p01);
+      pa[1] = pack_half2(p02, p03);
+      pa[2] = pack_half2(p10, p11);
+      pa[3] = pack_half2(p12, p13);
+    }
+    // ---- O += P V ----
+#pragma unroll
+    for (int n = 0; n < D / 16; ++n) {
+      uint32_t b0, b1, b2, b3;
+      const int mi = lane >> 3, rr = lane & 7;
+      ldmatrix_x4_trans(sV + tile_offset<D>(tok_in_tile + (mi & 1) * 8 + rr, n * 2 + (mi >> 1)), b0,
+                        b1, b2, b3);
+      mma_16816(oacc[2 * n], pa, b0, b1);
+      mma_16816(oacc[2 * n + 1], pa, b2, b3);
+    }
+  }
+};
+
 template <int D>
 __global__ void __launch_bounds__(kDecodeThreads, (D == 128) ? 2 : 2)
-decode_kernel(const __grid_constant__ DecodeParams p) {
+decode_split_kernel(const __grid_constant__ DecodeParams p) {
   using C = DCfg<D>;
   extern __shared__ uint8_t smem_raw[];
   const int split = blockIdx.x;
@@ -127,14 +272,8 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
   const int len = length.len;
   if (length.report && threadIdx.x == 0 && p.status) atomicOr(p.status, kStatusCapacityClamped);
   const int n_tiles = (len + kTileTokens - 1) / kTileTokens;
-  int tile_begin, tile_end;
-  if (p.chunk_tiles > 0) {
-    tile_begin = min(n_tiles, split * p.chunk_tiles);
-    tile_end = min(n_tiles, tile_begin + p.chunk_tiles);
-  } else {
-    tile_begin = static_cast<int>(static_cast<int64_t>(n_tiles) * split / p.num_splits);
-    tile_end = static_cast<int>(static_cast<int64_t>(n_tiles) * (split + 1) / p.num_splits);
-  }
+  const int tile_begin = static_cast<int>(static_cast<int64_t>(n_tiles) * split / p.num_splits);
+  const int tile_end = static_cast<int>(static_cast<int64_t>(n_tiles) * (split + 1) / p.num_splits);
   const int my_tiles = tile_end - tile_begin;
 
   // row r of the M tile -> (query position, head); output row index in (b, h, seqlen_q) order
@@ -217,37 +356,8 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
     // =========================== consumers ===========================
     const int g = lane >> 2;   // fragment row (and row + 8)
     const int t4 = lane & 3;   // fragment column pair
-    // Q fragments (A operand, 16 x D), straight from global memory; rows >= `rows` are zero.
-    uint32_t qa[D / 16][4];
-    {
-      auto q_ptr = [&](int r) -> const __half* {
-        const int q_pos = r / p.group;
-        const int head = head_k * p.group + (r - q_pos * p.group);
-        return p.q + batch * p.q_batch_stride + q_pos * p.q_row_stride + head * p.q_head_stride;
-      };
-      const __half* r0p = g < rows ? q_ptr(g) : nullptr;
-      const __half* r1p = (g + 8) < rows ? q_ptr(g + 8) : nullptr;
-#pragma unroll
-      for (int k = 0; k < D / 16; ++k) {
-        const int c = k * 16 + t4 * 2;
-        qa[k][0] = r0p ? *reinterpret_cast<const uint32_t*>(r0p + c) : 0u;
-        qa[k][1] = r1p ? *reinterpret_cast<const uint32_t*>(r1p + c) : 0u;
-        qa[k][2] = r0p ? *reinterpret_cast<const uint32_t*>(r0p + c + 8) : 0u;
-        qa[k][3] = r1p ? *reinterpret_cast<const uint32_t*>(r1p + c + 8) : 0u;
-      }
-    }
-    // causal limit per fragment row: key j visible iff j <= q_pos + len - seqlen_q
-    int lim0 = len - 1, lim1 = len - 1;
-    if (p.is_causal) {
-      lim0 = min(lim0, g / p.group + len - p.seqlen_q);
-      lim1 = min(lim1, (g + 8) / p.group + len - p.seqlen_q);
-    }
-
-    float oacc[D / 8][4];
-#pragma unroll
-    for (int n = 0; n < D / 8; ++n) oacc[n][0] = oacc[n][1] = oacc[n][2] = oacc[n][3] = 0.f;
-    float m0 = -INFINITY, m1 = -INFINITY;  // reference maxima of rows g and g + 8 (raw score units)
-    float l0 = 0.f, l1 = 0.f;              // per-thread partial row sums
+    WarpRows<D> w;
+    w.begin(p, batch, head_k, len, rows, lane);
     const float c = p.scale_log2;
     const int tok_in_tile = warp * 16;     // this warp's 16 tokens of every tile
     bool ok = true;
@@ -259,122 +369,34 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       const uint32_t sK = smem_u32(smem + s * C::kStageBytes);
-      const uint32_t sV = sK + C::kTileBytes;
       const int tok0 = (tile_begin + i) * kTileTokens + tok_in_tile;  // first token of this warp
-
-      if (tok0 < len) {
-        // ---- S = Q K^T for 16 tokens: two n8 tiles ----
-        float sacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          uint32_t b0, b1, b2, b3;
-          const int mi = lane >> 3, rr = lane & 7;
-          ldmatrix_x4(sK + tile_offset<D>(tok_in_tile + (mi >> 1) * 8 + rr, k * 2 + (mi & 1)), b0, b1,
-                      b2, b3);
-          mma_16816(sacc[0], qa[k], b0, b1);
-          mma_16816(sacc[1], qa[k], b2, b3);
-        }
-        // ---- mask the tail / causal limit ----
-        if (tok0 + 15 > min(lim0, lim1)) {
-#pragma unroll
-          for (int n = 0; n < 2; ++n) {
-            const int col = tok0 + n * 8 + t4 * 2;
-            if (col > lim0) sacc[n][0] = -INFINITY;
-            if (col + 1 > lim0) sacc[n][1] = -INFINITY;
-            if (col > lim1) sacc[n][2] = -INFINITY;
-            if (col + 1 > lim1) sacc[n][3] = -INFINITY;
-          }
-        }
-        // Rows of V past the end of the sequence may hold anything (uninitialised cache memory):
-        // zero them so that 0 * garbage cannot produce NaN.  Only this warp reads these rows.
-        // (warp-uniform condition)
-        if (tok0 + 15 >= len) {
-          for (int idx = lane; idx < 16 * (D / 8); idx += 32) {
-            const int r = idx / (D / 8), c8 = idx - r * (D / 8);
-            if (tok0 + r >= len)
-              *reinterpret_cast<uint4*>(smem + s * C::kStageBytes + C::kTileBytes +
-                                        tile_offset<D>(tok_in_tile + r, c8)) = make_uint4(0, 0, 0, 0);
-          }
-          fence_proxy_async_smem();  // order these generic writes before the next TMA refill
-          __syncwarp();
-        }
-        // ---- online softmax with a lazy reference maximum ----
-        float mx0 = fmaxf(fmaxf(sacc[0][0], sacc[0][1]), fmaxf(sacc[1][0], sacc[1][1]));
-        float mx1 = fmaxf(fmaxf(sacc[0][2], sacc[0][3]), fmaxf(sacc[1][2], sacc[1][3]));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        float a0 = 1.f, a1 = 1.f;
-        bool need = false;
-        if (mx0 > m0) {
-          if (m0 == -INFINITY) m0 = mx0;
-          else if ((mx0 - m0) * c > 8.f) { a0 = ex2f((m0 - mx0) * c); m0 = mx0; need = true; }
-        }
-        if (mx1 > m1) {
-          if (m1 == -INFINITY) m1 = mx1;
-          else if ((mx1 - m1) * c > 8.f) { a1 = ex2f((m1 - mx1) * c); m1 = mx1; need = true; }
-        }
-        if (__any_sync(0xffffffffu, need)) {
-          l0 *= a0;
-          l1 *= a1;
-#pragma unroll
-          for (int n = 0; n < D / 8; ++n) {
-            oacc[n][0] *= a0; oacc[n][1] *= a0;
-            oacc[n][2] *= a1; oacc[n][3] *= a1;
-          }
-        }
-        const float nm0 = (m0 == -INFINITY) ? 0.f : -m0 * c;
-        const float nm1 = (m1 == -INFINITY) ? 0.f : -m1 * c;
-        uint32_t pa[4];
-        {
-          const float p00 = ex2f(fmaf(sacc[0][0], c, nm0)), p01 = ex2f(fmaf(sacc[0][1], c, nm0));
-          const float p02 = ex2f(fmaf(sacc[0][2], c, nm1)), p03 = ex2f(fmaf(sacc[0][3], c, nm1));
-          const float p10 = ex2f(fmaf(sacc[1][0], c, nm0)), p11 = ex2f(fmaf(sacc[1][1], c, nm0));
-          const float p12 = ex2f(fmaf(sacc[1][2], c, nm1)), p13 = ex2f(fmaf(sacc[1][3], c, nm1));
-          l0 += (p00 + p01) + (p10 + p11);
-          l1 += (p02 + p03) + (p12 + p13);
-          pa[0] = pack_half2(p00, p01);
-          pa[1] = pack_half2(p02, p03);
-          pa[2] = pack_half2(p10, p11);
-          pa[3] = pack_half2(p12, p13);
-        }
-        // ---- O += P V ----
-#pragma unroll
-        for (int n = 0; n < D / 16; ++n) {
-          uint32_t b0, b1, b2, b3;
-          const int mi = lane >> 3, rr = lane & 7;
-          ldmatrix_x4_trans(sV + tile_offset<D>(tok_in_tile + (mi & 1) * 8 + rr, n * 2 + (mi >> 1)), b0,
-                            b1, b2, b3);
-          mma_16816(oacc[2 * n], pa, b0, b1);
-          mma_16816(oacc[2 * n + 1], pa, b2, b3);
-        }
-      }
+      if (tok0 < len)
+        w.tokens(sK, sK + C::kTileBytes, smem + s * C::kStageBytes + C::kTileBytes, tok_in_tile, tok0, len, c, lane);
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->empty[s]);
     }
 
     // ---- merge the four warps: (m, l, O) through shared memory (aliases the stage ring) ----
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+    w.l0 += __shfl_xor_sync(0xffffffffu, w.l0, 1);
+    w.l0 += __shfl_xor_sync(0xffffffffu, w.l0, 2);
+    w.l1 += __shfl_xor_sync(0xffffffffu, w.l1, 1);
+    w.l1 += __shfl_xor_sync(0xffffffffu, w.l1, 2);
     named_barrier_sync(1, kConsumerWarps * 32);  // every warp is done reading the ring
     float* mbuf = reinterpret_cast<float*>(smem);
     // layout: [warp][row][D + 2] with the last two floats = (m, l)
     {
-      float* w = mbuf + warp * kMaxRows * (D + 2);
+      float* dst = mbuf + warp * kMaxRows * (D + 2);
 #pragma unroll
       for (int n = 0; n < D / 8; ++n) {
         const int col = n * 8 + t4 * 2;
-        *reinterpret_cast<float2*>(w + g * (D + 2) + col) = make_float2(oacc[n][0], oacc[n][1]);
-        *reinterpret_cast<float2*>(w + (g + 8) * (D + 2) + col) = make_float2(oacc[n][2], oacc[n][3]);
+        *reinterpret_cast<float2*>(dst + g * (D + 2) + col) = make_float2(w.oacc[n][0], w.oacc[n][1]);
+        *reinterpret_cast<float2*>(dst + (g + 8) * (D + 2) + col) = make_float2(w.oacc[n][2], w.oacc[n][3]);
       }
       if (t4 == 0) {
-        w[g * (D + 2) + D] = m0;
-        w[g * (D + 2) + D + 1] = l0;
-        w[(g + 8) * (D + 2) + D] = m1;
-        w[(g + 8) * (D + 2) + D + 1] = l1;
+        dst[g * (D + 2) + D] = w.m0;
+        dst[g * (D + 2) + D + 1] = w.l0;
+        dst[(g + 8) * (D + 2) + D] = w.m1;
+        dst[(g + 8) * (D + 2) + D + 1] = w.l1;
       }
     }
     named_barrier_sync(1, kConsumerWarps * 32);
@@ -448,6 +470,398 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// num_splits == 0: the tiles of the whole batch shared out evenly
+// ---------------------------------------------------------------------------------------------
+// The host does not know the lengths.  Every CTA reads them, counts the 64-token tiles of the sequences, laid end to end, and takes
+// its share of them for one KV head: an equal number of tiles whatever the spread of the lengths, one set-up per CTA, and the ring of
+// stages runs on from one sequence into the next.  The CTAs of all heads go over the same tokens at the same time, whose rows lie
+// next to each other in memory (a share of (sequence, head) pairs laid end to end, with heads far apart in time, read 3-10 % more slowly).
+// A share holds the end of a sequence, whole ones and the beginning of another; the parts of a sequence that several CTAs
+// share go to scratch memory (at most two per CTA), and the CTA that arrives last merges them, in the order of the tiles, so that the
+// result does not depend on who that is.
+// Bound by the K / V bytes for large batches, by a chain of latencies (lengths, Q and K / V tiles, merge) for small ones.  Append and
+// attention, us, chunks of a fixed size per CTA and a merge kernel against this: 1 x 1500 tokens (Hq32 Hkv8 D128) 13.2 -> 10.4,
+// 1 x 30000 42.1 -> 32.8, 16 x 1000-8000 56.3 -> 49.6 (6.0 TB/s), 64 x 1024-32768 620 -> 621 (6.9 TB/s), 128 x 20-64 (H32) 69.8 -> 43.1,
+// 128 x 200-3000 (Hq8 Hkv2 D64) 34.4 -> 28.6; slower: 2 x 6000-9000 (Hq8 Hkv2 D128) 14.5 -> 16.5.
+constexpr int kBalancedCtas = 2 * 148;  // two per SM are resident
+constexpr int kMinShare = 2;            // tiles of a CTA at least
+// A share of a sequence of n tiles is at least sqrt(kShareSlope * n) of them: what a tile takes its CTA and what a part takes the CTA that
+// merges the sequence are then about least together.  One sequence of 30000 tokens, Hkv1 D128, slopes 0.2 / 0.4: 18.6 / 20.3 us.
+constexpr float kShareSlope = 0.2f;
+static_assert(kBalancedCtas <= kArrivalSlots, "a counter per CTA");
+
+__device__ __forceinline__ int kv_tiles(const DecodeParams& p, int batch, int& len) {
+  len = cache_length(p.cache_seqlens[batch], p.seqlen_new, p.capacity, p.checked).len;
+  return max(1, (len + kTileTokens - 1) / kTileTokens);  // an empty sequence has a share too: its rows are zero
+}
+
+// Tiles [begin, end) of CTA i of a head out of `ctas` that share `total`: the first `more` have one more than `each`.
+struct Shares {
+  int64_t total;
+  int ctas, more;
+  int64_t each;
+  __device__ __forceinline__ Shares(int64_t total_, int ctas_) : total(total_), ctas(ctas_) {
+    each = total / ctas;
+    more = static_cast<int>(total - each * ctas);
+  }
+  __device__ __forceinline__ int64_t begin(int i) const { return i * each + min(i, more); }
+  __device__ __forceinline__ int owner(int64_t tile) const {
+    const int64_t first = more * (each + 1);
+    return static_cast<int>(tile < first ? tile / (each + 1) : more + (tile - first) / each);
+  }
+};
+
+// Walks a CTA's share sequence by sequence.
+struct ShareWalk {
+  int batch, tile, n_tiles, len;
+  int64_t at, end;   // tiles counted over the batch
+  // by a whole warp
+  __device__ __forceinline__ ShareWalk(const DecodeParams& p, int64_t begin, int64_t end_, int lane) : at(begin), end(end_) {
+    int64_t before = 0;  // tiles of the sequences before the current 32
+    batch = 0;
+    for (int b0 = 0; b0 < p.b; b0 += 32) {
+      int unused, sum = b0 + lane < p.b ? kv_tiles(p, b0 + lane, unused) : 0;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int other = __shfl_up_sync(0xffffffffu, sum, off);
+        if (lane >= off) sum += other;
+      }
+      const uint32_t past = __ballot_sync(0xffffffffu, before + sum > begin);
+      if (past != 0) {
+        const int first = __ffs(past) - 1;
+        const int skipped = __shfl_sync(0xffffffffu, sum, max(first - 1, 0));
+        batch = b0 + first;
+        before += first > 0 ? skipped : 0;
+        break;
+      }
+      before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    n_tiles = kv_tiles(p, batch, len);
+    tile = static_cast<int>(begin - before);
+  }
+  __device__ __forceinline__ int count() const { return static_cast<int>(min(static_cast<int64_t>(n_tiles - tile), end - at)); }
+  __device__ __forceinline__ void next(const DecodeParams& p) {
+    at += count();
+    tile = 0;
+    if (at < end) n_tiles = kv_tiles(p, ++batch, len);
+  }
+};
+
+// The tiles of the batch and of its longest sequence.
+__device__ __forceinline__ int64_t all_tiles(const DecodeParams& p, int lane, int& longest) {
+  int64_t sum = 0;
+  longest = 0;
+  for (int b0 = 0; b0 < p.b; b0 += 32) {
+    int unused;
+    const int n = b0 + lane < p.b ? kv_tiles(p, b0 + lane, unused) : 0;
+    sum += __reduce_add_sync(0xffffffffu, n);
+    longest = max(longest, __reduce_max_sync(0xffffffffu, n));
+  }
+  return sum;
+}
+
+// N (2 or 4) consecutive floats, aligned to their size
+template <int N>
+__device__ __forceinline__ void load_floats(const float* src, float (&x)[N]) {
+  if constexpr (N == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(src);
+    x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+  } else {
+    const float2 v = *reinterpret_cast<const float2*>(src);
+    x[0] = v.x, x[1] = v.y;
+  }
+}
+template <int N>
+__device__ __forceinline__ void store_floats(float* dst, const float (&x)[N], float mul) {
+  if constexpr (N == 4) {
+    *reinterpret_cast<float4*>(dst) = make_float4(x[0] * mul, x[1] * mul, x[2] * mul, x[3] * mul);
+  } else {
+    *reinterpret_cast<float2*>(dst) = make_float2(x[0] * mul, x[1] * mul);
+  }
+}
+
+// `bytes` (8 or 16) from global to shared memory, by each thread for itself
+template <int kBytes>
+__device__ __forceinline__ void async_copy(void* smem_dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(smem_dst)), "l"(src), "n"(kBytes) : "memory");
+}
+__device__ __forceinline__ void async_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// One row of the merged parts of a sequence, by a warp: this lane's D / 32 columns, and the LSE.  first_slot: where the sequence begins;
+// the later parts lie 2 * heads apart, from the slot before that on.  kPartsAtOnce rows are in flight at a time, through `buf` in shared
+// memory (a lane reads what it copied itself): four at a time in registers, as many as they hold, took twice as long.
+constexpr int kPartsAtOnce = 16;
+template <int D>
+__device__ __forceinline__ float merge_row(const float* o_accum, const float* lse_accum, int first_slot, int heads, int parts, int r,
+                                           float* buf, int lane, float (&acc)[D / 32]) {
+  constexpr int kPerLane = D / 32;
+  auto slot_of = [&](int j) { return static_cast<int64_t>(first_slot + (j > 0 ? 2 * heads * j - 1 : 0)) * kMaxRows + r; };
+  auto lse_of = [&](int j) { return j < parts ? __ldcg(lse_accum + slot_of(j)) : -INFINITY; };
+  float* mine = buf + lane * kPerLane;
+  auto fetch = [&](int j0) {
+#pragma unroll 4
+    for (int u = 0; u < min(kPartsAtOnce, parts - j0); ++u)
+      async_copy<kPerLane * 4>(mine + u * D, o_accum + slot_of(j0 + u) * D + lane * kPerLane);
+  };
+  fetch(0);
+  const float first = lse_of(lane);
+  float mx = first;
+  for (int j = lane + 32; j < parts; j += 32) mx = fmaxf(mx, lse_of(j));
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  const bool dead = mx == -INFINITY;
+  float sum = 0.f, weight = 0.f;
+#pragma unroll
+  for (int e = 0; e < kPerLane; ++e) acc[e] = 0.f;
+  for (int j0 = 0; j0 < parts; j0 += kPartsAtOnce) {
+    if (j0 > 0) fetch(j0);
+    if (j0 % 32 == 0) {  // the weights of 32 parts sit in the lanes; 0 for a part without a visible key
+      weight = dead ? 0.f : __expf((j0 == 0 ? first : lse_of(j0 + lane)) - mx);
+      sum += weight;
+    }
+    async_copy_wait();
+    for (int u = 0; u < min(kPartsAtOnce, parts - j0); ++u) {
+      const float wu = __shfl_sync(0xffffffffu, weight, j0 % 32 + u);
+      float x[kPerLane];
+      load_floats(mine + u * D, x);
+#pragma unroll
+      for (int e = 0; e < kPerLane; ++e) acc[e] = fmaf(wu, x[e], acc[e]);
+    }
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  const float inv = dead ? 0.f : 1.f / sum;
+#pragma unroll
+  for (int e = 0; e < kPerLane; ++e) acc[e] *= inv;
+  return dead ? 0.f : mx + __logf(sum);
+}
+
+template <int D>
+__global__ void __launch_bounds__(kDecodeThreads, 2)
+decode_balanced_kernel(const __grid_constant__ DecodeParams p) {
+  using C = DCfg<D>;
+  extern __shared__ uint8_t smem_raw[];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int rows = p.seqlen_q * p.group;  // valid rows of the 16-row M tile
+  const int stop_probe = stop_probe_begin(p.status);
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  DBarriers* bars = reinterpret_cast<DBarriers*>(smem + C::kStages * C::kStageBytes);
+  float2* ml_of_seqs = reinterpret_cast<float2*>(bars + 1);  // (m, l) of [sequence & 1][warp][row]: a warp may be a sequence ahead
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::kStages; ++s) {
+      mbar_init(&bars->full[s], 1);
+      mbar_init(&bars->empty[s], kConsumerWarps);
+    }
+    bars->abort_flag = 0;
+    fence_mbar_init();
+  }
+  int longest;
+  const int64_t total = all_tiles(p, lane, longest);
+  const int least = max(kMinShare, static_cast<int>(sqrtf(kShareSlope * longest)));
+  const Shares shares(total, static_cast<int>(min(static_cast<int64_t>(gridDim.y), (total + least - 1) / least)));
+  const int cta = blockIdx.y, head_k = blockIdx.x;
+  const bool stop = __syncthreads_or(stop_probe) != 0;
+  if (cta >= shares.ctas) return;
+  WaitCtx ctx{&bars->abort_flag, p.status};
+  ShareWalk w(p, shares.begin(cta), shares.begin(cta + 1), lane);
+
+  // row r of the M tile -> (query position, head)
+  auto row_head = [&](int r, int& q_pos) {
+    q_pos = r / p.group;
+    return head_k * p.group + (r - q_pos * p.group);
+  };
+
+  if (stop) {  // sticky time-out bit: zeros, by the CTA where a sequence begins
+    if (threadIdx.x == 0) grid_dependency_wait();
+    for (; w.at < w.end; w.next(p)) {
+      if (w.tile != 0) continue;
+      for (int idx = threadIdx.x; idx < rows * (D / 8); idx += blockDim.x) {
+        int q_pos;
+        const int head = row_head(idx / (D / 8), q_pos);
+        *reinterpret_cast<uint4*>(p.o + w.batch * p.o_batch_stride + q_pos * p.o_row_stride + head * p.o_head_stride +
+                                  idx % (D / 8) * 8) = make_uint4(0, 0, 0, 0);
+        if (idx % (D / 8) == 0) p.lse[(static_cast<int64_t>(w.batch) * p.h + head) * p.seqlen_q + q_pos] = 0.f;
+      }
+    }
+    return;
+  }
+
+  if (warp == kConsumerWarps) {
+    // =========================== TMA producer ===========================
+    if (lane == 0) {
+      prefetch_tensormap(&p.tm_k);
+      prefetch_tensormap(&p.tm_v);
+      grid_dependency_wait();  // the appended rows; nothing else here depends on the kernel before
+      bool ok = true;
+      int i = 0;  // ring position
+      for (; ok && w.at < w.end; w.next(p)) {
+        const int cache_row = p.cache_batch_idx ? p.cache_batch_idx[w.batch] : w.batch;
+        const int n = w.len > 0 ? w.count() : 0;
+        for (int t = 0; t < n; ++t, ++i) {
+          const int s = i % C::kStages;
+          const int tok = (w.tile + t) * kTileTokens;
+          int row = tok, blk = cache_row;
+          if (p.block_table) {
+            blk = p.block_table[w.batch * p.block_table_batch_stride + tok / p.page_size];
+            row = tok % p.page_size;
+          }
+          if (!(ok = mbar_wait(&bars->empty[s], ((i / C::kStages) & 1) ^ 1, ctx))) break;
+          mbar_arrive_expect_tx(&bars->full[s], C::kStageBytes);
+          uint8_t* dst = smem + s * C::kStageBytes;
+#pragma unroll
+          for (int c = 0; c < C::kChunks; ++c)
+            tma_load_4d(dst + c * C::kChunkBytes, &p.tm_k, &bars->full[s], c * 64, head_k, row, blk);
+#pragma unroll
+          for (int c = 0; c < C::kChunks; ++c)
+            tma_load_4d(dst + C::kTileBytes + c * C::kChunkBytes, &p.tm_v, &bars->full[s], c * 64, head_k, row, blk);
+        }
+        // the stage behind the last tile of a sequence is where the consumers merge their rows
+        if (ok && (ok = mbar_wait(&bars->empty[i % C::kStages], ((i / C::kStages) & 1) ^ 1, ctx))) {
+          mbar_arrive(&bars->full[i % C::kStages]);
+          ++i;
+        }
+      }
+    }
+  } else {
+    // =========================== consumers ===========================
+    const int g = lane >> 2;   // fragment row (and row + 8)
+    const int t4 = lane & 3;   // fragment column pair
+    const int tok_in_tile = warp * 16;  // this warp's 16 tokens of every tile
+    const float c = p.scale_log2;
+    constexpr int kPerLane = D / 32;    // columns of a lane when a warp merges a row
+    auto wait_full = [&](int i) {
+      const bool ok = mbar_wait(&bars->full[i % C::kStages], (i / C::kStages) & 1, ctx);
+      return __all_sync(0xffffffffu, ok) != 0;
+    };
+    auto release = [&](int i) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->empty[i % C::kStages]);
+    };
+    int i = 0, n_seqs = 0;
+    float2* ml = ml_of_seqs;
+    bool ok = true;
+    for (; ok && w.at < w.end; w.next(p)) {
+      const int count = w.count(), n = w.len > 0 ? count : 0;
+      const bool whole = count == w.n_tiles;
+      if (w.tile == 0 && head_k == 0 && threadIdx.x == 0 && p.status &&
+          cache_length(p.cache_seqlens[w.batch], p.seqlen_new, p.capacity, p.checked).report)
+        atomicOr(p.status, kStatusCapacityClamped);
+      WarpRows<D> mine;
+      mine.begin(p, w.batch, head_k, w.len, rows, lane);
+      for (int t = 0; t < n; ++t, ++i) {
+        if (!(ok = wait_full(i))) break;
+        uint8_t* stage = smem + (i % C::kStages) * C::kStageBytes;
+        const uint32_t sK = smem_u32(stage);
+        const int tok0 = (w.tile + t) * kTileTokens + tok_in_tile;
+        if (tok0 < w.len) mine.tokens(sK, sK + C::kTileBytes, stage + C::kTileBytes, tok_in_tile, tok0, w.len, c, lane);
+        release(i);
+      }
+      if (!ok || !(ok = wait_full(i))) break;
+
+      // ---- merge the four warps through the stage that holds no tile: [warp][row][D], the columns of row r xor 8 * (r % 8) so
+      // that the eight rows of a fragment column lie in different banks ----
+      float* mbuf = reinterpret_cast<float*>(smem + (i % C::kStages) * C::kStageBytes);
+      mine.l0 += __shfl_xor_sync(0xffffffffu, mine.l0, 1);
+      mine.l0 += __shfl_xor_sync(0xffffffffu, mine.l0, 2);
+      mine.l1 += __shfl_xor_sync(0xffffffffu, mine.l1, 1);
+      mine.l1 += __shfl_xor_sync(0xffffffffu, mine.l1, 2);
+      float* dst = mbuf + warp * kMaxRows * D;
+#pragma unroll
+      for (int k = 0; k < D / 8; ++k) {
+        const int col = ((k * 8) ^ (g * 8)) + t4 * 2;
+        if (g < rows) *reinterpret_cast<float2*>(dst + g * D + col) = make_float2(mine.oacc[k][0], mine.oacc[k][1]);
+        if (g + 8 < rows) *reinterpret_cast<float2*>(dst + (g + 8) * D + col) = make_float2(mine.oacc[k][2], mine.oacc[k][3]);
+      }
+      ml = ml_of_seqs + (n_seqs++ & 1) * kConsumerWarps * kMaxRows;
+      if (t4 == 0) {
+        ml[warp * kMaxRows + g] = make_float2(mine.m0, mine.l0);
+        ml[warp * kMaxRows + g + 8] = make_float2(mine.m1, mine.l1);
+      }
+      named_barrier_sync(1, kConsumerWarps * 32);
+
+      // a warp per row, a lane per kPerLane columns
+      auto store = [&](int r, const float (&acc)[kPerLane], float mul, float lse) {
+        int q_pos;
+        const int head = row_head(r, q_pos);
+        __half* out = p.o + w.batch * p.o_batch_stride + q_pos * p.o_row_stride + head * p.o_head_stride + lane * kPerLane;
+        if constexpr (kPerLane == 4) {
+          *reinterpret_cast<uint2*>(out) = make_uint2(pack_half2(acc[0] * mul, acc[1] * mul), pack_half2(acc[2] * mul, acc[3] * mul));
+        } else {
+          *reinterpret_cast<uint32_t*>(out) = pack_half2(acc[0] * mul, acc[1] * mul);
+        }
+        if (lane == 0) p.lse[(static_cast<int64_t>(w.batch) * p.h + head) * p.seqlen_q + q_pos] = lse;
+      };
+      // part of a sequence in scratch memory: slot 1 of the CTA where the sequence begins, slot 0 of the others
+      auto part = [&](int owner, bool begins) { return 2 * (owner * static_cast<int>(gridDim.x) + head_k) + (begins ? 1 : 0); };
+      for (int r = warp; r < rows; r += kConsumerWarps) {
+        float2 of[kConsumerWarps];
+        float mt = -INFINITY;
+#pragma unroll
+        for (int u = 0; u < kConsumerWarps; ++u) {
+          of[u] = ml[u * kMaxRows + r];
+          mt = fmaxf(mt, of[u].x);
+        }
+        float lt = 0.f, acc[kPerLane];
+#pragma unroll
+        for (int e = 0; e < kPerLane; ++e) acc[e] = 0.f;
+        const int col = (lane * kPerLane) ^ ((r & 7) * 8);
+#pragma unroll
+        for (int u = 0; u < kConsumerWarps; ++u) {
+          const float scale = of[u].x == -INFINITY ? 0.f : ex2f((of[u].x - mt) * c);
+          lt += of[u].y * scale;
+          float x[kPerLane];
+          load_floats(mbuf + (u * kMaxRows + r) * D + col, x);
+#pragma unroll
+          for (int e = 0; e < kPerLane; ++e) acc[e] = fmaf(x[e], scale, acc[e]);
+        }
+        const bool dead = mt == -INFINITY || lt == 0.f;
+        const float inv = dead ? 0.f : 1.f / lt;
+        const float lse = dead ? -INFINITY : (mt * c + __log2f(lt)) * kLn2;
+        if (whole) {
+          store(r, acc, inv, dead ? 0.f : lse);
+        } else {
+          const int slot = part(cta, w.tile == 0);
+          store_floats(p.o_accum + (static_cast<int64_t>(slot) * kMaxRows + r) * D + lane * kPerLane, acc, inv);
+          if (lane == 0) p.lse_accum[slot * kMaxRows + r] = lse;
+        }
+      }
+      if (!whole) {
+        // ---- the last of the CTAs that share the sequence merges its parts ----
+        const int64_t first_tile = w.at - w.tile;
+        const int c0 = shares.owner(first_tile), parts = shares.owner(first_tile + w.n_tiles - 1) - c0 + 1;
+        named_barrier_sync(1, kConsumerWarps * 32);
+        if (threadIdx.x == 0) {  // release: the barrier's other threads' writes too; acquire: those of the CTAs that came before
+          int* arrivals = p.arrivals + c0 * gridDim.x + head_k;
+          const bool last = atomic_add_acq_rel_gpu(arrivals, 1) == parts - 1;
+          if (last) *arrivals = 0;  // for the launch that takes the counters next
+          bars->last = last;
+        }
+        named_barrier_sync(1, kConsumerWarps * 32);
+        if (bars->last) {
+          for (int r = warp; r < rows; r += kConsumerWarps) {
+            float acc[kPerLane];
+            const float lse = merge_row<D>(p.o_accum, p.lse_accum, part(c0, true), gridDim.x, parts, r, mbuf + warp * kPartsAtOnce * D, lane, acc);
+            store(r, acc, 1.f, lse);
+          }
+        }
+      }
+      fence_proxy_async_smem();  // the merge buffer's writes, before TMA fills the stage again
+      release(i);
+      ++i;
+    }
+  }
+  __syncthreads();
+  if (bars->abort_flag) {
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 200000ull) {
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // append: k_new/v_new (b, s_new, h_k, d) -> cache rows / pages at cache_seqlens[b] + t
 // ---------------------------------------------------------------------------------------------
 struct AppendParams {
@@ -489,44 +903,53 @@ __global__ void __launch_bounds__(256) check_lengths_kernel(const int* lengths, 
   if (threadIdx.x == 0) tell_host(verdict, token, fits);
 }
 
-__global__ void __launch_bounds__(256) append_kernel(const AppendParams p) {
+// The 16-byte units of the first step are fetched before the lengths are looked at: two memory latencies in a row instead of four
+// (lengths, the length again, the unit, the store), which is most of what a small append takes.
+__global__ void __launch_bounds__(256) append_kernel(const __grid_constant__ AppendParams p) {
   grid_launch_dependents();
+  const int unit_bits = p.d == 128 ? 4 : 3;  // d / 8 units of 16 bytes per (token, head)
+  const int64_t total = (static_cast<int64_t>(p.b) * p.seqlen_new * p.h_k) << unit_bits;
+  int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  int u, head, t, batch, cached;
+  uint4 kv, vv;
+  auto fetch = [&]() {
+    u = static_cast<int>(idx) & ((1 << unit_bits) - 1);
+    if (total <= 0x7fffffff) {  // divisions in 32 bits
+      const int rest = static_cast<int>(idx) >> unit_bits, token = rest / p.h_k;
+      head = rest - token * p.h_k, batch = token / p.seqlen_new, t = token - batch * p.seqlen_new;
+    } else {
+      const int64_t rest = idx >> unit_bits, token = rest / p.h_k;
+      head = static_cast<int>(rest - token * p.h_k);
+      batch = static_cast<int>(token / p.seqlen_new), t = static_cast<int>(token - static_cast<int64_t>(batch) * p.seqlen_new);
+    }
+    cached = p.cache_seqlens[batch];
+    kv = *reinterpret_cast<const uint4*>(p.k_new + batch * p.kn_batch_stride + t * p.kn_row_stride + head * p.kn_head_stride + u * 8);
+    vv = *reinterpret_cast<const uint4*>(p.v_new + batch * p.vn_batch_stride + t * p.vn_row_stride + head * p.vn_head_stride + u * 8);
+  };
+  if (idx < total) fetch();
   if (p.verdict != nullptr) {  // every block looks at all lengths (b loads by its 256 threads, from L2 but for the first): no launch in between
     const bool fits = lengths_fit(p.cache_seqlens, p.b, p.max_length);
     if (blockIdx.x == 0 && threadIdx.x == 0) tell_host(p.verdict, p.token, fits);
     if (!fits) return;
   }
-  const int units_per_row = p.d / 8;  // 16-byte units per (token, head)
-  const int64_t total = static_cast<int64_t>(p.b) * p.seqlen_new * p.h_k * units_per_row;
-  for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int u = static_cast<int>(idx % units_per_row);
-    int64_t rest = idx / units_per_row;
-    const int head = static_cast<int>(rest % p.h_k);
-    rest /= p.h_k;
-    const int t = static_cast<int>(rest % p.seqlen_new);
-    const int batch = static_cast<int>(rest / p.seqlen_new);
-    const int pos = static_cast<int>(static_cast<uint32_t>(p.cache_seqlens[batch]) + t);  // past 2^31: negative, not written
-    int64_t blk, row;
+  while (idx < total) {
+    const int pos = static_cast<int>(static_cast<uint32_t>(cached) + t);  // past 2^31: negative, not written
+    int64_t blk = -1, row = pos;
     if (p.block_table) {
       const int slot = pos / p.seqlen_cache;
-      if (pos < 0 || slot >= p.max_blocks_per_seq) continue;  // beyond capacity: never written
-      blk = p.block_table[batch * p.block_table_batch_stride + slot];
-      row = pos - slot * p.seqlen_cache;
-    } else {
-      if (pos < 0 || pos >= p.seqlen_cache) continue;
+      if (pos >= 0 && slot < p.max_blocks_per_seq) {  // beyond capacity: never written
+        blk = p.block_table[batch * p.block_table_batch_stride + slot];
+        row = pos - slot * p.seqlen_cache;
+      }
+    } else if (pos >= 0 && pos < p.seqlen_cache) {
       blk = p.cache_batch_idx ? p.cache_batch_idx[batch] : batch;
-      row = pos;
     }
-    if (blk < 0 || blk >= p.cache_batch) continue;
-    const uint4 kv = *reinterpret_cast<const uint4*>(p.k_new + batch * p.kn_batch_stride + t * p.kn_row_stride +
-                                                     head * p.kn_head_stride + u * 8);
-    const uint4 vv = *reinterpret_cast<const uint4*>(p.v_new + batch * p.vn_batch_stride + t * p.vn_row_stride +
-                                                     head * p.vn_head_stride + u * 8);
-    *reinterpret_cast<uint4*>(p.k_cache + blk * p.kc_batch_stride + row * p.kc_row_stride +
-                              head * p.kc_head_stride + u * 8) = kv;
-    *reinterpret_cast<uint4*>(p.v_cache + blk * p.vc_batch_stride + row * p.vc_row_stride +
-                              head * p.vc_head_stride + u * 8) = vv;
+    if (blk >= 0 && blk < p.cache_batch) {
+      *reinterpret_cast<uint4*>(p.k_cache + blk * p.kc_batch_stride + row * p.kc_row_stride + head * p.kc_head_stride + u * 8) = kv;
+      *reinterpret_cast<uint4*>(p.v_cache + blk * p.vc_batch_stride + row * p.vc_row_stride + head * p.vc_head_stride + u * 8) = vv;
+    }
+    idx += static_cast<int64_t>(gridDim.x) * blockDim.x;
+    if (idx < total) fetch();
   }
 }
 
@@ -538,43 +961,53 @@ int capacity_tokens(const FaKvcacheParams* p) {
   return p->block_table ? p->max_blocks_per_seq * p->seqlen_cache : p->seqlen_cache;
 }
 
-// Split plan.  An explicit request is honoured as given (proportional ranges per sequence).  With
-// num_splits == 0 the lengths are unknown on the host (no synchronisation), so work is cut into
-// fixed chunks of tiles instead: every CTA gets at most `chunk` tiles and the grid covers the cache
-// capacity; CTAs past a sequence's end return at once.  The chunk is chosen so that the sequences at
-// full capacity would give about four CTAs per SM-slot (2 resident CTAs x 148 SMs), with a floor of
-// 8 tiles (512 tokens) so that the merge traffic stays small against the K/V bytes.  Floors of 4 / 2 / 1 tiles against 8,
-// one token each: one sequence of 1500 (Hq32 Hkv8 D128, capacity 4096) 13.6 / 15.6 / 17.7 against 14.6 us, one of 30000 62 / 62 /
-// 62 against 45, four of up to 4000 22.3 / 29.4 / 29.1 against 20.7.
-void plan_splits(const FaKvcacheParams* p, int* num_splits, int* chunk_tiles) {
-  if (!uses_decode_kernel(p)) {
-    *num_splits = 1;
-    *chunk_tiles = 0;
-    return;
-  }
-  if (p->num_splits > 0) {
-    *num_splits = std::min(p->num_splits, 256);
-    *chunk_tiles = 0;
-    return;
-  }
-  const int cap_tiles = std::max(1, (capacity_tokens(p) + p->seqlen_new + kTileTokens - 1) / kTileTokens);
-  const int64_t base_ctas = static_cast<int64_t>(p->b) * p->h_k;
-  const int64_t target_ctas = 4 * 2 * 148;
-  int64_t want = (target_ctas + base_ctas - 1) / base_ctas;  // splits per (sequence, KV head)
-  want = std::max<int64_t>(1, std::min<int64_t>(want, 256));
-  int chunk = static_cast<int>((cap_tiles + want - 1) / want);
-  chunk = std::max(chunk, 8);
-  int splits = (cap_tiles + chunk - 1) / chunk;
-  if (splits <= 1) {
-    *num_splits = 1;
-    *chunk_tiles = 0;
-  } else {
-    *num_splits = splits;
-    *chunk_tiles = chunk;
-  }
+// num_splits == 0: the balanced kernel.  An explicit request is honoured as given (proportional ranges per sequence).
+bool uses_balanced_kernel(const FaKvcacheParams* p) { return uses_decode_kernel(p) && p->num_splits == 0; }
+
+int64_t capacity_tiles(const FaKvcacheParams* p) {
+  return std::max<int64_t>(1, (static_cast<int64_t>(capacity_tokens(p)) + p->seqlen_new + kTileTokens - 1) / kTileTokens);
+}
+
+// CTAs per KV head: as many as are resident together, and no more than can have a share
+int balanced_shares(const FaKvcacheParams* p) {
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(kBalancedCtas / p->h_k, capacity_tiles(p) * p->b)));
+}
+
+// Parts in scratch memory: two per CTA
+size_t balanced_slots(const FaKvcacheParams* p) { return 2 * static_cast<size_t>(balanced_shares(p)) * p->h_k; }
+
+// Calls for which no scratch memory was asked before the balanced kernel: without any they run as a single split.
+bool may_lack_workspace(const FaKvcacheParams* p) {
+  return capacity_tiles(p) <= 8 || static_cast<int64_t>(p->b) * p->h_k >= 8 * 148;
+}
+
+// Parts that the keys of a sequence are attended in (balanced kernel: at most)
+int effective_splits(const FaKvcacheParams* p) {
+  if (!uses_decode_kernel(p)) return 1;
+  if (p->num_splits > 0) return std::min(p->num_splits, 256);
+  return static_cast<int>(std::min<int64_t>(balanced_shares(p), capacity_tiles(p)));
 }
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+template <int D>
+int launch_balanced(const DecodeParams& dp, dim3 grid, bool after_append, cudaStream_t stream) {
+  using C = DCfg<D>;
+  static bool configured[64] = {};
+  int dev = 0;
+  FA_CHECK_CUDA(cudaGetDevice(&dev));
+  if (!configured[dev & 63]) {
+    FA_CHECK_CUDA(cudaFuncSetAttribute(decode_balanced_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+    configured[dev & 63] = true;
+  }
+  if (after_append) {
+    FA_CHECK_CUDA(launch_overlapped(decode_balanced_kernel<D>, grid, kDecodeThreads, C::kSmemBytes, stream, dp));
+  } else {
+    decode_balanced_kernel<D><<<grid, kDecodeThreads, C::kSmemBytes, stream>>>(dp);
+    FA_CHECK_CUDA(cudaGetLastError());
+  }
+  return FA_OK;
+}
 
 template <int D>
 int launch_decode(const DecodeParams& dp, int b, int h_k, bool after_append, cudaStream_t stream) {
@@ -583,15 +1016,15 @@ int launch_decode(const DecodeParams& dp, int b, int h_k, bool after_append, cud
   int dev = 0;
   FA_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    FA_CHECK_CUDA(cudaFuncSetAttribute(decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    FA_CHECK_CUDA(cudaFuncSetAttribute(decode_split_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        C::kSmemBytes));
     configured[dev & 63] = true;
   }
   dim3 grid(dp.num_splits, h_k, b);
   if (after_append) {
-    FA_CHECK_CUDA(launch_overlapped(decode_kernel<D>, grid, kDecodeThreads, C::kSmemBytes, stream, dp));
+    FA_CHECK_CUDA(launch_overlapped(decode_split_kernel<D>, grid, kDecodeThreads, C::kSmemBytes, stream, dp));
   } else {
-    decode_kernel<D><<<grid, kDecodeThreads, C::kSmemBytes, stream>>>(dp);
+    decode_split_kernel<D><<<grid, kDecodeThreads, C::kSmemBytes, stream>>>(dp);
     FA_CHECK_CUDA(cudaGetLastError());
   }
   return FA_OK;
@@ -620,16 +1053,19 @@ extern "C" int fa_kvcache_num_splits(const FaKvcacheParams* p) {
   using namespace fa;
   int rc = validate(p, "fa_kvcache_num_splits");
   if (rc != FA_OK) return rc;
-  int splits, chunk;
-  plan_splits(p, &splits, &chunk);
-  return splits;
+  return effective_splits(p);
 }
 
 extern "C" size_t fa_kvcache_workspace_bytes(const FaKvcacheParams* p) {
   using namespace fa;
   if (validate(p, "fa_kvcache_workspace_bytes") != FA_OK) return 0;
-  int splits, chunk;
-  plan_splits(p, &splits, &chunk);
+  if (uses_balanced_kernel(p)) {
+    const int shares = balanced_shares(p);
+    if (shares <= 1) return 0;  // no sequence is shared
+    const size_t slot_rows = balanced_slots(p) * kMaxRows;
+    return align_up(slot_rows * p->d * sizeof(float), 256) + align_up(slot_rows * sizeof(float), 256);
+  }
+  const int splits = effective_splits(p);
   if (splits <= 1) return 0;
   const size_t rows = static_cast<size_t>(p->b) * p->h * p->seqlen_q;
   return align_up(static_cast<size_t>(splits) * rows * p->d * sizeof(float), 256) +
@@ -653,9 +1089,8 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   rc = check_device_sm100();
   if (rc != FA_OK) return rc;
 
-  // The three launches overlap (launch_overlapped): each kernel's set-up and launch run under its predecessor, and it waits inside
-  // for what that writes.  Append + attend + merge, one after the other against overlapped and with the batched merge: one
-  // sequence of 1500 tokens (Hq32 Hkv8 D128) 21.2 -> 14.6 us, four of up to 4000 24.8 -> 20.7, 16 of up to 8000 77.6 -> 71.4.
+  // The launches overlap (launch_overlapped): each kernel's set-up and launch run under its predecessor, and it waits inside for
+  // what that writes.
   // ---- 1. append ----
   const bool appends = p->k_new && p->seqlen_new > 0;
   const int64_t max_length = (p->block_table ? static_cast<int64_t>(p->max_blocks_per_seq) : 1) * p->seqlen_cache - p->seqlen_new;
@@ -715,8 +1150,8 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
     return run_fwd(&f, p->seqlen_new, stream, appends, verdict != nullptr);
   }
 
-  int splits, chunk;
-  plan_splits(p, &splits, &chunk);
+  const bool balanced = uses_balanced_kernel(p) && (p->workspace != nullptr || balanced_shares(p) == 1 || !may_lack_workspace(p));
+  const int splits = p->num_splits == 0 && !balanced ? 1 : effective_splits(p);
   const int64_t rows_total = static_cast<int64_t>(p->b) * p->h * p->seqlen_q;
   DecodeParams dp;
   rc = make_tensor_map_4d(&dp.tm_k, p->k_cache, p->d, p->h_k, p->seqlen_cache, p->cache_batch,
@@ -740,7 +1175,8 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
     dp.o_accum = static_cast<float*>(p->workspace);
     dp.lse_accum = reinterpret_cast<float*>(
         static_cast<uint8_t*>(p->workspace) +
-        align_up(static_cast<size_t>(splits) * rows_total * p->d * sizeof(float), 256));
+        align_up((balanced ? balanced_slots(p) * kMaxRows : static_cast<size_t>(splits) * rows_total) * p->d *
+                     sizeof(float), 256));
   }
   dp.q_batch_stride = p->q_batch_stride; dp.q_row_stride = p->q_row_stride; dp.q_head_stride = p->q_head_stride;
   dp.o_batch_stride = p->o_batch_stride; dp.o_row_stride = p->o_row_stride; dp.o_head_stride = p->o_head_stride;
@@ -756,9 +1192,16 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   dp.page_size = p->seqlen_cache;
   dp.capacity = capacity_tokens(p);
   dp.num_splits = splits;
-  dp.chunk_tiles = chunk;
+  dp.b = p->b;
+  dp.arrivals = nullptr;
   dp.checked = verdict != nullptr;
   dp.status = device_status_ptr();
+  if (balanced) {
+    dp.arrivals = next_arrival_slots();
+    if (dp.arrivals == nullptr) return set_error(FA_ERR_CUDA, "fa_kvcache: device attributes not available");
+    const dim3 grid(p->h_k, balanced_shares(p));
+    return p->d == 128 ? launch_balanced<128>(dp, grid, appends, stream) : launch_balanced<64>(dp, grid, appends, stream);
+  }
   rc = (p->d == 128) ? launch_decode<128>(dp, p->b, p->h_k, appends, stream) : launch_decode<64>(dp, p->b, p->h_k, appends, stream);
   if (rc != FA_OK) return rc;
 

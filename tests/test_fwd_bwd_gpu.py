@@ -1153,6 +1153,9 @@ def test_transforms_and_modes_still_go_to_the_class(ext, which):
         dual = torch.autograd.forward_ad.make_dual(inputs[0], torch.ones_like(inputs[0]))
         with pytest.raises((RuntimeError, NotImplementedError)):
             call(dual, *inputs[1:])
+    traced = torch.jit.trace(call, tuple(inputs), check_trace=False)
+    other = [x.flip(0).contiguous() for x in inputs]
+    assert torch.equal(traced(*other), call(*other))
     applied = []
     real = cls.apply
     try:

@@ -480,3 +480,55 @@ def test_an_error_behind_the_launch_is_not_hidden_by_a_second_try(ext, monkeypat
     monkeypatch.setattr(iface, "_gpu", NoAnswer)
     with pytest.raises(RuntimeError, match="gave no answer"):
         iface.flash_attn_with_kvcache(q, kv, kv.clone(), cache_seqlens=lens)
+
+
+@pytest.mark.parametrize("d,h,hk,new,page,lens", [
+    (128, 6, 3, 1, 0, (5000,)),                                          # one sequence over many shares
+    (64, 2, 1, 1, 256, (0, 8000, 1, 64)),                                # parts of several CTAs, empty and one-tile sequences
+    (128, 16, 4, 4, 256, (700, 63, 64, 65, 2100)),                       # sixteen rows
+    (64, 5, 5, 3, 0, tuple((37 * i) % 450 for i in range(70))),          # three rounds of lengths, shares of several sequences
+    (128, 32, 32, 1, 0, tuple(1 + (53 * i) % 130 for i in range(40))),   # nine shares per head
+    (64, 300, 300, 1, 0, (70, 1, 200)),                                  # more heads than CTAs: a share per head
+])
+def test_even_shares_equal_single_splits(ext, d, h, hk, new, page, lens):
+    """num_splits = 0 against 1.  P is rounded to fp16 against another reference maximum and O once more: 2^-11 (2 max|V| + max|O|)."""
+    from flash_attention_turing_b200 import flash_attn_with_kvcache
+
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    r = lambda *s: torch.randn(*s, generator=gen, device=DEV, dtype=torch.half)  # noqa: E731
+    b, cap = len(lens), -(-(max(lens) + new) // 256) * 256
+    q, k, v = r(b, new, h, d), r(b, new, hk, d), r(b, new, hk, d)
+    rows = (b * cap // page, page) if page else (b, cap)
+    kc, vc = r(*rows, hk, d), r(*rows, hk, d)
+    table = torch.randperm(rows[0], generator=gen, device=DEV).int().view(b, -1) if page else None
+    seqlens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+
+    def run(splits):
+        return flash_attn_with_kvcache(q, kc, vc, k, v, cache_seqlens=seqlens, block_table=table, causal=True, num_splits=splits,
+                                       return_softmax_lse=True)
+
+    (out, lse), (want, want_lse) = run(0), run(1)
+    assert (out - want).abs().max() <= 2.0 ** -11 * (2 * vc.abs().max() + want.abs().max())
+    assert (lse - want_lse).abs().max() <= 1e-4
+    for _ in range(1100 // b + 3):  # the pool of arrival counters comes round (and is left clean)
+        again, again_lse = run(0)
+    assert torch.equal(again, out) and torch.equal(again_lse, lse)
+
+
+def test_even_shares_without_scratch_memory(ext):
+    """The calls that needed no scratch memory when num_splits = 0 meant a split count from the shape still need none; others are refused."""
+    import ctypes
+    from flash_attention_turing_b200 import capi, flash_attn_with_kvcache
+
+    lib, stream = capi.lib(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    r = lambda *s: torch.randn(*s, device=DEV, dtype=torch.half)  # noqa: E731
+    for cap, ok in ((512, True), (1024, False)):
+        q, kc, vc = r(2, 1, 4, 64), r(2, cap, 2, 64), r(2, cap, 2, 64)
+        out, lse = torch.empty_like(q), torch.empty(2, 4, 1, device=DEV)
+        lens = torch.tensor([cap, 100], dtype=torch.int32, device=DEV)
+        p = capi.kvcache_params(q, kc, vc, None, None, out, lse, lens, None, 0.125, True, 0)
+        rc = lib.fa_kvcache(ctypes.byref(p), stream)
+        assert rc == (0 if ok else -3)  # FA_ERR_WORKSPACE
+        if ok:
+            want = flash_attn_with_kvcache(q, kc, vc, cache_seqlens=lens, causal=True, num_splits=1)
+            assert torch.equal(out, want)
