@@ -248,16 +248,11 @@ __device__ __forceinline__ void warp_arrive_loaded(uint64_t* bar, int lane) {
   if (lane == 0) mbar_arrive(bar);
 }
 
-__device__ __forceinline__ void store_row_fp16(__half* dst, const uint32_t (&r)[32], float mul) {
+__device__ __forceinline__ void store_scaled_rows(__half* to, int64_t row_stride, int rows, const uint32_t (&r)[32], float mul, int lane) {
+  uint32_t pk[16];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint4 v;
-    v.x = pack_half2(__uint_as_float(r[8 * i + 0]) * mul, __uint_as_float(r[8 * i + 1]) * mul);
-    v.y = pack_half2(__uint_as_float(r[8 * i + 2]) * mul, __uint_as_float(r[8 * i + 3]) * mul);
-    v.z = pack_half2(__uint_as_float(r[8 * i + 4]) * mul, __uint_as_float(r[8 * i + 5]) * mul);
-    v.w = pack_half2(__uint_as_float(r[8 * i + 6]) * mul, __uint_as_float(r[8 * i + 7]) * mul);
-    *reinterpret_cast<uint4*>(dst + i * 8) = v;
-  }
+  for (int i = 0; i < 16; ++i) pk[i] = pack_half2(__uint_as_float(r[2 * i]) * mul, __uint_as_float(r[2 * i + 1]) * mul);
+  store_rows_fp16(to, row_stride, rows, pk, lane);
 }
 
 }  // namespace

@@ -370,7 +370,7 @@ bwd_fused_kernel(const __grid_constant__ BwdKernelParams p) {
           uint32_t r[32];
           tmem_ld32(tmem_base + lane_base + kFColAcc + which * D + col_half * (D / 2) + q * 32, r);
           tmem_wait_ld();
-          if (key < sk) store_row_fp16(dst + q * 32, r, mul);
+          store_scaled_rows(dst - lane * rs + q * 32, rs, sk - (key - lane), r, mul, lane);
         }
       } else if (key < sk) {
         const uint4 z = make_uint4(0, 0, 0, 0);

@@ -507,7 +507,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
           tmem_ld32(tmem_base + lane_base + kColAcc + cq * 32, r);
           tmem_wait_ld();
           tc_fence_before_sync();
-          if (row < sq) store_row_fp16(p.dq + dq_idx, r, p.scale);
+          store_scaled_rows(p.dq + dq_idx - lane * p.dq_row_stride, p.dq_row_stride, sq - (row - lane), r, p.scale, lane);
         } else if (row < sq) {
           const uint4 z = make_uint4(0, 0, 0, 0);
 #pragma unroll
@@ -1015,7 +1015,7 @@ bwd_dkdv_kernel(const __grid_constant__ BwdKernelParams p) {
           uint32_t r[32];
           tmem_ld32(tmem_base + lane_base + kColAcc + which * D + col_half * (D / 2) + q * 32, r);
           tmem_wait_ld();
-          if (key < w.sk) store_row_fp16(dst + q * 32, r, mul);
+          store_scaled_rows(dst - lane * rs + q * 32, rs, w.sk - (key - lane), r, mul, lane);
         }
         tc_fence_before_sync();
       } else if (key < w.sk) {
@@ -1373,7 +1373,7 @@ bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
           uint32_t r[32];
           tmem_ld32(tmem_base + lane_base + kColAcc + which * D + col_half * (D / 2) + q * 32, r);
           tmem_wait_ld();
-          if (key < sk) store_row_fp16(dst + q * 32, r, mul);
+          store_scaled_rows(dst - lane * rs + q * 32, rs, sk - (key - lane), r, mul, lane);
         }
       } else if (key < sk) {
         const uint4 z = make_uint4(0, 0, 0, 0);
