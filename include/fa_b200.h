@@ -202,9 +202,9 @@ int fa_bwd_stages(const FaBwdParams* p, int stage_mask, fa_stream_t stream);
 /* (:995-1218) with kvcache_decode_split_kernel / kvcache_split_kernel /                         */
 /* kvcache_split_kernel_legacy (:148-674) and kvcache_combine_kernel (:676-780).                 */
 /* No host synchronisation: the capacity check of the reference (flash_api.cpp:627) is the       */
-/* caller's responsibility.  num_splits == 0: the keys of the whole batch are shared out evenly   */
-/* over the GPU, on the device, from the lengths (choose_num_splits, kvcache_native.cu:913-952,    */
-/* picks a count from the shape).                                                                */
+/* caller's responsibility.  num_splits == 0: up to 8 query rows per KV head, the keys of the     */
+/* whole batch are shared out evenly over the GPU, on the device, from the lengths; more rows: a  */
+/* split count from the shape (choose_num_splits, kvcache_native.cu:913-952, for 148 SMs).         */
 /* Scratch: fa_kvcache_workspace_bytes() bytes when the effective split count exceeds 1.  With     */
 /* num_splits == 0, at most 512 tokens of capacity or at least 1184 (sequence, KV head) pairs,     */
 /* workspace may be NULL: every sequence is then attended in one piece.                           */
