@@ -169,6 +169,13 @@ constexpr int kDqSchedWarp = 19;
 constexpr int kDqReaders = kComputeWarps + 3;  // elementwise warps, producer warp, two MMA threads
 static_assert((kDqThreads / 32 + 3) / 4 * 32 * 96 <= 16384, "register file of one SM sub-partition");
 
+// dQ of an item is stored at the end of the first block of the next one: its last product ends 900 to 2500 clocks after its last dS, and
+// the elementwise warps, who have the next S and dP waiting, do not stand by.  The accumulator is written again only behind that
+// (acc_free).  Three items are in shared memory then: the one to be stored, the current one, and the next, whose tiles are being fetched.
+// dQ kernel: 64 texts H16 D64 98.9 -> 96.0 us, D128 133.7 -> 130.4, B4 S4096 H32 D128 710 -> 670 (power-capped), B16 S1024 251 -> 247, long
+// rows the same.  The dK/dV kernel got slower by as much in the same form (B16 S1024 347 -> 372: more code, spills in packed batches).
+constexpr int kItemSlots = 3;
+
 // A work item with everything the roles derive from it, filled in once by the scheduler thread.
 struct __align__(16) DqItem {
   int nb;  // key blocks to visit; < 0: no more work
@@ -183,8 +190,9 @@ struct DqBarriers {
   // the arithmetic of block g (S and dP are handed back before it), and on one barrier its second arrival would stand for the other
   // warp's first: dQ(g) on half a dS.  For block g + 2, the next on the same barrier, dP(g+2) has waited for dQ(g).
   uint64_t ds_full[2];
-  uint64_t sched_full[2], sched_empty[2], sched_go;
-  DqItem items[2];
+  uint64_t acc_free;        // the accumulator of the item before has been read (see kItemSlots)
+  uint64_t sched_full[kItemSlots], sched_empty[kItemSlots], sched_go;
+  DqItem items[kItemSlots];
 };
 static_assert(sizeof(DqBarriers) <= 1024, "barrier block");
 
@@ -229,8 +237,9 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
   if (warp == kProducerWarp && lane == 0) {
     init_barriers(bars, C::kStagesK, 2, 1);
     mbar_init(&xb->q_free, 1 + kComputeWarps);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&xb->ds_full[i], kComputeWarps);
+    mbar_init(&xb->acc_free, kComputeWarps);
+    for (int i = 0; i < 2; ++i) mbar_init(&xb->ds_full[i], kComputeWarps);
+    for (int i = 0; i < kItemSlots; ++i) {
       mbar_init(&xb->sched_full[i], 1);
       mbar_init(&xb->sched_empty[i], kDqReaders);
     }
@@ -250,8 +259,8 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
   const uint32_t tmem_base = bars->tmem_base;
   WaitCtx ctx{&bars->abort_flag, p.status};
 
-  auto wait_item = [&](int n) -> bool { return mbar_wait(&xb->sched_full[n & 1], (n >> 1) & 1, ctx); };
-  auto release_item = [&](int n) { mbar_arrive(&xb->sched_empty[n & 1]); };
+  auto wait_item = [&](int n) -> bool { return mbar_wait(&xb->sched_full[n % kItemSlots], (n / kItemSlots) & 1, ctx); };
+  auto release_item = [&](int n) { mbar_arrive(&xb->sched_empty[n % kItemSlots]); };
 
   if (stop) {
   } else if (warp == kDqSchedWarp) {
@@ -288,9 +297,9 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
           }
           next = gridDim.x + atomicAdd(p.sched, 1);
         }
-        if (!mbar_wait(&xb->sched_empty[n & 1], ((n >> 1) & 1) ^ 1, ctx)) break;
-        xb->items[n & 1] = it;
-        mbar_arrive(&xb->sched_full[n & 1]);
+        if (!mbar_wait(&xb->sched_empty[n % kItemSlots], ((n / kItemSlots) & 1) ^ 1, ctx)) break;
+        xb->items[n % kItemSlots] = it;
+        mbar_arrive(&xb->sched_full[n % kItemSlots]);
         if (it.nb < 0) {
           finished = true;
           break;
@@ -309,7 +318,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
     for (int n = 0;; ++n) {
       bool ok = wait_item(n);
       if (!__all_sync(0xffffffffu, ok)) break;
-      const DqItem w = xb->items[n & 1];
+      const DqItem w = xb->items[n % kItemSlots];
       __syncwarp();
       if (lane == 0) release_item(n);
       if (w.nb < 0) break;
@@ -348,10 +357,10 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
         const int g = G + w.nb - 1, s = g % C::kStagesK;
         if (!mbar_wait_warp(&bars->a_full[s], (g / C::kStagesK) & 1, ctx)) break;
         zero_tile_rows_from<D>(sK + s * C::kTileBytes, w.sk - (w.nb - 1) * kBlock, lane);
-        // Two barriers in turn: with short items this warp can be a whole item ahead of the accumulating thread, and
-        // on one barrier that thread would then wait for a phase that is over and comes round only after it has
-        // moved on.  It cannot be two ahead: item n + 2 is published when the epilogue of item n is done.
-        if (lane == 0) mbar_arrive(&bars->tail_fixed[nf & 1]);
+        // Barriers in turn: with short items this warp can be ahead of the accumulating thread, and on one barrier that thread
+        // would then wait for a phase that is over and comes round only after it has moved on.  It cannot be kItemSlots items
+        // ahead: that item is published when dQ of this one has been stored.
+        if (lane == 0) mbar_arrive(&bars->tail_fixed[nf % kItemSlots]);
         ++nf;
       }
       G += w.nb;
@@ -366,7 +375,7 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
       bool ok = true;
       for (int n = 0; ok; ++n) {
         if (!(ok = wait_item(n))) break;
-        const int nb = xb->items[n & 1].nb;
+        const int nb = xb->items[n % kItemSlots].nb;
         release_item(n);
         if (nb < 0) break;
         if (nb <= 2) mbar_arrive(&xb->sched_go);  // short item: claim the next one right away
@@ -398,11 +407,11 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
   } else if (warp == kAccMmaWarp) {
     if (elect_one()) {
       constexpr uint32_t idesc_acc = make_idesc_f16(128, D, false, true);
-      int G = 0, nf = 0;
+      int G = 0, nf = 0, na = 0;
       bool ok = true;
       for (int n = 0; ok; ++n) {
         if (!(ok = wait_item(n))) break;
-        const int nb = xb->items[n & 1].nb, fix_k_tail = xb->items[n & 1].fix_k_tail;
+        const int nb = xb->items[n % kItemSlots].nb, fix_k_tail = xb->items[n % kItemSlots].fix_k_tail;
         release_item(n);
         if (nb < 0) break;
         if (nb == 0) continue;
@@ -411,9 +420,10 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
           // dS(g) written implies that K(g) has landed: S(g) read it, and the elementwise warps have seen S(g)
           if (!(ok = mbar_wait(&xb->ds_full[g & 1], (g >> 1) & 1, ctx))) break;
           if (fix_k_tail && j == nb - 1) {
-            if (!(ok = mbar_wait(&bars->tail_fixed[nf & 1], (nf >> 1) & 1, ctx))) break;
+            if (!(ok = mbar_wait(&bars->tail_fixed[nf % kItemSlots], (nf / kItemSlots) & 1, ctx))) break;
             ++nf;
           }
+          if (j == 0 && na++ > 0 && !(ok = mbar_wait(&xb->acc_free, na & 1, ctx))) break;  // phase na - 2 of the items before
           tc_fence_after_sync();
           gemm_ts<D>(tmem_base + kColAcc, tmem_base + kColPacked + (g & 1) * 64, smem_u32(sK + s * C::kTileBytes),
                      idesc_acc, j == 0);
@@ -433,90 +443,101 @@ bwd_dq_kernel(const __grid_constant__ BwdKernelParams p) {
     const uint32_t tDP = tmem_base + lane_base + kColDP + cq * 32;
     const float c = p.scale_log2;
     const float2 c2 = make_float2(c, c);
-    int G = 0, ni = 0;
+    int G = 0, ni = 0, pending = -1;  // pending: the item whose dQ is still to be stored
     bool ok = true;
     for (int n = 0; ok; ++n) {
       ok = wait_item(n);
       if (!(ok = __all_sync(0xffffffffu, ok))) break;
-      const DqItem* it = &xb->items[n & 1];  // stays in its slot until this warp releases it
+      const DqItem* it = &xb->items[n % kItemSlots];  // stays in its slot until this warp has stored its dQ
       const int nb = it->nb, sk = it->sk, shift = it->shift, row = it->row0 + row_in_tile;
-      if (nb < 0) break;
       float2 nl2 = make_float2(0.f, 0.f), nd2 = make_float2(0.f, 0.f);
-      for (int j = 0; j < nb; ++j) {
-        const int g = G + j;
-        // dP(g) complete: S and dP are there and packed-dS buffer g & 1 is free.  S and dP are fetched at once and handed back together, then the arithmetic of the block runs under the next products.
-        if (!(ok = mbar_wait_warp(&bars->dp_full, g & 1, ctx))) break;
-        tc_fence_after_sync();
-        uint32_t sr[32], dr[32];
-        tmem_ld32(tS, sr);
-        tmem_ld32(tDP, dr);
-        if (j == 0) {  // S(0) of the item was issued after its statistics had landed
-          const float l = sStats[row_in_tile], dl = sStats[128 + row_in_tile];
-          nl2 = make_float2(l, l), nd2 = make_float2(dl, dl);
-        }
-        tmem_wait_ld();
-        warp_arrive_loaded(&bars->s_loaded, lane);
-        if (j == 0 && lane == 0) mbar_arrive(&xb->q_free);  // the statistics are in registers
-        schedule_barrier(lane);
-        const int col0 = j * kBlock + cq * 32;
-        int limit = sk - 1 - col0;
-        if (p.is_causal) limit = min(limit, row + shift - col0);
-        float2 pr[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float2 x = ffma2(make_float2(__uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1])), c2, nl2);
-          pr[i] = exp2_pair(x);
-        }
-        if (limit < 31) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            if (2 * i > limit) pr[i].x = 0.f;
-            if (2 * i + 1 > limit) pr[i].y = 0.f;
-          }
-        }
-        uint32_t pk[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float2 d = fmul2(pr[i], fadd2(make_float2(__uint_as_float(dr[2 * i]), __uint_as_float(dr[2 * i + 1])), nd2));
-          pk[i] = pack_half2(d.x, d.y);
-        }
-        if (limit < 31) {  // by selection: dP of a masked column may be NaN/Inf (rows of the next sequence in V)
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            if (2 * i > limit) pk[i] &= 0xffff0000u;
-            if (2 * i + 1 > limit) pk[i] &= 0x0000ffffu;
-          }
-        }
-        tmem_st16(tmem_base + lane_base + kColPacked + (g & 1) * 64 + cq * 16, pk);
-        warp_arrive(&xb->ds_full[g & 1], lane);
-      }
-      if (!ok) break;
-      // ---- epilogue: dQ = scale * acc ----
-      const bool stores = cq < D / 32;
-      const int64_t dq_idx = it->bq * p.dq_batch_stride + static_cast<int64_t>(it->q_off + row) * p.dq_row_stride +
-                             it->head * p.dq_head_stride + cq * 32;
-      const int sq = it->sq;
-      if (nb > 0) {
-        if (!(ok = mbar_wait_warp(&bars->acc_full, ni & 1, ctx))) break;
-        ++ni;
-      }
-      if (stores) {
-        if (nb > 0) {
+      int j = 0;
+      do {
+        if (j < nb) {
+          const int g = G + j;
+          // dP(g) complete: S and dP are there and packed-dS buffer g & 1 is free.  S and dP are fetched at once and handed back together, then the arithmetic of the block runs under the next products.
+          if (!(ok = mbar_wait_warp(&bars->dp_full, g & 1, ctx)))
+            break;
           tc_fence_after_sync();
-          uint32_t r[32];
-          tmem_ld32(tmem_base + lane_base + kColAcc + cq * 32, r);
+          uint32_t sr[32], dr[32];
+          tmem_ld32(tS, sr);
+          tmem_ld32(tDP, dr);
+          if (j == 0) {  // S(0) of the item was issued after its statistics had landed
+            const float l = sStats[row_in_tile], dl = sStats[128 + row_in_tile];
+            nl2 = make_float2(l, l), nd2 = make_float2(dl, dl);
+          }
           tmem_wait_ld();
-          tc_fence_before_sync();
-          store_scaled_rows(p.dq + dq_idx - lane * p.dq_row_stride, p.dq_row_stride, sq - (row - lane), r, p.scale, lane);
-        } else if (row < sq) {
-          const uint4 z = make_uint4(0, 0, 0, 0);
+          warp_arrive_loaded(&bars->s_loaded, lane);
+          if (j == 0 && lane == 0) mbar_arrive(&xb->q_free);  // the statistics are in registers
+          schedule_barrier(lane);
+          const int col0 = j * kBlock + cq * 32;
+          int limit = sk - 1 - col0;
+          if (p.is_causal) limit = min(limit, row + shift - col0);
+          float2 pr[16];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(p.dq + dq_idx + i * 8) = z;
+          for (int i = 0; i < 16; ++i) {
+            const float2 x = ffma2(make_float2(__uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1])), c2, nl2);
+            pr[i] = exp2_pair(x);
+          }
+          if (limit < 31) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              if (2 * i > limit) pr[i].x = 0.f;
+              if (2 * i + 1 > limit) pr[i].y = 0.f;
+            }
+          }
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float2 d = fmul2(pr[i], fadd2(make_float2(__uint_as_float(dr[2 * i]), __uint_as_float(dr[2 * i + 1])), nd2));
+            pk[i] = pack_half2(d.x, d.y);
+          }
+          if (limit < 31) {  // by selection: dP of a masked column may be NaN/Inf (rows of the next sequence in V)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              if (2 * i > limit) pk[i] &= 0xffff0000u;
+              if (2 * i + 1 > limit) pk[i] &= 0x0000ffffu;
+            }
+          }
+          tmem_st16(tmem_base + lane_base + kColPacked + (g & 1) * 64 + cq * 16, pk);
+          warp_arrive(&xb->ds_full[g & 1], lane);
         }
+        // ---- epilogue of the item before: dQ = scale * acc ----
+        if (j == 0 && pending >= 0) {
+          if (!(ok = mbar_wait_warp(&bars->acc_full, ni & 1, ctx))) break;
+          ++ni;
+          tc_fence_after_sync();
+          if (cq < D / 32) {
+            const DqItem* done = &xb->items[pending % kItemSlots];
+            const int first = done->row0 + quarter * 32;
+            uint32_t r[32];
+            tmem_ld32(tmem_base + lane_base + kColAcc + cq * 32, r);
+            tmem_wait_ld();
+            store_scaled_rows(p.dq + done->bq * p.dq_batch_stride + static_cast<int64_t>(done->q_off + first) * p.dq_row_stride +
+                                  done->head * p.dq_head_stride + cq * 32,
+                              p.dq_row_stride, done->sq - first, r, p.scale, lane);
+          }
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&xb->acc_free);
+          if (lane == 0) release_item(pending);
+          pending = -1;
+        }
+      } while (++j < nb);
+      if (!ok || nb < 0) break;
+      if (nb > 0) {
+        pending = n;
+        G += nb;
+      } else {  // no key is visible to any row
+        if (cq < D / 32 && row < it->sq) {
+          __half* to = p.dq + it->bq * p.dq_batch_stride + static_cast<int64_t>(it->q_off + row) * p.dq_row_stride +
+                       it->head * p.dq_head_stride + cq * 32;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(to + i * 8) = make_uint4(0, 0, 0, 0);
+        }
+        __syncwarp();
+        if (lane == 0) release_item(n);
       }
-      G += nb;
-      __syncwarp();
-      if (lane == 0) release_item(n);
     }
   }
 

@@ -134,6 +134,96 @@ def _walk_v_tail(n_fixed):
     return len(seen)
 
 
+def _walk_deferred_store(lengths, gate, n_tail, slots):
+    """dQ of an item is read by the elementwise warps at the end of the first block of the next item (or at the very end); every item
+    has a tail to zero.  gate: the accumulating thread waits until it has been read; n_tail: barriers of the zeroed tail in turn;
+    slots: items published at a time.  Faults: an accumulator written before it is read, a wait that never ends."""
+    first = [sum(lengths[:k]) for k in range(len(lengths))]
+    total, items = sum(lengths), len(lengths)
+    item_of = [k for k, n in enumerate(lengths) for _ in range(n)]
+    names = ["dp_full", "s_loaded", "ds_free0", "ds_free1", "ds_full0", "ds_full1", "acc_full", "acc_free"] + [f"tail{i}" for i in range(n_tail)]
+    need = {n: WARPS if n in ("s_loaded", "ds_full0", "ds_full1", "acc_free") else 1 for n in names}
+    index = {n: i for i, n in enumerate(names)}
+
+    def arrive(bars, name):
+        phases, count = bars[index[name]]
+        state = ((phases + 1) % 4, 0) if count + 1 == need[name] else (phases, count + 1)
+        return bars[: index[name]] + (state,) + bars[index[name] + 1:]
+
+    def passed(bars, name, phase):
+        return bars[index[name]][0] % 2 != phase % 2
+
+    # warp: (block, step), steps 0 load, 1 dS handed over, 2 read dQ of the item before; block `total`: only step 2 is left
+    start = (((0, 0),) * WARPS, 0, 0, 0, 0, 0, tuple((0, 0) for _ in names))
+    seen, todo = {start}, [start]
+    while todo:
+        state = todo.pop()
+        warps, prod, ss, acc, ss_flying, dq_flying, bars = state
+        nexts = []
+        read = lambda w: (item_of[w[0]] if w[0] < total else items) - (1 if w[1] < 3 else 0)  # noqa: E731  items a warp has read
+        done = [read(w) if w[0] < total and w[0] == first[item_of[w[0]]] else item_of[w[0]] if w[0] < total else
+                items - (w[1] < 3) for w in warps]
+        for w, (g, step) in enumerate(warps):
+            put = lambda v, b: nexts.append((warps[:w] + (v,) + warps[w + 1:], prod, ss, acc, ss_flying, dq_flying, b))  # noqa: E731
+            starts = g < total and g == first[item_of[g]] and g > 0
+            if g < total and step == 0 and passed(bars, "dp_full", g):
+                put((g, 1), arrive(bars, "s_loaded"))
+            elif g < total and step == 1:
+                put((g, 2) if starts else (g + 1, 2 if g + 1 == total else 0), arrive(bars, f"ds_full{g % 2}"))
+            elif step == 2 and passed(bars, "acc_full", (items if g == total else item_of[g]) - 1):
+                put((g, 3) if g == total else (g + 1, 2 if g + 1 == total else 0), arrive(bars, "acc_free"))
+        # the tiles of an item: its slot is free, Q and dO of the item before have been read, its statistics too
+        if prod < items and (prod < slots or min(done) > prod - slots) and (
+                prod == 0 or (ss >= first[prod - 1] + lengths[prod - 1] and all(w[0] > first[prod - 1] or w[1] > 0 and w[0] == first[prod - 1] for w in warps))):
+            nexts.append((warps, prod + 1, ss, acc, ss_flying, dq_flying, arrive(bars, f"tail{prod % n_tail}")))
+        if ss < total and prod > item_of[ss] and (ss == 0 or passed(bars, "s_loaded", ss - 1)) and (
+                ss < 2 or passed(bars, f"ds_free{ss % 2}", ss // 2 - 1)):
+            nexts.append((warps, prod, ss + 1, acc, ss_flying + 1, dq_flying, bars))
+        if acc < total and passed(bars, f"ds_full{acc % 2}", acc // 2):
+            k = item_of[acc]
+            begins, ends = acc == first[k], acc == first[k] + lengths[k] - 1
+            if (not ends or passed(bars, f"tail{k % n_tail}", k // n_tail)) and (
+                    not (gate and begins and k > 0) or passed(bars, "acc_free", k - 1)):
+                if begins and min(done) < k:
+                    raise _Fault(f"dQ of item {k} written over that of item {min(done)}")
+                nexts.append((warps, prod, ss, acc + 1, ss_flying, dq_flying + 1, bars))
+        if ss_flying:
+            nexts.append((warps, prod, ss, acc, ss_flying - 1, dq_flying, arrive(bars, "dp_full")))
+        if dq_flying:
+            g = acc - dq_flying
+            after = arrive(bars, f"ds_free{g % 2}")
+            if g == first[item_of[g]] + lengths[item_of[g]] - 1:
+                after = arrive(after, "acc_full")
+            nexts.append((warps, prod, ss, acc, ss_flying, dq_flying - 1, after))
+        if not nexts and any(w != (total, 3) for w in warps):
+            raise _Fault(f"stuck: warps {warps}, dQ({acc}) next, producer at item {prod}")
+        for n in nexts:
+            if n not in seen:
+                seen.add(n)
+                todo.append(n)
+    return len(seen)
+
+
+def _item_slots():
+    return int(re.search(r"constexpr int kItemSlots = (\d+);", (CSRC / "bwd_sm100.cu").read_text()).group(1))
+
+
+LENGTHS = [(1, 1, 1, 1, 1, 1, 1), (2, 1, 1, 2, 1, 1), (1, 3, 1, 1, 2)]
+
+
+@pytest.mark.parametrize("lengths", LENGTHS)
+def test_dq_of_an_item_is_stored_before_the_next_one_writes_over_it(lengths):
+    assert re.search(r"&xb->acc_free, na & 1", (CSRC / "bwd_sm100.cu").read_text())
+    assert _walk_deferred_store(lengths, True, _item_slots(), _item_slots()) > 20
+
+
+def test_the_deferred_store_needs_its_barriers():
+    with pytest.raises(_Fault, match="written over"):
+        _walk_deferred_store(LENGTHS[0], False, 3, 3)
+    with pytest.raises(_Fault, match="stuck"):
+        _walk_deferred_store(LENGTHS[0], True, 1, 3)
+
+
 HANDOVERS = [(_walk_dq, "bwd_sm100.cu", "DqBarriers", "ds_full"), (_walk_v_tail, "fwd_sm100.cu", "Barriers", "v_fixed")]
 
 
