@@ -998,6 +998,11 @@ int balanced_shares(const FaKvcacheParams* p) {
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(kBalancedCtas / p->h_k, capacity_tiles(p) * p->b)));
 }
 
+// Whatever the lengths, no sequence is cut: each is in one CTA's share
+bool never_cut(const FaKvcacheParams* p) {
+  return balanced_shares(p) == 1 || (capacity_tiles(p) <= kWholeTiles && p->b <= balanced_shares(p));
+}
+
 // Parts in scratch memory: two per CTA
 size_t balanced_slots(const FaKvcacheParams* p) { return 2 * static_cast<size_t>(balanced_shares(p)) * p->h_k; }
 
@@ -1041,7 +1046,7 @@ void plan_splits(const FaKvcacheParams* p, int* num_splits, int* chunk_tiles) {
 
 // Parts that the keys of a sequence are attended in (balanced kernel: at most)
 int effective_splits(const FaKvcacheParams* p) {
-  if (uses_balanced_kernel(p)) return static_cast<int>(std::min<int64_t>(balanced_shares(p), capacity_tiles(p)));
+  if (uses_balanced_kernel(p)) return never_cut(p) ? 1 : static_cast<int>(std::min<int64_t>(balanced_shares(p), capacity_tiles(p)));
   int splits, chunk;
   plan_splits(p, &splits, &chunk);
   return splits;
@@ -1119,8 +1124,7 @@ extern "C" size_t fa_kvcache_workspace_bytes(const FaKvcacheParams* p) {
   using namespace fa;
   if (validate(p, "fa_kvcache_workspace_bytes") != FA_OK) return 0;
   if (uses_balanced_kernel(p)) {
-    const int shares = balanced_shares(p);
-    if (shares <= 1) return 0;  // no sequence is shared
+    if (never_cut(p)) return 0;
     const size_t slot_rows = balanced_slots(p) * kMaxRows;
     return align_up(slot_rows * p->d * sizeof(float), 256) + align_up(slot_rows * sizeof(float), 256);
   }
@@ -1209,7 +1213,7 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
     return run_fwd(&f, p->seqlen_new, stream, appends, verdict != nullptr);
   }
 
-  const bool balanced = uses_balanced_kernel(p) && (p->workspace != nullptr || balanced_shares(p) == 1 || !may_lack_workspace(p));
+  const bool balanced = uses_balanced_kernel(p) && (p->workspace != nullptr || never_cut(p) || !may_lack_workspace(p));
   int splits = effective_splits(p), chunk = 0;
   if (!balanced && !uses_balanced_kernel(p)) plan_splits(p, &splits, &chunk);
   if (!balanced && uses_balanced_kernel(p)) splits = 1;  // no scratch memory (may_lack_workspace)
