@@ -148,11 +148,11 @@ std::vector<at::Tensor> mha_varlen_fwd(at::Tensor q, at::Tensor k, at::Tensor v,
   c10::cuda::CUDAGuard guard(q.device());
 
   at::Tensor out = torch::empty_like(q);
-  at::Tensor l = torch::zeros({batch_size, num_heads, max_seqlen_q}, q.options().dtype(torch::kFloat32));
-  if (q.size(0) == 0 || k.size(0) == 0 || max_seqlen_q <= 0) return {out.zero_(), l};
+  at::Tensor l = torch::empty({batch_size, num_heads, max_seqlen_q}, q.options().dtype(torch::kFloat32));
+  if (q.size(0) == 0 || k.size(0) == 0 || max_seqlen_q <= 0) return {out.zero_(), l.zero_()};
 
   FaFwdParams p = {};
-  p.flags = FA_FWD_ZERO_UNUSED_ROWS;  // rows outside every sequence are zero, as in the reference
+  p.flags = FA_FWD_ZERO_UNUSED_ROWS;  // rows outside every sequence are zero, as in the reference, in O and in the LSE
   p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr(); p.o = out.data_ptr();
   p.lse = l.data_ptr<float>();
   p.q_row_stride = q.stride(0); p.q_head_stride = q.stride(1); p.q_batch_stride = 0;

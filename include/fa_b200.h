@@ -31,8 +31,8 @@ extern "C" {
 /* Same underlying type as cudaStream_t (struct CUstream_st*); void* keeps the header CUDA-free. */
 typedef void* fa_stream_t;
 
-/* FaFwdParams.flags: packed (varlen) calls also set the rows of o outside every sequence to zero; without it they are left
- * as they are.  FA_BWD_ZERO_UNUSED_ROWS does the same for dq, dk, dv (and for keys past max_seqlen_k). */
+/* FaFwdParams.flags: packed (varlen) calls also set the rows of o outside every sequence to zero, and lse from the end of each
+ * sequence up to seqlen_q; without it they are left as they are.  FA_BWD_ZERO_UNUSED_ROWS does the same for dq, dk, dv (and for keys past max_seqlen_k). */
 #define FA_FWD_ZERO_UNUSED_ROWS 1
 
 #define FA_CAUSAL_SHIFT 2 /* value of is_causal: the causal diagonal is given by causal_shift */

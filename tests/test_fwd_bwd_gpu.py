@@ -1174,3 +1174,29 @@ def test_transforms_and_modes_still_go_to_the_class(ext, which):
     finally:
         del cls.apply
     assert torch.equal(call(*inputs), cls.apply(*inputs, *extra, *rest, False))
+
+
+@pytest.mark.parametrize("lens", [(1, 1023, 1024), (1025, 0, 3), (2100, 700), (5,) * 300])
+def test_lse_past_the_end_of_a_sequence_is_zero(ext, lens):
+    """Whatever the memory held before, by the binding and by the flag of the C entry; without the flag it is left alone."""
+    from flash_attention_turing_b200 import capi
+
+    gen = torch.Generator().manual_seed(4)
+    h, d, longest = 3, 64, max(lens) + 1
+    q, k, v = (randn_half(gen, sum(lens), h, d).to(DEV) for _ in range(3))
+    cu = torch.tensor([0, *lens], dtype=torch.int32).cumsum(0, dtype=torch.int32).to(DEV)
+    inside = torch.arange(longest, device=DEV)[None, None] < torch.tensor(lens, device=DEV)[:, None, None].expand(-1, h, 1)
+    for _ in range(3):
+        junk = [torch.full((len(lens), h, longest), float("nan"), device=DEV) for _ in range(4)]
+        torch.cuda.synchronize()
+        del junk  # the allocator hands this memory out for the LSE
+        _, lse = ext.varlen_fwd(q, k, v, cu, cu, longest, longest, d ** -0.5, True)
+        assert torch.isfinite(lse).all() and (lse[~inside] == 0).all()
+    for flags in (0, capi.FA_FWD_ZERO_UNUSED_ROWS):
+        out, got = torch.empty_like(q), torch.full_like(lse, 7.0)
+        p = capi.fwd_params(*(x[None] for x in (q, k, v, out)), got, d ** -0.5, True)
+        p.b, p.seqlen_q, p.seqlen_k, p.lse_row_stride = len(lens), longest, longest, longest
+        p.cu_seqlens_q = p.cu_seqlens_k = cu.data_ptr()
+        p.total_q, p.total_k, p.flags = q.shape[0], k.shape[0], flags
+        capi.check(capi.lib().fa_fwd(ctypes.byref(p), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        assert torch.equal(got[inside], lse[inside]) and (got[~inside] == (0 if flags else 7)).all()
