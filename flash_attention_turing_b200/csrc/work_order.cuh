@@ -15,9 +15,10 @@ namespace fa {
 // Bytes of streamed rows (K and V; for dK/dV Q and dO) per section: well below the 126 MB of L2, half of which is each die's.
 constexpr int64_t kSectionBytes = 32 << 20;
 
-// Host: rows of `row_bytes` that a section may hold.  Without a causal mask all items of a head are equal: one head per section.
-inline int section_rows(bool causal, int64_t row_bytes) {
-  return causal ? static_cast<int>(kSectionBytes / row_bytes) : 0;
+// Host: rows of `row_bytes` that a section may hold; 0, a head (or group) per section, where the order gains nothing because all items of a
+// head are equal or nearly so: no causal mask, or few queries at the end of many keys.
+inline int section_rows(bool causal, int seqlen_q, int seqlen_k, int64_t row_bytes) {
+  return causal && 4 * static_cast<int64_t>(seqlen_q) >= seqlen_k ? static_cast<int>(kSectionBytes / row_bytes) : 0;
 }
 
 #ifdef __CUDACC__
@@ -26,6 +27,10 @@ struct HeadPlace {
 };
 // Item r of `heads` heads with `count` items each, in units of `unit` heads that share their streamed rows (of which there are `rows`).
 __device__ __forceinline__ HeadPlace section_item(int r, int heads, int count, int unit, int rows, int rows_per_section) {
+  if (rows_per_section == 0) {
+    const int group = r / (unit * count), rest = r - group * unit * count, place = unit == 1 ? rest : rest / unit;
+    return {group * unit + rest - place * unit, place};
+  }
   if (static_cast<int64_t>(rows) * heads <= static_cast<int64_t>(rows_per_section) * unit) {  // one section: a division, not four (64 packed texts 103 -> 100 us)
     const int place = r / heads;
     return {r - place * heads, place};
