@@ -17,14 +17,11 @@ thread_local std::string g_last_error;
 __device__ int g_device_status;
 
 __device__ int g_sched_slots[2 * kSchedSlots];
-__device__ int g_arrival_slots[kArrivalLaunches * kArrivalSlots];
 
 constexpr int kMaxDevices = 64;
 int* g_status_ptr[kMaxDevices] = {};
 int* g_sched_ptr[kMaxDevices] = {};
 unsigned g_sched_next[kMaxDevices] = {};
-int* g_arrival_ptr[kMaxDevices] = {};
-unsigned g_arrival_next[kMaxDevices] = {};
 int g_sm_count[kMaxDevices] = {};
 int g_sm100_ok[kMaxDevices] = {};  // 0 unknown, 1 yes, -1 no
 std::mutex g_mutex;
@@ -123,18 +120,6 @@ int* next_sched_slot() {
   return g_sched_ptr[dev] + 2 * (g_sched_next[dev]++ % kSchedSlots);
 }
 
-int* next_arrival_slots() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-  std::lock_guard<std::mutex> lock(g_mutex);
-  if (!g_arrival_ptr[dev]) {
-    void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_arrival_slots) != cudaSuccess) return nullptr;
-    g_arrival_ptr[dev] = static_cast<int*>(p);
-  }
-  return g_arrival_ptr[dev] + kArrivalSlots * (g_arrival_next[dev]++ % kArrivalLaunches);
-}
-
 int device_sm_count() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
@@ -167,8 +152,6 @@ int fa_device_status(int reset) {
     void* slots = nullptr;  // a launch that gave up leaves its work counters dirty
     FA_CHECK_CUDA(cudaGetSymbolAddress(&slots, fa::g_sched_slots));
     FA_CHECK_CUDA(cudaMemset(slots, 0, sizeof(int) * 2 * fa::kSchedSlots));
-    FA_CHECK_CUDA(cudaGetSymbolAddress(&slots, fa::g_arrival_slots));
-    FA_CHECK_CUDA(cudaMemset(slots, 0, sizeof(int) * fa::kArrivalLaunches * fa::kArrivalSlots));
   }
   return value;
 }

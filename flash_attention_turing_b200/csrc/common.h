@@ -50,12 +50,6 @@ int* device_status_ptr();
 constexpr int kSchedSlots = 1024;
 int* next_sched_slot();
 
-// The same for the balanced decode kernel: kArrivalSlots zeroed counters per launch (a launch has at most that many CTAs), a pool of
-// kArrivalLaunches launches.
-constexpr int kArrivalSlots = 296;
-constexpr int kArrivalLaunches = 1024;
-int* next_arrival_slots();
-
 // Number of SMs of the current device (cached); 0 on error.
 int device_sm_count();
 

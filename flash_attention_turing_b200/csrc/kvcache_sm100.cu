@@ -61,7 +61,7 @@ struct DecodeParams {
   int checked;       // the host refuses lengths beyond the capacity: neither read nor reported
   int chunk_tiles;   // split kernel: > 0: split s owns tiles [s*chunk, (s+1)*chunk); 0: proportional ranges
   int b;             // sequences
-  int* arrivals;     // balanced kernel: one zeroed counter per CTA, zero again at the end
+  int* arrivals;     // balanced kernel: a counter per CTA in scratch memory, zeroed by the kernel before
   int* status;
 };
 
@@ -485,7 +485,8 @@ decode_split_kernel(const __grid_constant__ DecodeParams p) {
 // next to each other in memory (a share of (sequence, head) pairs laid end to end, with heads far apart in time, read 3-10 % more slowly).
 // A share holds the end of a sequence, whole ones and the beginning of another; the parts of a sequence that several CTAs
 // share go to scratch memory (at most two per CTA), and the CTA that arrives last merges them, in the order of the tiles, so that the
-// result does not depend on who that is.
+// result does not depend on who that is.  Arrivals are counted in the call's own scratch memory, which calls that overlap do not share,
+// and which the kernel before this one (append or prepare kernel) has zeroed.
 // Bound by the K / V bytes for large batches, by a chain of latencies (lengths, Q and K / V tiles, merge) for small ones.  Append and
 // attention, us, chunks of a fixed size per CTA and a merge kernel against this: 1 x 1500 tokens (Hq32 Hkv8 D128) 13.2 -> 10.4,
 // 1 x 30000 42.1 -> 32.8, 16 x 1000-8000 56.3 -> 49.6 (6.0 TB/s), 64 x 1024-32768 620 -> 621 (6.9 TB/s), 128 x 20-64 (H32) 69.8 -> 43.1,
@@ -498,7 +499,6 @@ constexpr int kMinShare = 2;            // tiles of a CTA at least
 // tokens (Hq8 Hkv2 D64) 12.4 -> 8.3.
 constexpr float kShareSlope = 0.05f;
 constexpr int kWholeTiles = 12;
-static_assert(kBalancedCtas <= kArrivalSlots, "a counter per CTA");
 
 __device__ __forceinline__ int kv_tiles(const DecodeParams& p, int batch, int& len) {
   len = cache_length(p.cache_seqlens[batch], p.seqlen_new, p.capacity, p.checked).len;
@@ -854,10 +854,8 @@ decode_balanced_kernel(const __grid_constant__ DecodeParams p) {
         const int c0 = shares.owner(first_tile), parts = shares.owner(first_tile + w.n_tiles - 1) - c0 + 1;
         named_barrier_sync(1, kConsumerWarps * 32);
         if (threadIdx.x == 0) {  // release: the barrier's other threads' writes too; acquire: those of the CTAs that came before
-          int* arrivals = p.arrivals + c0 * gridDim.x + head_k;
-          const bool last = atomic_add_acq_rel_gpu(arrivals, 1) == parts - 1;
-          if (last) *arrivals = 0;  // for the launch that takes the counters next
-          bars->last = last;
+          grid_dependency_wait();  // the zeros; over long ago, the producer has waited for the same before the first tile
+          bars->last = atomic_add_acq_rel_gpu(p.arrivals + c0 * gridDim.x + head_k, 1) == parts - 1;
         }
         named_barrier_sync(1, kConsumerWarps * 32);
         if (bars->last) {
@@ -905,7 +903,15 @@ struct AppendParams {
   int* verdict;
   int token;
   int64_t max_length;
+  // balanced kernel behind this one: its arrival counters, to be zeroed
+  int* arrivals;
+  int num_arrivals;
 };
+
+// By the threads of one block.
+__device__ __forceinline__ void zero_arrivals(int* arrivals, int n) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) arrivals[i] = 0;
+}
 
 // By all threads of a block.
 __device__ __forceinline__ bool lengths_fit(const int* lengths, int b, int64_t max_length) {
@@ -918,10 +924,15 @@ __device__ __forceinline__ void tell_host(int* verdict, int token, bool fits) {
   __threadfence_system();
 }
 
-// fa_kvcache_checked() without new tokens
-__global__ void __launch_bounds__(256) check_lengths_kernel(const int* lengths, int b, int64_t max_length, int* verdict, int token) {
-  const bool fits = lengths_fit(lengths, b, max_length);
-  if (threadIdx.x == 0) tell_host(verdict, token, fits);
+// Calls without new tokens: what the append kernel does besides appending
+__global__ void __launch_bounds__(256) prepare_kernel(const int* lengths, int b, int64_t max_length, int* verdict, int token, int* arrivals,
+                                                      int num_arrivals) {
+  grid_launch_dependents();
+  zero_arrivals(arrivals, num_arrivals);
+  if (verdict != nullptr) {
+    const bool fits = lengths_fit(lengths, b, max_length);
+    if (threadIdx.x == 0) tell_host(verdict, token, fits);
+  }
 }
 
 // The 16-byte units of the first step are fetched before the lengths are looked at: two memory latencies in a row instead of four
@@ -948,6 +959,7 @@ __global__ void __launch_bounds__(256) append_kernel(const __grid_constant__ App
     vv = *reinterpret_cast<const uint4*>(p.v_new + batch * p.vn_batch_stride + t * p.vn_row_stride + head * p.vn_head_stride + u * 8);
   };
   if (idx < total) fetch();
+  if (blockIdx.x == 0) zero_arrivals(p.arrivals, p.num_arrivals);
   if (p.verdict != nullptr) {  // every block looks at all lengths (b loads by its 256 threads, from L2 but for the first): no launch in between
     const bool fits = lengths_fit(p.cache_seqlens, p.b, p.max_length);
     if (blockIdx.x == 0 && threadIdx.x == 0) tell_host(p.verdict, p.token, fits);
@@ -1003,8 +1015,19 @@ bool never_cut(const FaKvcacheParams* p) {
   return balanced_shares(p) == 1 || (capacity_tiles(p) <= kWholeTiles && p->b <= balanced_shares(p));
 }
 
-// Parts in scratch memory: two per CTA
-size_t balanced_slots(const FaKvcacheParams* p) { return 2 * static_cast<size_t>(balanced_shares(p)) * p->h_k; }
+size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+// Scratch memory of the balanced kernel: the parts (two per CTA), their LSE, an arrival counter per CTA
+struct BalancedScratch {
+  size_t lse, arrivals, bytes;  // offsets of the second and third, and the size
+  int num_arrivals;
+  explicit BalancedScratch(const FaKvcacheParams* p) : num_arrivals(balanced_shares(p) * p->h_k) {
+    const size_t rows = 2 * static_cast<size_t>(num_arrivals) * kMaxRows;
+    lse = align_up(rows * p->d * sizeof(float), 256);
+    arrivals = lse + align_up(rows * sizeof(float), 256);
+    bytes = arrivals + align_up(num_arrivals * sizeof(int), 256);
+  }
+};
 
 // Calls for which no scratch memory was asked before the balanced kernel: without any they run as a single split.
 bool may_lack_workspace(const FaKvcacheParams* p) {
@@ -1052,10 +1075,8 @@ int effective_splits(const FaKvcacheParams* p) {
   return splits;
 }
 
-size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-
 template <int D>
-int launch_balanced(const DecodeParams& dp, dim3 grid, bool after_append, cudaStream_t stream) {
+int launch_balanced(const DecodeParams& dp, dim3 grid, bool overlap, cudaStream_t stream) {
   using C = DCfg<D>;
   static bool configured[64] = {};
   int dev = 0;
@@ -1064,7 +1085,7 @@ int launch_balanced(const DecodeParams& dp, dim3 grid, bool after_append, cudaSt
     FA_CHECK_CUDA(cudaFuncSetAttribute(decode_balanced_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
     configured[dev & 63] = true;
   }
-  if (after_append) {
+  if (overlap) {
     FA_CHECK_CUDA(launch_overlapped(decode_balanced_kernel<D>, grid, kDecodeThreads, C::kSmemBytes, stream, dp));
   } else {
     decode_balanced_kernel<D><<<grid, kDecodeThreads, C::kSmemBytes, stream>>>(dp);
@@ -1124,9 +1145,7 @@ extern "C" size_t fa_kvcache_workspace_bytes(const FaKvcacheParams* p) {
   using namespace fa;
   if (validate(p, "fa_kvcache_workspace_bytes") != FA_OK) return 0;
   if (uses_balanced_kernel(p)) {
-    if (never_cut(p)) return 0;
-    const size_t slot_rows = balanced_slots(p) * kMaxRows;
-    return align_up(slot_rows * p->d * sizeof(float), 256) + align_up(slot_rows * sizeof(float), 256);
+    return never_cut(p) ? 0 : BalancedScratch(p).bytes;
   }
   const int splits = effective_splits(p);
   if (splits <= 1) return 0;
@@ -1152,13 +1171,32 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   rc = check_device_sm100();
   if (rc != FA_OK) return rc;
 
+  const bool balanced = uses_balanced_kernel(p) && (p->workspace != nullptr || never_cut(p) || !may_lack_workspace(p));
+  int splits = effective_splits(p), chunk = 0;
+  if (!balanced && !uses_balanced_kernel(p)) plan_splits(p, &splits, &chunk);
+  if (!balanced && uses_balanced_kernel(p)) splits = 1;  // no scratch memory (may_lack_workspace)
+  uint8_t* scratch = nullptr;
+  if (splits > 1) {
+    const size_t need = fa_kvcache_workspace_bytes(p);
+    if (p->workspace == nullptr || p->workspace_bytes < need)
+      return set_error(FA_ERR_WORKSPACE, "fa_kvcache: workspace smaller than fa_kvcache_workspace_bytes()");
+    FA_CHECK_ARG(aligned16(p->workspace), "fa_kvcache: workspace must be 16-byte aligned");
+    scratch = static_cast<uint8_t*>(p->workspace);
+  }
+  int* arrivals = nullptr;
+  int num_arrivals = 0;
+  if (balanced && splits > 1) {
+    const BalancedScratch layout(p);
+    arrivals = reinterpret_cast<int*>(scratch + layout.arrivals), num_arrivals = layout.num_arrivals;
+  }
+
   // The launches overlap (launch_overlapped): each kernel's set-up and launch run under its predecessor, and it waits inside for
   // what that writes.
   // ---- 1. append ----
   const bool appends = p->k_new && p->seqlen_new > 0;
   const int64_t max_length = (p->block_table ? static_cast<int64_t>(p->max_blocks_per_seq) : 1) * p->seqlen_cache - p->seqlen_new;
-  if (verdict != nullptr && !appends) {
-    check_lengths_kernel<<<1, 256, 0, stream>>>(p->cache_seqlens, p->b, max_length, verdict, token);
+  if (!appends && (verdict != nullptr || num_arrivals > 0)) {
+    prepare_kernel<<<1, 256, 0, stream>>>(p->cache_seqlens, p->b, max_length, verdict, token, arrivals, num_arrivals);
     FA_CHECK_CUDA(cudaGetLastError());
   }
   if (appends) {
@@ -1184,6 +1222,7 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
     ap.block_table = p->block_table; ap.block_table_batch_stride = p->block_table_batch_stride;
     ap.max_blocks_per_seq = p->max_blocks_per_seq;
     ap.verdict = verdict; ap.token = token; ap.max_length = max_length;
+    ap.arrivals = arrivals; ap.num_arrivals = num_arrivals;
     const int64_t total = static_cast<int64_t>(p->b) * p->seqlen_new * p->h_k * (p->d / 8);
     const int blocks = static_cast<int>(std::min<int64_t>((total + 255) / 256, 148 * 8));
     append_kernel<<<blocks, 256, 0, stream>>>(ap);
@@ -1213,10 +1252,6 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
     return run_fwd(&f, p->seqlen_new, stream, appends, verdict != nullptr);
   }
 
-  const bool balanced = uses_balanced_kernel(p) && (p->workspace != nullptr || never_cut(p) || !may_lack_workspace(p));
-  int splits = effective_splits(p), chunk = 0;
-  if (!balanced && !uses_balanced_kernel(p)) plan_splits(p, &splits, &chunk);
-  if (!balanced && uses_balanced_kernel(p)) splits = 1;  // no scratch memory (may_lack_workspace)
   const int64_t rows_total = static_cast<int64_t>(p->b) * p->h * p->seqlen_q;
   DecodeParams dp;
   rc = make_tensor_map_4d(&dp.tm_k, p->k_cache, p->d, p->h_k, p->seqlen_cache, p->cache_batch,
@@ -1230,19 +1265,11 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   dp.q = static_cast<const __half*>(p->q);
   dp.o = static_cast<__half*>(p->o);
   dp.lse = p->lse;
-  dp.o_accum = nullptr;
+  dp.o_accum = reinterpret_cast<float*>(scratch);
   dp.lse_accum = nullptr;
-  if (splits > 1) {
-    const size_t need = fa_kvcache_workspace_bytes(p);
-    if (p->workspace == nullptr || p->workspace_bytes < need)
-      return set_error(FA_ERR_WORKSPACE, "fa_kvcache: workspace smaller than fa_kvcache_workspace_bytes()");
-    FA_CHECK_ARG(aligned16(p->workspace), "fa_kvcache: workspace must be 16-byte aligned");
-    dp.o_accum = static_cast<float*>(p->workspace);
+  if (splits > 1)
     dp.lse_accum = reinterpret_cast<float*>(
-        static_cast<uint8_t*>(p->workspace) +
-        align_up((balanced ? balanced_slots(p) * kMaxRows : static_cast<size_t>(splits) * rows_total) * p->d *
-                     sizeof(float), 256));
-  }
+        scratch + (balanced ? BalancedScratch(p).lse : align_up(static_cast<size_t>(splits) * rows_total * p->d * sizeof(float), 256)));
   dp.q_batch_stride = p->q_batch_stride; dp.q_row_stride = p->q_row_stride; dp.q_head_stride = p->q_head_stride;
   dp.o_batch_stride = p->o_batch_stride; dp.o_row_stride = p->o_row_stride; dp.o_head_stride = p->o_head_stride;
   dp.seqlen_q = p->seqlen_q; dp.seqlen_new = p->seqlen_new; dp.h = p->h; dp.h_k = p->h_k;
@@ -1259,14 +1286,13 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   dp.num_splits = splits;
   dp.chunk_tiles = chunk;
   dp.b = p->b;
-  dp.arrivals = nullptr;
+  dp.arrivals = arrivals;
   dp.checked = verdict != nullptr;
   dp.status = device_status_ptr();
   if (balanced) {
-    dp.arrivals = next_arrival_slots();
-    if (dp.arrivals == nullptr) return set_error(FA_ERR_CUDA, "fa_kvcache: device attributes not available");
     const dim3 grid(p->h_k, balanced_shares(p));
-    return p->d == 128 ? launch_balanced<128>(dp, grid, appends, stream) : launch_balanced<64>(dp, grid, appends, stream);
+    const bool overlap = appends || num_arrivals > 0;
+    return p->d == 128 ? launch_balanced<128>(dp, grid, overlap, stream) : launch_balanced<64>(dp, grid, overlap, stream);
   }
   rc = (p->d == 128) ? launch_decode<128>(dp, p->b, p->h_k, appends, stream) : launch_decode<64>(dp, p->b, p->h_k, appends, stream);
   if (rc != FA_OK) return rc;

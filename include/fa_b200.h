@@ -205,8 +205,8 @@ int fa_bwd_stages(const FaBwdParams* p, int stage_mask, fa_stream_t stream);
 /* caller's responsibility.  num_splits == 0: up to 8 query rows per KV head, the keys of the     */
 /* whole batch are shared out evenly over the GPU, on the device, from the lengths; more rows: a  */
 /* split count from the shape (choose_num_splits, kvcache_native.cu:913-952, for 148 SMs).         */
-/* The shares are merged by the CTA that arrives last, counted in a pool inside the library (1024  */
-/* launches; a launch leaves its counters zero, so captured launches can be replayed).            */
+/* The shares are merged by the CTA that arrives last, counted in the call's scratch memory (zeroed by  */
+/* the kernel before): calls that may overlap on the GPU need scratch of their own, as ever.        */
 /* Scratch: fa_kvcache_workspace_bytes() bytes when the effective split count exceeds 1.  With     */
 /* num_splits == 0, at most 512 tokens of capacity or at least 1184 (sequence, KV head) pairs,     */
 /* workspace may be NULL: every sequence is then attended in one piece.                           */

@@ -1,4 +1,4 @@
-"""Two hand-overs of the kernels, walked through exhaustively: every interleaving of small models that have the kernels' waits and
+"""Hand-overs of the kernels, walked through exhaustively: every interleaving of small models that have the kernels' waits and
 arrivals.  Barriers behave as mbarriers do: a phase ends with the last expected arrival, and a wait sees only the parity of the
 phase.  How many barriers a hand-over has is read from the kernels' source.
 
@@ -222,6 +222,64 @@ def test_the_deferred_store_needs_its_barriers():
         _walk_deferred_store(LENGTHS[0], False, 3, 3)
     with pytest.raises(_Fault, match="stuck"):
         _walk_deferred_store(LENGTHS[0], True, 1, 3)
+
+
+PARTS = 3
+
+
+def _walk_arrivals(own_counters, ordered=True):
+    """Two calls on two streams, in each of which PARTS CTAs share a sequence (decode_balanced_kernel, csrc/kvcache_sm100.cu): a kernel
+    that zeroes the counter, CTAs that store their part and count themselves, and the last of them merges.  own_counters: each call
+    counts in its own scratch memory; else both in one counter, zero at first and put back to zero by the CTA that merges.  ordered: the
+    CTAs count only behind the kernel that zeroes (each may start before it has finished).  Faults: a merge of parts that are not there,
+    a call that nobody merges."""
+    # call: (zeroed?, step of each CTA: 0 store, 1 count, 2 merge, 3 done); counters: None is what the memory held before
+    start = (((not own_counters, (0,) * PARTS),) * 2, (None, None) if own_counters else (0, 0), (0, 0))
+    seen, todo = {start}, [start]
+    while todo:
+        calls, counters, merged = todo.pop()
+        nexts = []
+        for c, (zeroed, ctas) in enumerate(calls):
+            at = c if own_counters else 0
+
+            def put(new_ctas, value, merges, new_zeroed=zeroed):
+                nexts.append((calls[:c] + ((new_zeroed, new_ctas),) + calls[c + 1:], counters[:at] + (value,) + counters[at + 1:],
+                              merged[:c] + (merged[c] + merges,) + merged[c + 1:]))
+
+            if not zeroed:
+                put(ctas, 0, 0, True)
+            for i, step in enumerate(ctas):
+                moved = lambda to: ctas[:i] + (to,) + ctas[i + 1:]  # noqa: E731
+                if step == 0:
+                    put(moved(1), counters[at], 0)
+                elif step == 1 and (zeroed or not ordered):
+                    old = counters[at]
+                    put(moved(2 if old == PARTS - 1 else 3), None if old is None else old + 1, 0)
+                elif step == 2:
+                    if 0 in ctas:
+                        raise _Fault(f"call {c} merges parts that are not there")
+                    put(moved(3), counters[at] if own_counters else 0, 1)
+        if not nexts and merged != (1, 1):
+            raise _Fault(f"merges: {merged}")
+        for n in nexts:
+            if n not in seen:
+                seen.add(n)
+                todo.append(n)
+    return len(seen)
+
+
+def test_arrivals_are_counted_in_the_scratch_memory_of_the_call():
+    source = (CSRC / "kvcache_sm100.cu").read_text()
+    shared = re.search(r"arrivals = next_\w+\(\)", source) is not None
+    wait = re.search(r"grid_dependency_wait\(\);[^\n]*\n\s*bars->last = atomic_add", source) is not None
+    assert _walk_arrivals(not shared, shared or wait) > 100
+
+
+def test_arrivals_need_counters_of_their_own_and_the_wait():
+    with pytest.raises(_Fault, match="not there|merges:"):
+        _walk_arrivals(False)
+    with pytest.raises(_Fault, match="merges:"):
+        _walk_arrivals(True, ordered=False)
 
 
 HANDOVERS = [(_walk_dq, "bwd_sm100.cu", "DqBarriers", "ds_full"), (_walk_v_tail, "fwd_sm100.cu", "Barriers", "v_fixed")]

@@ -532,3 +532,44 @@ def test_even_shares_without_scratch_memory(ext):
         if ok:
             want = flash_attn_with_kvcache(q, kc, vc, cache_seqlens=lens, causal=True, num_splits=1)
             assert torch.equal(out, want)
+
+
+def test_captured_decode_beside_eager_decode(ext, monkeypatch):
+    """Sequences over many shares: replays of two graphs, captured more than 1024 launches apart, beside each other and beside eager
+    calls on a third stream.  Every result is that of a call by itself, bit for bit."""
+    import flash_attention_turing_b200.flash_attention_interface as iface
+
+    monkeypatch.setattr(iface, "HOST_CAPACITY_CHECK", False)
+    gen = torch.Generator(device=DEV).manual_seed(12)
+    r = lambda *s: torch.randn(*s, generator=gen, device=DEV, dtype=torch.half)  # noqa: E731
+
+    def inputs(lens, new):
+        return r(len(lens), 1, 8, 128), r(len(lens), 8192, 2, 128), r(len(lens), 8192, 2, 128), *(
+            (r(len(lens), 1, 2, 128), r(len(lens), 1, 2, 128)) if new else (None, None)), torch.tensor(lens, dtype=torch.int32, device=DEV)
+
+    def call(q, kc, vc, k, v, lens):
+        return iface.flash_attn_with_kvcache(q, kc, vc, k, v, cache_seqlens=lens, causal=True, return_softmax_lse=True)
+
+    sets = [inputs((8000, 3000), True), inputs((5000, 7000, 600), False), inputs((100, 6500), True)]
+    want = [[x.clone() for x in call(*s)] for s in sets]
+    streams = [torch.cuda.Stream() for _ in sets]
+    graphs = []
+    for s, stream in zip(sets[:2], streams):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            out = call(*s)
+        graphs.append((g, out))
+        for _ in range(1023):  # a pool of 1024 counters would come round to the same one
+            call(*sets[2])
+    torch.cuda.synchronize()
+    for _ in range(20):
+        eager = []
+        for _ in range(20):
+            for (g, _), stream in zip(graphs, streams):
+                with torch.cuda.stream(stream):
+                    g.replay()
+            with torch.cuda.stream(streams[2]):
+                eager.append(call(*sets[2]))
+        torch.cuda.synchronize()
+        for got, expected in [(graphs[0][1], want[0]), (graphs[1][1], want[1]), *((e, want[2]) for e in eager)]:
+            assert all(torch.equal(x, y) for x, y in zip(got, expected))
