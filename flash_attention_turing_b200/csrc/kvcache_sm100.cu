@@ -779,7 +779,7 @@ decode_balanced_kernel(const __grid_constant__ DecodeParams p) {
         if (tok0 < w.len) mine.tokens(sK, sK + C::kTileBytes, stage + C::kTileBytes, tok_in_tile, tok0, w.len, c, lane);
         release(i);
       }
-      if (!ok || !(ok = wait_full(i))) break;
+      ok = ok && wait_full(i);
 
       // ---- merge the four warps through the stage that holds no tile: [warp][row][D], the columns of row r xor 8 * (r % 8) so
       // that the eight rows of a fragment column lie in different banks ----
@@ -789,18 +789,22 @@ decode_balanced_kernel(const __grid_constant__ DecodeParams p) {
       mine.l1 += __shfl_xor_sync(0xffffffffu, mine.l1, 1);
       mine.l1 += __shfl_xor_sync(0xffffffffu, mine.l1, 2);
       float* dst = mbuf + warp * kMaxRows * D;
-#pragma unroll
-      for (int k = 0; k < D / 8; ++k) {
-        const int col = ((k * 8) ^ (g * 8)) + t4 * 2;
-        if (g < rows) *reinterpret_cast<float2*>(dst + g * D + col) = make_float2(mine.oacc[k][0], mine.oacc[k][1]);
-        if (g + 8 < rows) *reinterpret_cast<float2*>(dst + (g + 8) * D + col) = make_float2(mine.oacc[k][2], mine.oacc[k][3]);
-      }
       ml = ml_of_seqs + (n_seqs++ & 1) * kConsumerWarps * kMaxRows;
-      if (t4 == 0) {
-        ml[warp * kMaxRows + g] = make_float2(mine.m0, mine.l0);
-        ml[warp * kMaxRows + g + 8] = make_float2(mine.m1, mine.l1);
+      if (ok) {
+#pragma unroll
+        for (int k = 0; k < D / 8; ++k) {
+          const int col = ((k * 8) ^ (g * 8)) + t4 * 2;
+          if (g < rows) *reinterpret_cast<float2*>(dst + g * D + col) = make_float2(mine.oacc[k][0], mine.oacc[k][1]);
+          if (g + 8 < rows) *reinterpret_cast<float2*>(dst + (g + 8) * D + col) = make_float2(mine.oacc[k][2], mine.oacc[k][3]);
+        }
+        if (t4 == 0) {
+          ml[warp * kMaxRows + g] = make_float2(mine.m0, mine.l0);
+          ml[warp * kMaxRows + g + 8] = make_float2(mine.m1, mine.l1);
+        }
       }
-      named_barrier_sync(1, kConsumerWarps * 32);
+      // A warp may give up on a phase that the others see complete: all come here, and all leave or none (a warp that left by itself
+      // would be at the end of the kernel while the others wait for it at this barrier, without a limit).
+      if (!(ok = named_barrier_and(1, kConsumerWarps * 32, ok))) break;
 
       // a warp per row, a lane per kPerLane columns
       auto store = [&](int r, const float (&acc)[kPerLane], float mul, float lse) {

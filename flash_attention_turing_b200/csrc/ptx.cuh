@@ -564,6 +564,21 @@ __device__ __forceinline__ void store_rows_fp16(__half* to, int64_t row_stride, 
 __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+// The same; true in all threads when `ok` was true in all of them
+__device__ __forceinline__ bool named_barrier_and(int id, int nthreads, bool ok) {
+  int all;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred mine, every;\n\t"
+      "setp.ne.s32 mine, %3, 0;\n\t"
+      "bar.red.and.pred every, %1, %2, mine;\n\t"
+      "selp.s32 %0, 1, 0, every;\n\t"
+      "}"
+      : "=r"(all)
+      : "r"(id), "r"(nthreads), "r"(static_cast<int>(ok))
+      : "memory");
+  return all != 0;
+}
 
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;

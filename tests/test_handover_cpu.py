@@ -282,6 +282,54 @@ def test_arrivals_need_counters_of_their_own_and_the_wait():
         _walk_arrivals(True, ordered=False)
 
 
+def _walk_give_up(agree, warps=3, seqs=2, waits=2):
+    """Consumer warps of decode_balanced_kernel (csrc/kvcache_sm100.cu) when bounded waits run out: per sequence `waits` of them, each
+    of which a warp may give up or see complete, whatever the others see, then the barriers of the merge, which have no limit.  agree: every
+    warp goes to the first of these, and all leave if one has given up; else a warp that gives up goes to the end of the kernel at once.
+    Fault: a warp that waits at a barrier for one that does not come."""
+    merge = 2  # barriers of a merge
+    end = (seqs, 0, True)
+    start = ((0, 0, True),) * warps  # sequence, step (waits, then barriers), no wait given up
+    seen, todo = {start}, [start]
+    while todo:
+        state = todo.pop()
+        nexts = []
+        for w, (seq, step, ok) in enumerate(state):
+            if seq < seqs and step < waits:
+                gave_up = (seq, waits, False) if agree else end
+                for to in ((seq, step + 1, ok), gave_up):
+                    nexts.append(state[:w] + (to,) + state[w + 1:])
+        at = [(seq, step) for seq, step, _ in state if seq < seqs]
+        if len(at) == warps and len(set(at)) == 1 and at[0][1] >= waits:  # all are at the same barrier
+            seq, step = at[0]
+            if not all(ok for _, _, ok in state):
+                nexts.append((end,) * warps)
+            else:
+                nexts.append(((seq, step + 1, True) if step + 1 < waits + merge else (seq + 1, 0, True),) * warps)
+        if not nexts and any(w != end for w in state):
+            raise _Fault(f"stuck: {state}")
+        for n in nexts:
+            if n not in seen:
+                seen.add(n)
+                todo.append(n)
+    return len(seen)
+
+
+def test_consumers_that_give_up_leave_together():
+    body = re.search(r"decode_balanced_kernel\(const.*?\n\}\n", (CSRC / "kvcache_sm100.cu").read_text(), re.S).group(0)
+    merge = body[body.index("WarpRows<D> mine"):]
+    first = re.search(r"named_barrier_\w+\([^;]*;", merge)
+    leaves = [m for m in re.finditer(r"\bbreak;", merge[:first.start()])]
+    # the only way out ahead of the barrier is that of the tile loop
+    agree = first.group(0).startswith("named_barrier_and") and len(leaves) == 1 and "ok = ok && wait_full(i);" in merge[:first.start()]
+    assert _walk_give_up(agree) > 100
+
+
+def test_a_consumer_that_leaves_by_itself_is_waited_for():
+    with pytest.raises(_Fault, match="stuck"):
+        _walk_give_up(False)
+
+
 HANDOVERS = [(_walk_dq, "bwd_sm100.cu", "DqBarriers", "ds_full"), (_walk_v_tail, "fwd_sm100.cu", "Barriers", "v_fixed")]
 
 
