@@ -842,6 +842,10 @@ decode_balanced_kernel(const __grid_constant__ DecodeParams p) {
           for (int e = 0; e < kPerLane; ++e) acc[e] = fmaf(x[e], scale, acc[e]);
         }
         const bool dead = mt == -INFINITY || lt == 0.f;
+        if (dead) {  // no visible key: 0 times a value that is hidden may be NaN
+#pragma unroll
+          for (int e = 0; e < kPerLane; ++e) acc[e] = 0.f;
+        }
         const float inv = dead ? 0.f : 1.f / lt;
         const float lse = dead ? -INFINITY : (mt * c + __log2f(lt)) * kLn2;
         if (whole) {

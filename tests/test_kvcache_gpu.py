@@ -573,3 +573,30 @@ def test_captured_decode_beside_eager_decode(ext, monkeypatch):
         torch.cuda.synchronize()
         for got, expected in [(graphs[0][1], want[0]), (graphs[1][1], want[1]), *((e, want[2]) for e in eager)]:
             assert all(torch.equal(x, y) for x, y in zip(got, expected))
+
+
+def _share_begins(tiles, rows):
+    """First tiles of the even shares of sequences of `tiles` 64-token tiles laid end to end, one KV head (csrc/kvcache_sm100.cu)."""
+    total, least = sum(tiles), max(2, int((0.05 * max(tiles) * max(rows, 4)) ** 0.5))
+    n = min(296, -(-total // least))
+    return [i * (total // n) + min(i, total % n) for i in range(n)]
+
+
+def test_hidden_values_of_a_part_without_visible_keys_stay_out(ext):
+    """V that is not finite, causally hidden from a query row and in a part (or a sequence) in which that row sees no key at all: the row
+    is that of a cache with finite values there, bit for bit; a row without any visible key is zero."""
+    from flash_attention_turing_b200 import flash_attn_with_kvcache
+
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    r = lambda *s: torch.randn(*s, generator=gen, device=DEV, dtype=torch.half)  # noqa: E731
+    d, cap, first = 64, 400 * 64, 40  # tiles of sequence 0; its last one holds a single key
+    second = next(n for n in range(20, 200) if first - 1 in _share_begins((first, n, 30, 1), 2))
+    lens = torch.tensor([(first - 1) * 64 + 1, second * 64, 30 * 64, 1], dtype=torch.int32, device=DEV)
+    q, kc, vc = r(4, 2, 1, d), r(4, cap, 1, d), r(4, cap, 1, d)
+    want, want_lse = flash_attn_with_kvcache(q, kc, vc, cache_seqlens=lens, causal=True, return_softmax_lse=True)
+    for i in (0, 3):
+        vc[i, lens[i] - 1] = float("nan")
+    out, lse = flash_attn_with_kvcache(q, kc, vc, cache_seqlens=lens, causal=True, return_softmax_lse=True)
+    assert torch.equal(out[:, 0], want[:, 0]) and torch.equal(out[1:3], want[1:3]) and torch.equal(lse, want_lse)
+    assert (out[3, 0] == 0).all() and lse[3, 0, 0] == 0
+    assert out[0, 1].isnan().all() and out[3, 1].isnan().all()
