@@ -544,7 +544,7 @@ def test_captured_decode_beside_eager_decode(ext, monkeypatch):
     r = lambda *s: torch.randn(*s, generator=gen, device=DEV, dtype=torch.half)  # noqa: E731
 
     def inputs(lens, new):
-        return r(len(lens), 1, 8, 128), r(len(lens), 8192, 2, 128), r(len(lens), 8192, 2, 128), *(
+        return r(len(lens), 1, 8, 128), r(len(lens), 20480, 2, 128), r(len(lens), 20480, 2, 128), *(
             (r(len(lens), 1, 2, 128), r(len(lens), 1, 2, 128)) if new else (None, None)), torch.tensor(lens, dtype=torch.int32, device=DEV)
 
     def call(q, kc, vc, k, v, lens):
