@@ -1074,7 +1074,7 @@ struct BalancedScratch {
   }
 };
 
-// Calls for which the chunk plan asks for no scratch memory: without any they run as a single split.
+// Calls for which the chunk plan asks for no scratch memory: without what the balanced kernel would use they run as a single split.
 bool may_lack_workspace(const FaKvcacheParams* p) {
   int splits, chunk;
   plan_chunks(p, &splits, &chunk);
@@ -1197,13 +1197,14 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   rc = check_device_sm100();
   if (rc != FA_OK) return rc;
 
-  const bool balanced = uses_balanced_kernel(p) && (p->workspace != nullptr || never_cut(p) || !may_lack_workspace(p));
+  const size_t need = fa_kvcache_workspace_bytes(p);
+  const bool enough = need == 0 || (p->workspace != nullptr && p->workspace_bytes >= need && aligned16(p->workspace));
+  const bool balanced = uses_balanced_kernel(p) && (enough || !may_lack_workspace(p));
   int splits = effective_splits(p), chunk = 0;
   if (!balanced && !uses_balanced_kernel(p)) plan_splits(p, &splits, &chunk);
-  if (!balanced && uses_balanced_kernel(p)) splits = 1;  // no scratch memory (may_lack_workspace)
+  if (!balanced && uses_balanced_kernel(p)) splits = 1;
   uint8_t* scratch = nullptr;
   if (splits > 1) {
-    const size_t need = fa_kvcache_workspace_bytes(p);
     if (p->workspace == nullptr || p->workspace_bytes < need)
       return set_error(FA_ERR_WORKSPACE, "fa_kvcache: workspace smaller than fa_kvcache_workspace_bytes()");
     FA_CHECK_ARG(aligned16(p->workspace), "fa_kvcache: workspace must be 16-byte aligned");

@@ -202,14 +202,16 @@ int fa_bwd_stages(const FaBwdParams* p, int stage_mask, fa_stream_t stream);
 /* (:995-1218) with kvcache_decode_split_kernel / kvcache_split_kernel /                         */
 /* kvcache_split_kernel_legacy (:148-674) and kvcache_combine_kernel (:676-780).                 */
 /* No host synchronisation: the capacity check of the reference (flash_api.cpp:627) is the       */
-/* caller's responsibility.  num_splits == 0: up to 8 query rows per KV head, the keys of the     */
-/* whole batch are shared out evenly over the GPU, on the device, from the lengths; more rows: a  */
-/* split count from the shape (choose_num_splits, kvcache_native.cu:913-952, for 148 SMs).         */
+/* caller's responsibility.  num_splits == 0: a split count from the shape (choose_num_splits,     */
+/* kvcache_native.cu:913-952, for 148 SMs), or, where the shape makes that the faster way, the keys */
+/* of the whole batch shared out evenly over the GPU, on the device, from the lengths; the last bits */
+/* of a sequence's rows then depend on the lengths of the others.                                */
 /* The shares are merged by the CTA that arrives last, counted in the call's scratch memory (zeroed by  */
 /* the kernel before): calls that may overlap on the GPU need scratch of their own, as ever.        */
 /* Scratch: fa_kvcache_workspace_bytes() bytes when the effective split count exceeds 1.  With     */
-/* num_splits == 0, at most 512 tokens of capacity or at least 1184 (sequence, KV head) pairs,     */
-/* workspace may be NULL: every sequence is then attended in one piece.                           */
+/* num_splits == 0 and either capacity + seqlen_new <= 512 tokens or at least 1184 (sequence, KV   */
+/* head) pairs, none has to be given (NULL, or fewer bytes): every sequence is then attended in    */
+/* one piece.                                                                                   */
 /* ------------------------------------------------------------------------------------------- */
 typedef struct FaKvcacheParams {
   const void* q;       /* (b, seqlen_q, h, d)                                                   */

@@ -600,3 +600,34 @@ def test_hidden_values_of_a_part_without_visible_keys_stay_out(ext):
     assert torch.equal(out[:, 0], want[:, 0]) and torch.equal(out[1:3], want[1:3]) and torch.equal(lse, want_lse)
     assert (out[3, 0] == 0).all() and lse[3, 0, 0] == 0
     assert out[0, 1].isnan().all() and out[3, 1].isnan().all()
+
+
+@pytest.mark.parametrize("b,hk,cap,new,given,ok", [
+    (160, 8, 512, 0, "none", True), (160, 8, 512, 0, "few", True), (160, 8, 512, 0, "odd", True),  # even shares with scratch
+    (160, 8, 1024, 1, "few", True),
+    (200, 4, 511, 1, "none", True), (200, 4, 512, 1, "none", False), (200, 4, 512, 1, "few", False),
+])
+def test_scratch_memory_that_does_not_suffice(ext, b, hk, cap, new, given, ok):
+    """Calls whose chunk plan is one split a sequence (capacity + new tokens <= 512, or 1184 pairs) never look at a workspace that is
+    missing, too small or not aligned; others are refused without it, and then nothing has been appended."""
+    import ctypes
+    from flash_attention_turing_b200 import capi, flash_attn_with_kvcache
+
+    lib, stream = capi.lib(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    r = lambda *s: torch.randn(*s, device=DEV, dtype=torch.half)  # noqa: E731
+    q, kc, vc = r(b, 1, hk, 64), r(b, cap, hk, 64), r(b, cap, hk, 64)
+    k, v = (r(b, 1, hk, 64), r(b, 1, hk, 64)) if new else (None, None)
+    out, lse = torch.empty_like(q), torch.empty(b, hk, 1, device=DEV)
+    lens = (torch.arange(b, device=DEV, dtype=torch.int32) * 37) % (cap - new)
+    want = flash_attn_with_kvcache(q, kc.clone(), vc.clone(), k, v, cache_seqlens=lens, causal=True, num_splits=1)
+    p = capi.kvcache_params(q, kc, vc, k, v, out, lse, lens, None, 0.125, True, 0)
+    need = lib.fa_kvcache_workspace_bytes(ctypes.byref(p))
+    room = torch.empty(need + 64, dtype=torch.uint8, device=DEV)
+    if given == "few":
+        p.workspace, p.workspace_bytes = room.data_ptr(), max(0, need - 1)
+    elif given == "odd":
+        p.workspace, p.workspace_bytes = room.data_ptr() + 8, need
+    before = kc.clone()
+    rc = lib.fa_kvcache(ctypes.byref(p), stream)
+    assert rc == (0 if ok else -3)  # FA_ERR_WORKSPACE
+    assert torch.equal(out, want) if ok else torch.equal(kc, before)
