@@ -1471,7 +1471,7 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
     }
     BwdKernelParams kq = kp;
     const int sms = device_sm_count();
-    kq.sched = next_sched_slot();
+    kq.sched = next_sched_slot(stream);
     if (sms <= 0 || kq.sched == nullptr) return set_error(FA_ERR_CUDA, "fa_bwd: device attributes not available");
     kq.items_x = (p->seqlen_q + kBlock - 1) / kBlock;
     kq.b = p->b;
@@ -1509,7 +1509,7 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
     } else {
       BwdKernelParams kk = kp;
       const int sms = device_sm_count();
-      kk.sched = next_sched_slot();
+      kk.sched = next_sched_slot(stream);
       if (sms <= 0 || kk.sched == nullptr) return set_error(FA_ERR_CUDA, "fa_bwd: device attributes not available");
       kk.items_x = (p->seqlen_k + kBlock - 1) / kBlock;
       kk.b = p->b;

@@ -16,12 +16,12 @@ thread_local std::string g_last_error;
 // One status word per device; kernels receive its address as a parameter.
 __device__ int g_device_status;
 
-__device__ int g_sched_slots[2 * kSchedSlots];
+__device__ int g_sched_slots[2][2 * kSchedSlots];  // eager, captured
 
 constexpr int kMaxDevices = 64;
 int* g_status_ptr[kMaxDevices] = {};
 int* g_sched_ptr[kMaxDevices] = {};
-unsigned g_sched_next[kMaxDevices] = {};
+unsigned g_sched_next[kMaxDevices][2] = {};
 int g_sm_count[kMaxDevices] = {};
 int g_sm100_ok[kMaxDevices] = {};  // 0 unknown, 1 yes, -1 no
 std::mutex g_mutex;
@@ -108,7 +108,13 @@ int* device_status_ptr() {
   return g_status_ptr[dev];
 }
 
-int* next_sched_slot() {
+int* next_sched_slot(cudaStream_t stream) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {  // the null stream beside a capture: the launch will say so
+    cudaGetLastError();
+    capture = cudaStreamCaptureStatusNone;
+  }
+  const int pool = capture == cudaStreamCaptureStatusNone ? 0 : 1;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
   std::lock_guard<std::mutex> lock(g_mutex);
@@ -117,7 +123,7 @@ int* next_sched_slot() {
     if (cudaGetSymbolAddress(&p, g_sched_slots) != cudaSuccess) return nullptr;
     g_sched_ptr[dev] = static_cast<int*>(p);
   }
-  return g_sched_ptr[dev] + 2 * (g_sched_next[dev]++ % kSchedSlots);
+  return g_sched_ptr[dev] + 2 * (pool * kSchedSlots + g_sched_next[dev][pool]++ % kSchedSlots);
 }
 
 int device_sm_count() {
@@ -151,7 +157,7 @@ int fa_device_status(int reset) {
     FA_CHECK_CUDA(cudaMemcpy(p, &zero, sizeof(int), cudaMemcpyHostToDevice));
     void* slots = nullptr;  // a launch that gave up leaves its work counters dirty
     FA_CHECK_CUDA(cudaGetSymbolAddress(&slots, fa::g_sched_slots));
-    FA_CHECK_CUDA(cudaMemset(slots, 0, sizeof(int) * 2 * fa::kSchedSlots));
+    FA_CHECK_CUDA(cudaMemset(slots, 0, sizeof(int) * 2 * 2 * fa::kSchedSlots));
   }
   return value;
 }

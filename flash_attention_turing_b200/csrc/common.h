@@ -42,13 +42,14 @@ int check_device_sm100();
 // Address of the per-device status word kernels write when a bounded wait gives up.
 int* device_status_ptr();
 
-// Work counters of the persistent kernels: a pool of {next item, finished CTAs} pairs in device memory, all zero
-// between launches (the last CTA of a launch to finish puts its pair back to zero).  Every launch takes the next
-// pair of the pool in turn, so launches that overlap on different streams do not share one unless kSchedSlots
-// launches lie between them.  fa_device_status(1) clears the pool together with a non-zero status word (a
-// launch that gave up on a wait leaves its pair dirty).
-constexpr int kSchedSlots = 1024;
-int* next_sched_slot();
+// Work counters of the persistent kernels: {next item, finished CTAs} pairs in device memory, all zero between launches (the last CTA of a
+// launch to finish puts its pair back to zero).  Two launches that run at the same time must not have the same pair: items would be
+// computed by neither.  Launches take the next pair in turn from one of two pools, by whether `stream` is being captured: a captured launch
+// keeps its pair for as long as its graph lives, and with a single pool eager launches came round to it.  So two eager launches share a
+// pair only with kSchedSlots others issued between them, and two captured ones with kSchedSlots captured between them.
+// fa_device_status(1) clears the pools together with a non-zero status word (a launch that gave up on a wait leaves its pair dirty).
+constexpr int kSchedSlots = 16384;
+int* next_sched_slot(cudaStream_t stream);
 
 // Number of SMs of the current device (cached); 0 on error.
 int device_sm_count();

@@ -88,11 +88,12 @@ int fa_selftest_wait_timeout(uint32_t limit_us, fa_stream_t stream);
 /* Also serves the tiled path of mha_fwd_kvcache (flash_api.cpp:686-714) through seqused_k,      */
 /* cache_batch_idx and block_table, without the index_select copy the reference makes.           */
 /* The kernel is persistent: one CTA per SM takes items of 256 (small dense batches: 128) rows from a counter in device */
-/* memory (a pool of 1024 counter pairs inside the library; a launch takes the next pair and     */
-/* leaves it zero), where the reference launches one CTA per row block of a max_seqlen-sized     */
+/* memory (16384 counter pairs inside the library for launches and 16384 for captured ones; a    */
+/* launch takes the next pair in turn and leaves it zero), where the reference launches one CTA per row block of a max_seqlen-sized     */
 /* grid (src/flash_fwd_launch_template.h:60-75).  Nothing for the host to manage: launches may   */
 /* overlap on different streams and may be captured in CUDA graphs (first call on a device       */
-/* outside the capture).  The dQ and dK/dV kernels of fa_bwd take their work the same way.       */
+/* outside the capture), as long as no two that run at the same time have 16384 others of their  */
+/* kind, captured or not, issued between them.  The dQ and dK/dV kernels of fa_bwd take their work the same way. */
 /* ------------------------------------------------------------------------------------------- */
 typedef struct FaFwdParams {
   const void* q; /* dense (b, seqlen_q, h, d); varlen (total_q, h, d)                           */

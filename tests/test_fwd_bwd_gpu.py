@@ -622,13 +622,13 @@ def _multi_wave_case(seed, causal=True, d=128):
 
 
 def test_forward_work_counters_are_left_clean_over_many_launches(ext):
-    """The persistent forward takes a {next item, finished CTAs} pair from a pool of 1024 and its last CTA puts
-    the pair back to zero.  2200 launches go round the pool twice: a pair left dirty by an earlier launch would
+    """The persistent forward takes a {next item, finished CTAs} pair from a pool of 16384 and its last CTA puts
+    the pair back to zero.  33000 launches go round the pool twice: a pair left dirty by an earlier launch would
     make a later one skip items, i.e. leave rows of O unwritten."""
     q, k, v, scale, causal = _multi_wave_case(31)
     want, want_lse = ext.fwd(q, k, v, scale, causal)
     out, lse = torch.empty_like(want), torch.empty_like(want_lse)
-    for i in range(2200):
+    for i in range(33000):
         if i % 550 == 0:
             out.fill_(float("nan"))
         ext.fwd(q, k, v, scale, causal, out=out, lse=lse)
@@ -676,6 +676,56 @@ def test_forward_in_a_cuda_graph_replays(ext):
         want, _ = ext.fwd(q, k, v, scale, causal)
         assert torch.equal(got, want)
     assert ext.device_status(True) == 0
+
+
+def _kernel_arguments(graph):
+    """The argument bytes of the kernels of a captured graph, in order."""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert int(result[0]) == 0, result
+        return result[1:] if len(result) != 2 else result[1]
+
+    n = ok(driver.cuGraphGetNodes(graph.raw_cuda_graph()))[1]
+    found = []
+    for node in ok(driver.cuGraphGetNodes(graph.raw_cuda_graph(), n))[0]:
+        if ok(driver.cuGraphNodeGetType(node)) == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = ok(driver.cuGraphKernelNodeGetParams(node))
+            _, size = (ok(driver.cuFuncGetParamInfo(params.func, 0)) if int(params.func)
+                       else ok(driver.cuKernelGetParamInfo(params.kern, 0)))
+            found.append(ctypes.string_at(ctypes.cast(params.kernelParams, ctypes.POINTER(ctypes.c_void_p))[0], size))
+    return found
+
+
+def test_graphs_captured_many_launches_apart_have_work_counters_of_their_own(ext):
+    """The same calls captured twice, 1024 launches apart: the arguments of the three persistent kernels differ, and only in the
+    pointer to the work counters (a pool that eager and captured launches shared came round after 1024)."""
+    from flash_attention_turing_b200 import capi
+
+    q, k, v, scale, causal = _multi_wave_case(36)
+    dout, (dq, dk, dv) = torch.randn_like(q), (torch.empty_like(x) for x in (q, k, v))
+    out, lse = ext.fwd(q, k, v, scale, causal)
+    fwd = capi.fwd_params(q, k, v, out, lse, scale, causal)
+    room = torch.empty(1 << 20, dtype=torch.uint8, device=DEV)
+    bwd = capi.bwd_params(q, k, v, out, dout, lse, dq, dk, dv, room, scale, causal)
+
+    def capture(what):
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+            for call, params in what:
+                capi.check(call(ctypes.byref(params), stream))
+        return graph
+
+    both = [(capi.lib().fa_fwd, fwd), (capi.lib().fa_bwd, bwd)]  # three pairs of counters
+    first = capture(both)
+    between = capture([both[0]] * 1021)
+    second = capture(both)
+    words = [[(x, y) for x, y in zip(memoryview(a[:len(a) // 8 * 8]).cast("Q"), memoryview(b[:len(b) // 8 * 8]).cast("Q")) if x != y]
+             for a, b in zip(_kernel_arguments(first), _kernel_arguments(second))]
+    assert [len(w) for w in words if w] == [1, 1, 1]
+    assert all(abs(y - x) == 1024 * 8 for w in words for x, y in w)
+    del between
 
 
 @pytest.mark.parametrize("causal", [False, True])
