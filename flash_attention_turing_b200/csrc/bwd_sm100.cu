@@ -1104,17 +1104,21 @@ bwd_dkdv_packed_kernel(const __grid_constant__ BwdKernelParams p) {
   static_assert(kColDPT<D> == kColS && !C::kStatsWithQ, "S^T and dP^T share a region, the statistics have a ring of their own");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int batch = sequence_by_size(p.cu_seqlens_q, p.cu_seqlens_k, p.b, blockIdx.z);
-  const int nblk = blockIdx.x / p.h_k, head_k = blockIdx.x - nblk * p.h_k;  // the heaviest key tiles of all heads first
   const int q_off = p.cu_seqlens_q[batch];
   const int sq = p.cu_seqlens_q[batch + 1] - q_off;
   const int k_off = p.cu_seqlens_k[batch];
   const int sk = p.cu_seqlens_k[batch + 1] - k_off;
-  const int key0 = nblk * kBlock;
   const bool first_cta = (blockIdx.x | blockIdx.z) == 0;
-  if (key0 >= sk) {
+  int nblk = blockIdx.x / p.h_k, head_k = blockIdx.x - nblk * p.h_k;  // the heaviest key tiles of all heads first
+  if (nblk * kBlock >= sk) {
     if (first_cta) grid_dependency_wait();
     return;
   }
+  if (static_cast<int64_t>(sq) * p.h_k > p.section_rows) {  // section by section
+    const HeadPlace at = section_item(blockIdx.x, p.h_k, min((sk + kBlock - 1) / kBlock, static_cast<int>(gridDim.x) / p.h_k), 1, sq, p.section_rows);
+    nblk = at.place, head_k = at.head;
+  }
+  const int key0 = nblk * kBlock;
   const int stop_probe = stop_probe_begin(p.status);
   const int group = p.group;
   const int nq = (sq + kBlock - 1) / kBlock;
@@ -1497,13 +1501,20 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
     // dK and dV may be written over K and V (a CTA reads its own tile before it writes it): then the dQ kernel, which reads
     // K and V too, has to be over first.
     const bool overlap = (stage_mask & 2) != 0 && !gradients_over_keys(p);
+    const int rows = section_rows(p->is_causal != 0, p->seqlen_q, p->seqlen_k, static_cast<int64_t>(4 * D) * kp.group);
     if (D == 128 && kp.cu_seqlens_q != nullptr && p->h != p->h_k) {  // one CTA per key tile: see bwd_dkdv_packed_kernel
       if constexpr (D == 128) {
+        BwdKernelParams kk = kp;
+        // Sections as elsewhere, but of eight heads at least: 18 CTAs to a head still read its rows together, and fewer heads leave the
+        // heaviest items of the last ones for the end.  All heads of a sequence at once, sections of the common rule, these (us, causal): 4 x
+        // 8000-16384 Hkv4 (group 4) 4567 : 4770 : 4576; 30000 Hkv16 13528 : 13067 : 13254; without the mask all heads at once read from
+        // memory what a head by itself reads from L2: 30000 Hkv16 29832 : 25804, 2 x 8192 Hkv32 8690 : 7835.
+        kk.section_rows = rows == 0 ? 0 : std::max(rows, 8 * p->seqlen_q);
         dim3 grid_k((p->seqlen_k + kBlock - 1) / kBlock * p->h_k, 1, p->b);
         if (overlap) {
-          FA_CHECK_CUDA(launch_overlapped(bwd_dkdv_packed_kernel, grid_k, kNumThreads, C::kSmemBytesDkdv, stream, kp));
+          FA_CHECK_CUDA(launch_overlapped(bwd_dkdv_packed_kernel, grid_k, kNumThreads, C::kSmemBytesDkdv, stream, kk));
         } else {
-          bwd_dkdv_packed_kernel<<<grid_k, kNumThreads, C::kSmemBytesDkdv, stream>>>(kp);
+          bwd_dkdv_packed_kernel<<<grid_k, kNumThreads, C::kSmemBytesDkdv, stream>>>(kk);
         }
       }
     } else {
@@ -1517,7 +1528,7 @@ int launch_bwd(const BwdKernelParams& kp, const FaBwdParams* p, int stage_mask, 
                                             : static_cast<int64_t>(kk.items_x) * p->h_k * p->b;
       FA_CHECK_ARG(total < (1ll << 30), "fa_bwd: too many work items");
       kk.total_items = static_cast<int>(total);
-      kk.section_rows = section_rows(p->is_causal != 0, p->seqlen_q, p->seqlen_k, static_cast<int64_t>(4 * D) * kp.group);
+      kk.section_rows = rows;
       const int grid = kk.total_items < sms ? kk.total_items : sms;
       const auto kernel = kk.cu_seqlens_q ? bwd_dkdv_kernel<D, true> : bwd_dkdv_kernel<D, false>;
       if (overlap) {
