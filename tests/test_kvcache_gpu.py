@@ -482,26 +482,32 @@ def test_an_error_behind_the_launch_is_not_hidden_by_a_second_try(ext, monkeypat
         iface.flash_attn_with_kvcache(q, kv, kv.clone(), cache_seqlens=lens)
 
 
-@pytest.mark.parametrize("d,h,hk,new,page,lens", [
-    (128, 6, 3, 1, 0, (5000,)),                                          # one sequence over many shares
-    (64, 2, 1, 1, 256, (0, 8000, 1, 64)),                                # parts of several CTAs, empty and one-tile sequences
-    (128, 16, 4, 4, 256, (700, 63, 64, 65, 2100)),                       # sixteen rows
-    (64, 5, 5, 3, 0, tuple((37 * i) % 450 for i in range(70))),          # three rounds of lengths, shares of several sequences
-    (128, 32, 32, 1, 0, tuple(1 + (53 * i) % 130 for i in range(40))),   # nine shares per head
-    (64, 300, 300, 1, 0, (70, 1, 200)),                                  # more heads than CTAs: a share per head
+@pytest.mark.parametrize("d,h,hk,new,page,cap,lens", [
+    (128, 6, 3, 1, 0, 5120, (5000,)),                                        # one sequence over many shares
+    (64, 2, 1, 1, 256, 20480, (0, 8000, 1, 64)),                             # parts of several CTAs, empty and one-tile sequences
+    (128, 32, 4, 1, 0, 30208, (30000,)),                                     # eight rows, 37 parts: two rounds of rows, two of weights
+    (64, 8, 2, 2, 256, 12800, (700, 63, 64, 12000, 2100)),                   # eight rows at two positions, several sequences cut
+    (128, 5, 1, 1, 0, 20480, (6000, 10, 15000, 64)),                         # five rows: one warp has two
+    (64, 5, 5, 3, 0, 512, tuple((37 * i) % 450 for i in range(70))),         # three rounds of lengths, shares of several sequences
+    (128, 32, 32, 1, 0, 256, tuple(1 + (53 * i) % 130 for i in range(40))),  # nine shares per head
+    (64, 300, 300, 1, 0, 768, (700,)),                                       # more heads than CTAs: a share per head
 ])
-def test_even_shares_equal_single_splits(ext, d, h, hk, new, page, lens):
+def test_even_shares_equal_single_splits(ext, d, h, hk, new, page, cap, lens):
     """num_splits = 0 against 1.  P is rounded to fp16 against another reference maximum and O once more: 2^-11 (2 max|V| + max|O|)."""
-    from flash_attention_turing_b200 import flash_attn_with_kvcache
+    import ctypes
+    from flash_attention_turing_b200 import capi, flash_attn_with_kvcache
 
     gen = torch.Generator(device=DEV).manual_seed(9)
     r = lambda *s: torch.randn(*s, generator=gen, device=DEV, dtype=torch.half)  # noqa: E731
-    b, cap = len(lens), -(-(max(lens) + new) // 256) * 256
+    b = len(lens)
     q, k, v = r(b, new, h, d), r(b, new, hk, d), r(b, new, hk, d)
     rows = (b * cap // page, page) if page else (b, cap)
     kc, vc = r(*rows, hk, d), r(*rows, hk, d)
     table = torch.randperm(rows[0], generator=gen, device=DEV).int().view(b, -1) if page else None
     seqlens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    # the most parts of the even shares: the call does not go to the chunks
+    p = capi.kvcache_params(q, kc, vc, k, v, torch.empty_like(q), torch.empty(b, h, new, device=DEV), seqlens, table, d ** -0.5, True, 0)
+    assert capi.lib().fa_kvcache_num_splits(ctypes.byref(p)) == max(1, min(296 // hk, -(-(cap + new) // 64)))
 
     def run(splits):
         return flash_attn_with_kvcache(q, kc, vc, k, v, cache_seqlens=seqlens, block_table=table, causal=True, num_splits=splits,
@@ -510,9 +516,10 @@ def test_even_shares_equal_single_splits(ext, d, h, hk, new, page, lens):
     (out, lse), (want, want_lse) = run(0), run(1)
     assert (out - want).abs().max() <= 2.0 ** -11 * (2 * vc.abs().max() + want.abs().max())
     assert (lse - want_lse).abs().max() <= 1e-4
-    for _ in range(1100 // b + 3):  # the pool of arrival counters comes round (and is left clean)
+    for _ in range(20):  # whoever merges, and whatever the scratch memory held before
+        torch.full((1 << 20,), -1, dtype=torch.int32, device=DEV)
         again, again_lse = run(0)
-    assert torch.equal(again, out) and torch.equal(again_lse, lse)
+        assert torch.equal(again, out) and torch.equal(again_lse, lse)
 
 
 def test_even_shares_without_scratch_memory(ext):
