@@ -1095,41 +1095,21 @@ int effective_splits(const FaKvcacheParams* p) {
   return splits;
 }
 
-template <int D>
-int launch_balanced(const DecodeParams& dp, dim3 grid, bool overlap, cudaStream_t stream) {
+// kKernel: decode_split_kernel<D> or decode_balanced_kernel<D>
+template <int D, auto kKernel>
+int launch_decode(const DecodeParams& dp, dim3 grid, bool overlap, cudaStream_t stream) {
   using C = DCfg<D>;
   static bool configured[64] = {};
   int dev = 0;
   FA_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    FA_CHECK_CUDA(cudaFuncSetAttribute(decode_balanced_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+    FA_CHECK_CUDA(cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
     configured[dev & 63] = true;
   }
   if (overlap) {
-    FA_CHECK_CUDA(launch_overlapped(decode_balanced_kernel<D>, grid, kDecodeThreads, C::kSmemBytes, stream, dp));
+    FA_CHECK_CUDA(launch_overlapped(kKernel, grid, kDecodeThreads, C::kSmemBytes, stream, dp));
   } else {
-    decode_balanced_kernel<D><<<grid, kDecodeThreads, C::kSmemBytes, stream>>>(dp);
-    FA_CHECK_CUDA(cudaGetLastError());
-  }
-  return FA_OK;
-}
-
-template <int D>
-int launch_decode(const DecodeParams& dp, int b, int h_k, bool after_append, cudaStream_t stream) {
-  using C = DCfg<D>;
-  static bool configured[64] = {};
-  int dev = 0;
-  FA_CHECK_CUDA(cudaGetDevice(&dev));
-  if (!configured[dev & 63]) {
-    FA_CHECK_CUDA(cudaFuncSetAttribute(decode_split_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       C::kSmemBytes));
-    configured[dev & 63] = true;
-  }
-  dim3 grid(dp.num_splits, h_k, b);
-  if (after_append) {
-    FA_CHECK_CUDA(launch_overlapped(decode_split_kernel<D>, grid, kDecodeThreads, C::kSmemBytes, stream, dp));
-  } else {
-    decode_split_kernel<D><<<grid, kDecodeThreads, C::kSmemBytes, stream>>>(dp);
+    kKernel<<<grid, kDecodeThreads, C::kSmemBytes, stream>>>(dp);
     FA_CHECK_CUDA(cudaGetLastError());
   }
   return FA_OK;
@@ -1313,9 +1293,12 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   if (balanced) {
     const dim3 grid(p->h_k, balanced_shares(p));
     const bool overlap = appends || num_arrivals > 0;
-    return p->d == 128 ? launch_balanced<128>(dp, grid, overlap, stream) : launch_balanced<64>(dp, grid, overlap, stream);
+    return p->d == 128 ? launch_decode<128, decode_balanced_kernel<128>>(dp, grid, overlap, stream)
+                       : launch_decode<64, decode_balanced_kernel<64>>(dp, grid, overlap, stream);
   }
-  rc = (p->d == 128) ? launch_decode<128>(dp, p->b, p->h_k, appends, stream) : launch_decode<64>(dp, p->b, p->h_k, appends, stream);
+  const dim3 grid(splits, p->h_k, p->b);
+  rc = p->d == 128 ? launch_decode<128, decode_split_kernel<128>>(dp, grid, appends, stream)
+                   : launch_decode<64, decode_split_kernel<64>>(dp, grid, appends, stream);
   if (rc != FA_OK) return rc;
 
   // ---- 3. merge ----
