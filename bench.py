@@ -863,7 +863,7 @@ def main():
                 best = (splits, gbs, ms)
         decode["value"] = best[1]
         per_gpu = best[1] / world
-        roofline_decode = {"kernel": "decode_kernel<128> + combine_kernel<128> + append_kernel", "bound": "hbm",
+        roofline_decode = {"kernel": "decode_balanced_kernel<128> + append_kernel", "bound": "hbm",
                            "achieved": per_gpu, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": per_gpu / peaks["hbm_gbs"],
                            "frac_of_nominal_8000": per_gpu / 8000.0, "traffic": NCU_TRAFFIC_BYTES["decode"], "num_splits": best[0],
                            "peak_source": f"{peak_src} (copy bandwidth)", "ms_per_launch": best[2]}

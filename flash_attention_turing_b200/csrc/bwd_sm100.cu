@@ -172,8 +172,8 @@ static_assert((kDqThreads / 32 + 3) / 4 * 32 * 96 <= 16384, "register file of on
 // dQ of an item is stored at the end of the first block of the next one: its last product ends 900 to 2500 clocks after its last dS, and
 // the elementwise warps, who have the next S and dP waiting, do not stand by.  The accumulator is written again only behind that
 // (acc_free).  Three items are in shared memory then: the one to be stored, the current one, and the next, whose tiles are being fetched.
-// dQ kernel: 64 texts H16 D64 98.9 -> 96.0 us, D128 133.7 -> 130.4, B4 S4096 H32 D128 710 -> 670 (power-capped), B16 S1024 251 -> 247, long
-// rows the same.  The dK/dV kernel got slower by as much in the same form (B16 S1024 347 -> 372: more code, spills in packed batches).
+// dQ kernel, medians of 11 alternations: 64 texts H16 D64 99.4 -> 95.9 us, D128 135.8 -> 131.4, B16 S1024 H32 D128 243.9 -> 238.1; B4 S4096 H32
+// D128 683 -> 680 and B1 S16384 H16 D64 892 -> 908, inside the spread (power-capped).  The dK/dV kernel got slower by as much in the same form (B16 S1024 347 -> 372: more code, spills in packed batches).
 constexpr int kItemSlots = 3;
 
 // A work item with everything the roles derive from it, filled in once by the scheduler thread.

@@ -3,8 +3,8 @@
 //
 // The attend kernel is HBM-bound (every cached K and V byte is read exactly once per KV head; the
 // query heads of a GQA group share the read), so it is built around the memory system:
-//   * one CTA per (split, KV head, sequence), or for num_splits = 0 per even share of the batch (decode_balanced_kernel); a producer
-//     warp streams 64-token K and V tiles with
+//   * one CTA per (split, KV head, sequence), or for num_splits = 0, where that is faster, per even share of the batch
+//     (decode_balanced_kernel, see uses_balanced_kernel()); a producer warp streams 64-token K and V tiles with
 //     TMA (16-byte aligned bulk copies, 128-byte swizzle, no multicast) through a ring of
 //     mbarrier-guarded stages, pages looked up in block_table per tile;
 //   * four consumer warps each take 16 tokens of every tile: S = Q K^T and O += P V run on
@@ -486,7 +486,8 @@ decode_split_kernel(const __grid_constant__ DecodeParams p) {
 // next to each other in memory (a share of (sequence, head) pairs laid end to end, with heads far apart in time, read 3-10 % more slowly).
 // A share holds the end of a sequence, whole ones and the beginning of another; the parts of a sequence that several CTAs
 // share go to scratch memory (at most two per CTA), and the CTA that arrives last merges them, in the order of the tiles, so that the
-// result does not depend on who that is.  Arrivals are counted in the call's own scratch memory, which calls that overlap do not share,
+// result does not depend on who that is.  Where a sequence is cut depends on the lengths of the others, and with it the last bits of its rows
+// (P is rounded to fp16 against the maximum of a part).  Arrivals are counted in the call's own scratch memory, which calls that overlap do not share,
 // and which the kernel before this one (append or prepare kernel) has zeroed.
 // Bound by the K / V bytes for large batches, by a chain of latencies (lengths, Q and K / V tiles, merge) for small ones.  Append and
 // attention, us, chunks of a fixed size per CTA and a merge kernel against this: 1 x 1500 tokens (Hq32 Hkv8 D128) 13.2 -> 10.4,
@@ -495,8 +496,8 @@ decode_split_kernel(const __grid_constant__ DecodeParams p) {
 constexpr int kBalancedCtas = 2 * 148;  // two per SM are resident
 constexpr int kMinShare = 2;            // tiles of a CTA at least
 // A share of a sequence of n tiles is at least sqrt(kShareSlope * n * rows) of them (a warp merges a row): what a tile takes its CTA and
-// what a part takes the CTA that merges the sequence are then about least together.  One sequence of 30000 tokens, Hq1 Hkv1 D128, slopes
-// 0.05 / 0.1: 18.6 / 20.3 us.  Sequences of up to kWholeTiles are not cut while there is a CTA for each, the merge takes as long: 60 x 50-250
+// what a part takes the CTA that merges the sequence are then about least together.  Half and twice the slope: 1.000 and 1.003 of the time over
+// 400 shapes, 1.004 and 1.008 with one sequence, 1.004 and 1.005 with eight rows.  Sequences of up to kWholeTiles are not cut while there is a CTA for each, the merge takes as long: 60 x 50-250
 // tokens (Hq8 Hkv2 D64) 12.4 -> 8.3.
 constexpr float kShareSlope = 0.05f;
 constexpr int kWholeTiles = 12;

@@ -16,7 +16,8 @@ namespace fa {
 constexpr int64_t kSectionBytes = 32 << 20;
 
 // Host: rows of `row_bytes` that a section may hold; 0, a head (or group) per section, where the order gains nothing because all items of a
-// head are equal or nearly so: no causal mask, or few queries at the end of many keys.
+// head are equal or nearly so: no causal mask, or few queries at the end of many keys.  The heads of a group are then taken tile by tile; one
+// head after the other took the same, 17 grouped shapes without mask 0.98-1.02.
 inline int section_rows(bool causal, int seqlen_q, int seqlen_k, int64_t row_bytes) {
   return causal && 4 * static_cast<int64_t>(seqlen_q) >= seqlen_k ? static_cast<int>(kSectionBytes / row_bytes) : 0;
 }

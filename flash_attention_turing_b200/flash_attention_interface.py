@@ -363,7 +363,9 @@ def flash_attn_with_kvcache(
     ``q`` (batch, seqlen_q, nheads, d) against the first ``cache_seqlens + seqlen_new`` tokens.
     Cache layouts: contiguous (batch_cache, seqlen_cache, nheads_k, d), optionally indexed through
     ``cache_batch_idx``; or paged (num_pages, page_size, nheads_k, d) with ``block_table`` (batch,
-    max_pages) and page_size % 256 == 0.  ``num_splits`` 0 picks a split count from the shape.
+    max_pages) and page_size % 256 == 0.  ``num_splits`` 0 picks a split count from the shape, or, where
+    the shape makes that faster, shares the keys of the whole batch out evenly; the last bits of a
+    sequence's rows then depend on the other lengths too (not with an explicit split count).
     Rotary, ALiBi, local windows, softcap and cache_leftpad raise NotImplementedError.
     Returns ``out`` or ``(out, softmax_lse)``.
     """
