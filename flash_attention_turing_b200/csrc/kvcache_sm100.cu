@@ -1033,19 +1033,17 @@ void plan_chunks(const FaKvcacheParams* p, int* num_splits, int* chunk_tiles) {
 //  * A batch whose chunks all run at once, about one per SM: there is nothing to balance, and finer shares are more parts to merge.
 //    75 to 148 chunks 1.02-1.09 (2 x 6000-9000 Hq8 Hkv2 D128 16.5 : 14.4), with more than four rows up to 148 chunks 1.1-1.3, up to 296 of shorter
 //    sequences 1.05-1.13; beyond that 0.75-0.95 and 0.85-0.95.  One sequence alone gains from finer shares (0.85-0.95).
-bool uses_balanced_kernel(const FaKvcacheParams* p) {
+bool uses_balanced_kernel(const FaKvcacheParams* p, int splits) {  // splits: of the chunk plan
   const int64_t rows = static_cast<int64_t>(p->seqlen_q) * (p->h / p->h_k);
-  if (p->num_splits != 0 || rows > kBalancedRows) return false;
+  if (rows > kBalancedRows) return false;
   const int64_t tiles = capacity_tiles(p), pairs = static_cast<int64_t>(p->b) * p->h_k;
   if (p->b > 256 && (p->h_k < 4 || (p->h_k < 8 && tiles > 8))) return false;
   const int used = kBalancedCtas / p->h_k * p->h_k;  // of the CTAs that are resident together
   if (p->b > 1 && 5 * used < (p->b > 4 ? 4 : 3) * kBalancedCtas) return false;
   const bool two_rows_a_warp = rows > kConsumerWarps;
-  int splits, chunk;
-  plan_chunks(p, &splits, &chunk);
   if (splits == 1) return !two_rows_a_warp && pairs > 1200;
   if (tiles <= kWholeTiles) return true;  // not cut, or rarely: 0.6-0.95
-  const int64_t chunks = splits * pairs;
+  const int64_t chunks = static_cast<int64_t>(splits) * pairs;
   if (two_rows_a_warp) return p->b == 1 ? tiles < 64 || chunks > 148 : chunks > (tiles < 192 ? 296 : 148);
   return p->b == 1 || tiles >= 300 || chunks > 148 || chunks <= (tiles < 128 ? 74 : 40);
 }
@@ -1069,31 +1067,38 @@ struct BalancedScratch {
   }
 };
 
-// Calls for which the chunk plan asks for no scratch memory: without what the balanced kernel would use they run as a single split.
-bool may_lack_workspace(const FaKvcacheParams* p) {
-  int splits, chunk;
-  plan_chunks(p, &splits, &chunk);
-  return splits == 1;
-}
-
-// Split plan of the other kernel.  An explicit request is honoured as given (proportional ranges per sequence).
-void plan_splits(const FaKvcacheParams* p, int* num_splits, int* chunk_tiles) {
-  *num_splits = 1;
-  *chunk_tiles = 0;
-  if (!uses_decode_kernel(p)) return;
+// How a call is attended.  An explicit num_splits is honoured as given (proportional ranges per sequence).
+struct Plan {
+  bool balanced = false;  // the balanced kernel, else the split kernel (or the tiled forward: one split)
+  bool may_lack = false;  // chunk plan of one split: without scratch memory that the balanced kernel would use, that is what runs
+  int splits = 1;         // parts that the keys of a sequence are attended in (balanced kernel: at most)
+  int chunk = 0;          // tiles of a split; 0: proportional ranges
+  size_t lse = 0;         // scratch memory: offset of the LSE of the parts behind the parts, and the size
+  size_t bytes = 0;
+};
+Plan plan_call(const FaKvcacheParams* p) {
+  Plan plan;
+  if (!uses_decode_kernel(p)) return plan;
   if (p->num_splits > 0) {
-    *num_splits = std::min(p->num_splits, 256);
+    plan.splits = std::min(p->num_splits, 256);
   } else {
-    plan_chunks(p, num_splits, chunk_tiles);
+    plan_chunks(p, &plan.splits, &plan.chunk);
+    plan.may_lack = plan.splits == 1;
+    plan.balanced = uses_balanced_kernel(p, plan.splits);
+    if (plan.balanced) {
+      plan.splits = never_cut(p) ? 1 : static_cast<int>(std::min<int64_t>(balanced_shares(p), capacity_tiles(p)));
+      plan.chunk = 0;
+    }
   }
-}
-
-// Parts that the keys of a sequence are attended in (balanced kernel: at most)
-int effective_splits(const FaKvcacheParams* p) {
-  if (uses_balanced_kernel(p)) return never_cut(p) ? 1 : static_cast<int>(std::min<int64_t>(balanced_shares(p), capacity_tiles(p)));
-  int splits, chunk;
-  plan_splits(p, &splits, &chunk);
-  return splits;
+  if (plan.splits > 1 && plan.balanced) {
+    const BalancedScratch scratch(p);
+    plan.lse = scratch.lse, plan.bytes = scratch.bytes;
+  } else if (plan.splits > 1) {
+    const size_t rows = static_cast<size_t>(plan.splits) * p->b * p->h * p->seqlen_q;
+    plan.lse = align_up(rows * p->d * sizeof(float), 256);
+    plan.bytes = plan.lse + align_up(rows * sizeof(float), 256);
+  }
+  return plan;
 }
 
 // kKernel: decode_split_kernel<D> or decode_balanced_kernel<D>
@@ -1139,20 +1144,13 @@ extern "C" int fa_kvcache_num_splits(const FaKvcacheParams* p) {
   using namespace fa;
   int rc = validate(p, "fa_kvcache_num_splits");
   if (rc != FA_OK) return rc;
-  return effective_splits(p);
+  return plan_call(p).splits;
 }
 
 extern "C" size_t fa_kvcache_workspace_bytes(const FaKvcacheParams* p) {
   using namespace fa;
   if (validate(p, "fa_kvcache_workspace_bytes") != FA_OK) return 0;
-  if (uses_balanced_kernel(p)) {
-    return never_cut(p) ? 0 : BalancedScratch(p).bytes;
-  }
-  const int splits = effective_splits(p);
-  if (splits <= 1) return 0;
-  const size_t rows = static_cast<size_t>(p->b) * p->h * p->seqlen_q;
-  return align_up(static_cast<size_t>(splits) * rows * p->d * sizeof(float), 256) +
-         align_up(static_cast<size_t>(splits) * rows * sizeof(float), 256);
+  return plan_call(p).bytes;
 }
 
 namespace fa {
@@ -1172,22 +1170,21 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   rc = check_device_sm100();
   if (rc != FA_OK) return rc;
 
-  const size_t need = fa_kvcache_workspace_bytes(p);
-  const bool enough = need == 0 || (p->workspace != nullptr && p->workspace_bytes >= need && aligned16(p->workspace));
-  const bool balanced = uses_balanced_kernel(p) && (enough || !may_lack_workspace(p));
-  int splits = effective_splits(p), chunk = 0;
-  if (!balanced && !uses_balanced_kernel(p)) plan_splits(p, &splits, &chunk);
-  if (!balanced && uses_balanced_kernel(p)) splits = 1;
+  Plan plan = plan_call(p);
   uint8_t* scratch = nullptr;
-  if (splits > 1) {
-    if (p->workspace == nullptr || p->workspace_bytes < need)
-      return set_error(FA_ERR_WORKSPACE, "fa_kvcache: workspace smaller than fa_kvcache_workspace_bytes()");
-    FA_CHECK_ARG(aligned16(p->workspace), "fa_kvcache: workspace must be 16-byte aligned");
-    scratch = static_cast<uint8_t*>(p->workspace);
+  if (plan.bytes > 0) {
+    const bool enough = p->workspace != nullptr && p->workspace_bytes >= plan.bytes;
+    if (plan.may_lack && !(enough && aligned16(p->workspace))) {
+      plan = Plan{};
+    } else {
+      if (!enough) return set_error(FA_ERR_WORKSPACE, "fa_kvcache: workspace smaller than fa_kvcache_workspace_bytes()");
+      FA_CHECK_ARG(aligned16(p->workspace), "fa_kvcache: workspace must be 16-byte aligned");
+      scratch = static_cast<uint8_t*>(p->workspace);
+    }
   }
   int* arrivals = nullptr;
   int num_arrivals = 0;
-  if (balanced && splits > 1) {
+  if (plan.balanced && scratch != nullptr) {
     const BalancedScratch layout(p);
     arrivals = reinterpret_cast<int*>(scratch + layout.arrivals), num_arrivals = layout.num_arrivals;
   }
@@ -1268,10 +1265,7 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   dp.o = static_cast<__half*>(p->o);
   dp.lse = p->lse;
   dp.o_accum = reinterpret_cast<float*>(scratch);
-  dp.lse_accum = nullptr;
-  if (splits > 1)
-    dp.lse_accum = reinterpret_cast<float*>(
-        scratch + (balanced ? BalancedScratch(p).lse : align_up(static_cast<size_t>(splits) * rows_total * p->d * sizeof(float), 256)));
+  dp.lse_accum = scratch != nullptr ? reinterpret_cast<float*>(scratch + plan.lse) : nullptr;
   dp.q_batch_stride = p->q_batch_stride; dp.q_row_stride = p->q_row_stride; dp.q_head_stride = p->q_head_stride;
   dp.o_batch_stride = p->o_batch_stride; dp.o_row_stride = p->o_row_stride; dp.o_head_stride = p->o_head_stride;
   dp.seqlen_q = p->seqlen_q; dp.seqlen_new = p->seqlen_new; dp.h = p->h; dp.h_k = p->h_k;
@@ -1285,26 +1279,26 @@ int run_kvcache(const FaKvcacheParams* p, int* verdict, int token, cudaStream_t 
   dp.block_table_batch_stride = p->block_table_batch_stride;
   dp.page_size = p->seqlen_cache;
   dp.capacity = capacity_tokens(p);
-  dp.num_splits = splits;
-  dp.chunk_tiles = chunk;
+  dp.num_splits = plan.splits;
+  dp.chunk_tiles = plan.chunk;
   dp.b = p->b;
   dp.arrivals = arrivals;
   dp.checked = verdict != nullptr;
   dp.status = device_status_ptr();
-  if (balanced) {
+  if (plan.balanced) {
     const dim3 grid(p->h_k, balanced_shares(p));
     const bool overlap = appends || num_arrivals > 0;
     return p->d == 128 ? launch_decode<128, decode_balanced_kernel<128>>(dp, grid, overlap, stream)
                        : launch_decode<64, decode_balanced_kernel<64>>(dp, grid, overlap, stream);
   }
-  const dim3 grid(splits, p->h_k, p->b);
+  const dim3 grid(plan.splits, p->h_k, p->b);
   rc = p->d == 128 ? launch_decode<128, decode_split_kernel<128>>(dp, grid, appends, stream)
                    : launch_decode<64, decode_split_kernel<64>>(dp, grid, appends, stream);
   if (rc != FA_OK) return rc;
 
   // ---- 3. merge ----
-  if (splits > 1)
-    return launch_combine(dp.o_accum, dp.lse_accum, p->o, p->lse, rows_total, splits, p->h, p->seqlen_q, p->d,
+  if (plan.splits > 1)
+    return launch_combine(dp.o_accum, dp.lse_accum, p->o, p->lse, rows_total, plan.splits, p->h, p->seqlen_q, p->d,
                           p->o_batch_stride, p->o_row_stride, p->o_head_stride, stream, true);
   return FA_OK;
 }
