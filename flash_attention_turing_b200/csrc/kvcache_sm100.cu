@@ -1023,13 +1023,16 @@ void plan_chunks(const FaKvcacheParams* p, int* num_splits, int* chunk_tiles) {
 
 // Which kernel attends calls with num_splits == 0.  More than kBalancedRows rows per KV head: the chunks, because the balanced kernel's merge
 // by a single CTA takes longer than it saves: 16 rows, 6 x 1000-5000 tokens (Hkv1 D128) 22.7 us against 15.5, 3 x 3000-12000 (Hkv4) 26.8 : 22.7.
-// Else the balanced kernel, except where the chunks measured faster (append and attention, us, balanced : chunks; 3400 shapes of 1 to 4096
+// Else the balanced kernel, except where the chunks measured faster (append and attention, us, balanced : chunks; 4300 shapes of 1 to 4096
 // sequences and 64 to 32768 tokens):
 //  * Many sequences of one or two heads, since every CTA counts the tiles of all of them: 4096 x 10-100 (Hkv1) 95 : 77, 16384 x 1-60 374 : 199;
 //    2048 x 10-60 (Hkv8) 0.70 of the chunks' time, 1024 x 200-1000 (Hkv4) 1.07.
 //  * A head count that leaves resident CTAs over: 16 x 100-1500 (D64) Hkv149 1.49, Hkv99 1.19; Hkv120 and Hkv64 1.0 and 0.90.
 //  * Chunks that need no merge, until they are several rounds of CTAs (33 x 105-285, Hkv12, 16.5 : 13.0; 128 x 20-64, Hkv32, 42 : 69), and with
 //    more than four rows, two for a warp to merge, always.
+//  * Large batches, bound by HBM whichever way, where the shares of sequences of equal lengths read more slowly: at least 700 (D64: 500) pairs of sequence
+//    and head with 90000 tiles, and 1184 pairs whose chunks need no merge and are long: D64 97 x 3742 Hkv32 503 : 412, 137 x 8190 Hkv8 384 : 335,
+//    D128 54 x 8200 Hkv16 442 : 425; 24 x 2000 and shorter 0.85-1.0, 64 x 1024-32768 Hkv8 (512 pairs) 645 : 657.
 //  * A batch whose chunks all run at once, about one per SM: there is nothing to balance, and finer shares are more parts to merge.
 //    75 to 148 chunks 1.02-1.09 (2 x 6000-9000 Hq8 Hkv2 D128 16.5 : 14.4), with more than four rows up to 148 chunks 1.1-1.3, up to 296 of shorter
 //    sequences 1.05-1.13; beyond that 0.75-0.95 and 0.85-0.95.  One sequence alone gains from finer shares (0.85-0.95).
@@ -1041,7 +1044,8 @@ bool uses_balanced_kernel(const FaKvcacheParams* p, int splits) {  // splits: of
   const int used = kBalancedCtas / p->h_k * p->h_k;  // of the CTAs that are resident together
   if (p->b > 1 && 5 * used < (p->b > 4 ? 4 : 3) * kBalancedCtas) return false;
   const bool two_rows_a_warp = rows > kConsumerWarps;
-  if (splits == 1) return !two_rows_a_warp && pairs > 1200;
+  if (splits == 1) return !two_rows_a_warp && pairs > 1200 && tiles <= (p->d == 64 ? 28 : 12);
+  if (pairs >= (p->d == 64 ? 500 : 700) && tiles * pairs >= 90000) return false;
   if (tiles <= kWholeTiles) return true;  // not cut, or rarely: 0.6-0.95
   const int64_t chunks = static_cast<int64_t>(splits) * pairs;
   if (two_rows_a_warp) return p->b == 1 ? tiles < 64 || chunks > 148 : chunks > (tiles < 192 ? 296 : 148);

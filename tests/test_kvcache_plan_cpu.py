@@ -23,7 +23,7 @@ def _chunks(b, capacity, hk, new=0):
     return -(-tiles // chunk)
 
 
-# (sequences, capacity, KV heads, rows per KV head)
+# (sequences, capacity, KV heads, rows per KV head, head size 128 unless it follows)
 CHUNKS = [
     (2, 9200, 2, 4), (2, 9200, 2, 1), (9, 4738, 1, 1), (4, 3200, 4, 1),   # 75 to 148 chunks, all at once
     (2, 9200, 2, 8), (4, 3200, 4, 5), (4, 9200, 4, 8), (1, 9200, 8, 8),   # two rows a warp
@@ -31,29 +31,30 @@ CHUNKS = [
     (16384, 160, 1, 2), (4096, 200, 1, 4), (512, 1000, 4, 2),            # the tiles of many sequences are counted by every CTA
     (16, 1600, 149, 1), (16, 1600, 99, 1), (2, 1600, 300, 1),            # heads that leave CTAs over
     (4, 9200, 1, 16),                                                    # sixteen rows
+    (97, 3842, 32, 1, 64), (97, 1000, 32, 1), (60, 10240, 16, 1), (34, 22344, 16, 1, 64),  # large batches
 ]
 SHARES = [
     (1, 4096, 8, 4), (1, 30200, 8, 4), (1, 3200, 2, 8),                   # one sequence
     (2, 30200, 8, 4), (64, 33024, 8, 4), (2, 30200, 8, 8), (16, 9200, 4, 8), (4, 20000, 1, 1),
     (128, 164, 32, 1), (2048, 110, 8, 2), (1024, 110, 4, 2),              # short ones, several rounds of chunks
     (23, 600, 12, 1), (4, 700, 8, 8),                                    # never cut
-    (16, 1600, 64, 1), (16, 1600, 130, 1), (2, 3200, 2, 4), (2, 3200, 4, 1),
+    (16, 1600, 64, 1), (16, 1600, 130, 1, 64), (2, 3200, 2, 4), (2, 3200, 4, 1), (97, 1000, 32, 1, 64), (60, 5000, 16, 1),
 ]
 
 
 @pytest.mark.parametrize("case", CHUNKS)
 def test_chunks_where_they_are_faster(case):
-    b, capacity, hk, rows = case
+    b, capacity, hk, rows, d = (*case, 128)[:5]
     p = _params(*case)
     splits = _chunks(b, capacity, hk)
     assert capi.lib().fa_kvcache_num_splits(ctypes.byref(p)) == splits
-    need = 0 if splits == 1 else sum(-(-splits * b * hk * rows * n * 4 // 256) * 256 for n in (128, 1))
+    need = 0 if splits == 1 else sum(-(-splits * b * hk * rows * n * 4 // 256) * 256 for n in (d, 1))
     assert capi.lib().fa_kvcache_workspace_bytes(ctypes.byref(p)) == need
 
 
 @pytest.mark.parametrize("case", SHARES)
 def test_even_shares_elsewhere(case):
-    b, capacity, hk, _ = case
+    b, capacity, hk = case[:3]
     p = _params(*case)
     tiles, shares = -(-capacity // 64), max(1, min(296 // hk, -(-capacity // 64) * b))
     cut = shares > 1 and not (tiles <= 12 and b <= shares)
